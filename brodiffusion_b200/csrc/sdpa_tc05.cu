@@ -4,31 +4,35 @@
 // tiles (128 keys each).  Roles (12 warps, three warpgroups):
 //   warps 0-3  : softmax of query tile 0   (one thread per query row)
 //   warps 4-7  : softmax of query tile 1
-//   warp  8    : issues every tcgen05.mma (one lane), owns the TMEM allocation
+//   warp  8    : issues the Q.K^T MMAs (one lane), owns the TMEM allocation
 //   warp  9    : TMA producer for Q, K and V tiles (one lane)
-//   warps 10-11: with per-key scale vectors (kScale): multiply the rows of a K or
+//   warp  10   : issues the P.V MMAs (one lane)
+//   warp  11   : with per-key scale vectors (kScale): multiplies the rows of a K or
 //                V tile in shared memory by their factors before the MMAs read it;
-//                otherwise idle (they complete the third warpgroup so that
-//                registers can be moved to the softmax warpgroups with setmaxnreg)
-// Tensor memory (512 columns): S0 [0,128) S1 [128,256) O0 [256,256+HD)
-// O1 [256+HD,256+2HD).  P (the exponentiated scores, 16-bit, two per column)
-// is written back over the first 64 columns of its S tile and consumed from
-// tensor memory as the A operand of the P.V MMA.
+//                otherwise idle (it completes the third warpgroup, so that registers
+//                can be moved to the softmax warpgroups with setmaxnreg)
+// Tensor memory (512 columns) at head_dim 128:
+//   P0 [0,64)  S [64,192)  P1 [192,256)  O0 [256,384)  O1 [384,512)
+// and at 64: S0 [0,128) S1 [128,256) P0 [256,320) P1 [320,384) O0 [384,448)
+// O1 [448,512).  P is the exponentiated score tile (16-bit, two per column),
+// consumed from tensor memory as the A operand of the P.V MMA.
 //
-// Per key tile j and query tile t the tensor pipe runs, in this issue order,
-//   PV(t, j) then QK(t, j+1)
-// so the softmax of one query tile overlaps the MMAs of the other.  The
-// running maximum is only raised when it grew by more than 2^8 (the factor
+// What paces the kernel is the dependency chain of one query tile: scores ready ->
+// softmax -> P ready -> P.V.  P has columns of its own, so the scores of step j+1
+// are computed while step j is still exponentiated: Q.K^T of a tile is issued as
+// soon as the S buffer's last user has fetched its scores into registers, and the
+// softmax warps go from one step to the next without waiting for any MMA of their
+// own step.  At head_dim 128 there is room for one S buffer only; the two tiles, half
+// a step apart, take turns in it (it is occupied from the first MMA until the fetch
+// is over, about 1100 cycles of a step per tile).  A key step takes 2790 cycles (3550
+// when P overwrote S and Q.K^T of step j+1 had to wait for P.V of step j): 4608 x 4608,
+// 24 heads of 128, 224 -> 199 us before the power cap sets in; 16896 x 16896, two batch
+// items, under the cap (SM clock 1.48 GHz instead of 1.85) 6.34 -> 5.77 ms.
+// The running maximum is only raised when it grew by more than 2^8 (the factor
 // is carried by P and cancels in O / l), which makes the O rescale rare; the
 // rescale is done in tensor memory by the softmax warps themselves.
-//
-// What paces the kernel is the dependency chain of one query tile (scores ready
-// -> softmax -> P ready -> P.V and the next Q.K^T -> scores ready), of which the
-// softmax is the longest link, and the single MMA-issuing thread: tcgen05.mma
-// holds its issuing thread for as long as the MMA executes (64 cycles for
-// 128x128x16), so every wait, fence and commit of that thread is time the tensor
-// pipe idles.  The softmax arithmetic is therefore packed two floats per
-// instruction (fma/add .f32x2) and the row maximum uses the three-input max.
+// The softmax arithmetic is packed two floats per instruction (fma/add .f32x2)
+// and the row maximum uses the three-input max.
 //
 // Q, K and V are addressed through 4-D tensor maps (head element, head, row,
 // batch): a head narrower than the 64 / 128 columns the kernel computes with
@@ -47,20 +51,34 @@ namespace {
 
 constexpr int kBM = 128;           // query rows per tile
 constexpr int kBN = 128;           // keys per tile
-constexpr int kThreads = 384;
 constexpr int kChunkBytes = 128 * 128;  // one 64-column (128 B) x 128-row TMA box
-constexpr int kRegsSoftmax = 216;
-constexpr int kRegsOther = 64;
 
 template <int HD>
 struct Cfg {
     static constexpr int kChunks = HD / 64;
     static constexpr int kTileBytes = kBN * HD * 2;
     static constexpr int kQBytes = kBM * HD * 2;
-    static constexpr int kStages = HD == 128 ? 5 : 6;
-    static constexpr int kBarBytes = 256;
-    static constexpr int kSmemBytes = 2 * kQBytes + kStages * kTileBytes + kBarBytes + 1024;
+    // K and V tiles have a ring each: each ring is then read by one MMA warp only,
+    // which sees every phase of its barriers.
+    static constexpr int kKStages = HD == 128 ? 3 : 4;
+    static constexpr int kVStages = HD == 128 ? 2 : 4;
+    static constexpr int kBarBytes = 512;
+    static constexpr int kSmemBytes = 2 * kQBytes + (kKStages + kVStages) * kTileBytes + kBarBytes + 1024;
+    // Tensor memory columns (512 in all).  At 64 columns per head every tile has its
+    // own S; at 128 the two tiles take turns in one S buffer between their P tiles.
+    static constexpr uint32_t kColS0 = HD == 128 ? 64 : 0;
+    static constexpr uint32_t kColS1 = HD == 128 ? 64 : 128;
+    static constexpr uint32_t kColP0 = HD == 128 ? 0 : 256;
+    static constexpr uint32_t kColP1 = HD == 128 ? 192 : 320;
+    static constexpr uint32_t kColO0 = HD == 128 ? 256 : 384;
+    static constexpr uint32_t kColO1 = kColO0 + HD;
 };
+
+constexpr int kThreads = 384;
+// Registers per thread after the hand-over (setmaxnreg): 8 x 216 + 4 x 64 stays within
+// the 12 x 168 the CTA is launched with.
+constexpr int kRegsSoftmax = 216;
+constexpr int kRegsOther = 64;
 
 struct TileInfo {
     int seg;
@@ -138,22 +156,28 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                  const __grid_constant__ CUtensorMap tmV0, const __grid_constant__ CUtensorMap tmV1,
                  const SdpaDevArgs a) {
     using C = Cfg<HD>;
-    constexpr int ST = C::kStages;
+    constexpr int KS = C::kKStages;
+    constexpr int VS = C::kVStages;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
     uint8_t* smem_q = smem;
-    uint8_t* smem_kv = smem + 2 * C::kQBytes;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_kv + ST * C::kTileBytes);
+    uint8_t* smem_k = smem + 2 * C::kQBytes;
+    uint8_t* smem_v = smem_k + KS * C::kTileBytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_v + VS * C::kTileBytes);
     uint64_t* q_full = bars;             // [2]
-    uint64_t* kv_full = bars + 2;        // [ST]
-    uint64_t* kv_empty = kv_full + ST;   // [ST]
-    uint64_t* s_full = kv_empty + ST;    // [2]
-    uint64_t* p_full = s_full + 2;       // [2]
-    uint64_t* pv_done = p_full + 2;      // [2]
-    uint64_t* q_ready = pv_done + 2;     // [2]  Q tile normalised + rotated in place (fused Q path)
-    uint64_t* kv_ready = q_ready + 2;    // [ST] tile landed and, where needed, scaled (kScale)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(kv_ready + ST);
+    uint64_t* s_full = bars + 2;         // [2]  scores of the tile are in tensor memory
+    uint64_t* s_free = bars + 4;         // [2]  the tile's softmax warps hold them in registers
+    uint64_t* p_full = bars + 6;         // [2]
+    uint64_t* pv_done = bars + 8;        // [2]
+    uint64_t* q_ready = bars + 10;       // [2]  Q tile normalised + rotated in place (fused Q path)
+    uint64_t* k_full = bars + 12;        // [KS]
+    uint64_t* k_empty = k_full + KS;     // [KS]
+    uint64_t* k_ready = k_empty + KS;    // [KS] tile landed and, where needed, scaled (kScale)
+    uint64_t* v_full = k_ready + KS;     // [VS]
+    uint64_t* v_empty = v_full + VS;     // [VS]
+    uint64_t* v_ready = v_empty + VS;    // [VS]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_ready + VS);
 
     dependents_may_launch();
     const int warp = threadIdx.x >> 5;
@@ -178,16 +202,21 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
     }
 
     if (threadIdx.x == 0) {
-        mbar_init(&q_full[0], 1);
-        mbar_init(&q_full[1], 1);
-        for (int s = 0; s < ST; ++s) {
-            mbar_init(&kv_full[s], 1);
-            mbar_init(&kv_empty[s], 1);
-            mbar_init(&kv_ready[s], 2);           // warps 10 and 11
+        for (int i = 0; i < KS; ++i) {
+            mbar_init(&k_full[i], 1);
+            mbar_init(&k_empty[i], 1);
+            mbar_init(&k_ready[i], 1);
+        }
+        for (int i = 0; i < VS; ++i) {
+            mbar_init(&v_full[i], 1);
+            mbar_init(&v_empty[i], 1);
+            mbar_init(&v_ready[i], 1);
         }
         for (int t = 0; t < 2; ++t) {
+            mbar_init(&q_full[t], 1);
             mbar_init(&s_full[t], 1);
-            mbar_init(&p_full[t], 4);          // one arrival per softmax warp of the tile
+            mbar_init(&s_free[t], 4);          // one arrival per softmax warp of the tile
+            mbar_init(&p_full[t], 4);
             mbar_init(&pv_done[t], 1);
             mbar_init(&q_ready[t], 4);
         }
@@ -214,8 +243,9 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
         setmaxnreg_inc<kRegsSoftmax>();
         const int t = warp >> 2;
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t tS = tmem_base + lane_base + static_cast<uint32_t>(t * kBN);
-        const uint32_t tO = tmem_base + lane_base + static_cast<uint32_t>(256 + t * HD);
+        const uint32_t tS = tmem_base + lane_base + (t ? C::kColS1 : C::kColS0);
+        const uint32_t tP = tmem_base + lane_base + (t ? C::kColP1 : C::kColP0);
+        const uint32_t tO = tmem_base + lane_base + (t ? C::kColO1 : C::kColO0);
         const int row_in_tile = (warp & 3) * 32 + lane;
         const int row_in_seg = qrow0 + t * kBM + row_in_tile;
         const int q_glob = q_global0 + t * kBM + row_in_tile;
@@ -362,8 +392,10 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                     for (int w = 0; w < 4; ++w) mbits[w] = __ballot_sync(0xffffffffu, mv[w] != 0.0f);
                 }
             }
-            ok = mbar_wait(&s_full[t], static_cast<uint32_t>(j & 1));
-            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+            // A wait that runs out leaves `ok` false in its lane and the step goes on with
+            // whatever is there; the vote on the row maximum below ends the loop for the
+            // whole warp (one vote per step instead of one per wait).
+            ok = mbar_wait(&s_full[t], static_cast<uint32_t>(j & 1)) && ok;
             tc_fence_after();
             float s[kBN];
 #pragma unroll
@@ -371,6 +403,10 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                 tmem_ld32(tS + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[c * 32]));
             }
             tmem_wait_ld();
+            // the scores are in registers: the next Q.K^T may overwrite the buffer
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[t]);
 
             const TileInfo ti = kv_tile(a, j);
             if constexpr (kHooks == 2) {
@@ -385,9 +421,10 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                     }
                 }
             }
+            // (uniform over the CTA without the causal rule: no vote on whole tiles)
             int lim = ti.valid - 1;
             if (a.mask_mode == 1) lim = min(lim, q_glob + a.q_offset - ti.kbase);
-            if (__any_sync(0xffffffffu, lim < kBN - 1)) {
+            if (a.mask_mode == 1 ? __any_sync(0xffffffffu, lim < kBN - 1) : ti.valid < kBN) {
 #pragma unroll
                 for (int c = 0; c < kBN; ++c) s[c] = (c <= lim) ? s[c] : -INFINITY;
             }
@@ -417,7 +454,9 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
             const float m_new = fmaxf(m_ref, mx);
             const bool grow = (m_new - m_ref) * sl2 > 8.0f;
-            if (__any_sync(0xffffffffu, grow)) {
+            if (__any_sync(0xffffffffu, grow || !ok)) {
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
                 float alpha = 1.0f;
                 if (grow) {
                     alpha = (m_ref == -INFINITY) ? 0.0f : fast_exp2((m_ref - m_new) * sl2);
@@ -425,9 +464,10 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                 }
                 l_sum *= alpha;
                 if (j > 0) {
-                    // P.V of step j-1 has completed: the commit that made S of this step
-                    // visible was issued after it and covers every earlier MMA of the
-                    // issuing thread
+                    // the accumulator is at rest between P.V of step j-1 and that of step j
+                    ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[t], static_cast<uint32_t>((j - 1) & 1)));
+                    if (!ok) break;
+                    tc_fence_after();
 #pragma unroll
                     for (int c = 0; c < HD / 32; ++c) {
                         uint32_t o[32];
@@ -441,16 +481,17 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             }
             const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
             const float neg_ms = -m_use * sl2;
-            // p = 2^(s * scale_log2 - m * scale_log2); row sum in four packed chains
+            // p = 2^(s * scale_log2 - m * scale_log2); row sum in four packed chains.  The
+            // first half of P waits in registers until P.V of step j-1 has released the
+            // tile's P columns (it was issued when this step's scores were fetched, so the
+            // wait is over by then as a rule).
             float rs[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) rs[i] = 0.0f;
+            auto exp_pairs = [&](int c_begin, int n, uint32_t* pk) {
 #pragma unroll
-            for (int ch = 0; ch < 4; ++ch) {
-                uint32_t pk[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int c0 = ch * 32 + 2 * i;
+                for (int i = 0; i < n; ++i) {
+                    const int c0 = c_begin + 2 * i;
                     float x0, x1, p0, p1;
                     ffma2(x0, x1, s[c0], s[c0 + 1], sl2, sl2, neg_ms, neg_ms);
                     p0 = fast_exp2(x0);
@@ -458,7 +499,21 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                     fadd2(rs[2 * (i & 3)], rs[2 * (i & 3) + 1], rs[2 * (i & 3)], rs[2 * (i & 3) + 1], p0, p1);
                     pk[i] = pack2<kBf16>(p0, p1);
                 }
-                tmem_st16(tS + ch * 16, pk);
+            };
+            {
+                uint32_t pk[32];
+                exp_pairs(0, 32, pk);
+                if (j > 0) {
+                    ok = mbar_wait(&pv_done[t], static_cast<uint32_t>((j - 1) & 1));
+                    tc_fence_after();
+                }
+                tmem_st32(tP, pk);
+            }
+#pragma unroll
+            for (int ch = 2; ch < 4; ++ch) {
+                uint32_t pk[16];
+                exp_pairs(ch * 32, 16, pk);
+                tmem_st16(tP + ch * 16, pk);
             }
             l_sum += ((rs[0] + rs[1]) + (rs[2] + rs[3])) + ((rs[4] + rs[5]) + (rs[6] + rs[7]));
             tmem_wait_st();
@@ -469,8 +524,8 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             if (lane == 0) mbar_arrive(&p_full[t]);
         }
 
-        if (ok && n_kv > 0) {
-            ok = mbar_wait(&pv_done[t], 0u);       // committed once, after the last P.V
+        if (n_kv > 0) {
+            ok = mbar_wait(&pv_done[t], static_cast<uint32_t>((n_kv - 1) & 1)) && ok;
             ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
         }
@@ -546,95 +601,81 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
     } else {
         setmaxnreg_dec<kRegsOther>();
         if (warp == 8) {
-            // -------------------------------------------------- MMA issuer
-            // tcgen05.mma issue blocks while the pipe is busy, and everything this
-            // warp does between two batches of MMAs (barrier waits, commits, index
-            // arithmetic) is time the tensor pipe idles, so the loop is kept short:
-            // ring slots and phases are walked without divisions, the K/V waits sit
-            // before the wait for P, and descriptors are formed from per-tile bases.
-            // (Two issuing warps, one per query tile, were slower: MMAs of the two
-            // tiles then interleave in the pipe and lose their back-to-back runs on
-            // one accumulator.)
-            constexpr int kFmt = kBf16 ? 1 : 0;
-            constexpr uint32_t idesc_qk = make_idesc_f16(kFmt, kBM, kBN, 0, 0);
-            constexpr uint32_t idesc_pv = make_idesc_f16(kFmt, kBM, HD, 0, 1);
+            // -------------------------------------------------- Q.K^T issuer
+            // One tcgen05.mma costs its issuing thread 46-59 cycles and the pipe 64, the
+            // queue between them holds about sixteen, and every commit and completed wait
+            // costs another 46-50 cycles of the thread: a single warp issuing both products
+            // of both tiles could not keep the pipe fed, two warps can (65.5 cycles per MMA
+            // measured with a wait and a commit after every eight).
+            constexpr uint32_t idesc_qk = make_idesc_f16(kBf16 ? 1 : 0, kBM, kBN, 0, 0);
             const uint32_t q_base = smem_u32(smem_q);
-            const uint32_t kv_base = smem_u32(smem_kv);
-            uint64_t* const kv_rdy = kScale ? kv_ready : kv_full;
-
-            auto issue_qk = [&](int t, int slot) {
-                const uint32_t qa = q_base + t * C::kQBytes;
-                const uint32_t kb = kv_base + slot * C::kTileBytes;
-#pragma unroll
-                for (int kk = 0; kk < HD / 16; ++kk) {
-                    const uint32_t off = (kk >> 2) * kChunkBytes + (kk & 3) * 32;
-                    umma_ss(tmem_base + t * kBN, make_smem_desc_sw128(qa + off, 16, 1024),
-                            make_smem_desc_sw128(kb + off, 16, 1024), idesc_qk, kk > 0 ? 1u : 0u);
-                }
-            };
-            auto issue_pv = [&](int t, int slot, bool acc) {
-                const uint32_t vb = kv_base + slot * C::kTileBytes;
-#pragma unroll
-                for (int kk = 0; kk < kBN / 16; ++kk) {
-                    umma_ts(tmem_base + 256 + t * HD, tmem_base + t * kBN + kk * 8,
-                            make_smem_desc_sw128(vb + kk * 2048, kChunkBytes, 1024), idesc_pv,
-                            (acc || kk > 0) ? 1u : 0u);
-                }
-            };
-
-            bool ok = n_kv > 0;
-            if (ok) ok = mbar_wait(&q_full[0], 0) && mbar_wait(&q_full[1], 0);
-            if (ok && a.q_fused) ok = mbar_wait(&q_ready[0], 0) && mbar_wait(&q_ready[1], 0);
-            if (ok) ok = mbar_wait(&kv_rdy[0], 0);
-            if (ok) {
-                tc_fence_after();
-                if (lane == 0) {
-                    issue_qk(0, 0);
-                    umma_commit(&s_full[0]);
-                    issue_qk(1, 0);
-                    umma_commit(&s_full[1]);
-                    umma_commit(&kv_empty[0]);
-                }
-                __syncwarp();
-            }
-            // slot and phase of the V tile of step j (ring item 2j+1) and of the K tile
-            // of step j+1 (item 2j+2)
-            int vslot = 1 % ST, vphase = 0;
+            const uint32_t k_base = smem_u32(smem_k);
+            uint64_t* const k_rdy = kScale ? k_ready : k_full;
+            int slot = 0;
+            uint32_t phase = 0;
+            bool ok = true;
             for (int j = 0; ok && j < n_kv; ++j) {
-                int kslot = vslot + 1, kphase = vphase;
-                if (kslot == ST) { kslot = 0; kphase ^= 1; }
-                const bool more = j + 1 < n_kv;
-                ok = mbar_wait(&kv_rdy[vslot], static_cast<uint32_t>(vphase));
-                if (ok && more) ok = mbar_wait(&kv_rdy[kslot], static_cast<uint32_t>(kphase));
-                if (ok) ok = mbar_wait(&p_full[0], static_cast<uint32_t>(j & 1));
-                if (!ok) break;
-                tc_fence_after();
-                if (lane == 0) {
-                    issue_pv(0, vslot, j > 0);
-                    if (more) {
-                        issue_qk(0, kslot);
-                        umma_commit(&s_full[0]);
+                for (int t = 0; t < 2; ++t) {
+                    if (j == 0) {
+                        ok = mbar_wait(&q_full[t], 0);
+                        if (ok && a.q_fused) ok = mbar_wait(&q_ready[t], 0);
+                    }
+                    // the S buffer's last user holds its scores in registers: with one buffer
+                    // that is the other tile, else the tile itself one step earlier
+                    if (HD == 128) {
+                        if (ok && (j > 0 || t > 0)) ok = mbar_wait(&s_free[t ^ 1], static_cast<uint32_t>((t ? j : j - 1) & 1));
                     } else {
-                        umma_commit(&pv_done[0]);    // only the last step needs its own signal
+                        if (ok && j > 0) ok = mbar_wait(&s_free[t], static_cast<uint32_t>((j - 1) & 1));
                     }
-                }
-                __syncwarp();
-                ok = mbar_wait(&p_full[1], static_cast<uint32_t>(j & 1));
-                if (!ok) break;
-                tc_fence_after();
-                if (lane == 0) {
-                    issue_pv(1, vslot, j > 0);
-                    if (!more) umma_commit(&pv_done[1]);
-                    umma_commit(&kv_empty[vslot]);
-                    if (more) {
-                        issue_qk(1, kslot);
-                        umma_commit(&s_full[1]);
-                        umma_commit(&kv_empty[kslot]);
+                    if (ok && t == 0) ok = mbar_wait(&k_rdy[slot], phase);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (lane == 0) {
+                        const uint32_t qa = q_base + t * C::kQBytes;
+                        const uint32_t kb = k_base + slot * C::kTileBytes;
+                        const uint32_t d = tmem_base + (t ? C::kColS1 : C::kColS0);
+#pragma unroll
+                        for (int kk = 0; kk < HD / 16; ++kk) {
+                            const uint32_t off = (kk >> 2) * kChunkBytes + (kk & 3) * 32;
+                            umma_ss(d, make_smem_desc_sw128(qa + off, 16, 1024),
+                                    make_smem_desc_sw128(kb + off, 16, 1024), idesc_qk, kk > 0 ? 1u : 0u);
+                        }
+                        umma_commit(&s_full[t]);
+                        if (t == 1) umma_commit(&k_empty[slot]);
                     }
+                    __syncwarp();
                 }
-                __syncwarp();
-                vslot = kslot + 1; vphase = kphase;
-                if (vslot == ST) { vslot = 0; vphase ^= 1; }
+                if (++slot == KS) { slot = 0; phase ^= 1; }
+            }
+        } else if (warp == 10) {
+            // -------------------------------------------------- P.V issuer
+            constexpr uint32_t idesc_pv = make_idesc_f16(kBf16 ? 1 : 0, kBM, HD, 0, 1);
+            const uint32_t v_base = smem_u32(smem_v);
+            uint64_t* const v_rdy = kScale ? v_ready : v_full;
+            int slot = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int j = 0; ok && j < n_kv; ++j) {
+                ok = mbar_wait(&v_rdy[slot], phase);
+                for (int t = 0; t < 2; ++t) {
+                    if (ok) ok = mbar_wait(&p_full[t], static_cast<uint32_t>(j & 1));
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (lane == 0) {
+                        const uint32_t vb = v_base + slot * C::kTileBytes;
+                        const uint32_t d = tmem_base + (t ? C::kColO1 : C::kColO0);
+                        const uint32_t p = tmem_base + (t ? C::kColP1 : C::kColP0);
+#pragma unroll
+                        for (int kk = 0; kk < kBN / 16; ++kk) {
+                            umma_ts(d, p + kk * 8, make_smem_desc_sw128(vb + kk * 2048, kChunkBytes, 1024), idesc_pv,
+                                    (j > 0 || kk > 0) ? 1u : 0u);
+                        }
+                        umma_commit(&pv_done[t]);
+                        if (t == 1) umma_commit(&v_empty[slot]);
+                    }
+                    __syncwarp();
+                }
+                if (++slot == VS) { slot = 0; phase ^= 1; }
             }
         } else if (warp == 9) {
             // ------------------------------------------------ TMA producer
@@ -647,45 +688,51 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                                     c * 64, head, qrow0 + t * kBM, batch);
                     }
                 }
-                int issued = 0;
+                const int kv_head = head / a.kv_group;
+                int ks = 0, vs = 0, issued = 0;
+                uint32_t kph = 1, vph = 1;             // parity that a fresh barrier passes
                 bool ok = true;
-                for (int i = 0; i < 2 * n_kv; ++i) {
-                    const int slot = i % ST;
-                    if (i >= ST) {
-                        ok = mbar_wait(&kv_empty[slot], static_cast<uint32_t>(((i / ST) - 1) & 1));
-                        if (!ok) break;
-                    }
-                    const TileInfo ti = kv_tile(a, i >> 1);
-                    const int kv_head = head / a.kv_group;
-                    const CUtensorMap* m = (i & 1) ? (ti.seg ? &tmV1 : &tmV0) : (ti.seg ? &tmK1 : &tmK0);
-                    mbar_arrive_expect_tx(&kv_full[slot], C::kTileBytes);
+                for (int j = 0; j < n_kv; ++j) {
+                    const TileInfo ti = kv_tile(a, j);
+                    if (j >= KS) ok = mbar_wait(&k_empty[ks], kph);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(&k_full[ks], C::kTileBytes);
                     for (int c = 0; c < C::kChunks; ++c) {
-                        tma_load_4d(smem_kv + slot * C::kTileBytes + c * kChunkBytes, m, &kv_full[slot],
+                        tma_load_4d(smem_k + ks * C::kTileBytes + c * kChunkBytes, ti.seg ? &tmK1 : &tmK0, &k_full[ks],
                                     c * 64, kv_head, ti.row0, batch);
                     }
-                    issued = i + 1;
+                    issued = 2 * j + 1;
+                    if (++ks == KS) { ks = 0; kph ^= 1; }
+                    if (j >= VS) ok = mbar_wait(&v_empty[vs], vph);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(&v_full[vs], C::kTileBytes);
+                    for (int c = 0; c < C::kChunks; ++c) {
+                        tma_load_4d(smem_v + vs * C::kTileBytes + c * kChunkBytes, ti.seg ? &tmV1 : &tmV0, &v_full[vs],
+                                    c * 64, kv_head, ti.row0, batch);
+                    }
+                    issued = 2 * j + 2;
+                    if (++vs == VS) { vs = 0; vph ^= 1; }
                 }
                 if (!ok) {
                     // Unwinding after a wait ran out: let the copies already in
                     // flight land before the CTA gives its shared memory back.
                     mbar_wait(&q_full[0], 0);
                     mbar_wait(&q_full[1], 0);
-                    for (int i = max(0, issued - ST); i < issued; ++i) {
-                        mbar_wait(&kv_full[i % ST], static_cast<uint32_t>((i / ST) & 1));
-                    }
+                    const int nk = (issued + 1) / 2, nv = issued / 2;
+                    for (int i = max(0, nk - KS); i < nk; ++i) mbar_wait(&k_full[i % KS], static_cast<uint32_t>((i / KS) & 1));
+                    for (int i = max(0, nv - VS); i < nv; ++i) mbar_wait(&v_full[i % VS], static_cast<uint32_t>((i / VS) & 1));
                 }
             }
             __syncwarp();
-        } else if (warp >= 10) {
+        } else {
             // ------------------------------------------- K / V row scaling
-            // Warps 10 and 11 both walk the ring items in order (each sees every phase
-            // of the barriers it waits on) and take half of a tile each.  The row
+            // Warp 11 walks the K and V tiles in order (it sees every phase of the
+            // barriers it waits on).  The row
             // factors of an item are fetched before the wait for its tile.  A tile
             // none of whose factors differs from one is passed on as it is; otherwise
             // every row is multiplied by its factor (FP32 product rounded to the
             // storage type).
             if constexpr (kScale) {
-                const int half_id = warp - 10;
                 bool ok = true;
                 // row factors of item i (rows lane, lane + 32, ...), fetched one item ahead
                 auto fetch = [&](int i, float (&f)[4]) {
@@ -704,26 +751,26 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                 float f[4], fn[4];
                 fetch(0, fn);
                 for (int i = 0; ok && i < 2 * n_kv; ++i) {
-                    const int slot = i % ST;
+                    const int n = i >> 1;
+                    const int slot = (i & 1) ? n % VS : n % KS;
+                    const uint32_t phase = static_cast<uint32_t>(((i & 1) ? n / VS : n / KS) & 1);
 #pragma unroll
                     for (int w = 0; w < 4; ++w) f[w] = fn[w];
                     fetch(i + 1, fn);
                     const bool ne = f[0] != 1.0f || f[1] != 1.0f || f[2] != 1.0f || f[3] != 1.0f;
                     const bool scale_tile = __any_sync(0xffffffffu, ne);
-                    ok = mbar_wait(&kv_full[slot], static_cast<uint32_t>((i / ST) & 1));
+                    ok = mbar_wait((i & 1) ? &v_full[slot] : &k_full[slot], phase);
                     if (!ok) break;
                     if (scale_tile) {
-                        uint8_t* tile = smem_kv + slot * C::kTileBytes;
+                        uint8_t* tile = ((i & 1) ? smem_v : smem_k) + slot * C::kTileBytes;
                         // A lane owns whole rows (lane, lane + 32, ...: the rows whose factors it
                         // holds).  Within a 64-column chunk a row is one 128-byte line whose 16-byte
                         // pieces the swizzle permutes; the factor is the same for all of them, so
                         // the pieces are walked in physical order, rotated by the lane's row so that
-                        // the 32 rows of one access fall into different banks.  The (row group,
-                        // chunk) pairs alternate between the two warps.
+                        // the 32 rows of one access fall into different banks.
 #pragma unroll
                         for (int pi = 0; pi < 4 * C::kChunks; ++pi) {
                             const int w = pi / C::kChunks, ch = pi % C::kChunks;
-                            if ((pi & 1) != half_id) continue;
                             if (!__any_sync(0xffffffffu, f[w] != 1.0f)) continue;
                             uint8_t* line = tile + ch * kChunkBytes + (lane + 32 * w) * 128;
                             const float fw = f[w];
@@ -760,7 +807,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                         fence_proxy_async_smem();      // the MMA reads the tile through the async proxy
                     }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&kv_ready[slot]);
+                    if (lane == 0) mbar_arrive((i & 1) ? &v_ready[slot] : &k_ready[slot]);
                 }
             }
         }
