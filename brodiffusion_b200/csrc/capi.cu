@@ -466,27 +466,45 @@ int bdattn_sdpa_traced_fwd(const bdattn_sdpa_params* p, const bdattn_trace_param
     if (sdpa_fwd_impl(op, p, nullptr, nullptr, 0, t, stream)) return -1;
     if (t->attn_avg == nullptr) return 0;
     const int hd = p->head_dim;
-    bdattn::AttnMapArgs m;
-    std::memset(&m, 0, sizeof(m));
+    const bool bf16 = p->dtype == BDATTN_BF16;
+    bdattn::AttnMapLaunch L;
+    std::memset(&L, 0, sizeof(L));
+    bdattn::AttnMapArgs& m = L.args;
     for (int s = 0; s < 2; ++s) {
-        if (s < p->n_q_seg) { m.q[s] = p->q[s]; m.q_rows[s] = p->q_rows[s]; m.q_ld[s] = p->q_ld[s]; }
-        if (s < p->n_kv_seg) { m.k[s] = p->k[s]; m.kv_rows[s] = p->kv_rows[s]; m.k_ld[s] = p->k_ld[s]; }
+        const int qs = s < p->n_q_seg ? s : 0, ks = s < p->n_kv_seg ? s : 0;
+        if (make_map_heads(op, &L.tmQ[s], p->q[qs], bf16, hd, p->num_heads, p->q_rows[qs], 1, p->q_ld[qs], 0, 128) ||
+            make_map_heads(op, &L.tmK[s], p->k[ks], bf16, hd, p->num_heads, p->kv_rows[ks], 1, p->k_ld[ks], 0, 64))
+            return -1;
+        m.q_rows[s] = s < p->n_q_seg ? p->q_rows[s] : 0;
+        m.kv_rows[s] = s < p->n_kv_seg ? p->kv_rows[s] : 0;
+        const int base = s ? m.q_rows[0] : 0;
+        const int lo = t->map_row0 > base ? t->map_row0 - base : 0;
+        const int end = t->map_row0 + t->map_rows - base < m.q_rows[s] ? t->map_row0 + t->map_rows - base : m.q_rows[s];
+        m.row_lo[s] = lo;
+        m.row_n[s] = end > lo ? end - lo : 0;
     }
-    if (p->n_q_seg == 1) m.q_rows[0] = static_cast<int>(Lq);
-    if (p->n_kv_seg == 1) m.kv_rows[0] = static_cast<int>(Lk);
-    m.num_heads = p->num_heads; m.head_dim = hd;
+    m.key_n[0] = t->map_cols < m.kv_rows[0] ? t->map_cols : m.kv_rows[0];
+    m.key_n[1] = t->map_cols - m.key_n[0];
+    m.row_tiles0 = (m.row_n[0] + 127) / 128;
+    m.key_tiles0 = (m.key_n[0] + 63) / 64;
+    L.row_tiles = m.row_tiles0 + (m.row_n[1] + 127) / 128;
+    L.key_tiles = m.key_tiles0 + (m.key_n[1] + 63) / 64;
+    if (L.row_tiles > 65535) return fail("%s: map block of %d rows is too large", op, t->map_rows);
+    L.head_dim = hd <= 64 ? 64 : 128;
+    L.bf16 = bf16;
+    m.num_heads = p->num_heads;
     const float scale = p->softmax_scale > 0.0f ? p->softmax_scale : 1.0f / std::sqrt(static_cast<float>(hd));
     m.scale_log2 = scale * 1.4426950408889634f;
     m.lse = static_cast<const float*>(t->workspace); m.lq_total = static_cast<int>(Lq);
     m.bias = t->bias; m.bias_row0 = t->bias_row0; m.bias_rows = t->bias_rows; m.bias_cols = t->bias_cols;
     m.bias_ld = t->bias_ld > 0 ? t->bias_ld : t->bias_cols;
-    m.map = t->attn_avg; m.map_row0 = t->map_row0; m.map_rows = t->map_rows; m.map_cols = t->map_cols;
+    m.map = t->attn_avg; m.map_row0 = t->map_row0;
     m.map_ld = t->map_ld > 0 ? t->map_ld : t->map_cols;
     m.mask_mode = p->mask_mode;
     m.q_offset = static_cast<int>(Lk - Lq);
     m.key_mask = p->key_mask;
     m.key_scale = p->key_scale;
-    cudaError_t e = bdattn::launch_attn_map(m, p->dtype == BDATTN_BF16, reinterpret_cast<cudaStream_t>(stream));
+    cudaError_t e = bdattn::launch_attn_map(L, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(op, e);
     return 0;
 }

@@ -88,11 +88,8 @@ cudaError_t launch_sdpa_general(const SdpaGeneralArgs& a, int num_heads, int bat
 
 // Head-averaged attention map of a query-row range x leading key range.
 struct AttnMapArgs {
-    const void* q[2];
-    const void* k[2];
     int q_rows[2], kv_rows[2];
-    long long q_ld[2], k_ld[2];
-    int num_heads, head_dim;
+    int num_heads;
     float scale_log2;
     const float* lse;       // (heads, lq_total, 2)
     int lq_total;
@@ -100,8 +97,12 @@ struct AttnMapArgs {
     int bias_row0, bias_rows, bias_cols;
     long long bias_ld;
     float* map;             // (map_rows, map_cols) FP32
-    int map_row0, map_rows, map_cols;
+    int map_row0;
     long long map_ld;
+    // The block by segment: rows [row_lo, row_lo + row_n) of a query segment (128-row
+    // tiles), the first key_n keys of a key segment (64-key tiles).
+    int row_lo[2], row_n[2], row_tiles0;
+    int key_n[2], key_tiles0;
     // The visibility rules the attention kernel applied, so that the map agrees
     // with the output: a masked key has weight 0, a scaled key a scaled score.
     int mask_mode;          // 1: key j visible to query i iff j <= i + q_offset
@@ -109,7 +110,14 @@ struct AttnMapArgs {
     const float* key_mask;  // Lk floats, 0 = masked; or null
     const float* key_scale; // Lk floats or null
 };
-cudaError_t launch_attn_map(const AttnMapArgs& a, bool bf16, cudaStream_t stream);
+struct AttnMapLaunch {
+    CUtensorMap tmQ[2], tmK[2];   // boxes of 128 query rows, 64 keys
+    AttnMapArgs args;
+    int row_tiles, key_tiles;
+    int head_dim;                 // columns computed with: 64 or 128
+    bool bf16;
+};
+cudaError_t launch_attn_map(const AttnMapLaunch& L, cudaStream_t stream);
 
 // Per-head RMSNorm + RoPE.
 struct NormRopeJobDev {

@@ -179,7 +179,6 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
     uint64_t* v_ready = v_empty + VS;    // [VS]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_ready + VS);
 
-    dependents_may_launch();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int head = blockIdx.y;
@@ -235,6 +234,8 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // only now: a dependent CTA that took tensor memory first could keep this one from getting its own
+    dependents_may_launch();
     // barriers, tensor memory and descriptors are set up; from here on global memory is touched
     wait_for_prior_grid();
 

@@ -77,20 +77,30 @@ inline int sm_count() {
 // its set-up and then holds at wait_for_prior_grid() until the earlier grid has
 // completed and its writes are visible.  Every kernel launched this way calls
 // wait_for_prior_grid() before its first access to global memory.
+// With a cluster of more than one CTA, `cluster` gives its size.
 template <class... KArgs, class... Args>
-inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                    cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_dependent_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                            cudaStream_t stream, dim3 cluster, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster.x;
+    attr[1].val.clusterDim.y = cluster.y;
+    attr[1].val.clusterDim.z = cluster.z;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster.x * cluster.y * cluster.z > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <class... KArgs, class... Args>
+inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t stream, Args&&... args) {
+    return launch_dependent_cluster(kernel, grid, block, smem, stream, dim3(1), static_cast<Args&&>(args)...);
 }
 __device__ __forceinline__ void dependents_may_launch() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
