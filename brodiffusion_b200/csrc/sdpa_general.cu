@@ -1,9 +1,20 @@
-// Softmax attention forward for head dims the tensor-core kernel does not
-// take (any multiple of 8 up to 256): a plain tiled online-softmax kernel on
-// the CUDA cores with FP32 arithmetic.  One CTA = 32 query rows of one
-// (batch, head); key/value tiles of 32 rows are staged in shared memory as
-// FP32.  Thread (r, c) = (tid / 4, tid % 4) owns query row r: it computes 8 of
-// the 32 scores of a tile and accumulates output columns c, c+4, c+8, ...
+// Softmax attention forward for the head dims the tcgen05 kernel does not take (136
+// to 256; SD1.5's deepest levels have 160), with the probabilities kept to FP32.
+//
+// These calls are small (64 to 576 queries, 8 heads): what counts is how many SMs a
+// call reaches and how short a CTA's chain of loads and products is, so the tiles are
+// far below a tcgen05 tile.  One CTA = 16 * MT query rows of one (batch, head); its
+// four warps take the 16-key chunks of the sequence in turn, each with a ring of two
+// K / V chunks of its own (cp.async, no CTA barrier in the loop) and a running
+// maximum, sum and accumulator of its own, which are merged through shared memory at
+// the end.  Products run on mma.sync m16n8k16 with FP32 accumulation; a probability is
+// split into 16-bit parts that add up to it (two for FP16, three for BF16, where two
+// would keep 16 of its 24 bits), one product each, so that nothing is rounded to 16
+// bits before the output.
+// Two row tiles per CTA (MT = 2) halve the reads of K and V where there are still
+// enough CTAs for that.
+// A CUDA-core kernel stood here before: the two attention calls of a 64-token block
+// (8 heads of 160) took 250 of its 354 us.
 // Same arithmetic as src/dit/common.cpp:246-305 with FP32 scores.
 #include "sdpa_internal.h"
 #include "tc05.cuh"
@@ -11,165 +22,342 @@
 namespace bdattn {
 namespace {
 
-constexpr int kGRows = 32;
-constexpr int kGKeys = 32;
+constexpr int kGWarps = 4;
+constexpr int kGThreads = kGWarps * 32;
+constexpr int kGKeys = 16;     // keys of a chunk
 
+// Rows of HD elements, 16 bytes apart from a multiple of 32: an odd number of 16-byte
+// units, so that the eight rows of an ldmatrix fall into different banks.
+template <int HD>
+struct GenCfg {
+    static constexpr int kLd = HD + 8;                        // elements
+    static constexpr int kChunk = kGKeys * kLd;               // elements of a K or V chunk
+    static constexpr int kRing = kGWarps * 2 * 2 * kChunk * 2;   // bytes: two stages of K and V per warp
+    static constexpr int kMergeLd = HD + 4;                   // floats
+    static constexpr int smem(int mt) {
+        const int q = 16 * mt * kLd * 2;
+        const int merge = kGWarps * 16 * mt * (kMergeLd + 2) * 4;
+        return q + (kRing > merge ? kRing : merge);
+    }
+};
+
+__device__ __forceinline__ void gen_ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void gen_ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
 template <bool kBf16>
-__device__ __forceinline__ float ld16(const void* p, long long i) {
-    if constexpr (kBf16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
-    else return __half2float(reinterpret_cast<const __half*>(p)[i]);
+__device__ __forceinline__ void gen_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    if constexpr (kBf16)
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+            "{%0, %1, %2, %3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    else
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+            "{%0, %1, %2, %3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// 16 bytes global -> shared; zeros where `live` is false (the source is not read then)
+__device__ __forceinline__ void gen_cp16(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+// Takes the 16-bit part off a pair of floats: returns it packed, leaves the remainder.
+template <bool kBf16>
+__device__ __forceinline__ uint32_t gen_part(float& x, float& y) {
+    const uint32_t w = pack2<kBf16>(x, y);
+    if constexpr (kBf16) {
+        x -= __uint_as_float(w << 16);
+        y -= __uint_as_float(w & 0xffff0000u);
+    } else {
+        const __half2 h = *reinterpret_cast<const __half2*>(&w);
+        x -= __low2float(h);
+        y -= __high2float(h);
+    }
+    return w;
 }
 
-template <bool kBf16>
-__global__ void __launch_bounds__(128) sdpa_general_kernel(const SdpaGeneralArgs a, int q_ctas0) {
-    extern __shared__ float sm[];
-    const int hd = a.head_dim;
-    const int hdp = hd + 1;
-    float* Qs = sm;                      // [32][hdp]
-    float* Ks = Qs + kGRows * hdp;       // [32][hdp]
-    float* Vs = Ks + kGKeys * hdp;       // [32][hd]
-    float* Ps = Vs + kGKeys * hd;        // [32][33]
+template <int HD, int MT, bool kBf16>
+__global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGeneralArgs a, int q_ctas0) {
+    using C = GenCfg<HD>;
+    constexpr int kParts = kBf16 ? 3 : 2;
+    extern __shared__ __align__(16) uint8_t gsm[];
+    uint16_t* Qs = reinterpret_cast<uint16_t*>(gsm);                                    // [16 * MT][kLd]
+    uint8_t* ring = gsm + 16 * MT * C::kLd * 2;
 
-    const int tid = threadIdx.x;
-    const int r = tid >> 2;
-    const int c = tid & 3;
-    const int head = blockIdx.y;
-    const int batch = blockIdx.z;
+    dependents_may_launch();
+    wait_for_prior_grid();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, q4 = lane & 3;
+    const int hd = a.head_dim, vecs = hd >> 3;
+    const int head = blockIdx.y, batch = blockIdx.z;
     const int qseg = static_cast<int>(blockIdx.x) >= q_ctas0 ? 1 : 0;
-    const int qrow0 = (qseg ? static_cast<int>(blockIdx.x) - q_ctas0 : static_cast<int>(blockIdx.x)) * kGRows;
+    const int qrow0 = (qseg ? static_cast<int>(blockIdx.x) - q_ctas0 : static_cast<int>(blockIdx.x)) * (16 * MT);
     const int seg_rows = qseg ? a.q_rows[1] : a.q_rows[0];
     const int q_glob0 = (qseg ? a.q_rows[0] : 0) + qrow0;
-    const void* qp = qseg ? a.q[1] : a.q[0];
-    const long long q_ld = qseg ? a.q_ld[1] : a.q_ld[0];
-    const long long q_bs = qseg ? a.q_bs[1] : a.q_bs[0];
-
-    for (int i = tid; i < kGRows * hd; i += 128) {
-        const int rr = i / hd, d = i - rr * hd;
-        float v = 0.0f;
-        if (qrow0 + rr < seg_rows)
-            v = ld16<kBf16>(qp, batch * q_bs + static_cast<long long>(qrow0 + rr) * q_ld + head * hd + d);
-        Qs[rr * hdp + d] = v * a.scale;
-    }
-
     const int Lk = a.kv_rows[0] + a.kv_rows[1];
     int k_end = Lk;
     if (a.mask_mode == 1) {
-        const int last = q_glob0 + min(kGRows, seg_rows - qrow0) - 1;
+        const int last = q_glob0 + min(16 * MT, seg_rows - qrow0) - 1;
         k_end = max(0, min(Lk, last + a.q_offset + 1));
     }
-    const int q_glob = q_glob0 + r;
-    float m_run = -INFINITY, l_run = 0.0f;
-    float o[64];
-#pragma unroll
-    for (int i = 0; i < 64; ++i) o[i] = 0.0f;
+    const int n_chunks = (k_end + kGKeys - 1) / kGKeys;
+    const long long kv_col = static_cast<long long>(head / a.kv_group) * hd;
 
-    for (int k0 = 0; k0 < k_end; k0 += kGKeys) {
-        __syncthreads();
-        for (int i = tid; i < kGKeys * hd; i += 128) {
-            const int kk = i / hd, d = i - kk * hd;
-            const int kg = k0 + kk;
-            float kvv = 0.0f, vvv = 0.0f;
-            if (kg < Lk) {
-                const int seg = kg >= a.kv_rows[0] ? 1 : 0;
-                const int rr = seg ? kg - a.kv_rows[0] : kg;
-                const void* kp = seg ? a.k[1] : a.k[0];
-                const void* vp = seg ? a.v[1] : a.v[0];
-                const long long kld = seg ? a.k_ld[1] : a.k_ld[0];
-                const long long vld = seg ? a.v_ld[1] : a.v_ld[0];
-                const long long kbs = seg ? a.k_bs[1] : a.k_bs[0];
-                const long long vbs = seg ? a.v_bs[1] : a.v_bs[0];
-                kvv = ld16<kBf16>(kp, batch * kbs + static_cast<long long>(rr) * kld + (head / a.kv_group) * hd + d);
-                vvv = ld16<kBf16>(vp, batch * vbs + static_cast<long long>(rr) * vld + (head / a.kv_group) * hd + d);
-                if (a.key_scale != nullptr) kvv *= __ldg(a.key_scale + kg);
-                if (a.val_scale != nullptr) vvv *= __ldg(a.val_scale + kg);
-            }
-            Ks[kk * hdp + d] = kvv;
-            Vs[kk * hd + d] = vvv;
+    // K / V chunk `ch` into stage `st` of this warp's ring.  Columns past head_dim and keys past
+    // the sequence read as zero.
+    uint16_t* wring = reinterpret_cast<uint16_t*>(ring) + warp * 4 * C::kChunk;
+    auto fetch = [&](int ch, int st) {
+        const uint32_t kd = smem_u32(wring + st * 2 * C::kChunk);
+#pragma unroll 2
+        for (int i = lane; i < kGKeys * (HD / 8); i += 32) {
+            const int kk = i / (HD / 8), v = i - kk * (HD / 8);
+            const int kg = ch * kGKeys + kk;
+            const bool live = kg < Lk && v < vecs;
+            const int seg = live && kg >= a.kv_rows[0] ? 1 : 0;
+            const long long rr = live ? (seg ? kg - a.kv_rows[0] : kg) : 0;
+            const long long col = live ? kv_col + v * 8 : 0;
+            const uint16_t* kp = static_cast<const uint16_t*>(seg ? a.k[1] : a.k[0]) +
+                                 (batch * (seg ? a.k_bs[1] : a.k_bs[0]) + rr * (seg ? a.k_ld[1] : a.k_ld[0]) + col);
+            const uint16_t* vp = static_cast<const uint16_t*>(seg ? a.v[1] : a.v[0]) +
+                                 (batch * (seg ? a.v_bs[1] : a.v_bs[0]) + rr * (seg ? a.v_ld[1] : a.v_ld[0]) + col);
+            const uint32_t d = kd + (kk * C::kLd + v * 8) * 2;
+            gen_cp16(d, kp, live);
+            gen_cp16(d + C::kChunk * 2, vp, live);
         }
-        __syncthreads();
+    };
 
-        float s[8];
-        float mx = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int kk = c * 8 + i;
-            const int kg = k0 + kk;
-            float acc = 0.0f;
-            for (int d = 0; d < hd; ++d) acc = fmaf(Qs[r * hdp + d], Ks[kk * hdp + d], acc);
-            bool vis = kg < Lk;
-            if (a.mask_mode == 1) vis = vis && (kg <= q_glob + a.q_offset);
-            if (vis && a.key_mask != nullptr) vis = __ldg(a.key_mask + kg) != 0.0f;
-            s[i] = vis ? acc : -INFINITY;
-            mx = fmaxf(mx, s[i]);
-        }
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        const float m_new = fmaxf(m_run, mx);
-        const float m_use = (m_new == -INFINITY) ? 0.0f : m_new;
-        const float alpha = (m_run == -INFINITY) ? 0.0f : __expf(m_run - m_use);
-        float rs = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float p = __expf(s[i] - m_use);
-            rs += p;
-            Ps[r * 33 + c * 8 + i] = p;
-        }
-        rs += __shfl_xor_sync(0xffffffffu, rs, 1);
-        rs += __shfl_xor_sync(0xffffffffu, rs, 2);
-        l_run = l_run * alpha + rs;
-        m_run = m_new;
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-            const int d = c + 4 * i;
-            if (d < hd) {
-                float acc = o[i] * alpha;
-                for (int kk = 0; kk < kGKeys; ++kk) acc = fmaf(Ps[r * 33 + kk], Vs[kk * hd + d], acc);
-                o[i] = acc;
-            }
-        }
-        __syncwarp();
-    }
-
-    if (qrow0 + r < seg_rows) {
-        const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
-        void* op = qseg ? a.o[1] : a.o[0];
-        const long long o_ld = qseg ? a.o_ld[1] : a.o_ld[0];
-        const long long o_bs = qseg ? a.o_bs[1] : a.o_bs[0];
-        const long long base = batch * o_bs + static_cast<long long>(qrow0 + r) * o_ld + head * hd;
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-            const int d = c + 4 * i;
-            if (d < hd) {
-                if constexpr (kBf16) reinterpret_cast<__nv_bfloat16*>(op)[base + d] = __float2bfloat16_rn(o[i] * inv);
-                else reinterpret_cast<__half*>(op)[base + d] = __float2half_rn(o[i] * inv);
-            }
+    // Q rows (zero past the segment and past head_dim)
+    {
+        const uint16_t* qp = static_cast<const uint16_t*>(qseg ? a.q[1] : a.q[0]) + batch * (qseg ? a.q_bs[1] : a.q_bs[0]) +
+                             static_cast<long long>(head) * hd;
+        const long long q_ld = qseg ? a.q_ld[1] : a.q_ld[0];
+        for (int i = threadIdx.x; i < 16 * MT * (HD / 8); i += kGThreads) {
+            const int r = i / (HD / 8), v = i - r * (HD / 8);
+            const bool live = qrow0 + r < seg_rows && v < vecs;
+            gen_cp16(smem_u32(Qs + r * C::kLd + v * 8), qp + (live ? static_cast<long long>(qrow0 + r) * q_ld + v * 8 : 0), live);
         }
     }
+    if (warp < n_chunks) fetch(warp, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+
+    // FP16: probabilities carry a factor of 2^10 (it cancels in O / l), which keeps small ones out
+    // of the subnormals; with value scales they carry the power of two that brings the largest scale
+    // to at most one instead, so that no part overflows.
+    const float boost = kBf16 ? 0.0f : 10.0f;
+    float v_mul = 1.0f, v_undo = 1.0f;
+    if (!kBf16 && a.val_scale != nullptr) {
+        float mx = 0.0f;
+        for (int i = lane; i < Lk; i += 32) mx = fmaxf(mx, fabsf(__ldg(a.val_scale + i)));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (mx > 1.0f && mx < INFINITY) {
+            int e;
+            frexpf(mx, &e);                       // mx <= 2^e
+            v_mul = ldexpf(1.0f, -e / 2) * ldexpf(1.0f, -(e - e / 2));
+            v_undo = 1.0f / v_mul;
+        }
+    }
+
+    float o[MT][HD / 8][4];
+    float m_run[MT][2], l_run[MT][2];
+#pragma unroll
+    for (int t = 0; t < MT; ++t) {
+        m_run[t][0] = m_run[t][1] = -INFINITY;
+        l_run[t][0] = l_run[t][1] = 0.0f;
+#pragma unroll
+        for (int n = 0; n < HD / 8; ++n) o[t][n][0] = o[t][n][1] = o[t][n][2] = o[t][n][3] = 0.0f;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                             // Q from all warps
+
+    const float sl2 = a.scale * 1.4426950408889634f;
+    const uint32_t q_addr = smem_u32(Qs + (lane & 15) * C::kLd + (lane >> 4) * 8);
+    int st = 0;
+    for (int ch = warp; ch < n_chunks; ch += kGWarps, st ^= 1) {
+        if (ch + kGWarps < n_chunks) fetch(ch + kGWarps, st ^ 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");      // this chunk (all but the newest group)
+        __syncwarp();
+        const uint16_t* Kc = wring + st * 2 * C::kChunk;
+        // B fragments: K is (key, d) = (n, k) row-major; matrices keys 0-7 | 8-15 x d 0-7 | 8-15
+        const uint32_t k_addr = smem_u32(Kc + ((lane & 7) + ((lane >> 4) << 3)) * C::kLd + ((lane >> 3) & 1) * 8);
+        const uint32_t v_addr = smem_u32(Kc + C::kChunk + (lane & 15) * C::kLd + (lane >> 4) * 8);
+
+        float s[MT][2][4];
+#pragma unroll
+        for (int t = 0; t < MT; ++t)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) s[t][n][0] = s[t][n][1] = s[t][n][2] = s[t][n][3] = 0.0f;
+#pragma unroll
+        for (int kk = 0; kk < HD / 16; ++kk) {
+            uint32_t b[4];
+            gen_ldsm4(b, k_addr + kk * 32);
+#pragma unroll
+            for (int t = 0; t < MT; ++t) {
+                uint32_t qa[4];
+                gen_ldsm4(qa, q_addr + t * 16 * C::kLd * 2 + kk * 32);
+                gen_mma<kBf16>(s[t][0], qa, b[0], b[1]);
+                gen_mma<kBf16>(s[t][1], qa, b[2], b[3]);
+            }
+        }
+
+        // this thread's four keys: 2 * q4 + {0, 1} and the same + 8
+        float ks[4], vs[4];
+        bool seen[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int kg = ch * kGKeys + (i >> 1) * 8 + q4 * 2 + (i & 1);
+            const bool in = kg < Lk;
+            seen[i] = in && (a.key_mask == nullptr || __ldg(a.key_mask + kg) != 0.0f);
+            ks[i] = sl2 * (in && a.key_scale != nullptr ? __ldg(a.key_scale + kg) : 1.0f);
+            vs[i] = in && a.val_scale != nullptr ? __ldg(a.val_scale + kg) * v_mul : 1.0f;
+        }
+        uint32_t pa[MT][kParts][4];
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {                      // row g, row g + 8
+                const int q_glob = q_glob0 + t * 16 + hf * 8 + g;
+                float x[4];
+                float mx = -INFINITY;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int kg = ch * kGKeys + (i >> 1) * 8 + q4 * 2 + (i & 1);
+                    const bool vis = seen[i] && (a.mask_mode != 1 || kg <= q_glob + a.q_offset);
+                    x[i] = vis ? s[t][i >> 1][hf * 2 + (i & 1)] * ks[i] : -INFINITY;
+                    mx = fmaxf(mx, x[i]);
+                }
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                const float m_new = fmaxf(m_run[t][hf], mx);
+                const float m_use = m_new == -INFINITY ? 0.0f : m_new;
+                if (m_new != m_run[t][hf]) {
+                    const float alpha = m_run[t][hf] == -INFINITY ? 0.0f : fast_exp2(m_run[t][hf] - m_use);
+                    l_run[t][hf] *= alpha;
+#pragma unroll
+                    for (int n = 0; n < HD / 8; ++n) {
+                        o[t][n][hf * 2] *= alpha;
+                        o[t][n][hf * 2 + 1] *= alpha;
+                    }
+                    m_run[t][hf] = m_new;
+                }
+                float p[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    p[i] = fast_exp2(x[i] - m_use + boost);
+                    l_run[t][hf] += p[i];
+                    p[i] *= vs[i];
+                }
+#pragma unroll
+                for (int k = 0; k < kParts; ++k) {
+                    pa[t][k][hf] = gen_part<kBf16>(p[0], p[1]);          // keys 2 q4, 2 q4 + 1
+                    pa[t][k][2 + hf] = gen_part<kBf16>(p[2], p[3]);      // the same + 8
+                }
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < HD / 16; ++n) {
+            uint32_t b[4];
+            gen_ldsm4_t(b, v_addr + n * 32);
+#pragma unroll
+            for (int t = 0; t < MT; ++t) {
+#pragma unroll
+                for (int k = kParts - 1; k >= 0; --k) {                  // smallest part first
+                    gen_mma<kBf16>(o[t][2 * n], pa[t][k], b[0], b[1]);
+                    gen_mma<kBf16>(o[t][2 * n + 1], pa[t][k], b[2], b[3]);
+                }
+            }
+        }
+        __syncwarp();                            // the stage is refilled in the next step
+    }
+
+    // merge of the four warps' results (the ring is at rest)
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    constexpr int kRows = 16 * MT;
+    float* Om = reinterpret_cast<float*>(ring);                          // [warps][kRows][kMergeLd]
+    float* Sm = Om + kGWarps * kRows * C::kMergeLd;                      // [warps][kRows][2]
+#pragma unroll
+    for (int t = 0; t < MT; ++t) {
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const int r = t * 16 + hf * 8 + g;
+            float l = l_run[t][hf];
+            l += __shfl_xor_sync(0xffffffffu, l, 1);
+            l += __shfl_xor_sync(0xffffffffu, l, 2);
+            if (q4 == 0) {
+                Sm[(warp * kRows + r) * 2] = m_run[t][hf];
+                Sm[(warp * kRows + r) * 2 + 1] = l;
+            }
+            float* orow = Om + (warp * kRows + r) * C::kMergeLd + q4 * 2;
+#pragma unroll
+            for (int n = 0; n < HD / 8; ++n)
+                *reinterpret_cast<float2*>(orow + n * 8) = make_float2(o[t][n][hf * 2], o[t][n][hf * 2 + 1]);
+        }
+    }
+    __syncthreads();
+    uint16_t* op = static_cast<uint16_t*>(qseg ? a.o[1] : a.o[0]) + batch * (qseg ? a.o_bs[1] : a.o_bs[0]) +
+                   static_cast<long long>(head) * hd;
+    const long long o_ld = qseg ? a.o_ld[1] : a.o_ld[0];
+    for (int i = threadIdx.x; i < kRows * vecs; i += kGThreads) {
+        const int r = i / vecs, v = i - r * vecs;
+        if (qrow0 + r >= seg_rows) break;        // rows only grow from here on
+        float m = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < kGWarps; ++w) m = fmaxf(m, Sm[(w * kRows + r) * 2]);
+        float l = 0.0f, f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kGWarps; ++w) {
+            const float mw = Sm[(w * kRows + r) * 2];
+            const float c = mw == -INFINITY ? 0.0f : fast_exp2(mw - m);
+            l = fmaf(c, Sm[(w * kRows + r) * 2 + 1], l);
+            const float* src = Om + (w * kRows + r) * C::kMergeLd + v * 8;
+            const float4 u0 = *reinterpret_cast<const float4*>(src), u1 = *reinterpret_cast<const float4*>(src + 4);
+            f[0] = fmaf(c, u0.x, f[0]); f[1] = fmaf(c, u0.y, f[1]); f[2] = fmaf(c, u0.z, f[2]); f[3] = fmaf(c, u0.w, f[3]);
+            f[4] = fmaf(c, u1.x, f[4]); f[5] = fmaf(c, u1.y, f[5]); f[6] = fmaf(c, u1.z, f[6]); f[7] = fmaf(c, u1.w, f[7]);
+        }
+        const float inv = l > 0.0f ? v_undo / l : 0.0f;
+        uint4 w4;
+        w4.x = pack2<kBf16>(f[0] * inv, f[1] * inv); w4.y = pack2<kBf16>(f[2] * inv, f[3] * inv);
+        w4.z = pack2<kBf16>(f[4] * inv, f[5] * inv); w4.w = pack2<kBf16>(f[6] * inv, f[7] * inv);
+        *reinterpret_cast<uint4*>(op + static_cast<long long>(qrow0 + r) * o_ld + v * 8) = w4;
+    }
+}
+
+template <int HD, int MT, bool kBf16>
+cudaError_t launch_general_t(const SdpaGeneralArgs& a, int num_heads, int batch, cudaStream_t stream) {
+    auto kern = sdpa_general_kernel<HD, MT, kBf16>;
+    constexpr int smem = GenCfg<HD>::smem(MT);
+    cudaError_t e = set_max_smem_once(kern, smem);
+    if (e != cudaSuccess) return e;
+    const int q_ctas0 = (a.q_rows[0] + 16 * MT - 1) / (16 * MT);
+    const int q_ctas1 = (a.q_rows[1] + 16 * MT - 1) / (16 * MT);
+    dim3 grid(static_cast<unsigned>(q_ctas0 + q_ctas1), static_cast<unsigned>(num_heads),
+              static_cast<unsigned>(batch));
+    return launch_dependent(kern, grid, dim3(kGThreads), smem, stream, a, q_ctas0);
 }
 
 }  // namespace
 
 cudaError_t launch_sdpa_general(const SdpaGeneralArgs& a, int num_heads, int batch, bool bf16,
                                 cudaStream_t stream) {
-    const int hd = a.head_dim;
-    const size_t smem = sizeof(float) * (static_cast<size_t>(kGRows) * (hd + 1) + kGKeys * (hd + 1) +
-                                         kGKeys * hd + kGRows * 33);
-    const int q_ctas0 = (a.q_rows[0] + kGRows - 1) / kGRows;
-    const int q_ctas1 = (a.q_rows[1] + kGRows - 1) / kGRows;
-    dim3 grid(static_cast<unsigned>(q_ctas0 + q_ctas1), static_cast<unsigned>(num_heads),
-              static_cast<unsigned>(batch));
-    cudaError_t e;
-    if (bf16) {
-        e = set_max_smem_once(sdpa_general_kernel<true>, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-        sdpa_general_kernel<true><<<grid, 128, smem, stream>>>(a, q_ctas0);
-    } else {
-        e = set_max_smem_once(sdpa_general_kernel<false>, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-        sdpa_general_kernel<false><<<grid, 128, smem, stream>>>(a, q_ctas0);
-    }
-    return cudaGetLastError();
+    if (a.head_dim > 160)
+        return bf16 ? launch_general_t<256, 1, true>(a, num_heads, batch, stream)
+                    : launch_general_t<256, 1, false>(a, num_heads, batch, stream);
+    // two row tiles per CTA once that still leaves one CTA per SM
+    const long long rows = static_cast<long long>(a.q_rows[0]) + a.q_rows[1];
+    if ((rows + 31) / 32 * num_heads * batch >= sm_count())
+        return bf16 ? launch_general_t<160, 2, true>(a, num_heads, batch, stream)
+                    : launch_general_t<160, 2, false>(a, num_heads, batch, stream);
+    return bf16 ? launch_general_t<160, 1, true>(a, num_heads, batch, stream)
+                : launch_general_t<160, 1, false>(a, num_heads, batch, stream);
 }
 
 }  // namespace bdattn

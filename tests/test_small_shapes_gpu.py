@@ -1,5 +1,5 @@
-"""Calls whose shape decides the route: map blocks at the edges of their tiles and
-segments.  References: the CPU oracle."""
+"""Calls whose shape decides the route: head dims above 128 (mma.sync kernel) and map
+blocks at the edges of their tiles and segments.  References: the CPU oracle."""
 import numpy as np
 import pytest
 import torch
@@ -12,6 +12,51 @@ pytestmark = pytest.mark.gpu
 
 def _acts(shapes, seed, storage):
     return [synth.activations(s, seed + i, storage) for i, s in enumerate(shapes)]
+
+
+# Rows and keys around the 16-row / 16-key tiles, one and two row tiles per CTA (the
+# second where the call fills the SMs), both padded widths, every option of the kernel.
+# The probabilities keep FP32 and only the output is rounded: half an ulp of a value
+# below 4 is 2^-8 in BF16 and 2^-10 in FP16.
+@pytest.mark.parametrize("storage", ["bf16", "fp16"])
+@pytest.mark.parametrize("hd,nh,Lq,Lk,opt", [
+    (160, 8, 64, 64, ""), (160, 8, 1, 1, ""), (160, 2, 17, 15, "mask"), (160, 3, 33, 129, "causal"),
+    (160, 8, 576, 577, "mask"), (160, 8, 600, 77, "scale"), (136, 2, 70, 49, "scale"), (256, 2, 48, 130, "causal"),
+    (168, 5, 31, 200, "mask"), (200, 1, 16, 16, "scale"), (160, 2, 40, 24, "causal")])
+def test_head_dims_above_128(bd, oracle, storage, hd, nh, Lq, Lk, opt):
+    q, k, v = _acts([(Lq, nh * hd), (Lk, nh * hd), (Lk, nh * hd)], 9500 + hd + Lq, storage)
+    kw = {}
+    if opt == "causal":
+        kw["mask_mode"] = 1
+    if opt == "mask":
+        kw["key_mask"] = (synth.uniform01(Lk, 9501) > 0.3).astype(np.float32)
+    if opt == "scale":
+        kw["key_scale"] = 0.5 + synth.uniform01(Lk, 9502).astype(np.float32)
+        kw["val_scale"] = (100.0 * synth.uniform01(Lk, 9503)).astype(np.float32) ** 2 if storage == "fp16" else \
+            synth.uniform01(Lk, 9503).astype(np.float32)
+        if storage == "fp16":
+            v = synth.round_fp16(v * 1e-3)
+    dt = torch.bfloat16 if storage == "bf16" else torch.float16
+    got = G.sdpa(bd, q, k, v, nh, dtype=dt, **kw)
+    ks, vs = kw.pop("key_scale", None), kw.pop("val_scale", None)
+    if ks is not None:
+        k, v = k * ks[:, None], v * vs[:, None]
+    ref = oracle.sdpa(q, k, v, nh, **kw)
+    half_ulp = np.exp2(np.ceil(np.log2(np.abs(ref).max() + 1e-9))) * (2.0 ** -9 if storage == "bf16" else 2.0 ** -12)
+    assert np.abs(got - ref).max() <= half_ulp + 1e-4 * np.abs(ref).max()
+
+
+def test_head_dims_above_128_segments_and_groups(bd, oracle):
+    """Two segments on both sides whose border is inside a tile, two query heads per K/V head."""
+    hd, nh, nkv = 160, 4, 2
+    q = synth.activations((45, nh * hd), 9520)
+    k, v = _acts([(39, nkv * hd)] * 2, 9521, "bf16")
+    tq, tk, tv = G.dev(q), G.dev(k), G.dev(v)
+    out = torch.full_like(tq, float("nan"))
+    bd.sdpa_fwd([tq[:21], tq[21:]], [tk[:19], tk[19:]], [tv[:19], tv[19:]], [out[:21], out[21:]], nh, num_kv_heads=nkv)
+    assert bd.device_status() == 0
+    rep = lambda x: np.repeat(x.reshape(-1, nkv, hd), nh // nkv, axis=1).reshape(x.shape[0], -1)
+    G.check(G.host(out), oracle.sdpa(q, rep(k), rep(v), nh), what="segments and groups, head_dim 160")
 
 
 # Map blocks: rows and keys around the 128 x 64 tiles, blocks that begin inside a segment
