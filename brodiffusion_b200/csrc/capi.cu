@@ -144,80 +144,87 @@ int make_map_2d(const char* op, CUtensorMap* m, const void* base, bool bf16, lon
 
 int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
-// Width each head is padded to for the tensor-core attention kernel (0: the
-// general kernel is used and heads stay unpadded).
-int padded_head_dim(int hd) {
-    if (hd % 8 != 0) return 0;
-    if (hd <= 64) return 64;
-    if (hd <= 128) return 128;
-    return 0;
-}
-
-// One GEMM problem  C[M, N] = A[M, K] . W[N, K]^T (+ bias).  head_dim > 0 cuts
-// the N dimension into per-head tiles whose results land head_pad columns
-// apart (zero filled); head_dim == 0 uses plain 64-column tiles.
+// One GEMM problem  C[M, N] = A[M, K] . W[N, K]^T (+ bias).  head_dim > 0 asks for
+// tiles of whole heads (norm + RoPE epilogue).
 int add_gemm_problem(const char* op, bdattn::GemmLaunch& L, int idx, const void* A, long long lda,
                      const void* W, long long ldw, const void* bias, void* Cout, long long ldc, int M,
-                     int N, int K, int head_dim, int head_pad, int geglu_offset) {
+                     int N, int K, int head_dim, int geglu_offset) {
     if (A == nullptr || W == nullptr || Cout == nullptr) return fail("%s: null matrix pointer", op);
     if (M < 1 || N < 1 || K < 1) return fail("%s: empty matrix (M=%d N=%d K=%d)", op, M, N, K);
     if (K % 8 != 0 || lda % 8 != 0 || ldw % 8 != 0 || ldc % 8 != 0 || lda < K || ldw < K)
         return fail("%s: inner size and row strides must be multiples of 8 elements (K=%d lda=%lld ldw=%lld "
                     "ldc=%lld)", op, K, lda, ldw, ldc);
     if (!aligned16(A) || !aligned16(W) || !aligned16(Cout)) return fail("%s: matrices must be 16-byte aligned", op);
-    {
-        // columns one output row receives: N, or head_pad per head for head tiles
-        const long long written = head_dim > 0 ? static_cast<long long>(N / head_dim) * head_pad : N;
-        if (ldc < written)
-            return fail("%s: output row stride %lld is smaller than the %lld columns written per row", op, ldc, written);
-    }
+    if (ldc < N) return fail("%s: output row stride %lld is smaller than the %d columns written per row", op, ldc, N);
+    if (N % 8 != 0) return fail("%s: output width must be a multiple of 8 (got %d)", op, N);
     bdattn::GemmProblem& p = L.args.p[idx];
     p.M = M; p.N = N; p.K = K; p.C = Cout; p.ldc = ldc; p.bias = bias;
     p.tiles_m = (M + 127) / 128;
     p.geglu_offset = geglu_offset;
-    if (head_dim > 0) {
-        if (N % head_dim != 0) return fail("%s: output width %d is not a multiple of head_dim %d", op, N, head_dim);
-        p.n_tile = round_up(head_dim, 16);
-        p.n_step = head_dim;
-        p.n_valid = head_dim;
-        p.c_step = head_pad;
-        p.c_fill = head_pad;
-        p.tiles_n = N / head_dim;
-    } else {
-        if (N % 8 != 0) return fail("%s: output width must be a multiple of 8 (got %d)", op, N);
-        // 128-column tiles once the output is wide enough to fill the SMs with them
-        const int tile = (geglu_offset == 0 && static_cast<long long>((M + 127) / 128) * ((N + 127) / 128) >= 148) ? 128 : 64;
-        p.n_tile = tile;
-        p.n_step = tile;
-        p.n_valid = tile;
-        p.c_step = tile;
-        p.c_fill = tile;      // the epilogue stops at the matrix edge on a ragged last tile
-        p.tiles_n = (N + tile - 1) / tile;
-    }
+    p.n_tile = head_dim;       // 0: chosen at the launch
     if (make_map_2d(op, &L.tmA[idx], A, L.bf16, K, M, lda, 128)) return -1;
     // the weight matrix has N (+ D_out for GEGLU) rows
-    const long long w_rows = geglu_offset > 0 ? static_cast<long long>(N) + geglu_offset : N;
-    if (make_map_2d(op, &L.tmB[idx], W, L.bf16, K, w_rows, ldw, p.n_tile)) return -1;
-    // 128 x 256 tiles need whole tiles along N and, for head tiles, unpadded heads of 64 or 128
-    // (GEGLU: a tile is 128 value columns + their 128 gate columns, two 128-row boxes)
-    L.wide[idx] = geglu_offset > 0
-                      ? N % 128 == 0
-                      : N % 256 == 0 && (head_dim == 0 || (head_dim == head_pad && (head_dim == 64 || head_dim == 128)));
-    if (L.wide[idx] && make_map_2d(op, &L.tmBw[idx], W, L.bf16, K, w_rows, ldw, geglu_offset > 0 ? 128 : 256)) return -1;
+    L.W[idx] = W;
+    L.ldw[idx] = ldw;
+    L.w_rows[idx] = geglu_offset > 0 ? static_cast<long long>(N) + geglu_offset : N;
+    // the pair kernel's tiles are 256 columns (GEGLU: 128 value columns + their gate columns)
+    L.whole[idx] = N % (geglu_offset > 0 ? 128 : 256) == 0;
     return 0;
 }
 
-void finish_gemm_launch(bdattn::GemmLaunch& L, int n) {
+// Chooses the kernel, the tile width and the number of CTAs that share a tile's K
+// blocks for the launch's problems, makes the weight maps and launches.
+int launch_gemm(const char* op, bdattn::GemmLaunch& L, int n, cudaStream_t stream) {
     L.n_problems = n;
+    const int sms = bdattn::sm_count();
+    bool pair = true;
+    bool geglu = false, heads = false;
+    int k_max = 0;
+    for (int i = 0; i < n; ++i) {
+        pair = pair && L.whole[i];
+        geglu = geglu || L.args.p[i].geglu_offset > 0;
+        heads = heads || L.args.p[i].norm_rope;
+        k_max = L.args.p[i].K > k_max ? L.args.p[i].K : k_max;
+    }
+    pair = pair && (geglu || heads || bdattn::gemm_pair_tiles(L) >= sms / 2);
+    int width = 64, split = 1;
+    if (!pair) {
+        auto tiles = [&](int w) {
+            long long t = 0;
+            for (int i = 0; i < n; ++i) {
+                const bdattn::GemmProblem& p = L.args.p[i];
+                const int pw = p.n_tile > 0 ? p.n_tile : w;
+                t += static_cast<long long>(p.tiles_m) * ((p.N + pw - 1) / pw);
+            }
+            return t;
+        };
+        const int kb = (k_max + 63) / 64;
+        if (!geglu && tiles(128) >= sms) width = 128;
+        if (!heads)
+            while (split < 8 && tiles(width) * split * 2 <= sms * 5 / 4 && kb >= split * 2 * 4) split *= 2;
+    }
+#ifdef BDATTN_TUNE
+    if (const char* e = std::getenv("BD_W")) { const int v = std::atoi(e); if (v) { pair = v == 256; if (v < 256) width = v; else split = 1; } }
+    if (const char* e = std::getenv("BD_S")) { const int v = std::atoi(e); if (v && !pair && !heads) split = v; }
+#endif
+    L.args.split = split;
+    for (int i = 0; i < n; ++i) {
+        bdattn::GemmProblem& p = L.args.p[i];
+        if (p.n_tile == 0) p.n_tile = width;
+        p.tiles_n = (p.N + p.n_tile - 1) / p.n_tile;
+        // a CTA of a pair stages 128 weight rows
+        if (make_map_2d(op, &L.tmB[i], L.W[i], L.bf16, p.K, L.w_rows[i], L.ldw[i], pair ? 128 : p.n_tile)) return -1;
+    }
     for (int i = n; i < 3; ++i) {
         L.args.p[i] = L.args.p[0];
         L.args.p[i].tiles_m = 0;
         L.args.p[i].tiles_n = 0;
         L.tmA[i] = L.tmA[0];
         L.tmB[i] = L.tmB[0];
-        L.tmBw[i] = L.tmBw[0];
-        L.wide[i] = L.wide[0];
     }
+    const cudaError_t e = pair ? bdattn::launch_gemm_pair(L, stream) : bdattn::launch_gemm_tc05(L, stream);
+    if (e != cudaSuccess) return cuda_fail(op, e);
+    return 0;
 }
 
 }  // namespace
@@ -690,11 +697,8 @@ int bdattn_linear_fwd(const void* x, const void* w, const void* bias, void* y, i
     bdattn::GemmLaunch L;
     std::memset(&L, 0, sizeof(L));
     L.bf16 = dtype == BDATTN_BF16;
-    if (add_gemm_problem(op, L, 0, x, ldx, w, ldw, bias, y, ldy, M, N, K, 0, 0, 0)) return -1;
-    finish_gemm_launch(L, 1);
-    cudaError_t e = bdattn::launch_gemm(L, reinterpret_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) return cuda_fail(op, e);
-    return 0;
+    if (add_gemm_problem(op, L, 0, x, ldx, w, ldw, bias, y, ldy, M, N, K, 0, 0)) return -1;
+    return launch_gemm(op, L, 1, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int bdattn_qkv_norm_rope_fwd(const bdattn_qkv_proj_params* p, bdattn_stream_t stream) {
@@ -722,7 +726,7 @@ int bdattn_qkv_norm_rope_fwd(const bdattn_qkv_proj_params* p, bdattn_stream_t st
     for (int i = 0; i < 3; ++i) {
         if (w[i] == nullptr || out[i] == nullptr) continue;     // a projection may be left out
         if (add_gemm_problem(op, L, n, p->x, p->x_ld > 0 ? p->x_ld : p->in_features, w[i], p->in_features, b[i],
-                             out[i], ld[i], p->rows, N, p->in_features, p->head_dim, p->head_dim, 0))
+                             out[i], ld[i], p->rows, N, p->in_features, p->head_dim, 0))
             return -1;
         bdattn::GemmProblem& g = L.args.p[n];
         g.norm_rope = 1;
@@ -735,10 +739,7 @@ int bdattn_qkv_norm_rope_fwd(const bdattn_qkv_proj_params* p, bdattn_stream_t st
         ++n;
     }
     if (n == 0) return fail("%s: no projection requested", op);
-    finish_gemm_launch(L, n);
-    cudaError_t e = bdattn::launch_gemm(L, reinterpret_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) return cuda_fail(op, e);
-    return 0;
+    return launch_gemm(op, L, n, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int bdattn_linear_geglu_fwd(const void* x, const void* w, const void* bias, void* y, int dtype,
@@ -749,11 +750,8 @@ int bdattn_linear_geglu_fwd(const void* x, const void* w, const void* bias, void
     bdattn::GemmLaunch L;
     std::memset(&L, 0, sizeof(L));
     L.bf16 = dtype == BDATTN_BF16;
-    if (add_gemm_problem(op, L, 0, x, d_in, w, d_in, bias, y, d_out, rows, d_out, d_in, 0, 0, d_out)) return -1;
-    finish_gemm_launch(L, 1);
-    cudaError_t e = bdattn::launch_gemm(L, reinterpret_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) return cuda_fail(op, e);
-    return 0;
+    if (add_gemm_problem(op, L, 0, x, d_in, w, d_in, bias, y, d_out, rows, d_out, d_in, 0, d_out)) return -1;
+    return launch_gemm(op, L, 1, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int bdattn_add_inplace(void* y, const void* x, long long n, int dtype, bdattn_stream_t stream) {
@@ -795,7 +793,8 @@ int bdattn_add_row_bias(void* y, const void* bias, int rows, int cols, long long
 
 size_t bdattn_qkvo_workspace_bytes(int q_rows, int kv_rows, int num_heads, int head_dim) {
     if (q_rows < 0 || kv_rows < 0 || num_heads < 1 || head_dim < 1) return 0;
-    const int pad = padded_head_dim(head_dim) ? padded_head_dim(head_dim) : head_dim;
+    // room for heads padded to 64 or 128 columns, which the projections once wrote
+    const int pad = head_dim % 8 != 0 || head_dim > 128 ? head_dim : (head_dim <= 64 ? 64 : 128);
     const size_t wq = static_cast<size_t>(q_rows) * num_heads * pad * 2;
     const size_t wkv = static_cast<size_t>(kv_rows) * num_heads * pad * 2;
     const size_t wo = static_cast<size_t>(q_rows) * num_heads * head_dim * 2;
@@ -812,12 +811,9 @@ int bdattn_project_kv(const void* ctx, int ctx_rows, int ctx_cols, long long ctx
     bdattn::GemmLaunch L;
     std::memset(&L, 0, sizeof(L));
     L.bf16 = dtype == BDATTN_BF16;
-    if (add_gemm_problem(op, L, 0, ctx, ctx_ld, wk, ctx_cols, bk, k_out, kv_ld, ctx_rows, inner_dim, ctx_cols, 0, 0, 0)) return -1;
-    if (add_gemm_problem(op, L, 1, ctx, ctx_ld, wv, ctx_cols, bv, v_out, kv_ld, ctx_rows, inner_dim, ctx_cols, 0, 0, 0)) return -1;
-    finish_gemm_launch(L, 2);
-    cudaError_t e = bdattn::launch_gemm(L, reinterpret_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) return cuda_fail(op, e);
-    return 0;
+    if (add_gemm_problem(op, L, 0, ctx, ctx_ld, wk, ctx_cols, bk, k_out, kv_ld, ctx_rows, inner_dim, ctx_cols, 0, 0)) return -1;
+    if (add_gemm_problem(op, L, 1, ctx, ctx_ld, wv, ctx_cols, bv, v_out, kv_ld, ctx_rows, inner_dim, ctx_cols, 0, 0)) return -1;
+    return launch_gemm(op, L, 2, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int bdattn_qkvo_fwd(const bdattn_qkvo_params* p, bdattn_stream_t stream) {
@@ -851,57 +847,43 @@ int bdattn_qkvo_fwd(const bdattn_qkvo_params* p, bdattn_stream_t stream) {
     if (p->workspace == nullptr || p->workspace_bytes < need)
         return fail("%s: workspace of %zu bytes needed (got %zu)", op, need, p->workspace_bytes);
     if ((reinterpret_cast<uintptr_t>(p->workspace) & 255u) != 0) return fail("%s: workspace must be 256-byte aligned", op);
-    const int pad = padded_head_dim(hd);
-    const int P = pad ? pad : hd;
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     uint8_t* ws = static_cast<uint8_t*>(p->workspace);
+    const size_t q_bytes = up(static_cast<size_t>(Lq) * C * 2), kv_bytes = up(static_cast<size_t>(Lk) * C * 2);
     void* Qp = ws;
-    void* Kp = ws + up(static_cast<size_t>(Lq) * nh * P * 2);
-    void* Vp = static_cast<uint8_t*>(Kp) + up(static_cast<size_t>(Lk) * nh * P * 2);
-    void* Op = static_cast<uint8_t*>(Vp) + up(static_cast<size_t>(Lk) * nh * P * 2);
+    void* Kp = ws + q_bytes;
+    void* Vp = ws + q_bytes + kv_bytes;
+    void* Op = ws + q_bytes + 2 * kv_bytes;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const long long ldp = static_cast<long long>(nh) * P;
 
-    // 1. projections into head-padded Q / K / V
+    // 1. projections.  Heads stay unpadded: the attention kernel's tensor maps zero-fill a head
+    // of 40 or 80 columns to 64 or 128, so the projections are plain GEMMs with whole tiles and
+    // cached K / V are read where they are.
     {
         bdattn::GemmLaunch L;
         std::memset(&L, 0, sizeof(L));
         L.bf16 = bf16;
         int n = 0;
-        if (add_gemm_problem(op, L, n++, p->x, p->x_ld, p->wq, p->x_cols, p->bq, Qp, ldp, Lq, C, p->x_cols,
-                             pad ? hd : 0, P, 0)) return -1;
+        if (add_gemm_problem(op, L, n++, p->x, p->x_ld, p->wq, p->x_cols, p->bq, Qp, C, Lq, C, p->x_cols, 0, 0)) return -1;
         if (!cached) {
-            if (add_gemm_problem(op, L, n++, src, src_ld, p->wk, src_cols, p->bk, Kp, ldp, Lk, C, src_cols,
-                                 pad ? hd : 0, P, 0)) return -1;
-            if (add_gemm_problem(op, L, n++, src, src_ld, p->wv, src_cols, p->bv, Vp, ldp, Lk, C, src_cols,
-                                 pad ? hd : 0, P, 0)) return -1;
+            if (add_gemm_problem(op, L, n++, src, src_ld, p->wk, src_cols, p->bk, Kp, C, Lk, C, src_cols, 0, 0)) return -1;
+            if (add_gemm_problem(op, L, n++, src, src_ld, p->wv, src_cols, p->bv, Vp, C, Lk, C, src_cols, 0, 0)) return -1;
         }
-        finish_gemm_launch(L, n);
-        cudaError_t e = bdattn::launch_gemm(L, st);
-        if (e != cudaSuccess) return cuda_fail(op, e);
+        if (launch_gemm(op, L, n, st)) return -1;
     }
-    const void* Kin = Kp;
-    const void* Vin = Vp;
-    long long k_ld = ldp, v_ld = ldp;
-    if (cached) {
-        if (P != hd) {
-            cudaError_t e = bdattn::launch_pad_heads(p->k_cached, Kp, Lk, nh, hd, P, p->k_ld, st);
-            if (e == cudaSuccess) e = bdattn::launch_pad_heads(p->v_cached, Vp, Lk, nh, hd, P, p->v_ld, st);
-            if (e != cudaSuccess) return cuda_fail(op, e);
-        } else {
-            Kin = p->k_cached; Vin = p->v_cached; k_ld = p->k_ld; v_ld = p->v_ld;
-        }
-    }
+    const void* Kin = cached ? p->k_cached : Kp;
+    const void* Vin = cached ? p->v_cached : Vp;
+    const long long k_ld = cached ? p->k_ld : C, v_ld = cached ? p->v_ld : C;
 
     // 2. attention core
     const float scale = 1.0f / std::sqrt(static_cast<float>(hd));
-    if (pad) {
+    if (hd <= 128) {
         bdattn::SdpaLaunch L;
         std::memset(&L, 0, sizeof(L));
         for (int s = 0; s < 2; ++s) {
-            if (make_map_heads(op, &L.tmQ[s], Qp, bf16, P, nh, Lq, 1, ldp, 0, 128)) return -1;
-            if (make_map_heads(op, &L.tmK[s], Kin, bf16, P, nh, Lk, 1, k_ld, 0, 128)) return -1;
-            if (make_map_heads(op, &L.tmV[s], Vin, bf16, P, nh, Lk, 1, v_ld, 0, 128)) return -1;
+            if (make_map_heads(op, &L.tmQ[s], Qp, bf16, hd, nh, Lq, 1, C, 0, 128)) return -1;
+            if (make_map_heads(op, &L.tmK[s], Kin, bf16, hd, nh, Lk, 1, k_ld, 0, 128)) return -1;
+            if (make_map_heads(op, &L.tmV[s], Vin, bf16, hd, nh, Lk, 1, v_ld, 0, 128)) return -1;
         }
         bdattn::SdpaDevArgs& a = L.args;
         a.q_rows[0] = Lq; a.kv_rows[0] = Lk;
@@ -916,7 +898,7 @@ int bdattn_qkvo_fwd(const bdattn_qkvo_params* p, bdattn_stream_t stream) {
         a.key_mask = p->key_mask;
         a.scale_log2 = scale * 1.4426950408889634f;
         L.q_ctas = a.q_ctas0;
-        L.num_heads = nh; L.batch = 1; L.head_dim = P; L.bf16 = bf16;
+        L.num_heads = nh; L.batch = 1; L.head_dim = hd <= 64 ? 64 : 128; L.bf16 = bf16;
         cudaError_t e = bdattn::launch_sdpa_tc05(L, st);
         if (e != cudaSuccess) return cuda_fail(op, e);
     } else {
@@ -924,7 +906,7 @@ int bdattn_qkvo_fwd(const bdattn_qkvo_params* p, bdattn_stream_t stream) {
         std::memset(&g, 0, sizeof(g));
         g.q[0] = Qp; g.k[0] = Kin; g.v[0] = Vin; g.o[0] = Op;
         g.q_rows[0] = Lq; g.kv_rows[0] = Lk;
-        g.q_ld[0] = ldp; g.k_ld[0] = k_ld; g.v_ld[0] = v_ld; g.o_ld[0] = C;
+        g.q_ld[0] = C; g.k_ld[0] = k_ld; g.v_ld[0] = v_ld; g.o_ld[0] = C;
         g.mask_mode = p->causal ? 1 : 0;
         g.q_offset = Lk - Lq;
         g.head_dim = hd;
@@ -942,10 +924,8 @@ int bdattn_qkvo_fwd(const bdattn_qkvo_params* p, bdattn_stream_t stream) {
         std::memset(&L, 0, sizeof(L));
         L.bf16 = bf16;
         if (add_gemm_problem(op, L, 0, Op, C, p->wo, C, p->bo, p->out, p->out_ld > 0 ? p->out_ld : out_cols, Lq,
-                             out_cols, C, 0, 0, 0)) return -1;
-        finish_gemm_launch(L, 1);
-        cudaError_t e = bdattn::launch_gemm(L, st);
-        if (e != cudaSuccess) return cuda_fail(op, e);
+                             out_cols, C, 0, 0)) return -1;
+        if (launch_gemm(op, L, 1, st)) return -1;
     }
     return 0;
 }

@@ -3,9 +3,6 @@
 //   add_row_bias     Y[i, j] += b[j]   (src/fused_transformer.cu:413-428)
 //   axpby_inplace    Y = a*Y + b*X     (prefix-cache scale_kv / blend_from,
 //                    src/dit/qwenimage21_hooks.cpp:79-124; X null: Y = a*Y)
-//   pad_heads        (rows, nh*hd) -> (rows, nh*hd_pad), zero padded, for
-//                    feeding cached K/V of head_dim 40 / 80 to the tensor-core
-//                    attention kernel (which takes 64 / 128).
 // 16-byte vectors where alignment allows; grid sized to the SM count.
 #include "sdpa_internal.h"
 #include "tc05.cuh"
@@ -38,6 +35,8 @@ __device__ __forceinline__ uint16_t add1(uint16_t a, uint16_t b) {
 
 template <bool kBf16>
 __global__ void __launch_bounds__(256) add_inplace_kernel(uint16_t* y, const uint16_t* x, long long n, int vec_ok) {
+    dependents_may_launch();
+    wait_for_prior_grid();
     const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long long nthreads = static_cast<long long>(gridDim.x) * blockDim.x;
     long long done = 0;
@@ -90,6 +89,8 @@ __device__ __forceinline__ uint32_t axpby2(uint32_t y, uint32_t x, float a, floa
 template <bool kBf16>
 __global__ void __launch_bounds__(256) axpby_inplace_kernel(uint16_t* y, const uint16_t* x, long long n, float a,
                                                             float b, int vec_ok) {
+    dependents_may_launch();
+    wait_for_prior_grid();
     const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long long nthreads = static_cast<long long>(gridDim.x) * blockDim.x;
     long long done = 0;
@@ -115,28 +116,13 @@ __global__ void __launch_bounds__(256) axpby_inplace_kernel(uint16_t* y, const u
 template <bool kBf16>
 __global__ void __launch_bounds__(256) add_row_bias_kernel(uint16_t* y, const uint16_t* bias, long long rows,
                                                            long long cols, long long ld) {
+    dependents_may_launch();
+    wait_for_prior_grid();
     const long long n = rows * cols;
     const long long nthreads = static_cast<long long>(gridDim.x) * blockDim.x;
     for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += nthreads) {
         const long long r = i / cols, c = i - r * cols;
         y[r * ld + c] = add1<kBf16>(y[r * ld + c], bias[c]);
-    }
-}
-
-__global__ void __launch_bounds__(256) pad_heads_kernel(const uint16_t* src, uint16_t* dst, int rows, int nh,
-                                                        int hd, int hd_pad, long long src_ld) {
-    // one thread per 8-element (16-byte) group of the padded row
-    const int groups = hd_pad / 8;
-    const long long n = static_cast<long long>(rows) * nh * groups;
-    const long long nthreads = static_cast<long long>(gridDim.x) * blockDim.x;
-    for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += nthreads) {
-        const int gi = static_cast<int>(i % groups);
-        const long long rh = i / groups;
-        const int h = static_cast<int>(rh % nh);
-        const long long r = rh / nh;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (gi * 8 < hd) v = *reinterpret_cast<const uint4*>(src + r * src_ld + h * hd + gi * 8);
-        *reinterpret_cast<uint4*>(dst + (r * nh + h) * hd_pad + gi * 8) = v;
     }
 }
 
@@ -153,9 +139,9 @@ unsigned grid_for(long long work_items) {
 cudaError_t launch_add_inplace(void* y, const void* x, long long n, bool bf16, cudaStream_t stream) {
     const int vec_ok = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0;
     const unsigned g = grid_for(vec_ok ? (n + 7) / 8 : n);
-    if (bf16) add_inplace_kernel<true><<<g, 256, 0, stream>>>(static_cast<uint16_t*>(y), static_cast<const uint16_t*>(x), n, vec_ok);
-    else add_inplace_kernel<false><<<g, 256, 0, stream>>>(static_cast<uint16_t*>(y), static_cast<const uint16_t*>(x), n, vec_ok);
-    return cudaGetLastError();
+    if (bf16)
+        return launch_dependent(add_inplace_kernel<true>, dim3(g), dim3(256), 0, stream, static_cast<uint16_t*>(y), static_cast<const uint16_t*>(x), n, vec_ok);
+    return launch_dependent(add_inplace_kernel<false>, dim3(g), dim3(256), 0, stream, static_cast<uint16_t*>(y), static_cast<const uint16_t*>(x), n, vec_ok);
 }
 
 cudaError_t launch_axpby_inplace(void* y, const void* x, long long n, float a, float b, bool bf16,
@@ -163,25 +149,17 @@ cudaError_t launch_axpby_inplace(void* y, const void* x, long long n, float a, f
     const int vec_ok = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0;
     const unsigned g = grid_for(vec_ok ? (n + 7) / 8 : n);
     if (x == nullptr) b = 0.0f;
-    if (bf16) axpby_inplace_kernel<true><<<g, 256, 0, stream>>>(static_cast<uint16_t*>(y), static_cast<const uint16_t*>(x), n, a, b, vec_ok);
-    else axpby_inplace_kernel<false><<<g, 256, 0, stream>>>(static_cast<uint16_t*>(y), static_cast<const uint16_t*>(x), n, a, b, vec_ok);
-    return cudaGetLastError();
+    if (bf16)
+        return launch_dependent(axpby_inplace_kernel<true>, dim3(g), dim3(256), 0, stream, static_cast<uint16_t*>(y), static_cast<const uint16_t*>(x), n, a, b, vec_ok);
+    return launch_dependent(axpby_inplace_kernel<false>, dim3(g), dim3(256), 0, stream, static_cast<uint16_t*>(y), static_cast<const uint16_t*>(x), n, a, b, vec_ok);
 }
 
 cudaError_t launch_add_row_bias(void* y, const void* bias, long long rows, long long cols, long long ld,
                                 bool bf16, cudaStream_t stream) {
     const unsigned g = grid_for(rows * cols);
-    if (bf16) add_row_bias_kernel<true><<<g, 256, 0, stream>>>(static_cast<uint16_t*>(y), static_cast<const uint16_t*>(bias), rows, cols, ld);
-    else add_row_bias_kernel<false><<<g, 256, 0, stream>>>(static_cast<uint16_t*>(y), static_cast<const uint16_t*>(bias), rows, cols, ld);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pad_heads(const void* src, void* dst, int rows, int num_heads, int hd, int hd_pad,
-                             long long src_ld, cudaStream_t stream) {
-    const unsigned g = grid_for(static_cast<long long>(rows) * num_heads * (hd_pad / 8));
-    pad_heads_kernel<<<g, 256, 0, stream>>>(static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), rows,
-                                            num_heads, hd, hd_pad, src_ld);
-    return cudaGetLastError();
+    if (bf16)
+        return launch_dependent(add_row_bias_kernel<true>, dim3(g), dim3(256), 0, stream, static_cast<uint16_t*>(y), static_cast<const uint16_t*>(bias), rows, cols, ld);
+    return launch_dependent(add_row_bias_kernel<false>, dim3(g), dim3(256), 0, stream, static_cast<uint16_t*>(y), static_cast<const uint16_t*>(bias), rows, cols, ld);
 }
 
 }  // namespace bdattn

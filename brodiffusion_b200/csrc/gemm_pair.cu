@@ -1,67 +1,72 @@
-// Persistent wide-tile linear layer for the large projections (Q/K/V of a
-// DiT block: src/dit/flux.cpp:471-484; out-projection: src/dit/flux.cpp:519-525):
+// Persistent two-SM linear layer for the large projections (Q/K/V of a DiT block:
+// src/dit/flux.cpp:471-484; out-projection: src/dit/flux.cpp:519-525):
 //   C[M,N] = A[M,K] . W[N,K]^T (+ bias) [-> per-head RMSNorm -> RoPE]
-// Same operand layout and epilogue arithmetic as gemm_tc05_kernel; what differs
-// is the schedule, chosen for problems with at least one 128 x 256 tile per SM:
-//   * one CTA per SM walks a list of 128-row x 256-column tiles (up to three
-//     problems in one launch, tiles of one column block adjacent so that the
-//     CTAs running together share a few weight tiles in L2);
-//   * an MMA of N = 256 reads 12 KB of shared memory per 128 tensor-pipe
-//     cycles instead of 8 KB per 64, which keeps the operand reads and the TMA
-//     fill of the next stage inside the shared-memory bandwidth;
-//   * the accumulator is double-buffered in tensor memory (2 x 256 columns),
-//     so the epilogue of tile i (bias, RMSNorm, RoPE, stores) runs while the
-//     MMAs of tile i+1 are issued.
-// GEGLU (src/fused_transformer.cu:89-92,275-282) runs here too: a tile is then
-// 128 value columns + their 128 gate columns (weight rows n0.. and D_out + n0..
-// loaded as the two halves of the B stage), one N = 256 MMA computes both and
-// the epilogue stores value * gelu_exact(gate).
-// Roles: warp 0 = TMA producer, warp 1 = tcgen05.mma issuer and TMEM owner,
-// warps 2-9 = epilogue (warp w owns TMEM lanes 32 * (w % 4)..; warps 2-5 take
-// the first half of a tile's output columns, warps 6-9 the second half).
-#include <cstdlib>
-
+// Same operand layout and epilogue arithmetic as gemm_tc05_kernel; what differs is the
+// schedule, for problems that fill the SMs with 256 x 256 tiles:
+//   * a cluster of two CTAs owns a 256-row x 256-column tile and computes it with
+//     tcgen05.mma.cta_group::2: every CTA stages its 128 rows of A and 128 of the tile's 256
+//     weight rows, so a K block costs an SM 32 KB of L2 reads and 8 KB of operand reads per
+//     128 tensor-pipe cycles (48 KB and 12 KB with a 128 x 256 tile of its own), and six
+//     stages fit instead of four;
+//   * the pairs walk a list of tiles (up to three problems in one launch; tiles of one
+//     column block adjacent, in groups of sixteen row blocks, so that what runs together
+//     reads few weight and few activation tiles);
+//   * the accumulator is double-buffered in tensor memory (2 x 256 columns), so the epilogue
+//     of tile i (bias, RMSNorm, RoPE, stores) runs while the MMAs of tile i+1 are issued.
+// GEGLU (src/fused_transformer.cu:89-92,275-282) runs here too: a tile is then 128 value
+// columns + their 128 gate columns (the first CTA stages the value rows of the weight, the
+// second the gate rows), one MMA computes both and the epilogue stores
+// value * gelu_exact(gate).
+// Roles in each CTA: warp 0 = TMA producer, warp 1 = TMEM owner and, in the first CTA of
+// the pair, tcgen05.mma issuer for both, warps 2-9 = epilogue of the CTA's 128 rows (warp w
+// owns TMEM lanes 32 * (w % 4)..; warps 2-5 take the first half of a tile's output columns,
+// warps 6-9 the second half).
 #include "sdpa_internal.h"
 #include "tc05.cuh"
 
 namespace bdattn {
 namespace {
 
-constexpr int kWThreads = 320;
-constexpr int kWStages = 4;
-constexpr int kWTileN = 256;
-constexpr int kWABytes = 128 * 64 * 2;        // A stage: 128 rows x 64 columns
-constexpr int kWBBytes = kWTileN * 64 * 2;    // B stage: 256 weight rows x 64 columns
-constexpr int kWStageBytes = kWABytes + kWBBytes;
-constexpr int kWSmemBytes = kWStages * kWStageBytes + 256 + 3 * 128 * 4 + 1024;
+constexpr int kPThreads = 320;
+constexpr int kPStages = 6;
+constexpr int kPTile = 256;                   // rows and accumulator columns of a pair's tile
+constexpr int kPABytes = 128 * 64 * 2;        // A stage of a CTA: 128 rows x 64 columns
+constexpr int kPBBytes = 128 * 64 * 2;        // B stage of a CTA: 128 of the tile's 256 weight rows
+constexpr int kPStageBytes = kPABytes + kPBBytes;
+constexpr int kPSmemBytes = kPStages * kPStageBytes + 256 + 3 * 128 * 4 + 1024;
+constexpr int kPGroup = 16;                   // row blocks of a group
 
-struct WideTile {
+struct PairTile {
     int z, m0, n0;
 };
 
 // Output columns of one tile: 256, or 128 for GEGLU (the other 128 accumulator
 // columns hold the gate).
-__host__ __device__ __forceinline__ int wide_out_cols(const GemmProblem& p) {
-    return p.geglu_offset > 0 ? kWTileN / 2 : kWTileN;
+__host__ __device__ __forceinline__ int pair_out_cols(const GemmProblem& p) {
+    return p.geglu_offset > 0 ? kPTile / 2 : kPTile;
 }
+__host__ __device__ __forceinline__ int pair_tiles_m(const GemmProblem& p) { return (p.tiles_m + 1) / 2; }
 
-__device__ __forceinline__ WideTile wide_tile(const GemmArgs& g, int tile) {
+__device__ __forceinline__ PairTile pair_tile(const GemmArgs& g, int tile) {
     int z = 0;
     int local = tile;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const int cnt = g.p[i].tiles_m * (g.p[i].N / wide_out_cols(g.p[i]));
+        const int cnt = pair_tiles_m(g.p[i]) * (g.p[i].N / pair_out_cols(g.p[i]));
         if (z == i && local >= cnt) {
             local -= cnt;
             z = i + 1;
         }
     }
-    const int tm = z == 0 ? g.p[0].tiles_m : (z == 1 ? g.p[1].tiles_m : g.p[2].tiles_m);
-    const int wn = z == 0 ? wide_out_cols(g.p[0]) : (z == 1 ? wide_out_cols(g.p[1]) : wide_out_cols(g.p[2]));
-    WideTile t;
+    const GemmProblem& p = z == 0 ? g.p[0] : (z == 1 ? g.p[1] : g.p[2]);
+    const int cols = pair_out_cols(p), tm = pair_tiles_m(p), tn = p.N / cols;
+    const int first = local / (kPGroup * tn) * kPGroup;      // first row block of the group
+    const int rows = min(kPGroup, tm - first);
+    local -= first * tn;
+    PairTile t;
     t.z = z;
-    t.n0 = (local / tm) * wn;
-    t.m0 = (local % tm) * 128;
+    t.n0 = (local / rows) * cols;
+    t.m0 = (first + local % rows) * kPTile;
     return t;
 }
 
@@ -83,10 +88,10 @@ template <int HD, bool kBf16>
 __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t tacc, uint16_t* crow, int row,
                                                int n0, const float* gain_s, int half) {
     // this warp group's share of the tile: half of its heads
-    constexpr int kHeads = kWTileN / HD / 2;
-    tacc += static_cast<uint32_t>(half * (kWTileN / 2));
-    crow += half * (kWTileN / 2);
-    n0 += half * (kWTileN / 2);
+    constexpr int kHeads = kPTile / HD / 2;
+    tacc += static_cast<uint32_t>(half * (kPTile / 2));
+    crow += half * (kPTile / 2);
+    n0 += half * (kPTile / 2);
     float inv[kHeads];
 #pragma unroll
     for (int h = 0; h < kHeads; ++h) inv[h] = 1.0f;
@@ -167,18 +172,18 @@ __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t ta
 }
 
 template <bool kBf16>
-__global__ void __launch_bounds__(kWThreads, 1)
-gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                  const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB0,
                  const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmB2,
                  const GemmArgs g, const int total_tiles) {
-    extern __shared__ uint8_t gemm_wide_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_wide_raw) + 1023) &
+    extern __shared__ uint8_t gemm_pair_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_pair_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kWStages * kWStageBytes);
-    uint64_t* full = bars;                   // [kWStages]
-    uint64_t* empty = bars + kWStages;       // [kWStages]
-    uint64_t* acc_full = empty + kWStages;   // [2]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kPStages * kPStageBytes);
+    uint64_t* full = bars;                   // [kPStages]
+    uint64_t* empty = bars + kPStages;       // [kPStages]
+    uint64_t* acc_full = empty + kPStages;   // [2]
     uint64_t* acc_empty = acc_full + 2;      // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     float* gain_s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);   // [3][128]
@@ -187,127 +192,133 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kWStages; ++s) {
+        for (int s = 0; s < kPStages; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], 256);
+            mbar_init(&acc_empty[s], 16);       // the epilogue warps of both CTAs
         }
         fence_mbar_init();
     }
-    // RMSNorm gains of the three problems as FP32 (read by every epilogue thread)
-    for (int idx = threadIdx.x; idx < 3 * 128; idx += kWThreads) {
-        const GemmProblem& gp = idx < 128 ? g.p[0] : (idx < 256 ? g.p[1] : g.p[2]);
-        const int i = idx & 127;
-        float gv = 1.0f;
-        if (gp.norm_rope && gp.gain != nullptr && i < gp.n_tile)
-            gv = gp.gain_is_f32 ? __ldg(reinterpret_cast<const float*>(gp.gain) + i) : load16<kBf16>(gp.gain, i);
-        gain_s[idx] = gv;
-    }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, 512);
-        tmem_relinquish();
+        tmem_alloc_pair(tmem_slot, 512);
+        tmem_relinquish_pair();
     }
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmA0);
         tma_prefetch_desc(&tmB0);
     }
     tc_fence_before();
-    __syncthreads();
+    cluster_sync();       // the peer signals these barriers too
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // only now: a dependent CTA that took tensor memory first could keep this one from getting its own
+    dependents_may_launch();
+    // barriers, tensor memory and descriptors are set up; from here on global memory is touched
+    wait_for_prior_grid();
+    const int rank = static_cast<int>(cluster_ctarank());
+    const int pairs = static_cast<int>(gridDim.x) >> 1;
+    const int first_tile = static_cast<int>(blockIdx.x) >> 1;
 
     if (warp == 0) {
         // ---------------------------------------------------- TMA producer
+        // Both CTAs load their part of a stage; the copies of both complete on the first
+        // CTA's barrier, where the MMA issuer waits.
         if (lane == 0) {
-            int it = 0;          // stage uses so far, over all tiles of this CTA
+            int it = 0;          // stage uses so far, over all tiles of this pair
+            int slot = 0;
+            uint32_t phase = 1;  // parity that a fresh barrier passes
             bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                const WideTile t = wide_tile(g, tile);
+            for (int tile = first_tile; ok && tile < total_tiles; tile += pairs) {
+                const PairTile t = pair_tile(g, tile);
                 const CUtensorMap* tmA = t.z == 0 ? &tmA0 : (t.z == 1 ? &tmA1 : &tmA2);
                 const CUtensorMap* tmB = t.z == 0 ? &tmB0 : (t.z == 1 ? &tmB1 : &tmB2);
                 const int K = t.z == 0 ? g.p[0].K : (t.z == 1 ? g.p[1].K : g.p[2].K);
                 const int geglu_off = t.z == 0 ? g.p[0].geglu_offset : (t.z == 1 ? g.p[1].geglu_offset : g.p[2].geglu_offset);
                 const int k_blocks = (K + 63) / 64;
+                const int a_row = t.m0 + rank * 128;
+                const int b_row = t.n0 + rank * (geglu_off > 0 ? geglu_off : 128);
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const int s = it % kWStages;
-                    if (it >= kWStages) {
-                        ok = mbar_wait(&empty[s], static_cast<uint32_t>(((it / kWStages) - 1) & 1));
-                        if (!ok) break;
-                    }
-                    uint8_t* st = smem + s * kWStageBytes;
-                    mbar_arrive_expect_tx(&full[s], kWStageBytes);
-                    tma_load_2d(st, tmA, &full[s], kb * 64, t.m0);
-                    if (geglu_off > 0) {
-                        // value rows, then the gate rows of the same output columns (128-row boxes)
-                        tma_load_2d(st + kWABytes, tmB, &full[s], kb * 64, t.n0);
-                        tma_load_2d(st + kWABytes + kWBBytes / 2, tmB, &full[s], kb * 64, geglu_off + t.n0);
-                    } else {
-                        tma_load_2d(st + kWABytes, tmB, &full[s], kb * 64, t.n0);
-                    }
+                    ok = mbar_wait(&empty[slot], phase);
+                    if (!ok) break;
+                    uint8_t* st = smem + slot * kPStageBytes;
+                    if (rank == 0) mbar_arrive_expect_tx(&full[slot], 2 * kPStageBytes);
+                    const uint32_t bar = mapa(smem_u32(&full[slot]), 0);
+                    tma_load_2d_pair(st, tmA, bar, kb * 64, a_row);
+                    tma_load_2d_pair(st + kPABytes, tmB, bar, kb * 64, b_row);
+                    if (++slot == kPStages) { slot = 0; phase ^= 1; }
                 }
             }
-            if (!ok) {
-                // a wait ran out: let the copies in flight land before the CTA ends
-                for (int i = max(0, it - kWStages); i < it; ++i)
-                    mbar_wait(&full[i % kWStages], static_cast<uint32_t>((i / kWStages) & 1));
+            if (!ok && rank == 0) {
+                // a wait ran out: let the copies in flight land before the CTAs end
+                for (int i = max(0, it - kPStages); i < it; ++i)
+                    mbar_wait(&full[i % kPStages], static_cast<uint32_t>((i / kPStages) & 1));
             }
         }
         __syncwarp();
     } else if (warp == 1) {
-        // ------------------------------------------------------ MMA issuer
-        constexpr uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, 128, kWTileN, 0, 0);
-        int it = 0;
-        int ti = 0;              // tiles done by this CTA
-        bool ok = true;
-        for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++ti) {
-            const WideTile t = wide_tile(g, tile);
+        // ---------------------------------------- MMA issuer (first CTA of the pair)
+        constexpr uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, kPTile, kPTile, 0, 0);
+        const uint64_t a0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
+        const uint64_t b0 = make_smem_desc_sw128(smem_u32(smem) + kPABytes, 16, 1024);
+        int slot = 0;
+        uint32_t phase = 0;
+        int ti = 0;              // tiles done by this pair
+        bool ok = rank == 0;
+        for (int tile = first_tile; ok && tile < total_tiles; tile += pairs, ++ti) {
+            const PairTile t = pair_tile(g, tile);
             const int K = t.z == 0 ? g.p[0].K : (t.z == 1 ? g.p[1].K : g.p[2].K);
             const int k_blocks = (K + 63) / 64;
             const int as = ti & 1;
-            if (ti >= 2) {       // the epilogue must have drained this accumulator (tile ti - 2)
+            if (ti >= 2) {       // both epilogues must have drained this accumulator (tile ti - 2)
                 ok = mbar_wait(&acc_empty[as], static_cast<uint32_t>(((ti >> 1) - 1) & 1));
                 if (!ok) break;
                 tc_fence_after();
             }
-            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(as * kWTileN);
-            for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                const int s = it % kWStages;
-                ok = mbar_wait(&full[s], static_cast<uint32_t>((it / kWStages) & 1));
+            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(as * kPTile);
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                ok = mbar_wait(&full[slot], phase);
                 if (!ok) break;
                 tc_fence_after();
                 if (lane == 0) {
-                    const uint32_t ab = smem_u32(smem + s * kWStageBytes);
-                    const uint32_t bb = ab + kWABytes;
+                    const uint64_t ad = a0 + slot * (kPStageBytes >> 4), bd = b0 + slot * (kPStageBytes >> 4);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        umma_ss(d_tmem, make_smem_desc_sw128(ab + kk * 32, 16, 1024),
-                                make_smem_desc_sw128(bb + kk * 32, 16, 1024), idesc,
-                                (kb > 0 || kk > 0) ? 1u : 0u);
-                    }
-                    umma_commit(&empty[s]);
-                    if (kb == k_blocks - 1) umma_commit(&acc_full[as]);
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma_ss_pair(d_tmem, ad + 2 * kk, bd + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+                    umma_commit_pair(&empty[slot]);
+                    if (kb == k_blocks - 1) umma_commit_pair(&acc_full[as]);
                 }
                 __syncwarp();
+                if (++slot == kPStages) { slot = 0; phase ^= 1; }
             }
         }
     } else {
         // -------------------------------------------------------- epilogue
         const int q = warp & 3;             // TMEM lane quarter of this warp
         const int half = (warp - 2) >> 2;   // which half of the tile's output columns
+        // RMSNorm gains of the three problems as FP32 for the 256 threads of these warps
+        for (int idx = threadIdx.x - 64; idx < 3 * 128; idx += kPThreads - 64) {
+            const GemmProblem& gp = idx < 128 ? g.p[0] : (idx < 256 ? g.p[1] : g.p[2]);
+            const int i = idx & 127;
+            float gv = 1.0f;
+            if (gp.norm_rope && gp.gain != nullptr && i < gp.n_tile)
+                gv = gp.gain_is_f32 ? __ldg(reinterpret_cast<const float*>(gp.gain) + i) : load16<kBf16>(gp.gain, i);
+            gain_s[idx] = gv;
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
         int ti = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++ti) {
-            const WideTile t = wide_tile(g, tile);
+        for (int tile = first_tile; tile < total_tiles; tile += pairs, ++ti) {
+            const PairTile t = pair_tile(g, tile);
             const GemmProblem& p = t.z == 0 ? g.p[0] : (t.z == 1 ? g.p[1] : g.p[2]);
             const int as = ti & 1;
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[as], static_cast<uint32_t>((ti >> 1) & 1)));
             if (!ok) break;
             tc_fence_after();
-            const int row = t.m0 + q * 32 + lane;
-            const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(as * kWTileN);
+            const int row = t.m0 + rank * 128 + q * 32 + lane;
+            const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(as * kPTile);
             uint16_t* crow = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row) * p.ldc + t.n0;
             if (p.norm_rope) {
                 const float* gs = p.gain != nullptr ? gain_s + t.z * 128 : nullptr;
@@ -345,7 +356,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                     }
                 }
             } else {
-                for (int c = half * (kWTileN / 2); c < (half + 1) * (kWTileN / 2); c += 32) {
+                for (int c = half * (kPTile / 2); c < (half + 1) * (kPTile / 2); c += 32) {
                     uint32_t v[32];
                     tmem_ld32(tacc + c, v);
                     tmem_wait_ld();
@@ -371,57 +382,39 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             }
             // this accumulator may be overwritten by the MMAs of tile ti + 2
             tc_fence_before();
-            mbar_arrive(&acc_empty[as]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(mapa(smem_u32(&acc_empty[as]), 0));
         }
     }
 
     tc_fence_before();
-    __syncthreads();
+    cluster_sync();       // neither CTA leaves while the other may still signal or read it
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, 512);
+        tmem_dealloc_pair(tmem_base, 512);
     }
 }
 
 }  // namespace
 
-int gemm_wide_tiles(const GemmLaunch& L) {
+int gemm_pair_tiles(const GemmLaunch& L) {
     int total = 0;
-    for (int i = 0; i < L.n_problems; ++i) total += L.args.p[i].tiles_m * (L.args.p[i].N / wide_out_cols(L.args.p[i]));
+    for (int i = 0; i < L.n_problems; ++i)
+        total += pair_tiles_m(L.args.p[i]) * (L.args.p[i].N / pair_out_cols(L.args.p[i]));
     return total;
 }
 
-cudaError_t launch_gemm_wide(const GemmLaunch& L, cudaStream_t stream) {
-    const int total = gemm_wide_tiles(L);
-    const int sms = sm_count();
-    cudaError_t e;
-    const int grid = total < sms ? total : sms;
-    if (L.bf16) {
-        e = set_max_smem_once(gemm_wide_kernel<true>, kWSmemBytes);
+cudaError_t launch_gemm_pair(const GemmLaunch& L, cudaStream_t stream) {
+    const int total = gemm_pair_tiles(L);
+    const int pairs = sm_count() / 2;
+    const dim3 grid(static_cast<unsigned>(2 * (total < pairs ? total : pairs)));
+    auto go = [&](auto kern) {
+        cudaError_t e = set_max_smem_once(kern, kPSmemBytes);
         if (e != cudaSuccess) return e;
-        gemm_wide_kernel<true><<<grid, kWThreads, kWSmemBytes, stream>>>(
-            L.tmA[0], L.tmA[1], L.tmA[2], L.tmBw[0], L.tmBw[1], L.tmBw[2], L.args, total);
-    } else {
-        e = set_max_smem_once(gemm_wide_kernel<false>, kWSmemBytes);
-        if (e != cudaSuccess) return e;
-        gemm_wide_kernel<false><<<grid, kWThreads, kWSmemBytes, stream>>>(
-            L.tmA[0], L.tmA[1], L.tmA[2], L.tmBw[0], L.tmBw[1], L.tmBw[2], L.args, total);
-    }
-    return cudaGetLastError();
-}
-
-// BDATTN_GEMM_WIDE=0 keeps every problem on the one-tile-per-CTA kernel (tuning runs).
-cudaError_t launch_gemm(const GemmLaunch& L, cudaStream_t stream) {
-    static const int mode = [] {
-        const char* e = std::getenv("BDATTN_GEMM_WIDE");
-        return e != nullptr ? std::atoi(e) : 1;
-    }();
-    bool wide = mode != 0 && L.n_problems > 0;
-    for (int i = 0; i < L.n_problems; ++i) wide = wide && L.wide[i];
-    if (wide) {
-        if (gemm_wide_tiles(L) >= sm_count()) return launch_gemm_wide(L, stream);
-    }
-    return launch_gemm_tc05(L, stream);
+        return launch_dependent(kern, grid, dim3(kPThreads), kPSmemBytes, stream, L.tmA[0], L.tmA[1], L.tmA[2],
+                                L.tmB[0], L.tmB[1], L.tmB[2], L.args, total);
+    };
+    return L.bf16 ? go(gemm_pair_kernel<true>) : go(gemm_pair_kernel<false>);
 }
 
 }  // namespace bdattn

@@ -10,14 +10,17 @@
 //   warp 0     TMA producer (A tile 128 x 64, B tile n_tile x 64 per K block)
 //   warp 1     tcgen05.mma issuer, owns the TMEM allocation
 //   warps 2-5  epilogue: tcgen05.ld -> bias / GEGLU -> 16-byte stores
-// Tiles may be head-aligned: tile t starts at weight row t * n_step and its
-// n_valid columns land at output column t * c_step, zero-filled up to c_fill.
-// That writes Q/K/V with every head padded to the width the attention kernel
-// takes (40 -> 64, 80 -> 128) without a separate padding pass.
+// Where the tiles leave SMs idle (the 64- and 256-token levels of a U-Net, short
+// prompts), a cluster of up to eight CTAs shares one tile: each takes a part of the K
+// blocks, the partial sums meet in distributed shared memory, and every CTA finishes
+// 128 / split rows of the tile (kSplit).
 //
 // GEGLU mode (src/fused_transformer.cu:89-92,275-282): a second B tile from
 // weight row n0 + D_out feeds a second accumulator and the epilogue stores
 // value * gelu_exact(gate), so the (B, 2*D_out) intermediate never exists.
+#include <cooperative_groups.h>
+#include <type_traits>
+
 #include "sdpa_internal.h"
 #include "tc05.cuh"
 
@@ -25,7 +28,7 @@ namespace bdattn {
 namespace {
 
 constexpr int kGemmThreads = 192;
-constexpr int kGemmMaxStages = 4;
+constexpr int kGemmMaxStages = 8;
 constexpr int kGemmABytes = 128 * 64 * 2;   // A stage
 // A B (or gate) tile is n_tile rows x 128 B; a stage holds A, B and, for GEGLU,
 // the gate tile, rounded up to the 1024-byte swizzle period.  Sizing the stage by
@@ -35,16 +38,81 @@ __host__ __device__ inline int gemm_stage_bytes(int n_tile, bool geglu) {
     return kGemmABytes + (geglu ? 2 : 1) * gemm_b_bytes(n_tile);
 }
 
-// One instantiation per epilogue (plain, GEGLU, norm + RoPE): the GEGLU and the norm +
-// RoPE code are long, and an epilogue that only branches around them spent more time
-// fetching instructions than storing (5.6 us for one 128 x 128 tile against 2.3 us).
-template <bool kBf16, bool kGeglu, bool kNormRope>
+// Partial sums of a split tile in shared memory: row-major, four floats of padding per
+// row so that both a thread per row and several threads per row read and write
+// float4 without bank conflicts.
+__host__ __device__ inline int gemm_red_ld(int n_tile, bool geglu) { return (geglu ? 2 : 1) * n_tile + 4; }
+
+template <bool kBf16>
+__device__ __forceinline__ float gemm_ld16(const void* base, long long i) {
+    const uint16_t b = reinterpret_cast<const uint16_t*>(base)[i];
+    return kBf16 ? __uint_as_float(static_cast<uint32_t>(b) << 16)
+                 : __half2float(*reinterpret_cast<const __half*>(&b));
+}
+
+// Epilogue of a split tile.  Every CTA of the cluster holds a partial 128 x n_tile sum
+// at the same shared-memory address; this one finishes 128 / split rows, `split`
+// threads to a row with n_tile / split columns (a multiple of eight) each.
+template <bool kBf16, bool kGeglu>
+__device__ __forceinline__ void epilogue_split(const GemmProblem& p, cooperative_groups::cluster_group& cluster,
+                                               float* red, int split, int part, int tid, int m0, int n0) {
+    const int ld = gemm_red_ld(p.n_tile, kGeglu);
+    const int r = part * (128 / split) + tid / split;
+    const int per = p.n_tile / split;
+    const int row = m0 + r;
+    const int c_first = (tid % split) * per;
+    if (row >= p.M) return;
+    auto sum8 = [&](int c, float (&f)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = 0.0f;
+        for (int k = 0; k < split; ++k) {
+            const float4* src = reinterpret_cast<const float4*>(cluster.map_shared_rank(red, k) + r * ld + c);
+            const float4 u = src[0], v = src[1];
+            f[0] += u.x; f[1] += u.y; f[2] += u.z; f[3] += u.w;
+            f[4] += v.x; f[5] += v.y; f[6] += v.z; f[7] += v.w;
+        }
+    };
+    uint16_t* crow = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row) * p.ldc + n0;
+    const int n_valid = min(p.n_tile, p.N - n0);           // a multiple of eight
+    for (int c = c_first; c < c_first + per; c += 8) {
+        if (c >= n_valid) break;
+        float f[8];
+        sum8(c, f);
+        if (p.bias != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] += gemm_ld16<kBf16>(p.bias, n0 + c + i);
+        }
+        if constexpr (kGeglu) {
+            if (p.geglu_offset > 0) {
+                float gt[8];
+                sum8(p.n_tile + c, gt);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (p.bias != nullptr) gt[i] += gemm_ld16<kBf16>(p.bias, n0 + p.geglu_offset + c + i);
+                    f[i] *= 0.5f * gt[i] * (1.0f + erff(gt[i] * 0.7071067811865475f));
+                }
+            }
+        }
+        uint4 w;
+        w.x = pack2<kBf16>(f[0], f[1]); w.y = pack2<kBf16>(f[2], f[3]);
+        w.z = pack2<kBf16>(f[4], f[5]); w.w = pack2<kBf16>(f[6], f[7]);
+        *reinterpret_cast<uint4*>(crow + c) = w;
+    }
+}
+
+// One instantiation per epilogue (plain, GEGLU, norm + RoPE; whole or split tiles): the
+// GEGLU and the norm + RoPE code are long, and an epilogue that only branches around them
+// spent more time fetching instructions than storing (5.6 us for one 128 x 128 tile
+// against 2.3 us).
+template <bool kBf16, bool kGeglu, bool kNormRope, bool kSplit>
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                  const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB0,
                  const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmB2,
                  const GemmArgs g) {
-    const int z = blockIdx.z;
+    const int split = kSplit ? g.split : 1;
+    const int z = kSplit ? static_cast<int>(blockIdx.z) / split : static_cast<int>(blockIdx.z);
+    const int part = kSplit ? static_cast<int>(blockIdx.z) % split : 0;    // the cluster spans `split` CTAs of z
     const GemmProblem& p = z == 0 ? g.p[0] : (z == 1 ? g.p[1] : g.p[2]);
     const CUtensorMap* tmA = z == 0 ? &tmA0 : (z == 1 ? &tmA1 : &tmA2);
     const CUtensorMap* tmB = z == 0 ? &tmB0 : (z == 1 ? &tmB1 : &tmB2);
@@ -66,8 +134,10 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int k_blocks = (p.K + 63) / 64;
-    const int n0 = tile_n * p.n_step;
+    const int k_all = (p.K + 63) / 64;
+    const int k_begin = kSplit ? part * k_all / split : 0;
+    const int k_blocks = (kSplit ? (part + 1) * k_all / split : k_all) - k_begin;
+    const int n0 = tile_n * p.n_tile;
     const int m0 = tile_m * 128;
     const bool geglu = kGeglu && p.geglu_offset > 0;
     constexpr uint32_t kTmemCols = kGeglu ? 256 : 128;     // the gate accumulator sits 128 columns up
@@ -88,24 +158,28 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // only now: a dependent CTA that took tensor memory first could keep this one from getting its own
+    dependents_may_launch();
+    wait_for_prior_grid();
 
     if (warp == 0) {
         if (lane == 0) {
             const uint32_t bytes = kGemmABytes + (geglu ? 2u : 1u) * static_cast<uint32_t>(p.n_tile) * 128u;
             bool ok = true;
             int issued = 0;
+            int slot = 0;
+            uint32_t phase = 1;          // parity that a fresh barrier passes
             for (int kb = 0; kb < k_blocks; ++kb) {
-                const int s = kb % kGemmStages;
-                if (kb >= kGemmStages) {
-                    ok = mbar_wait(&empty[s], static_cast<uint32_t>(((kb / kGemmStages) - 1) & 1));
-                    if (!ok) break;
-                }
-                uint8_t* st = smem + s * kGemmStageBytes;
-                mbar_arrive_expect_tx(&full[s], bytes);
-                tma_load_2d(st, tmA, &full[s], kb * 64, m0);
-                tma_load_2d(st + kGemmABytes, tmB, &full[s], kb * 64, n0);
-                if (geglu) tma_load_2d(st + kGemmABytes + kGemmBBytes, tmB, &full[s], kb * 64, n0 + p.geglu_offset);
+                ok = mbar_wait(&empty[slot], phase);
+                if (!ok) break;
+                uint8_t* st = smem + slot * kGemmStageBytes;
+                mbar_arrive_expect_tx(&full[slot], bytes);
+                const int x = (k_begin + kb) * 64;
+                tma_load_2d(st, tmA, &full[slot], x, m0);
+                tma_load_2d(st + kGemmABytes, tmB, &full[slot], x, n0);
+                if (geglu) tma_load_2d(st + kGemmABytes + kGemmBBytes, tmB, &full[slot], x, n0 + p.geglu_offset);
                 issued = kb + 1;
+                if (++slot == kGemmStages) { slot = 0; phase ^= 1; }
             }
             if (!ok) {
                 for (int kb = max(0, issued - kGemmStages); kb < issued; ++kb)
@@ -114,29 +188,31 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         }
         __syncwarp();
     } else if (warp == 1) {
+        // The issuing thread is what a long K loop waits for (with the loads left out it ran no
+        // faster): the slot and its parity are counted on, a division by the runtime ring size
+        // cost more than the four MMAs.
         const uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, 128, p.n_tile, 0, 0);
-        bool ok = true;
-        for (int kb = 0; kb < k_blocks && ok; ++kb) {
-            const int s = kb % kGemmStages;
-            ok = mbar_wait(&full[s], static_cast<uint32_t>((kb / kGemmStages) & 1));
-            if (!ok) break;
+        const uint64_t a0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
+        const uint64_t b0 = make_smem_desc_sw128(smem_u32(smem) + kGemmABytes, 16, 1024);
+        const uint32_t stage_units = static_cast<uint32_t>(kGemmStageBytes) >> 4;   // descriptors count 16 bytes
+        const uint32_t gate_units = static_cast<uint32_t>(kGemmBBytes) >> 4;
+        int slot = 0;
+        uint32_t phase = 0;
+        for (int kb = 0; kb < k_blocks; ++kb) {
+            if (!mbar_wait(&full[slot], phase)) break;
             tc_fence_after();
             if (lane == 0) {
-                const uint32_t ab = smem_u32(smem + s * kGemmStageBytes);
-                const uint32_t bb = ab + kGemmABytes;
+                const uint64_t ad = a0 + slot * stage_units, bd = b0 + slot * stage_units;
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) {
-                    const uint64_t ad = make_smem_desc_sw128(ab + kk * 32, 16, 1024);
-                    umma_ss(tmem_base, ad, make_smem_desc_sw128(bb + kk * 32, 16, 1024), idesc,
-                            (kb > 0 || kk > 0) ? 1u : 0u);
-                    if (geglu)
-                        umma_ss(tmem_base + 128, ad, make_smem_desc_sw128(bb + kGemmBBytes + kk * 32, 16, 1024),
-                                idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+                    umma_ss(tmem_base, ad + 2 * kk, bd + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+                    if (geglu) umma_ss(tmem_base + 128, ad + 2 * kk, bd + gate_units + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
                 }
-                umma_commit(&empty[s]);
+                umma_commit(&empty[slot]);
                 if (kb == k_blocks - 1) umma_commit(acc_done);
             }
             __syncwarp();
+            if (++slot == kGemmStages) { slot = 0; phase ^= 1; }
         }
     } else {
         // epilogue: warp w reads TMEM lanes 32 * (w % 4) ..
@@ -146,12 +222,23 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
         const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-        const long long c0 = static_cast<long long>(tile_n) * p.c_step;
-        uint16_t* crow = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row) * p.ldc + c0;
-        const int n_valid = min(p.n_valid, p.N - n0);
-        // plain tiles stop at the matrix edge; head tiles own their padded slot
-        const int c_lim = p.c_step == p.n_step ? min(p.c_fill, p.N - n0) : p.c_fill;
-        if (kNormRope && ok && p.norm_rope) {
+        uint16_t* crow = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row) * p.ldc + n0;
+        const int n_valid = min(p.n_tile, p.N - n0);      // a ragged last tile stops at the matrix edge
+        if constexpr (kSplit) {
+            // partial sums to shared memory: the ring is at rest, its last MMA has completed
+            float* rrow = reinterpret_cast<float*>(smem) + (q * 32 + lane) * gemm_red_ld(p.n_tile, kGeglu);
+#pragma unroll 1
+            for (int c = 0; ok && c < (kGeglu ? 2 : 1) * p.n_tile; c += 32) {
+                const bool gate = kGeglu && c >= p.n_tile;
+                if (gate && !geglu) break;
+                uint32_t v[32];
+                tmem_ld32(tacc + (gate ? 128 + c - p.n_tile : c), v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    *reinterpret_cast<uint4*>(rrow + c + 4 * i) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            }
+        } else if (kNormRope && ok && p.norm_rope) {
             // The tile is one head and this thread holds one token's row of it:
             // RMSNorm over the head and the rotary embedding are thread-local
             // (src/dit/flux.cpp:462-469 + src/dit/common.cpp:192-193 fused into
@@ -223,16 +310,11 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 }
             }
         } else if (ok) {
-            for (int c = 0; c < c_lim; c += 32) {
+            for (int c = 0; c < n_valid; c += 32) {
                 uint32_t v[32], gt[32];
-                if (c < p.n_tile) {
-                    tmem_ld32(tacc + c, v);
-                    if (geglu) tmem_ld32(tacc + 128 + c, gt);
-                    tmem_wait_ld();
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = 0u;
-                }
+                tmem_ld32(tacc + c, v);
+                if (geglu) tmem_ld32(tacc + 128 + c, gt);
+                tmem_wait_ld();
                 // the 32 bias values of this piece (and of its gate), zero where there is none
                 float bx[32], bg[kGeglu ? 32 : 1];
                 const bool whole = c + 32 <= n_valid;
@@ -274,12 +356,12 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                             x *= 0.5f * gate * (1.0f + erff(gate * 0.7071067811865475f));
                         }
                     }
-                    f[i] = c + i < n_valid ? x : 0.0f;
+                    f[i] = x;
                 }
                 if (row < p.M) {
 #pragma unroll
                     for (int v8 = 0; v8 < 4; ++v8) {
-                        if (c + v8 * 8 < c_lim) {
+                        if (c + v8 * 8 < n_valid) {
                             uint4 w;
                             w.x = pack2<kBf16>(f[v8 * 8 + 0], f[v8 * 8 + 1]);
                             w.y = pack2<kBf16>(f[v8 * 8 + 2], f[v8 * 8 + 3]);
@@ -293,6 +375,16 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         }
     }
 
+    if constexpr (kSplit) {
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        if (warp >= 2)
+            epilogue_split<kBf16, kGeglu>(p, cluster, reinterpret_cast<float*>(smem), split, part,
+                                          static_cast<int>(threadIdx.x) - 64, m0, n0);
+        cluster.sync();      // the peers' shared memory stays until everyone has read it
+    }
+
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -304,44 +396,52 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
 }  // namespace
 
 cudaError_t launch_gemm_tc05(const GemmLaunch& L, cudaStream_t stream) {
-    int tn = 0, tm = 0, nt_max = 16, any_geglu = 0, any_norm_rope = 0;
+    int tn = 0, tm = 0, nt_max = 16, any_geglu = 0, any_norm_rope = 0, k_max = 0;
     for (int i = 0; i < L.n_problems; ++i) {
-        tn = L.args.p[i].tiles_n > tn ? L.args.p[i].tiles_n : tn;
-        tm = L.args.p[i].tiles_m > tm ? L.args.p[i].tiles_m : tm;
-        nt_max = L.args.p[i].n_tile > nt_max ? L.args.p[i].n_tile : nt_max;
-        any_geglu |= L.args.p[i].geglu_offset > 0 ? 1 : 0;
-        any_norm_rope |= L.args.p[i].norm_rope ? 1 : 0;
+        const GemmProblem& p = L.args.p[i];
+        tn = p.tiles_n > tn ? p.tiles_n : tn;
+        tm = p.tiles_m > tm ? p.tiles_m : tm;
+        nt_max = p.n_tile > nt_max ? p.n_tile : nt_max;
+        k_max = p.K > k_max ? p.K : k_max;
+        any_geglu |= p.geglu_offset > 0 ? 1 : 0;
+        any_norm_rope |= p.norm_rope ? 1 : 0;
     }
     GemmArgs args = L.args;
     args.n_tile_max = nt_max;
     args.any_geglu = any_geglu;
+    const long long ctas = static_cast<long long>(tn) * tm * L.n_problems * args.split;
+    const int stage = gemm_stage_bytes(nt_max, any_geglu != 0);
     // three stages with the gate tile: the stage ring stays below 114 KB and two CTAs fit per SM
-    args.stages = any_geglu ? 3 : kGemmMaxStages;
-    // Short K and more tiles than SMs: a ring of two (64 KB) lets up to three CTAs share an SM,
-    // so that one CTA's epilogue runs under the others' loads (4096 x 320 -> 960: 18.1 -> 12.2 us).
-    int k_max = 0;
-    for (int i = 0; i < L.n_problems; ++i) k_max = L.args.p[i].K > k_max ? L.args.p[i].K : k_max;
-    if (!any_geglu && k_max <= 512 && static_cast<long long>(tn) * tm * L.n_problems > sm_count()) args.stages = 2;
-    const int kGemmSmemBytes = args.stages * gemm_stage_bytes(nt_max, any_geglu != 0) + 256 + 1024;
-    dim3 grid(static_cast<unsigned>(tn), static_cast<unsigned>(tm), static_cast<unsigned>(L.n_problems));
+    args.stages = any_geglu ? 3 : 4;
+    if (ctas <= sm_count()) {
+        // a CTA has its SM to itself: the ring may take all of the shared memory
+        args.stages = 192 * 1024 / stage < kGemmMaxStages ? 192 * 1024 / stage : kGemmMaxStages;
+    } else if (!any_geglu && k_max <= 512 && args.split == 1) {
+        // Short K and more tiles than SMs: a ring of two (64 KB) lets up to three CTAs share an SM,
+        // so that one CTA's epilogue runs under the others' loads (4096 x 320 -> 960: 18.1 -> 12.2 us).
+        args.stages = 2;
+    }
+    const int smem = args.stages * stage + 256 + 1024;
+    const dim3 grid(static_cast<unsigned>(tn), static_cast<unsigned>(tm),
+                    static_cast<unsigned>(L.n_problems * args.split));
     cudaError_t e = cudaSuccess;
     auto go = [&](auto kern) {
         e = set_max_smem_once(kern, 227 * 1024);
         if (e != cudaSuccess) return;
-        kern<<<grid, kGemmThreads, kGemmSmemBytes, stream>>>(L.tmA[0], L.tmA[1], L.tmA[2], L.tmB[0], L.tmB[1],
-                                                            L.tmB[2], args);
+        e = launch_dependent_cluster(kern, grid, dim3(kGemmThreads), smem, stream, dim3(1, 1, args.split), L.tmA[0],
+                                     L.tmA[1], L.tmA[2], L.tmB[0], L.tmB[1], L.tmB[2], args);
     };
-    if (L.bf16) {
-        if (any_norm_rope) go(gemm_tc05_kernel<true, false, true>);
-        else if (any_geglu) go(gemm_tc05_kernel<true, true, false>);
-        else go(gemm_tc05_kernel<true, false, false>);
-    } else {
-        if (any_norm_rope) go(gemm_tc05_kernel<false, false, true>);
-        else if (any_geglu) go(gemm_tc05_kernel<false, true, false>);
-        else go(gemm_tc05_kernel<false, false, false>);
-    }
-    if (e != cudaSuccess) return e;
-    return cudaGetLastError();
+    auto pick = [&](auto bf16) {
+        constexpr bool kB = decltype(bf16)::value;
+        if (any_norm_rope) go(gemm_tc05_kernel<kB, false, true, false>);        // never split
+        else if (any_geglu && args.split > 1) go(gemm_tc05_kernel<kB, true, false, true>);
+        else if (any_geglu) go(gemm_tc05_kernel<kB, true, false, false>);
+        else if (args.split > 1) go(gemm_tc05_kernel<kB, false, false, true>);
+        else go(gemm_tc05_kernel<kB, false, false, false>);
+    };
+    if (L.bf16) pick(std::true_type{});
+    else pick(std::false_type{});
+    return e;
 }
 
 }  // namespace bdattn

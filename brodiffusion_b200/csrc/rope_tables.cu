@@ -12,6 +12,8 @@ namespace bdattn {
 namespace {
 
 __global__ void rope_tables_kernel(const RopeTableArgs a) {
+    dependents_may_launch();
+    wait_for_prior_grid();
     const int half = a.half;
     const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= static_cast<long long>(a.rows) * half) return;
@@ -66,8 +68,7 @@ cudaError_t launch_rope_tables(const RopeTableArgs& a, cudaStream_t stream) {
     const long long n = static_cast<long long>(a.rows) * a.half;
     const int threads = 256;
     const long long blocks = (n + threads - 1) / threads;
-    rope_tables_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(rope_tables_kernel, dim3(static_cast<unsigned>(blocks)), dim3(threads), 0, stream, a);
 }
 
 }  // namespace bdattn

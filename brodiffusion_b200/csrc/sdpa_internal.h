@@ -167,11 +167,7 @@ struct GemmProblem {
     long long ldc;
     const void* bias;   // N values of the output dtype, or null
     int tiles_m, tiles_n;
-    int n_tile;         // MMA N (multiple of 16, <= 128) = rows of the B box
-    int n_step;         // weight rows between tile starts
-    int n_valid;        // columns of a tile that carry results
-    int c_step;         // output columns between tile starts
-    int c_fill;         // output columns written per tile (zeros beyond n_valid)
+    int n_tile;         // MMA N of a tile, 64 or 128 = rows of the B box; the head_dim with norm_rope
     int geglu_offset;   // 0, or D_out
     // Per-head RMSNorm + RoPE epilogue (head tiles with n_tile == head_dim only):
     const void* gain;   // head_dim values, or null
@@ -187,22 +183,22 @@ struct GemmArgs {
     int n_tile_max;   // largest n_tile of the launch: sizes the shared-memory stages
     int any_geglu;
     int stages;
+    int split;        // CTAs (a cluster) that share the K blocks of a tile
 };
 struct GemmLaunch {
     CUtensorMap tmA[3], tmB[3];
-    CUtensorMap tmBw[3];   // weight maps with 256-row boxes (wide-tile kernel), valid where wide[i]
-    bool wide[3];          // problem i can run as 128 x 256 tiles
+    bool whole[3];         // problem i has whole 256-column tiles (128 for GEGLU)
+    const void* W[3];      // weights: their maps are made once the tile width is chosen
+    long long ldw[3], w_rows[3];
     GemmArgs args;
     int n_problems;
     bool bf16;
 };
 cudaError_t launch_gemm_tc05(const GemmLaunch& L, cudaStream_t stream);
-// Persistent 128 x 256-tile kernel; every problem of the launch must have wide[i] set.
-cudaError_t launch_gemm_wide(const GemmLaunch& L, cudaStream_t stream);
-int gemm_wide_tiles(const GemmLaunch& L);
-// Picks the wide-tile kernel when every problem allows it and there is at least
-// one wide tile per SM, the one-tile-per-CTA kernel otherwise.
-cudaError_t launch_gemm(const GemmLaunch& L, cudaStream_t stream);
+// Persistent kernel of CTA pairs and 256 x 256 tiles; every problem of the launch must
+// have whole[i] set.
+cudaError_t launch_gemm_pair(const GemmLaunch& L, cudaStream_t stream);
+int gemm_pair_tiles(const GemmLaunch& L);
 
 // Elementwise helpers.
 cudaError_t launch_add_inplace(void* y, const void* x, long long n, bool bf16, cudaStream_t stream);
@@ -210,8 +206,7 @@ cudaError_t launch_axpby_inplace(void* y, const void* x, long long n, float a, f
                                  cudaStream_t stream);
 cudaError_t launch_add_row_bias(void* y, const void* bias, long long rows, long long cols, long long ld,
                                 bool bf16, cudaStream_t stream);
-cudaError_t launch_pad_heads(const void* src, void* dst, int rows, int num_heads, int hd, int hd_pad,
-                             long long src_ld, cudaStream_t stream);
+
 
 // Device-side RoPE table build.
 constexpr int kMaxRopeSegments = 64;

@@ -1,5 +1,6 @@
-"""Calls whose shape decides the route: head dims above 128 (mma.sync kernel) and map
-blocks at the edges of their tiles and segments.  References: the CPU oracle."""
+"""Calls whose shape decides the route: head dims above 128 (mma.sync kernel), linear
+layers whose K blocks are shared by a cluster or whose tiles are shared by a pair of CTAs,
+and map blocks at the edges of their tiles and segments.  References: the CPU oracle."""
 import numpy as np
 import pytest
 import torch
@@ -57,6 +58,65 @@ def test_head_dims_above_128_segments_and_groups(bd, oracle):
     assert bd.device_status() == 0
     rep = lambda x: np.repeat(x.reshape(-1, nkv, hd), nh // nkv, axis=1).reshape(x.shape[0], -1)
     G.check(G.host(out), oracle.sdpa(q, rep(k), rep(v), nh), what="segments and groups, head_dim 160")
+
+
+# Few output tiles, so that 2, 4 or 8 CTAs share a tile: ragged rows and columns, K not a
+# multiple of a K block, the smallest K that is split and one just below it.
+@pytest.mark.parametrize("M,N,K", [(64, 1280, 1280), (64, 1280, 5120), (1, 72, 2048), (77, 1280, 768), (130, 200, 1000),
+                                   (256, 3072, 3072), (128, 64, 504), (128, 64, 448), (300, 640, 2560)])
+def test_linear_split_over_a_cluster(bd, oracle, M, N, K):
+    x, w, b = synth.activations((M, K), 9600 + M), synth.weights((N, K), 9601 + N), synth.weights((N,), 9602)
+    for bias in (b, None):
+        y = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+        bd.linear_fwd(G.dev(x), G.dev(w), G.dev(bias) if bias is not None else None, y)
+        assert bd.device_status() == 0
+        ref = oracle.linear(x, w, bias)
+        # half an ulp of the largest output, and FP32 sums in another order
+        assert np.abs(G.host(y) - ref).max() <= np.abs(ref).max() * (2.0 ** -8 + 1e-5)
+
+
+@pytest.mark.parametrize("B,Din,Dout", [(64, 1280, 5120), (33, 1280, 264), (130, 520, 72)])
+def test_geglu_split_over_a_cluster(bd, oracle, B, Din, Dout):
+    x, w = synth.activations((B, Din), 9700, "fp16"), synth.weights((2 * Dout, Din), 9701, "fp16")
+    b = synth.weights((2 * Dout,), 9702, "fp16")
+    y = torch.full((B, Dout), float("nan"), device="cuda", dtype=torch.float16)
+    bd.linear_geglu_fwd(G.dev(x, torch.float16), G.dev(w, torch.float16), G.dev(b, torch.float16), y)
+    assert bd.device_status() == 0
+    ref = oracle.linear_geglu(x, w, b)
+    assert np.abs(G.host(y) - ref).max() <= 0.01 * np.abs(ref).max() + 0.008   # as for the unsplit kernel
+
+
+# Tiles of 256 x 256 shared by two CTAs: row counts that leave the second CTA empty or
+# part-filled, more than one group of sixteen row blocks, K not a multiple of a K block.
+@pytest.mark.parametrize("M,N,K", [(4500, 1280, 72), (9473, 512, 200), (2304, 2560, 136)])
+def test_linear_on_cta_pairs(bd, oracle, M, N, K):
+    x, w, b = synth.activations((M, K), 9650 + M), synth.weights((N, K), 9651 + N), synth.weights((N,), 9652)
+    y = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    bd.linear_fwd(G.dev(x), G.dev(w), G.dev(b), y)
+    assert bd.device_status() == 0
+    ref = oracle.linear(x, w, b)
+    assert np.abs(G.host(y) - ref).max() <= np.abs(ref).max() * (2.0 ** -8 + 1e-5)
+
+
+@pytest.mark.parametrize("hd,nh,rows", [(128, 24, 16), (128, 4, 130), (64, 3, 77), (64, 8, 300), (128, 2, 1)])
+def test_qkv_norm_rope_few_rows(bd, oracle, hd, nh, rows):
+    D, d_in = nh * hd, 1024
+    x = synth.activations((rows, d_in), 9800)
+    ws = [synth.weights((D, d_in), 9801 + i) for i in range(3)]
+    bs = [synth.weights((D,), 9810 + i) for i in range(3)]
+    gq, gk = synth.gains(hd, 9820), synth.gains(hd, 9821)
+    ang = synth.uniform01(rows * hd // 2, 9822).reshape(rows, hd // 2) * 6.0
+    cos, sin = np.cos(ang).astype(np.float32), np.sin(ang).astype(np.float32)
+    outs = [torch.full((rows, D), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+    bd.qkv_norm_rope_fwd(G.dev(x), *[G.dev(w) for w in ws], *outs, nh, hd, gain_q=G.dev(gq), gain_k=G.dev(gk),
+                         cos=G.dev(cos, torch.float32), sin=G.dev(sin, torch.float32),
+                         bq=G.dev(bs[0]), bk=G.dev(bs[1]), bv=G.dev(bs[2]))
+    assert bd.device_status() == 0
+    for i, gain in enumerate((gq, gk, None)):
+        ref = oracle.linear(x, ws[i], bs[i])
+        if gain is not None:
+            ref = oracle.rope_apply(oracle.rms_norm_heads(ref, nh, hd, gain), nh, hd, cos, sin)
+        G.check(G.host(outs[i]), ref, max_abs=2.0 ** -8 * np.abs(ref).max() + 1e-4, what=f"projection {i}")
 
 
 # Map blocks: rows and keys around the 128 x 64 tiles, blocks that begin inside a segment
