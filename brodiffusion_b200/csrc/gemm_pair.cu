@@ -6,13 +6,18 @@
 //   * a cluster of two CTAs owns a 256-row x 256-column tile and computes it with
 //     tcgen05.mma.cta_group::2: every CTA stages its 128 rows of A and 128 of the tile's 256
 //     weight rows, so a K block costs an SM 32 KB of L2 reads and 8 KB of operand reads per
-//     128 tensor-pipe cycles (48 KB and 12 KB with a 128 x 256 tile of its own), and six
-//     stages fit instead of four;
+//     128 tensor-pipe cycles (48 KB and 12 KB with a 128 x 256 tile of its own);
+//   * a stage is 128 columns of K: the issuing thread spends 64 cycles on an MMA and about
+//     250 on the wait and the commit around a stage, which with four MMAs to a stage made
+//     610 cycles of a K block of 64 where the tensor pipe needs 512;
 //   * the pairs walk a list of tiles (up to three problems in one launch; tiles of one
 //     column block adjacent, in groups of sixteen row blocks, so that what runs together
 //     reads few weight and few activation tiles);
 //   * the accumulator is double-buffered in tensor memory (2 x 256 columns), so the epilogue
-//     of tile i (bias, RMSNorm, RoPE, stores) runs while the MMAs of tile i+1 are issued.
+//     of tile i (bias, RMSNorm, RoPE, stores) runs while the MMAs of tile i+1 are issued;
+//   * the cos / sin rows and the outputs go through 4 KB of shared memory per epilogue warp, so
+//     that global accesses are whole row pieces (a load or store with a row per lane touches 32
+//     cache lines; the exposed last epilogue of a short prompt's projections took ten of 30 us).
 // GEGLU (src/fused_transformer.cu:89-92,275-282) runs here too: a tile is then 128 value
 // columns + their 128 gate columns (the first CTA stages the value rows of the weight, the
 // second the gate rows), one MMA computes both and the epilogue stores
@@ -28,12 +33,14 @@ namespace bdattn {
 namespace {
 
 constexpr int kPThreads = 320;
-constexpr int kPStages = 6;
+constexpr int kPStages = 3;
 constexpr int kPTile = 256;                   // rows and accumulator columns of a pair's tile
-constexpr int kPABytes = 128 * 64 * 2;        // A stage of a CTA: 128 rows x 64 columns
-constexpr int kPBBytes = 128 * 64 * 2;        // B stage of a CTA: 128 of the tile's 256 weight rows
-constexpr int kPStageBytes = kPABytes + kPBBytes;
-constexpr int kPSmemBytes = kPStages * kPStageBytes + 256 + 3 * 128 * 4 + 1024;
+constexpr int kPChunk = 128 * 64 * 2;         // 128 rows x 64 columns: one TMA box of A or B
+// A stage of a CTA: two chunks (128 columns of K) of its 128 rows of A, two of its 128 weight rows
+constexpr int kPStageBytes = 4 * kPChunk;
+constexpr int kPStgBytes = 4096;              // staging of one epilogue warp
+constexpr int kPSmemBytes = kPStages * kPStageBytes + 8 * kPStgBytes + 256 + 3 * 128 * 4 + 1024;
+static_assert(kPSmemBytes <= 227 * 1024, "shared memory of one CTA");
 constexpr int kPGroup = 16;                   // row blocks of a group
 
 struct PairTile {
@@ -83,15 +90,14 @@ __device__ __forceinline__ float load16(const void* base, long long i) {
 // passes over the accumulator (tensor memory reads are cheap): sum of squares
 // per head first, then 32 columns at a time so that one load of the token's
 // cos / sin serves every head of the tile.  gain_s: the HD gains in shared
-// memory as FP32, or null for no RMSNorm.
+// memory as FP32, or null for no RMSNorm.  row0: the warp's first row; c0: the
+// first of the 128 output columns it takes.
 template <int HD, bool kBf16>
-__device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t tacc, uint16_t* crow, int row,
-                                               int n0, const float* gain_s, int half) {
-    // this warp group's share of the tile: half of its heads
+__device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t tacc, int row0, int c0,
+                                               const float* gain_s, uint8_t* stg, int lane) {
     constexpr int kHeads = kPTile / HD / 2;
-    tacc += static_cast<uint32_t>(half * (kPTile / 2));
-    crow += half * (kPTile / 2);
-    n0 += half * (kPTile / 2);
+    const int rows = min(32, p.M - row0);
+    uint16_t* cbase = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row0) * p.ldc + c0;
     float inv[kHeads];
 #pragma unroll
     for (int h = 0; h < kHeads; ++h) inv[h] = 1.0f;
@@ -99,54 +105,64 @@ __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t ta
 #pragma unroll
         for (int h = 0; h < kHeads; ++h) {
             float ss0 = 0.0f, ss1 = 0.0f;
-#pragma unroll
+#pragma unroll 1
             for (int c = 0; c < HD / 32; ++c) {
-                uint32_t v[32];
-                tmem_ld32(tacc + h * HD + c * 32, v);
+                float f[32];
+                tmem_ld32(tacc + h * HD + c * 32, reinterpret_cast<uint32_t(&)[32]>(f));
                 tmem_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float x0 = __uint_as_float(v[i]), x1 = __uint_as_float(v[i + 1]);
-                    if (p.bias != nullptr) {
-                        x0 += load16<kBf16>(p.bias, n0 + h * HD + c * 32 + i);
-                        x1 += load16<kBf16>(p.bias, n0 + h * HD + c * 32 + i + 1);
+                for (int i = 0; i < 32; i += 8) {
+                    if (p.bias != nullptr) add8_from16<kBf16>(p.bias, c0 + h * HD + c * 32 + i, f + i);
+#pragma unroll
+                    for (int k = 0; k < 8; k += 2) {
+                        ss0 = fmaf(f[i + k], f[i + k], ss0);
+                        ss1 = fmaf(f[i + k + 1], f[i + k + 1], ss1);
                     }
-                    ss0 = fmaf(x0, x0, ss0);
-                    ss1 = fmaf(x1, x1, ss1);
                 }
             }
             inv[h] = rsqrtf((ss0 + ss1) / static_cast<float>(HD) + p.eps);
         }
     }
     const bool rope = p.cos != nullptr;
-    const long long tb = static_cast<long long>(p.rope_row0 + row) * (HD / 2);
-#pragma unroll
+    // lane -> (row lane / 4 of a group of eight, 16-byte piece lane % 4) for the table rows
+    const int tr = lane >> 2, tq = lane & 3;
+    const long long tb = static_cast<long long>(p.rope_row0 + row0) * (HD / 2) + tq * 4;
+#pragma unroll 1
     for (int c = 0; c < HD / 32; ++c) {
         float cs[16], sn[16];
-        if (rope && row < p.M) {
+        if (rope) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float4 a = __ldg(reinterpret_cast<const float4*>(p.cos + tb + c * 16) + i);
-                const float4 b = __ldg(reinterpret_cast<const float4*>(p.sin + tb + c * 16) + i);
+                const int r = i * 8 + tr;
+                if (r < rows) {
+                    const float4 a = __ldg(reinterpret_cast<const float4*>(p.cos + tb + static_cast<long long>(r) * (HD / 2) + c * 16));
+                    const float4 b = __ldg(reinterpret_cast<const float4*>(p.sin + tb + static_cast<long long>(r) * (HD / 2) + c * 16));
+                    *reinterpret_cast<float4*>(stg + r * 128 + ((tq ^ (r & 7)) << 4)) = a;
+                    *reinterpret_cast<float4*>(stg + r * 128 + (((tq + 4) ^ (r & 7)) << 4)) = b;
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(stg + lane * 128 + ((i ^ (lane & 7)) << 4));
+                const float4 b = *reinterpret_cast<const float4*>(stg + lane * 128 + (((i + 4) ^ (lane & 7)) << 4));
                 cs[4 * i] = a.x; cs[4 * i + 1] = a.y; cs[4 * i + 2] = a.z; cs[4 * i + 3] = a.w;
                 sn[4 * i] = b.x; sn[4 * i + 1] = b.y; sn[4 * i + 2] = b.z; sn[4 * i + 3] = b.w;
             }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) { cs[i] = 1.0f; sn[i] = 0.0f; }
+            __syncwarp();
         }
 #pragma unroll
         for (int h = 0; h < kHeads; ++h) {
-            uint32_t v[32];
-            tmem_ld32(tacc + h * HD + c * 32, v);
-            tmem_wait_ld();
             float f[32];
+            tmem_ld32(tacc + h * HD + c * 32, reinterpret_cast<uint32_t(&)[32]>(f));
+            tmem_wait_ld();
+            if (p.bias != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                float x = __uint_as_float(v[i]);
-                if (p.bias != nullptr) x += load16<kBf16>(p.bias, n0 + h * HD + c * 32 + i);
-                if (gain_s != nullptr) x *= inv[h] * gain_s[c * 32 + i];
-                f[i] = x;
+                for (int i = 0; i < 32; i += 8) add8_from16<kBf16>(p.bias, c0 + h * HD + c * 32 + i, f + i);
+            }
+            if (gain_s != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) f[i] *= inv[h] * gain_s[c * 32 + i];
             }
             if (rope) {
 #pragma unroll
@@ -156,17 +172,7 @@ __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t ta
                     f[2 * i + 1] = a0 * sn[i] + b0 * cs[i];
                 }
             }
-            if (row < p.M) {
-#pragma unroll
-                for (int v8 = 0; v8 < 4; ++v8) {
-                    uint4 w;
-                    w.x = pack2<kBf16>(f[v8 * 8 + 0], f[v8 * 8 + 1]);
-                    w.y = pack2<kBf16>(f[v8 * 8 + 2], f[v8 * 8 + 3]);
-                    w.z = pack2<kBf16>(f[v8 * 8 + 4], f[v8 * 8 + 5]);
-                    w.w = pack2<kBf16>(f[v8 * 8 + 6], f[v8 * 8 + 7]);
-                    *reinterpret_cast<uint4*>(crow + h * HD + c * 32 + v8 * 8) = w;
-                }
-            }
+            store_tile32<kBf16>(f, stg, lane, cbase + h * HD + c * 32, p.ldc, rows, 32);
         }
     }
 }
@@ -180,7 +186,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     extern __shared__ uint8_t gemm_pair_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_pair_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kPStages * kPStageBytes);
+    uint8_t* stg_all = smem + kPStages * kPStageBytes;      // [8][kPStgBytes]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(stg_all + 8 * kPStgBytes);
     uint64_t* full = bars;                   // [kPStages]
     uint64_t* empty = bars + kPStages;       // [kPStages]
     uint64_t* acc_full = empty + kPStages;   // [2]
@@ -237,17 +244,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 const CUtensorMap* tmB = t.z == 0 ? &tmB0 : (t.z == 1 ? &tmB1 : &tmB2);
                 const int K = t.z == 0 ? g.p[0].K : (t.z == 1 ? g.p[1].K : g.p[2].K);
                 const int geglu_off = t.z == 0 ? g.p[0].geglu_offset : (t.z == 1 ? g.p[1].geglu_offset : g.p[2].geglu_offset);
-                const int k_blocks = (K + 63) / 64;
+                const int chunks = (K + 63) / 64;
                 const int a_row = t.m0 + rank * 128;
                 const int b_row = t.n0 + rank * (geglu_off > 0 ? geglu_off : 128);
-                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                for (int c = 0; c < chunks; c += 2, ++it) {
                     ok = mbar_wait(&empty[slot], phase);
                     if (!ok) break;
                     uint8_t* st = smem + slot * kPStageBytes;
-                    if (rank == 0) mbar_arrive_expect_tx(&full[slot], 2 * kPStageBytes);
+                    const int n = min(2, chunks - c);          // an odd last chunk stands alone
+                    if (rank == 0) mbar_arrive_expect_tx(&full[slot], n * 2 * 2 * kPChunk);
                     const uint32_t bar = mapa(smem_u32(&full[slot]), 0);
-                    tma_load_2d_pair(st, tmA, bar, kb * 64, a_row);
-                    tma_load_2d_pair(st + kPABytes, tmB, bar, kb * 64, b_row);
+                    for (int i = 0; i < n; ++i) {
+                        tma_load_2d_pair(st + i * kPChunk, tmA, bar, (c + i) * 64, a_row);
+                        tma_load_2d_pair(st + (2 + i) * kPChunk, tmB, bar, (c + i) * 64, b_row);
+                    }
                     if (++slot == kPStages) { slot = 0; phase ^= 1; }
                 }
             }
@@ -262,7 +272,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         // ---------------------------------------- MMA issuer (first CTA of the pair)
         constexpr uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, kPTile, kPTile, 0, 0);
         const uint64_t a0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
-        const uint64_t b0 = make_smem_desc_sw128(smem_u32(smem) + kPABytes, 16, 1024);
+        const uint64_t b0 = make_smem_desc_sw128(smem_u32(smem) + 2 * kPChunk, 16, 1024);
         int slot = 0;
         uint32_t phase = 0;
         int ti = 0;              // tiles done by this pair
@@ -270,7 +280,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         for (int tile = first_tile; ok && tile < total_tiles; tile += pairs, ++ti) {
             const PairTile t = pair_tile(g, tile);
             const int K = t.z == 0 ? g.p[0].K : (t.z == 1 ? g.p[1].K : g.p[2].K);
-            const int k_blocks = (K + 63) / 64;
+            const int chunks = (K + 63) / 64;
             const int as = ti & 1;
             if (ti >= 2) {       // both epilogues must have drained this accumulator (tile ti - 2)
                 ok = mbar_wait(&acc_empty[as], static_cast<uint32_t>(((ti >> 1) - 1) & 1));
@@ -278,7 +288,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 tc_fence_after();
             }
             const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(as * kPTile);
-            for (int kb = 0; kb < k_blocks; ++kb) {
+            for (int c = 0; c < chunks; c += 2) {
                 ok = mbar_wait(&full[slot], phase);
                 if (!ok) break;
                 tc_fence_after();
@@ -286,9 +296,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                     const uint64_t ad = a0 + slot * (kPStageBytes >> 4), bd = b0 + slot * (kPStageBytes >> 4);
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        umma_ss_pair(d_tmem, ad + 2 * kk, bd + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+                        umma_ss_pair(d_tmem, ad + 2 * kk, bd + 2 * kk, idesc, (c > 0 || kk > 0) ? 1u : 0u);
+                    if (c + 1 < chunks) {
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            umma_ss_pair(d_tmem, ad + (kPChunk >> 4) + 2 * kk, bd + (kPChunk >> 4) + 2 * kk, idesc, 1u);
+                    }
                     umma_commit_pair(&empty[slot]);
-                    if (kb == k_blocks - 1) umma_commit_pair(&acc_full[as]);
+                    if (c + 2 >= chunks) umma_commit_pair(&acc_full[as]);
                 }
                 __syncwarp();
                 if (++slot == kPStages) { slot = 0; phase ^= 1; }
@@ -298,6 +313,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         // -------------------------------------------------------- epilogue
         const int q = warp & 3;             // TMEM lane quarter of this warp
         const int half = (warp - 2) >> 2;   // which half of the tile's output columns
+        uint8_t* const stg = stg_all + (warp - 2) * kPStgBytes;
         // RMSNorm gains of the three problems as FP32 for the 256 threads of these warps
         for (int idx = threadIdx.x - 64; idx < 3 * 128; idx += kPThreads - 64) {
             const GemmProblem& gp = idx < 128 ? g.p[0] : (idx < 256 ? g.p[1] : g.p[2]);
@@ -317,67 +333,48 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[as], static_cast<uint32_t>((ti >> 1) & 1)));
             if (!ok) break;
             tc_fence_after();
-            const int row = t.m0 + rank * 128 + q * 32 + lane;
+            const int row0 = t.m0 + rank * 128 + q * 32;
+            const int rows = min(32, p.M - row0);
             const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(as * kPTile);
-            uint16_t* crow = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row) * p.ldc + t.n0;
-            if (p.norm_rope) {
+            uint16_t* cbase = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row0) * p.ldc + t.n0;
+            if (rows <= 0) {
+                // rows past the matrix: nothing to store
+            } else if (p.norm_rope) {
                 const float* gs = p.gain != nullptr ? gain_s + t.z * 128 : nullptr;
-                if (p.n_tile == 128) epilogue_heads<128, kBf16>(p, tacc, crow, row, t.n0, gs, half);
-                else epilogue_heads<64, kBf16>(p, tacc, crow, row, t.n0, gs, half);
+                const int c0 = half * (kPTile / 2);
+                if (p.n_tile == 128) epilogue_heads<128, kBf16>(p, tacc + c0, row0, t.n0 + c0, gs, stg, lane);
+                else epilogue_heads<64, kBf16>(p, tacc + c0, row0, t.n0 + c0, gs, stg, lane);
             } else if (p.geglu_offset > 0) {
                 // value in accumulator columns [0, 128), gate in [128, 256); this group
                 // stores 64 of the tile's 128 output columns
+#pragma unroll 1
                 for (int c = half * 64; c < half * 64 + 64; c += 32) {
-                    uint32_t v[32], gt[32];
-                    tmem_ld32(tacc + c, v);
-                    tmem_ld32(tacc + 128 + c, gt);
+                    float f[32], gt[32];
+                    tmem_ld32(tacc + c, reinterpret_cast<uint32_t(&)[32]>(f));
+                    tmem_ld32(tacc + 128 + c, reinterpret_cast<uint32_t(&)[32]>(gt));
                     tmem_wait_ld();
-                    float f[32];
+                    if (p.bias != nullptr) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        float x = __uint_as_float(v[i]);
-                        float gate = __uint_as_float(gt[i]);
-                        if (p.bias != nullptr) {
-                            x += load16<kBf16>(p.bias, t.n0 + c + i);
-                            gate += load16<kBf16>(p.bias, p.geglu_offset + t.n0 + c + i);
-                        }
-                        f[i] = x * (0.5f * gate * (1.0f + erff(gate * 0.7071067811865475f)));
-                    }
-                    if (row < p.M) {
-#pragma unroll
-                        for (int v8 = 0; v8 < 4; ++v8) {
-                            uint4 w;
-                            w.x = pack2<kBf16>(f[v8 * 8 + 0], f[v8 * 8 + 1]);
-                            w.y = pack2<kBf16>(f[v8 * 8 + 2], f[v8 * 8 + 3]);
-                            w.z = pack2<kBf16>(f[v8 * 8 + 4], f[v8 * 8 + 5]);
-                            w.w = pack2<kBf16>(f[v8 * 8 + 6], f[v8 * 8 + 7]);
-                            *reinterpret_cast<uint4*>(crow + c + v8 * 8) = w;
+                        for (int i = 0; i < 32; i += 8) {
+                            add8_from16<kBf16>(p.bias, t.n0 + c + i, f + i);
+                            add8_from16<kBf16>(p.bias, p.geglu_offset + t.n0 + c + i, gt + i);
                         }
                     }
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) f[i] *= 0.5f * gt[i] * (1.0f + erff(gt[i] * 0.7071067811865475f));
+                    store_tile32<kBf16>(f, stg, lane, cbase + c, p.ldc, rows, 32);
                 }
             } else {
+#pragma unroll 1
                 for (int c = half * (kPTile / 2); c < (half + 1) * (kPTile / 2); c += 32) {
-                    uint32_t v[32];
-                    tmem_ld32(tacc + c, v);
-                    tmem_wait_ld();
                     float f[32];
+                    tmem_ld32(tacc + c, reinterpret_cast<uint32_t(&)[32]>(f));
+                    tmem_wait_ld();
+                    if (p.bias != nullptr) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        float x = __uint_as_float(v[i]);
-                        if (p.bias != nullptr) x += load16<kBf16>(p.bias, t.n0 + c + i);
-                        f[i] = x;
+                        for (int i = 0; i < 32; i += 8) add8_from16<kBf16>(p.bias, t.n0 + c + i, f + i);
                     }
-                    if (row < p.M) {
-#pragma unroll
-                        for (int v8 = 0; v8 < 4; ++v8) {
-                            uint4 w;
-                            w.x = pack2<kBf16>(f[v8 * 8 + 0], f[v8 * 8 + 1]);
-                            w.y = pack2<kBf16>(f[v8 * 8 + 2], f[v8 * 8 + 3]);
-                            w.z = pack2<kBf16>(f[v8 * 8 + 4], f[v8 * 8 + 5]);
-                            w.w = pack2<kBf16>(f[v8 * 8 + 6], f[v8 * 8 + 7]);
-                            *reinterpret_cast<uint4*>(crow + c + v8 * 8) = w;
-                        }
-                    }
+                    store_tile32<kBf16>(f, stg, lane, cbase + c, p.ldc, rows, 32);
                 }
             }
             // this accumulator may be overwritten by the MMAs of tile ti + 2

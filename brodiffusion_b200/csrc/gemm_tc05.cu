@@ -222,7 +222,8 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
         const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-        uint16_t* crow = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row) * p.ldc + n0;
+        uint16_t* crow0 = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(m0 + q * 32) * p.ldc + n0;
+        uint16_t* crow = crow0 + static_cast<long long>(lane) * p.ldc;
         const int n_valid = min(p.n_tile, p.N - n0);      // a ragged last tile stops at the matrix edge
         if constexpr (kSplit) {
             // partial sums to shared memory: the ring is at rest, its last MMA has completed
@@ -358,19 +359,8 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                     }
                     f[i] = x;
                 }
-                if (row < p.M) {
-#pragma unroll
-                    for (int v8 = 0; v8 < 4; ++v8) {
-                        if (c + v8 * 8 < n_valid) {
-                            uint4 w;
-                            w.x = pack2<kBf16>(f[v8 * 8 + 0], f[v8 * 8 + 1]);
-                            w.y = pack2<kBf16>(f[v8 * 8 + 2], f[v8 * 8 + 3]);
-                            w.z = pack2<kBf16>(f[v8 * 8 + 4], f[v8 * 8 + 5]);
-                            w.w = pack2<kBf16>(f[v8 * 8 + 6], f[v8 * 8 + 7]);
-                            *reinterpret_cast<uint4*>(crow + c + v8 * 8) = w;
-                        }
-                    }
-                }
+                // (the ring is at rest, its last MMA has completed: it holds the staging)
+                store_tile32<kBf16>(f, smem + q * 2048, lane, crow0 + c, p.ldc, p.M - m0 - q * 32, n_valid - c);
             }
         }
     }
