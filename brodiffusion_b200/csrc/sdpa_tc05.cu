@@ -542,6 +542,9 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
         // read: all Q.K^T MMAs have completed) so that global stores are whole
         // rows: 16-byte chunk c of row r sits at chunk c ^ (r mod chunks) to keep
         // the row-per-thread writes and the row-major reads free of bank conflicts.
+        // A warp stores the 32 rows it wrote (no CTA barrier), a lane the same chunk of every
+        // row, eight loads in flight: a row-by-row loop over the tile took 5500 cycles of
+        // a CTA's 11700 outside the key steps.
         constexpr int kRowChunks = HD / 8;
         uint8_t* stg = smem_q + t * C::kQBytes;
 #pragma unroll
@@ -565,37 +568,50 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                 *reinterpret_cast<uint4*>(stg + row_in_tile * (HD * 2) + ((cg ^ (row_in_tile & (kRowChunks - 1))) << 4)) = w;
             }
         }
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + t) : "memory");   // the 128 threads of this query tile
-        if (ok) {
-            uint8_t* obase = reinterpret_cast<uint8_t*>(qseg ? a.o[1] : a.o[0]);
-            const long long o_ld = qseg ? a.o_ld[1] : a.o_ld[0];
-            const long long o_bs = qseg ? a.o_bs[1] : a.o_bs[0];
-            const int out_chunks = a.hd_out >> 3;
-            for (int idx = row_in_tile; idx < kBM * kRowChunks; idx += kBM) {
-                const int r = idx / kRowChunks;
-                const int cg = idx - r * kRowChunks;
-                const int rs = qrow0 + t * kBM + r;
-                if (rs < seg_rows && cg < out_chunks) {
-                    const uint4 w = *reinterpret_cast<const uint4*>(stg + r * (HD * 2) + ((cg ^ (r & (kRowChunks - 1))) << 4));
-                    const long long off = 2 * (static_cast<long long>(batch) * o_bs + static_cast<long long>(rs) * o_ld +
-                                               static_cast<long long>(head) * a.hd_out + cg * 8);
-                    uint8_t* const mc = reinterpret_cast<uint8_t*>(qseg ? a.o_mc[1] : a.o_mc[0]);
-                    if (mc != nullptr) {
-                        // fused all-gather through the switch: one store to the multicast
-                        // address lands in every GPU's copy of the output, this one's included
-                        asm volatile("multimem.st.relaxed.sys.global.v4.f32 [%0], {%1, %2, %3, %4};"
-                                     ::"l"(mc + off), "f"(__uint_as_float(w.x)), "f"(__uint_as_float(w.y)),
-                                       "f"(__uint_as_float(w.z)), "f"(__uint_as_float(w.w))
-                                     : "memory");
-                    } else {
-                        *reinterpret_cast<uint4*>(obase + off) = w;
-                        // fused all-gather: the same vector goes to every peer's copy of the
-                        // output (plain stores over NVLink; no TMA, no peer reads)
-                        for (int pi = 0; pi < a.n_peers; ++pi) {
-                            uint8_t* pb = reinterpret_cast<uint8_t*>(qseg ? a.o_peer[1][pi] : a.o_peer[0][pi]);
-                            *reinterpret_cast<uint4*>(pb + off) = w;
-                        }
+        __syncwarp();
+        const int cg = lane & (kRowChunks - 1);
+        if (ok && cg < (a.hd_out >> 3)) {
+            constexpr int kRowsPer = 32 / kRowChunks;           // rows of one access: 2 or 4
+            const int r0 = (warp & 3) * 32 + lane / kRowChunks;
+            const int rows_left = seg_rows - (qrow0 + t * kBM + r0);
+            const long long o_ld = 2 * (qseg ? a.o_ld[1] : a.o_ld[0]);
+            const long long off0 = 2 * (static_cast<long long>(batch) * (qseg ? a.o_bs[1] : a.o_bs[0]) +
+                                        static_cast<long long>(head) * a.hd_out + cg * 8) +
+                                   (qrow0 + t * kBM + r0) * o_ld;
+            uint8_t* const obase = reinterpret_cast<uint8_t*>(qseg ? a.o[1] : a.o[0]);
+            uint8_t* const mc = reinterpret_cast<uint8_t*>(qseg ? a.o_mc[1] : a.o_mc[0]);
+            auto chunk = [&](int i) {
+                const int r = r0 + i * kRowsPer;
+                return *reinterpret_cast<const uint4*>(stg + r * (HD * 2) + ((cg ^ (r & (kRowChunks - 1))) << 4));
+            };
+            if (mc == nullptr) {
+#pragma unroll
+                for (int i0 = 0; i0 < kRowChunks; i0 += 8) {
+                    uint4 w[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) w[i] = chunk(i0 + i);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        if ((i0 + i) * kRowsPer < rows_left)
+                            *reinterpret_cast<uint4*>(obase + off0 + (i0 + i) * kRowsPer * o_ld) = w[i];
                     }
+                }
+                // fused all-gather: the same vectors go to every peer's copy of the
+                // output (plain stores over NVLink; no TMA, no peer reads)
+                for (int pi = 0; pi < a.n_peers; ++pi) {
+                    uint8_t* const pb = reinterpret_cast<uint8_t*>(qseg ? a.o_peer[1][pi] : a.o_peer[0][pi]);
+                    for (int i = 0; i < kRowChunks && i * kRowsPer < rows_left; ++i)
+                        *reinterpret_cast<uint4*>(pb + off0 + i * kRowsPer * o_ld) = chunk(i);
+                }
+            } else {
+                // fused all-gather through the switch: one store to the multicast
+                // address lands in every GPU's copy of the output, this one's included
+                for (int i = 0; i < kRowChunks && i * kRowsPer < rows_left; ++i) {
+                    const uint4 w = chunk(i);
+                    asm volatile("multimem.st.relaxed.sys.global.v4.f32 [%0], {%1, %2, %3, %4};"
+                                 ::"l"(mc + off0 + i * kRowsPer * o_ld), "f"(__uint_as_float(w.x)), "f"(__uint_as_float(w.y)),
+                                   "f"(__uint_as_float(w.z)), "f"(__uint_as_float(w.w))
+                                 : "memory");
                 }
             }
         }
@@ -682,13 +698,14 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             // ------------------------------------------------ TMA producer
             if (lane == 0 && n_kv > 0) {
                 const CUtensorMap* mq = qseg ? &tmQ1 : &tmQ0;
-                for (int t = 0; t < 2; ++t) {
+                auto load_q = [&](int t) {
                     mbar_arrive_expect_tx(&q_full[t], C::kQBytes);
                     for (int c = 0; c < C::kChunks; ++c) {
                         tma_load_4d(smem_q + t * C::kQBytes + c * kChunkBytes, mq, &q_full[t],
                                     c * 64, head, qrow0 + t * kBM, batch);
                     }
-                }
+                };
+                load_q(0);
                 const int kv_head = head / a.kv_group;
                 int ks = 0, vs = 0, issued = 0;
                 uint32_t kph = 1, vph = 1;             // parity that a fresh barrier passes
@@ -702,6 +719,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                         tma_load_4d(smem_k + ks * C::kTileBytes + c * kChunkBytes, ti.seg ? &tmK1 : &tmK0, &k_full[ks],
                                     c * 64, kv_head, ti.row0, batch);
                     }
+                    if (j == 0) load_q(1);         // after what the first scores need
                     issued = 2 * j + 1;
                     if (++ks == KS) { ks = 0; kph ^= 1; }
                     if (j >= VS) ok = mbar_wait(&v_empty[vs], vph);
