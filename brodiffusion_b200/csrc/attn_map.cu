@@ -238,7 +238,7 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
 #pragma unroll
             for (int c = 0; c < kMapKeys; ++c) red[c * kMapRows + row] = acc[c];
         }
-        cluster.sync();
+        cluster_sync();
         if (warp >= 2 && row < rows) {
             const int per = kMapKeys / cs;
             for (int c = rank * per; c < (rank + 1) * per; ++c) {
@@ -247,7 +247,7 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
                 if (c < keys) out[c] = sum * inv_h;
             }
         }
-        cluster.sync();      // the peers' shared memory stays until everyone has read it
+        cluster_sync_relaxed();      // the peers' shared memory stays until everyone has read it
     }
 
     tc_fence_before();

@@ -218,7 +218,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         tma_prefetch_desc(&tmB0);
     }
     tc_fence_before();
-    cluster_sync();       // the peer signals these barriers too
+    __syncthreads();
+    cluster_sync_relaxed();       // the peer signals these barriers too
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // only now: a dependent CTA that took tensor memory first could keep this one from getting its own
@@ -385,7 +386,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     }
 
     tc_fence_before();
-    cluster_sync();       // neither CTA leaves while the other may still signal or read it
+    cluster_sync_relaxed();       // neither CTA leaves while the other may still signal or read it
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, 512);

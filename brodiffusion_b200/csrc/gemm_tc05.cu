@@ -368,11 +368,11 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     if constexpr (kSplit) {
         namespace cg = cooperative_groups;
         cg::cluster_group cluster = cg::this_cluster();
-        cluster.sync();
+        cluster_sync();
         if (warp >= 2)
             epilogue_split<kBf16, kGeglu>(p, cluster, reinterpret_cast<float*>(smem), split, part,
                                           static_cast<int>(threadIdx.x) - 64, m0, n0);
-        cluster.sync();      // the peers' shared memory stays until everyone has read it
+        cluster_sync_relaxed();      // the peers' shared memory stays until everyone has read it
     }
 
     tc_fence_before();

@@ -24,7 +24,9 @@
 // softmax warps go from one step to the next without waiting for any MMA of their
 // own step.  At head_dim 128 there is room for one S buffer only; the two tiles, half
 // a step apart, take turns in it (it is occupied from the first MMA until the fetch
-// is over, about 1100 cycles of a step per tile).  A key step takes 2790 cycles (3550
+// is over, about 1100 cycles of a step per tile).  At 64 each tile has its own, and the
+// scores are issued in turns all the same: two tiles in step want the exponential unit at
+// the same time (4096 x 4096, 8 heads of 40, FP16: 57.9 us in step, 53.9 in turns).  A key step takes 2790 cycles (3550
 // when P overwrote S and Q.K^T of step j+1 had to wait for P.V of step j): 4608 x 4608,
 // 24 heads of 128, 224 -> 199 us before the power cap sets in; 16896 x 16896, two batch
 // items, under the cap (SM clock 1.48 GHz instead of 1.85) 6.34 -> 5.77 ms.
@@ -637,13 +639,9 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                         ok = mbar_wait(&q_full[t], 0);
                         if (ok && a.q_fused) ok = mbar_wait(&q_ready[t], 0);
                     }
-                    // the S buffer's last user holds its scores in registers: with one buffer
-                    // that is the other tile, else the tile itself one step earlier
-                    if (HD == 128) {
-                        if (ok && (j > 0 || t > 0)) ok = mbar_wait(&s_free[t ^ 1], static_cast<uint32_t>((t ? j : j - 1) & 1));
-                    } else {
-                        if (ok && j > 0) ok = mbar_wait(&s_free[t], static_cast<uint32_t>((j - 1) & 1));
-                    }
+                    // the other tile holds the scores before these in registers: with one buffer it
+                    // was that buffer's last user, with two this keeps the tiles in turns
+                    if (ok && (j > 0 || t > 0)) ok = mbar_wait(&s_free[t ^ 1], static_cast<uint32_t>((t ? j : j - 1) & 1));
                     if (ok && t == 0) ok = mbar_wait(&k_rdy[slot], phase);
                     if (!ok) break;
                     tc_fence_after();

@@ -314,6 +314,13 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same without ordering memory: for the start (behind fence_mbar_init) and for the end of a
+// kernel, where a CTA only has to outlive its peers' accesses.  The release of the other
+// form waits for the global stores in flight.
+__device__ __forceinline__ void cluster_sync_relaxed() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // The address of this CTA's shared-memory address `addr` in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
     uint32_t r;
