@@ -362,7 +362,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                         }
                     }
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) f[i] *= 0.5f * gt[i] * (1.0f + erff(gt[i] * 0.7071067811865475f));
+                    for (int i = 0; i < 32; ++i) f[i] *= gelu_exact(gt[i]);
                     store_tile32<kBf16>(f, stg, lane, cbase + c, p.ldc, rows, 32);
                 }
             } else {

@@ -89,7 +89,7 @@ __device__ __forceinline__ void epilogue_split(const GemmProblem& p, cooperative
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     if (p.bias != nullptr) gt[i] += gemm_ld16<kBf16>(p.bias, n0 + p.geglu_offset + c + i);
-                    f[i] *= 0.5f * gt[i] * (1.0f + erff(gt[i] * 0.7071067811865475f));
+                    f[i] *= gelu_exact(gt[i]);
                 }
             }
         }
@@ -354,7 +354,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                     if constexpr (kGeglu) {
                         if (geglu) {
                             const float gate = __uint_as_float(gt[i]) + bg[i];
-                            x *= 0.5f * gate * (1.0f + erff(gate * 0.7071067811865475f));
+                            x *= gelu_exact(gate);
                         }
                     }
                     f[i] = x;

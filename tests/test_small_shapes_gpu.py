@@ -63,7 +63,7 @@ def test_head_dims_above_128_segments_and_groups(bd, oracle):
 # Few output tiles, so that 2, 4 or 8 CTAs share a tile: ragged rows and columns, K not a
 # multiple of a K block, the smallest K that is split and one just below it.
 @pytest.mark.parametrize("M,N,K", [(64, 1280, 1280), (64, 1280, 5120), (1, 72, 2048), (77, 1280, 768), (130, 200, 1000),
-                                   (256, 3072, 3072), (128, 64, 504), (128, 64, 448), (300, 640, 2560)])
+                                   (256, 3072, 3072), (128, 64, 384), (128, 64, 320), (300, 640, 2560)])
 def test_linear_split_over_a_cluster(bd, oracle, M, N, K):
     x, w, b = synth.activations((M, K), 9600 + M), synth.weights((N, K), 9601 + N), synth.weights((N,), 9602)
     for bias in (b, None):
