@@ -189,23 +189,40 @@ def _check(rc: int) -> None:
         raise BdattnError(last_error())
 
 
-def _stream(stream=None):
-    """Raw cudaStream_t of a torch stream (default: torch's current stream)."""
+_torch = None            # the torch module, its dtype codes and raw-stream getter, looked up once
+_dtype_codes = {}
+_raw_stream = None
+
+
+def _bind_torch():
+    global _torch, _raw_stream
     import torch
+    _dtype_codes.update({torch.bfloat16: BF16, torch.float16: F16, torch.float32: F32})
+    _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    _torch = torch
+
+
+def _stream(stream=None):
+    """Raw cudaStream_t of a torch stream (default: torch's current stream).
+
+    The default goes past torch.cuda.current_stream(), whose Stream object costs more than
+    the argument marshalling of a whole call."""
+    if _torch is None:
+        _bind_torch()
     if stream is None:
-        stream = torch.cuda.current_stream()
+        if _raw_stream is not None:
+            return C.c_void_p(_raw_stream(_torch.cuda.current_device()))
+        stream = _torch.cuda.current_stream()
     return C.c_void_p(stream.cuda_stream)
 
 
 def _dtype_code(t) -> int:
-    import torch
-    if t.dtype == torch.bfloat16:
-        return BF16
-    if t.dtype == torch.float16:
-        return F16
-    if t.dtype == torch.float32:
-        return F32
-    raise BdattnError(f"unsupported tensor dtype {t.dtype}")
+    if _torch is None:
+        _bind_torch()
+    code = _dtype_codes.get(t.dtype)
+    if code is None:
+        raise BdattnError(f"unsupported tensor dtype {t.dtype}")
+    return code
 
 
 def _rows2d(t):

@@ -356,19 +356,21 @@ static int sdpa_fwd_impl(const char* op, const bdattn_sdpa_params* p, void* cons
         const int hd_kernel = hd <= 64 ? 64 : 128;
         bdattn::SdpaLaunch L;
         std::memset(&L, 0, sizeof(L));
-        for (int s = 0; s < 2; ++s) {
-            const int qs = s < p->n_q_seg ? s : 0;
-            const int ks = s < p->n_kv_seg ? s : 0;
-            if (make_map_heads(op, &L.tmQ[s], p->q[qs], bf16, hd, p->num_heads, p->q_rows[qs], p->batch,
-                               p->q_ld[qs], p->q_batch_stride[qs], 128))
-                return -1;
-            if (make_map_heads(op, &L.tmK[s], p->k[ks], bf16, hd, nkv, p->kv_rows[ks], p->batch,
-                               p->k_ld[ks], p->k_batch_stride[ks], 128))
-                return -1;
-            if (make_map_heads(op, &L.tmV[s], p->v[ks], bf16, hd, nkv, p->kv_rows[ks], p->batch,
-                               p->v_ld[ks], p->v_batch_stride[ks], 128))
+        for (int s = 0; s < p->n_q_seg; ++s) {
+            if (make_map_heads(op, &L.tmQ[s], p->q[s], bf16, hd, p->num_heads, p->q_rows[s], p->batch,
+                               p->q_ld[s], p->q_batch_stride[s], 128))
                 return -1;
         }
+        for (int s = 0; s < p->n_kv_seg; ++s) {
+            if (make_map_heads(op, &L.tmK[s], p->k[s], bf16, hd, nkv, p->kv_rows[s], p->batch,
+                               p->k_ld[s], p->k_batch_stride[s], 128))
+                return -1;
+            if (make_map_heads(op, &L.tmV[s], p->v[s], bf16, hd, nkv, p->kv_rows[s], p->batch,
+                               p->v_ld[s], p->v_batch_stride[s], 128))
+                return -1;
+        }
+        if (p->n_q_seg == 1) L.tmQ[1] = L.tmQ[0];
+        if (p->n_kv_seg == 1) { L.tmK[1] = L.tmK[0]; L.tmV[1] = L.tmV[0]; }
         bdattn::SdpaDevArgs& a = L.args;
         for (int s = 0; s < 2; ++s) {
             const bool have_q = s < p->n_q_seg;
@@ -918,11 +920,13 @@ int bdattn_qkvo_fwd(const bdattn_qkvo_params* p, bdattn_stream_t stream) {
     if (hd <= 128) {
         bdattn::SdpaLaunch L;
         std::memset(&L, 0, sizeof(L));
-        for (int s = 0; s < 2; ++s) {
-            if (make_map_heads(op, &L.tmQ[s], Qp, bf16, hd, nh, Lq, 1, C, 0, 128)) return -1;
-            if (make_map_heads(op, &L.tmK[s], Kin, bf16, hd, nh, Lk, 1, k_ld, 0, 128)) return -1;
-            if (make_map_heads(op, &L.tmV[s], Vin, bf16, hd, nh, Lk, 1, v_ld, 0, 128)) return -1;
-        }
+        if (make_map_heads(op, &L.tmQ[0], Qp, bf16, hd, nh, Lq, 1, C, 0, 128) ||
+            make_map_heads(op, &L.tmK[0], Kin, bf16, hd, nh, Lk, 1, k_ld, 0, 128) ||
+            make_map_heads(op, &L.tmV[0], Vin, bf16, hd, nh, Lk, 1, v_ld, 0, 128))
+            return -1;
+        L.tmQ[1] = L.tmQ[0];
+        L.tmK[1] = L.tmK[0];
+        L.tmV[1] = L.tmV[0];
         bdattn::SdpaDevArgs& a = L.args;
         a.q_rows[0] = Lq; a.kv_rows[0] = Lk;
         a.o[0] = Op; a.o_ld[0] = C; a.o_bs[0] = 0;
