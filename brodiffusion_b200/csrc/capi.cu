@@ -722,7 +722,6 @@ int bdattn_linear_attn_relu_fwd(const void* q, const void* k, const void* v, voi
     // sequences once more so that two 8-warp CTAs share an SM was slower at every shape
     // tried (28.6 against 30.6 us at 4096 tokens, batch 2): it buys a cluster barrier
     // and a second reduction where the 16 warps of one CTA already hide the latencies.
-    a.stages = 8;
     cudaError_t e = bdattn::launch_linear_attn(a, tq, tk, tv, to, cs, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(op, e);
     return 0;

@@ -40,7 +40,8 @@ constexpr int kLaWarps = 16;                  // consumer warps: two groups of 8
 constexpr int kLaThreads = (kLaWarps + 1) * 32;
 constexpr int kLaGroups = kLaWarps / kLaItemWarps;
 constexpr int kLaChunk = 128;                 // tokens per ring item
-constexpr int kLaMaxStages = 8;               // ring of 16 KB items; a multiple of the number of warp groups, so that
+constexpr int kLaStages = 8;                  // ring of 16 KB items, a compile-time power of two (the slot and
+                                              // parity of an item cost two divisions otherwise); a multiple of the number of warp groups, so that
                                               // a group always meets the same slots and sees every phase of their
                                               // barriers (a ring of nine, where the groups alternate on every slot,
                                               // ended one run with a launch failure and is refused by the launcher)
@@ -59,9 +60,9 @@ struct LaSmem {
     };
     float local_state[kLaState];
     float state[48 * kLaStLd];   // rows 33..47 zero
-    uint64_t full[kLaMaxStages];
-    uint64_t empty[kLaMaxStages];
-    alignas(1024) uint8_t ring[1][kLaSlotBytes];   // a.stages items follow (dynamic shared memory)
+    uint64_t full[kLaStages];
+    uint64_t empty[kLaStages];
+    alignas(1024) uint8_t ring[1][kLaSlotBytes];   // kLaStages items in all (dynamic shared memory)
 };
 
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2,
@@ -134,8 +135,7 @@ linear_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int n_b = (n_mine + 1) / 2;  // pass B items carry two 128-token Q chunks (16 KB, like a pass A item)
     const int n_items = n_mine + n_b;  // pass A items (K + V chunks), then pass B items
     const int row0 = head * 32;
-    const int kLaStages = a.stages;
-    uint8_t* const ring_base = &sm.ring[0][0];     // a.stages items of kLaSlotBytes
+    uint8_t* const ring_base = &sm.ring[0][0];     // kLaStages items of kLaSlotBytes
 
     // Programmatic dependent launch: the next kernel of the stream (if it was
     // launched with the same attribute) may become resident as CTAs of this one
@@ -430,19 +430,15 @@ linear_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 cudaError_t launch_linear_attn(const LinearAttnArgs& a, const CUtensorMap& tmQ, const CUtensorMap& tmK,
                                const CUtensorMap& tmV, const CUtensorMap& tmO, int cluster_size,
                                cudaStream_t stream) {
-    const size_t smem = sizeof(LaSmem) + static_cast<size_t>(a.stages - 1) * kLaSlotBytes + 1024;
-    // the largest ring is set once per device; every launch fits under it
-    constexpr int kMaxSmem = static_cast<int>(sizeof(LaSmem) + (kLaMaxStages - 1) * kLaSlotBytes + 1024);
-    static_assert(kLaMaxStages % kLaGroups == 0, "every warp group must own a fixed set of ring slots");
-    if (a.stages < kLaGroups || a.stages % kLaGroups != 0 || static_cast<int>(smem) > kMaxSmem)
-        return cudaErrorInvalidValue;
-    cudaError_t e = set_max_smem_once(linear_attn_kernel, kMaxSmem);
+    constexpr int kSmem = static_cast<int>(sizeof(LaSmem) + (kLaStages - 1) * kLaSlotBytes + 1024);
+    static_assert(kLaStages % kLaGroups == 0, "every warp group must own a fixed set of ring slots");
+    cudaError_t e = set_max_smem_once(linear_attn_kernel, kSmem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(cluster_size), static_cast<unsigned>(a.num_heads),
                        static_cast<unsigned>(a.batch));
     cfg.blockDim = dim3(kLaThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = kSmem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
