@@ -937,7 +937,7 @@ def run_proj(args):
                        "l2": "rotating 6 activation sets (170 MB > 126 MB L2)",
                        "timing": "CUDA-graph replay of the steps, median of 5"},
             "clocks": sampler.summary(), "gpu_launches": args.steps * 5,
-            "roofline": {"bound": "tensor", "kernel": "gemm_wide_kernel", "achieved": tf, "peak": peak_tf,
+            "roofline": {"bound": "tensor", "kernel": "gemm_pair_kernel", "achieved": tf, "peak": peak_tf,
                          "unit": "TFLOP/s", "frac": tf / peak_tf, "peak_kind": f"{kind} cuBLAS BF16 burst",
                          "traffic": None}}
     print(json.dumps(line), flush=True)

@@ -186,7 +186,9 @@ struct GemmPlan {
 //   64 x 1280 x 5120   64 columns 27.2 us, split over four 10.6, pairs 28.9
 //   256 x 1280 x 1280  64 columns  8.8 us, split over two 8.1, over four 9.6
 //   4096 x 320 x 320   64 columns  6.4 us, 128 columns 5.5
-//   1024 x 3072 x 3072 64 columns 36.8 us, 128 columns 37.9, pairs 23.4
+//   1024 x 3072 x 3072 64 columns 36.8 us, 128 columns 37.9, pairs 21.8
+// GEGLU: 64 x 1280 -> 5120 64 columns 16.0 us, pairs 14; 256 x 320 -> 1280 8.5 and 9.
+// None is split: the two accumulators of a tile double the exchange.
 GemmPlan plan_gemm(const bdattn::GemmLaunch& L) {
     const int sms = bdattn::sm_count();
     bool whole = true, geglu = false, heads = false;
@@ -198,8 +200,7 @@ GemmPlan plan_gemm(const bdattn::GemmLaunch& L) {
         heads = heads || p.norm_rope != 0;
         k_max = p.K > k_max ? p.K : k_max;
     }
-    // whole heads with norm + RoPE are faster on pairs at any size (16 rows of 3072: 31 against 23 us),
-    // and so is GEGLU from some hundred rows on; both are left whole
+    // whole heads with norm + RoPE are faster on pairs at any size (16 rows of 3072: 31 against 24 us)
     if (heads) return {whole, 64, 1};
     const int kb = (k_max + 63) / 64;
     auto tiles = [&](int w) {
@@ -230,7 +231,7 @@ GemmPlan plan_gemm(const bdattn::GemmLaunch& L) {
     }
     if (whole) {
         const double x = (bdattn::gemm_pair_tiles(L) + sms / 2 - 1) / (sms / 2);
-        offer({true, 64, 1}, x * (kb * 0.28 + (geglu ? 3.0 : 0.0)) + 7.5);
+        offer({true, 64, 1}, x * (kb * 0.28 + (geglu ? 2.5 : 0.0)) + (geglu ? 5.3 : 7.5));
     }
     return best;
 }

@@ -107,17 +107,18 @@ __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t ta
             float ss0 = 0.0f, ss1 = 0.0f;
 #pragma unroll 1
             for (int c = 0; c < HD / 32; ++c) {
-                float f[32];
-                tmem_ld32(tacc + h * HD + c * 32, reinterpret_cast<uint32_t(&)[32]>(f));
+                uint32_t v[32];
+                tmem_ld32(tacc + h * HD + c * 32, v);
                 tmem_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    if (p.bias != nullptr) add8_from16<kBf16>(p.bias, c0 + h * HD + c * 32 + i, f + i);
-#pragma unroll
-                    for (int k = 0; k < 8; k += 2) {
-                        ss0 = fmaf(f[i + k], f[i + k], ss0);
-                        ss1 = fmaf(f[i + k + 1], f[i + k + 1], ss1);
+                for (int i = 0; i < 32; i += 2) {
+                    float x0 = __uint_as_float(v[i]), x1 = __uint_as_float(v[i + 1]);
+                    if (p.bias != nullptr) {
+                        x0 += load16<kBf16>(p.bias, c0 + h * HD + c * 32 + i);
+                        x1 += load16<kBf16>(p.bias, c0 + h * HD + c * 32 + i + 1);
                     }
+                    ss0 = fmaf(x0, x0, ss0);
+                    ss1 = fmaf(x1, x1, ss1);
                 }
             }
             inv[h] = rsqrtf((ss0 + ss1) / static_cast<float>(HD) + p.eps);
@@ -153,16 +154,16 @@ __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t ta
         }
 #pragma unroll
         for (int h = 0; h < kHeads; ++h) {
-            float f[32];
-            tmem_ld32(tacc + h * HD + c * 32, reinterpret_cast<uint32_t(&)[32]>(f));
+            uint32_t v[32];
+            tmem_ld32(tacc + h * HD + c * 32, v);
             tmem_wait_ld();
-            if (p.bias != nullptr) {
+            float f[32];
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) add8_from16<kBf16>(p.bias, c0 + h * HD + c * 32 + i, f + i);
-            }
-            if (gain_s != nullptr) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) f[i] *= inv[h] * gain_s[c * 32 + i];
+            for (int i = 0; i < 32; ++i) {
+                float x = __uint_as_float(v[i]);
+                if (p.bias != nullptr) x += load16<kBf16>(p.bias, c0 + h * HD + c * 32 + i);
+                if (gain_s != nullptr) x *= inv[h] * gain_s[c * 32 + i];
+                f[i] = x;
             }
             if (rope) {
 #pragma unroll
@@ -315,6 +316,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         const int q = warp & 3;             // TMEM lane quarter of this warp
         const int half = (warp - 2) >> 2;   // which half of the tile's output columns
         uint8_t* const stg = stg_all + (warp - 2) * kPStgBytes;
+        float* const bias_w = reinterpret_cast<float*>(stg + 2048);    // behind the output staging
         // RMSNorm gains of the three problems as FP32 for the 256 threads of these warps
         for (int idx = threadIdx.x - 64; idx < 3 * 128; idx += kPThreads - 64) {
             const GemmProblem& gp = idx < 128 ? g.p[0] : (idx < 256 ? g.p[1] : g.p[2]);
@@ -331,6 +333,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             const PairTile t = pair_tile(g, tile);
             const GemmProblem& p = t.z == 0 ? g.p[0] : (t.z == 1 ? g.p[1] : g.p[2]);
             const int as = ti & 1;
+            if (!p.norm_rope) {
+                // the 128 bias values this warp needs (GEGLU: 64 and those of their gates), fetched
+                // while the tile is computed
+                const int lc = lane * 4;
+                const long long at = p.geglu_offset > 0
+                                         ? t.n0 + half * 64 + (lc < 64 ? lc : static_cast<long long>(p.geglu_offset) + lc - 64)
+                                         : t.n0 + half * 128 + lc;
+                float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (p.bias != nullptr)
+                    b = make_float4(load16<kBf16>(p.bias, at), load16<kBf16>(p.bias, at + 1), load16<kBf16>(p.bias, at + 2),
+                                    load16<kBf16>(p.bias, at + 3));
+                *reinterpret_cast<float4*>(bias_w + lc) = b;
+                __syncwarp();
+            }
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[as], static_cast<uint32_t>((ti >> 1) & 1)));
             if (!ok) break;
             tc_fence_after();
@@ -350,31 +366,27 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 // stores 64 of the tile's 128 output columns
 #pragma unroll 1
                 for (int c = half * 64; c < half * 64 + 64; c += 32) {
-                    float f[32], gt[32];
-                    tmem_ld32(tacc + c, reinterpret_cast<uint32_t(&)[32]>(f));
-                    tmem_ld32(tacc + 128 + c, reinterpret_cast<uint32_t(&)[32]>(gt));
+                    uint32_t v[32], gt[32];
+                    tmem_ld32(tacc + c, v);
+                    tmem_ld32(tacc + 128 + c, gt);
                     tmem_wait_ld();
-                    if (p.bias != nullptr) {
+                    const float* bv = bias_w + (c - half * 64);
+                    float f[32];
 #pragma unroll
-                        for (int i = 0; i < 32; i += 8) {
-                            add8_from16<kBf16>(p.bias, t.n0 + c + i, f + i);
-                            add8_from16<kBf16>(p.bias, p.geglu_offset + t.n0 + c + i, gt + i);
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) f[i] *= gelu_exact(gt[i]);
+                    for (int i = 0; i < 32; ++i)
+                        f[i] = (__uint_as_float(v[i]) + bv[i]) * gelu_exact(__uint_as_float(gt[i]) + bv[64 + i]);
                     store_tile32<kBf16>(f, stg, lane, cbase + c, p.ldc, rows, 32);
                 }
             } else {
 #pragma unroll 1
                 for (int c = half * (kPTile / 2); c < (half + 1) * (kPTile / 2); c += 32) {
-                    float f[32];
-                    tmem_ld32(tacc + c, reinterpret_cast<uint32_t(&)[32]>(f));
+                    uint32_t v[32];
+                    tmem_ld32(tacc + c, v);
                     tmem_wait_ld();
-                    if (p.bias != nullptr) {
+                    const float* bv = bias_w + (c - half * (kPTile / 2));
+                    float f[32];
 #pragma unroll
-                        for (int i = 0; i < 32; i += 8) add8_from16<kBf16>(p.bias, t.n0 + c + i, f + i);
-                    }
+                    for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]) + bv[i];
                     store_tile32<kBf16>(f, stg, lane, cbase + c, p.ldc, rows, 32);
                 }
             }

@@ -504,36 +504,6 @@ __device__ __forceinline__ void load32_as_float(const void* base, long long i, f
     }
 }
 
-// Adds eight consecutive 16-bit values from element i of `base` to f[0..8) (one 16-byte
-// load, the same for every lane, where the address allows).
-template <bool kBf16>
-__device__ __forceinline__ void add8_from16(const void* base, long long i, float* f) {
-    const uint16_t* p = reinterpret_cast<const uint16_t*>(base) + i;
-    uint4 w;
-    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
-        w = __ldg(reinterpret_cast<const uint4*>(p));
-    } else {
-        w.x = __ldg(p) | (static_cast<uint32_t>(__ldg(p + 1)) << 16);
-        w.y = __ldg(p + 2) | (static_cast<uint32_t>(__ldg(p + 3)) << 16);
-        w.z = __ldg(p + 4) | (static_cast<uint32_t>(__ldg(p + 5)) << 16);
-        w.w = __ldg(p + 6) | (static_cast<uint32_t>(__ldg(p + 7)) << 16);
-    }
-    auto add2 = [](uint32_t h, float& lo, float& hi) {
-        if constexpr (kBf16) {
-            lo += __uint_as_float(h << 16);
-            hi += __uint_as_float(h & 0xffff0000u);
-        } else {
-            const __half2 v = *reinterpret_cast<const __half2*>(&h);
-            lo += __low2float(v);
-            hi += __high2float(v);
-        }
-    };
-    add2(w.x, f[0], f[1]);
-    add2(w.y, f[2], f[3]);
-    add2(w.z, f[4], f[5]);
-    add2(w.w, f[6], f[7]);
-}
-
 // Stores a warp's 32 x 32 tile (thread = row) as 16-bit values: through `stg` (2 KB of this
 // warp's shared memory), so that four lanes write 64 consecutive bytes of a row.  Straight
 // from the registers a store instruction touches 32 rows, 32 cache lines.
