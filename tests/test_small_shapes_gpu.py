@@ -136,3 +136,21 @@ def test_map_block_edges(bd, oracle, hd, nh, L, split, row0, rows, cols):
     _, ref = oracle.sdpa(q, k, v, nh, bias=bias, bias_row0=row0, want_avg=True)
     # FP32 scores on both sides; 2^-22 from each exponential and 1e-5 from the sums
     assert np.abs(G.host(amap) - ref[row0:row0 + rows, :cols]).max() <= 1e-4 * ref.max()
+
+
+# Key masks that leave whole key tiles out: the first, the last, all but one, every one, more
+# tiles than the list of visible tiles holds.
+@pytest.mark.parametrize("hd,Lk,first,last", [(128, 700, 300, 700), (128, 700, 0, 100), (64, 1000, 390, 395),
+                                              (128, 300, 0, 0), (64, 512 * 128 + 77, 65000, 65600)])
+def test_key_tiles_without_a_visible_key(bd, oracle, hd, Lk, first, last):
+    nh, Lq = 2, 150
+    q, k, v = _acts([(Lq, nh * hd), (Lk, nh * hd), (Lk, nh * hd)], 9560 + Lk, "bf16")
+    mask = np.zeros(Lk, np.float32)
+    mask[first:last] = 1.0
+    got = G.sdpa(bd, q, k, v, nh, key_mask=mask)
+    if last == first:
+        assert not got.any()
+        return
+    ref = oracle.sdpa(q, k[first:last], v[first:last], nh)
+    # probabilities are rounded to BF16 (2^-9 of each), then the output
+    assert np.abs(got - ref).max() <= 2.0 ** -7 * np.abs(ref).max()
