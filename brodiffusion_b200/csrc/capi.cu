@@ -240,19 +240,13 @@ GemmPlan plan_gemm(const bdattn::GemmLaunch& L) {
 int launch_gemm(const char* op, bdattn::GemmLaunch& L, int n, cudaStream_t stream) {
     L.n_problems = n;
     const GemmPlan plan = plan_gemm(L);
-    bool pair = plan.pair;
-    int width = plan.width, split = plan.split;
-#ifdef BDATTN_TUNE
-    if (const char* e = std::getenv("BD_W")) { const int v = std::atoi(e); if (v) { pair = v == 256; if (v < 256) width = v; split = 1; } }
-    if (const char* e = std::getenv("BD_S")) { const int v = std::atoi(e); if (v && !pair && !L.args.p[0].norm_rope) split = v; }
-#endif
-    L.args.split = split;
+    L.args.split = plan.split;
     for (int i = 0; i < n; ++i) {
         bdattn::GemmProblem& p = L.args.p[i];
-        if (p.n_tile == 0) p.n_tile = width;
+        if (p.n_tile == 0) p.n_tile = plan.width;
         p.tiles_n = (p.N + p.n_tile - 1) / p.n_tile;
         // a CTA of a pair stages 128 weight rows
-        if (make_map_2d(op, &L.tmB[i], L.W[i], L.bf16, p.K, L.w_rows[i], L.ldw[i], pair ? 128 : p.n_tile)) return -1;
+        if (make_map_2d(op, &L.tmB[i], L.W[i], L.bf16, p.K, L.w_rows[i], L.ldw[i], plan.pair ? 128 : p.n_tile)) return -1;
     }
     for (int i = n; i < 3; ++i) {
         L.args.p[i] = L.args.p[0];
@@ -261,7 +255,7 @@ int launch_gemm(const char* op, bdattn::GemmLaunch& L, int n, cudaStream_t strea
         L.tmA[i] = L.tmA[0];
         L.tmB[i] = L.tmB[0];
     }
-    const cudaError_t e = pair ? bdattn::launch_gemm_pair(L, stream) : bdattn::launch_gemm_tc05(L, stream);
+    const cudaError_t e = plan.pair ? bdattn::launch_gemm_pair(L, stream) : bdattn::launch_gemm_tc05(L, stream);
     if (e != cudaSuccess) return cuda_fail(op, e);
     return 0;
 }

@@ -372,8 +372,8 @@ int bdattn_linear_attn_relu_fwd(const void* q, const void* k, const void* v, voi
  *   wo (out_cols, inner_dim); biases have one value per output feature, the
  *   tensor dtype, and may be NULL; out (x_rows, out_cols).
  * Weights are dense row-major (out_features, in_features).  Heads of 40 or
- * 80 columns are projected straight into a 64 / 128-wide padded layout in the
- * workspace so that the attention core runs on the tcgen05 kernel.
+ * 80 columns stay as they are in the workspace: the attention core's tensor
+ * maps zero-fill them to 64 / 128.
  * The workspace (device memory, 256-byte aligned, size from
  * bdattn_qkvo_workspace_bytes) holds Q, K, V and the attention output
  * between the three steps; the call does not allocate.
