@@ -9,6 +9,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "gemm_plan.h"
 #include "sdpa_internal.h"
 #include "tc05.cuh"
 
@@ -172,74 +173,15 @@ int add_gemm_problem(const char* op, bdattn::GemmLaunch& L, int idx, const void*
     return 0;
 }
 
-// Which kernel, tile width and number of CTAs per tile a GEMM launch gets.
-struct GemmPlan {
-    bool pair;
-    int width, split;
-};
-
-// The least of the modelled times, fitted to FP16 calls of 64 x 1280 x 1280 to 9216 x 320 x 1280
-// (M x N x K) on one B200.  A K block of 64 costs a CTA 0.30 us with 64 or 128 columns and a
-// pair 0.28 us; the rest of a call is 3 us (64 columns, one CTA per SM), 4.3 (64, several), 4.2
-// (128) or 7.5 (pairs), and the exchange of a split tile 1.5, as much again for a second wave.
-// Several CTAs of 64 columns share an SM and hide part of each other.  Examples, measured:
-//   64 x 1280 x 5120   64 columns 27.2 us, split over four 10.6, pairs 28.9
-//   256 x 1280 x 1280  64 columns  8.8 us, split over two 8.1, over four 9.6
-//   4096 x 320 x 320   64 columns  6.4 us, 128 columns 5.5
-//   1024 x 3072 x 3072 64 columns 36.8 us, 128 columns 37.9, pairs 21.8
-// GEGLU: 64 x 1280 -> 5120 64 columns 16.0 us, pairs 14; 256 x 320 -> 1280 8.5 and 9.
-// None is split: the two accumulators of a tile double the exchange.
-GemmPlan plan_gemm(const bdattn::GemmLaunch& L) {
-    const int sms = bdattn::sm_count();
-    bool whole = true, geglu = false, heads = false;
-    int k_max = 0;
-    for (int i = 0; i < L.n_problems; ++i) {
-        const bdattn::GemmProblem& p = L.args.p[i];
-        whole = whole && L.whole[i];
-        geglu = geglu || p.geglu_offset > 0;
-        heads = heads || p.norm_rope != 0;
-        k_max = p.K > k_max ? p.K : k_max;
-    }
-    // whole heads with norm + RoPE are faster on pairs at any size (16 rows of 3072: 31 against 24 us)
-    if (heads) return {whole, 64, 1};
-    const int kb = (k_max + 63) / 64;
-    auto tiles = [&](int w) {
-        long long t = 0;
-        for (int i = 0; i < L.n_problems; ++i)
-            t += static_cast<long long>(L.args.p[i].tiles_m) * ((L.args.p[i].N + w - 1) / w);
-        return t;
-    };
-    auto waves = [&](int w, int s) { return static_cast<double>((tiles(w) * s + sms - 1) / sms); };
-    GemmPlan best = {false, 64, 1};
-    double best_us;
-    {
-        const double x = waves(64, 1), b = kb * (geglu ? 0.45 : 0.30) * (geglu ? x : 1.0);
-        best_us = x <= 1.0 ? b + 3.0 : (geglu ? b : 0.62 * x * b) + 4.3;
-        if (geglu) best_us += 3.0 * x;
-    }
-    auto offer = [&](const GemmPlan& p, double us) {
-        if (us < best_us) { best = p; best_us = us; }
-    };
-    if (!geglu) {
-        offer({false, 128, 1}, waves(128, 1) * kb * 0.31 + 4.2);
-        // (beyond one and a half CTAs per SM a split only adds waves: 256 x 3072 x 3072 over four 21.4 us,
-        // over two 16.2)
-        for (int s = 2; s <= 8 && kb >= 3 * s && tiles(64) * s * 2 <= 3LL * sms; s *= 2) {
-            const double x = waves(64, s), b = 0.30 * kb / s;
-            offer({false, 64, s}, (x <= 1.0 ? b : 0.725 * x * b) + 4.5 + 1.5 * (x - 1.0));
-        }
-    }
-    if (whole) {
-        const double x = (bdattn::gemm_pair_tiles(L) + sms / 2 - 1) / (sms / 2);
-        offer({true, 64, 1}, x * (kb * 0.28 + (geglu ? 2.5 : 0.0)) + (geglu ? 5.3 : 7.5));
-    }
-    return best;
-}
-
 // Makes the weight maps for the plan and launches.
 int launch_gemm(const char* op, bdattn::GemmLaunch& L, int n, cudaStream_t stream) {
     L.n_problems = n;
-    const GemmPlan plan = plan_gemm(L);
+    bdattn::GemmShape shapes[3];
+    for (int i = 0; i < n; ++i) {
+        const bdattn::GemmProblem& p = L.args.p[i];
+        shapes[i] = {p.M, p.N, p.K, p.geglu_offset > 0, p.norm_rope != 0, L.whole[i]};
+    }
+    const bdattn::GemmPlan plan = bdattn::plan_gemm(shapes, n, bdattn::sm_count());
     L.args.split = plan.split;
     for (int i = 0; i < n; ++i) {
         bdattn::GemmProblem& p = L.args.p[i];

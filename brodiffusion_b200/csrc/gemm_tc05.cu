@@ -21,6 +21,7 @@
 #include <cooperative_groups.h>
 #include <type_traits>
 
+#include "gemm_plan.h"
 #include "sdpa_internal.h"
 #include "tc05.cuh"
 
@@ -134,9 +135,9 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int k_all = (p.K + 63) / 64;
-    const int k_begin = kSplit ? part * k_all / split : 0;
-    const int k_blocks = (kSplit ? (part + 1) * k_all / split : k_all) - k_begin;
+    const int k_all = gemm_k_blocks(p.K);
+    const int k_begin = kSplit ? gemm_part_begin(k_all, split, part) : 0;
+    const int k_blocks = (kSplit ? gemm_part_begin(k_all, split, part + 1) : k_all) - k_begin;
     const int n0 = tile_n * p.n_tile;
     const int m0 = tile_m * 128;
     const bool geglu = kGeglu && p.geglu_offset > 0;
@@ -387,6 +388,9 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
 
 cudaError_t launch_gemm_tc05(const GemmLaunch& L, cudaStream_t stream) {
     int tn = 0, tm = 0, nt_max = 16, any_geglu = 0, any_norm_rope = 0, k_max = 0;
+    // a CTA without a K block would wait for an accumulator that nobody computes
+    for (int i = 0; i < L.n_problems; ++i)
+        if (L.args.split > gemm_k_blocks(L.args.p[i].K)) return cudaErrorInvalidValue;
     for (int i = 0; i < L.n_problems; ++i) {
         const GemmProblem& p = L.args.p[i];
         tn = p.tiles_n > tn ? p.tiles_n : tn;

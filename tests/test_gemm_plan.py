@@ -1,0 +1,58 @@
+"""The rule that chooses kernel, tile width and split of a launch of linear layers, on the
+CPU: csrc/gemm_plan.h is plain C++ and is compiled here into a small library."""
+import ctypes as C
+import itertools
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("plan") / "plan.so")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-o", so,
+                           os.path.join(ROOT, "tests", "cpp", "gemm_plan_probe.cpp")])
+    lib = C.CDLL(so)
+
+    def run(shapes, geglu=False, heads=False, sms=148):
+        flat = (C.c_int * (3 * len(shapes)))(*itertools.chain(*shapes))
+        out = (C.c_int * 3)()
+        lib.probe_plan(flat, len(shapes), int(geglu), int(heads), sms, out)
+        return bool(out[0]), out[1], out[2]
+
+    run.fewest_blocks = lib.probe_fewest_blocks
+    return run
+
+
+def test_every_cta_of_a_split_tile_has_a_k_block(plan):
+    """Q, K and V of a cross-attention in one launch: K is x_cols for Q and ctx_cols for the others."""
+    splits = set()
+    for rows, ctx_rows, inner, x_cols, ctx_cols in itertools.product(
+            (1, 64, 256, 1000, 4096), (16, 77, 256, 512), (64, 128, 192, 256, 320, 640, 768, 1280, 3072),
+            (8, 64, 128, 192, 320, 640, 1280), (8, 64, 128, 320, 768, 1024, 2048, 4096)):
+        shapes = [(rows, inner, x_cols), (ctx_rows, inner, ctx_cols), (ctx_rows, inner, ctx_cols)]
+        pair, width, split = plan(shapes)
+        splits.add(split)
+        assert not (pair and split > 1)
+        for _, _, k in shapes:
+            assert plan.fewest_blocks(k, split) >= 1, (shapes, split)
+    assert splits == {1, 2, 4, 8}
+
+
+@pytest.mark.parametrize("shapes,split", [
+    ([(64, 64, 64), (77, 64, 768), (77, 64, 768)], 1),
+    ([(64, 192, 192), (77, 192, 768), (77, 192, 768)], 2),
+    ([(256, 256, 256), (77, 256, 2048), (77, 256, 2048)], 4),
+    ([(64, 1280, 1280), (77, 1280, 64), (77, 1280, 64)], 1),
+    ([(64, 1280, 5120)], 8), ([(256, 1280, 1280)], 2), ([(128, 64, 768)], 4), ([(128, 64, 704)], 2),
+    ([(128, 64, 640)], 1)])
+def test_split_is_bounded_by_the_shortest_k(plan, shapes, split):
+    assert plan(shapes)[2] == split
+
+
+def test_geglu_is_never_split(plan):
+    for rows, d_in, d_out in itertools.product((1, 64, 300, 4096), (64, 320, 1280, 5120), (72, 128, 1280, 5120)):
+        assert plan([(rows, d_out, d_in)], geglu=True)[2] == 1

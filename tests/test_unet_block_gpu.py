@@ -77,6 +77,20 @@ def test_sd15_cross_attention_uncached_cached_and_project_kv(bd, oracle):
     G.check(out_c, out, max_abs=1e-2, what="cached vs uncached")
 
 
+# A launch whose projections differ in K: 64 columns for one and 2048 or 4096 for the others are one
+# K block and many, so that the split is bounded by the shortest (one case per split it ends at).
+@pytest.mark.parametrize("L,C,nh,Lc,Cc", [(64, 64, 2, 77, 768), (64, 192, 3, 77, 768), (256, 128, 2, 77, 768),
+                                          (256, 256, 4, 77, 2048), (64, 320, 8, 77, 4096), (64, 1280, 8, 77, 64),
+                                          (64, 768, 12, 77, 128)])
+def test_cross_attention_with_projections_of_unequal_k(bd, oracle, L, C, nh, Lc, Cc):
+    x, ctx = synth.activations((L, C), 7150 + C), synth.activations((Lc, Cc), 7151 + Cc)
+    wq, wo = synth.weights((C, C), 7152), synth.weights((C, C), 7153)
+    wk, wv = synth.weights((C, Cc), 7154), synth.weights((C, Cc), 7155)
+    bo = synth.weights((C,), 7156)
+    ref = oracle.qkvo_attention(x, ctx, wq, wk, wv, wo, bo, nh)
+    G.check(_qkvo(bd, x, ctx, wq, wk, wv, wo, bo, nh), ref, what=f"cross {L}x{C}, context {Lc}x{Cc}")
+
+
 def test_fp16_self_attention(bd, oracle):
     """The reference runs SD1.5 in FP16 on the GPU."""
     L, C, nh = 512, 320, 8
