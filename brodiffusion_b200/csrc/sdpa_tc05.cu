@@ -292,10 +292,6 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             }
             __syncthreads();
             n_kv = n;
-            if (n == 0 && warp == 9 && lane == 0) {     // nobody else waits for the query tiles then
-                mbar_wait(&q_full[0], 0);
-                mbar_wait(&q_full[1], 0);
-            }
         }
     }
     // the j-th key tile of this CTA
@@ -608,6 +604,10 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             ok = mbar_wait(&pv_done[t], static_cast<uint32_t>((n_kv - 1) & 1)) && ok;
             ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
+        } else if (listed) {
+            // no visible key: the query tile may still be on its way into the buffer that the epilogue
+            // stages its zeros in
+            ok = __all_sync(0xffffffffu, mbar_wait(&q_full[t], 0));
         }
         const float inv = (l_sum > 0.0f) ? 1.0f / l_sum : 0.0f;
         if constexpr (kHooks == 2) {

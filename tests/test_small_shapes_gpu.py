@@ -154,3 +154,30 @@ def test_key_tiles_without_a_visible_key(bd, oracle, hd, Lk, first, last):
     ref = oracle.sdpa(q, k[first:last], v[first:last], nh)
     # probabilities are rounded to BF16 (2^-9 of each), then the output
     assert np.abs(got - ref).max() <= 2.0 ** -7 * np.abs(ref).max()
+
+
+# Query tiles all of whose keys are masked (a left-padded prompt under the causal rule, a mask without a
+# visible key): their rows are zero however late the query tile arrives.  Enough CTAs to fill the SMs,
+# queries that come from HBM (L2 is flushed), several repeats.
+@pytest.mark.parametrize("hd,nh", [(128, 24), (64, 24), (40, 8)])
+@pytest.mark.parametrize("masked,causal", [(300, True), (700, False)])
+def test_query_tiles_without_a_visible_key(bd, oracle, hd, nh, masked, causal):
+    B, L = 3, 700
+    q, k, v = (synth.activations((B, L, nh * hd), 9580 + i) for i in range(3))
+    mask = np.ones(L, np.float32)
+    mask[:masked] = 0.0
+    tq, tk, tv, tm = G.dev(q), G.dev(k), G.dev(v), G.dev(mask, torch.float32)
+    flush = torch.empty(256 << 20, device="cuda", dtype=torch.uint8)
+    first = None
+    for _ in range(8):
+        out = torch.full_like(tq, float("nan"))
+        flush.fill_(1)
+        bd.sdpa_fwd(tq, tk, tv, out, nh, key_mask=tm, mask_mode=bd.MASK_CAUSAL if causal else bd.MASK_NONE)
+        assert bd.device_status() == 0
+        assert not out[:, :masked].any()
+        first = out if first is None else first
+        assert torch.equal(out, first)
+    if masked < L:
+        ref = oracle.sdpa(q[1, masked:], k[1, masked:], v[1, masked:], nh, mask_mode=1)
+        # probabilities are rounded to BF16 (2^-9 of each), then the output
+        assert np.abs(G.host(first[1, masked:]) - ref).max() <= 2.0 ** -7 * np.abs(ref).max()
