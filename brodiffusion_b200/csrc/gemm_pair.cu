@@ -26,6 +26,7 @@
 // the pair, tcgen05.mma issuer for both, warps 2-9 = epilogue of the CTA's 128 rows (warp w
 // owns TMEM lanes 32 * (w % 4)..; warps 2-5 take the first half of a tile's output columns,
 // warps 6-9 the second half).
+#include "gemm_plan.h"
 #include "sdpa_internal.h"
 #include "tc05.cuh"
 
@@ -263,7 +264,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                     if (++slot == kPStages) { slot = 0; phase ^= 1; }
                 }
             }
-            if (!ok && rank == 0) {
+            if (ok) {
+                // the last commits arrive here too: both CTAs see them before they end
+                for (int i = max(0, it - kPStages); i < it; ++i)
+                    mbar_wait(&empty[i % kPStages], static_cast<uint32_t>((i / kPStages) & 1));
+            } else if (rank == 0) {
                 // a wait ran out: let the copies in flight land before the CTAs end
                 for (int i = max(0, it - kPStages); i < it; ++i)
                     mbar_wait(&full[i % kPStages], static_cast<uint32_t>((i / kPStages) & 1));
@@ -390,15 +395,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                     store_tile32<kBf16>(f, stg, lane, cbase + c, p.ldc, rows, 32);
                 }
             }
-            // this accumulator may be overwritten by the MMAs of tile ti + 2
+            // this accumulator may be overwritten by the MMAs of tile ti + 2; where there is none, nobody
+            // would wait for the arrival, and the first CTA could have left before it comes
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa(smem_u32(&acc_empty[as]), 0));
+            if (lane == 0 && pair_acc_reused(tile, pairs, total_tiles))
+                mbar_arrive_cluster(mapa(smem_u32(&acc_empty[as]), 0));
         }
     }
 
     tc_fence_before();
-    cluster_sync_relaxed();       // neither CTA leaves while the other may still signal or read it
+    // Neither CTA leaves while the other may still signal or read it.  (Every arrival at a peer's barrier
+    // has been waited for by then: the barrier itself orders none.)
+    cluster_sync_relaxed();
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, 512);

@@ -33,6 +33,12 @@ BDATTN_HD constexpr int gemm_row_tiles(int M) { return (M + 127) / 128; }
 BDATTN_HD constexpr int gemm_pair_row_tiles(int row_tiles) { return (row_tiles + 1) / 2; }
 BDATTN_HD constexpr int gemm_pair_cols(bool geglu) { return geglu ? 128 : 256; }
 
+// A pair of CTAs takes the tiles  first, first + pairs, ...  and its two accumulators in turn: whether the
+// accumulator of `tile` is used again, so that its release is waited for.
+BDATTN_HD constexpr bool pair_acc_reused(int tile, int pairs, int total_tiles) {
+    return tile + 2 * pairs < total_tiles;
+}
+
 // The least of the modelled times, fitted to FP16 calls of 64 x 1280 x 1280 to 9216 x 320 x 1280
 // (M x N x K) on one B200.  A K block of 64 costs a CTA 0.30 us with 64 or 128 columns and a
 // pair 0.28 us; the rest of a call is 3 us (64 columns, one CTA per SM), 4.3 (64, several), 4.2

@@ -1,4 +1,4 @@
-// The plan of a launch of linear layers as C functions, for tests/test_gemm_plan.py.
+// The plan of a launch of linear layers and the pair kernel's tile rules as C functions, for tests/test_gemm_plan.py.
 #include "../../brodiffusion_b200/csrc/gemm_plan.h"
 
 using namespace bdattn;
@@ -27,5 +27,7 @@ int probe_fewest_blocks(int K, int split) {
     }
     return least;
 }
+
+int probe_acc_reused(int tile, int pairs, int total_tiles) { return pair_acc_reused(tile, pairs, total_tiles); }
 
 }

@@ -24,6 +24,7 @@ def plan(tmp_path_factory):
         return bool(out[0]), out[1], out[2]
 
     run.fewest_blocks = lib.probe_fewest_blocks
+    run.acc_reused = lib.probe_acc_reused
     return run
 
 
@@ -56,3 +57,14 @@ def test_split_is_bounded_by_the_shortest_k(plan, shapes, split):
 def test_geglu_is_never_split(plan):
     for rows, d_in, d_out in itertools.product((1, 64, 300, 4096), (64, 320, 1280, 5120), (72, 128, 1280, 5120)):
         assert plan([(rows, d_out, d_in)], geglu=True)[2] == 1
+
+
+@pytest.mark.parametrize("pairs", [1, 2, 74])
+@pytest.mark.parametrize("total", [1, 2, 3, 4, 5, 73, 74, 75, 147, 148, 149, 222, 223, 1000])
+def test_every_release_of_an_accumulator_is_waited_for(plan, pairs, total):
+    """The MMA issuer of a pair waits, before its tile ti >= 2, for the release of tile ti - 2.  A release
+    that it does not wait for could reach a CTA that has ended."""
+    for first in range(min(pairs, total)):
+        tiles = list(range(first, total, pairs))
+        released = [ti for ti, tile in enumerate(tiles) if plan.acc_reused(tile, pairs, total)]
+        assert released == [ti - 2 for ti in range(2, len(tiles))]
