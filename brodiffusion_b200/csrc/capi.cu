@@ -25,7 +25,10 @@ int fail(const char* fmt, ...) {
     return -1;
 }
 
+// Reports a failed CUDA call and takes its error off the thread's last-error state, where the check of a
+// later, sound launch would find it.
 int cuda_fail(const char* op, cudaError_t e) {
+    cudaGetLastError();
     return fail("%s: CUDA error: %s", op, cudaGetErrorString(e));
 }
 

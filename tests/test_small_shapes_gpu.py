@@ -181,3 +181,15 @@ def test_query_tiles_without_a_visible_key(bd, oracle, hd, nh, masked, causal):
         ref = oracle.sdpa(q[1, masked:], k[1, masked:], v[1, masked:], nh, mask_mode=1)
         # probabilities are rounded to BF16 (2^-9 of each), then the output
         assert np.abs(G.host(first[1, masked:]) - ref).max() <= 2.0 ** -7 * np.abs(ref).max()
+
+
+def test_a_refused_launch_leaves_the_next_call_alone(bd):
+    """More heads than a grid has rows is refused, and the next call does not report that error again."""
+    x = torch.zeros(1, 65536 * 136, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(bd.BdattnError, match=r"^bdattn_sdpa_fwd: CUDA error"):
+        bd.sdpa_fwd(x, x, x, torch.empty_like(x), 65536)
+    t = torch.ones(4, 256, device="cuda", dtype=torch.bfloat16)
+    cos, sin = torch.ones(4, 64, device="cuda"), torch.zeros(4, 64, device="cuda")
+    out = torch.empty_like(t)
+    bd.rmsnorm_rope([dict(x=t, out=out, cos=cos, sin=sin)], 2, 128, pair_mode=1)
+    assert torch.equal(out, t)
