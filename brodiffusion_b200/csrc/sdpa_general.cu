@@ -8,9 +8,9 @@
 // K / V chunks of its own (cp.async, no CTA barrier in the loop) and a running
 // maximum, sum and accumulator of its own, which are merged through shared memory at
 // the end.  Products run on mma.sync m16n8k16 with FP32 accumulation; a probability is
-// split into 16-bit parts that add up to it (two for FP16, three for BF16, where two
-// would keep 16 of its 24 bits), one product each, so that nothing is rounded to 16
-// bits before the output.
+// split into 16-bit parts, one product each, so that nothing is rounded to 16 bits before the
+// output: three for BF16 (they add up to it exactly) and two for FP16 (23 of its 24 bits; the
+// exponential itself is good to 2^-22.5).
 // Two row tiles per CTA (MT = 2) halve the reads of K and V where there are still
 // enough CTAs for that.
 // 64 x 64 with 8 heads of 160: 4.2 us, 576 x 576: 22.8 us (97 and 840 on the CUDA-core kernel
@@ -145,10 +145,11 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
     if (warp < n_chunks) fetch(warp, 0);
     asm volatile("cp.async.commit_group;" ::: "memory");
 
-    // FP16: probabilities carry a factor of 2^10 (it cancels in O / l), which keeps small ones out
-    // of the subnormals; with value scales they carry the power of two that brings the largest scale
-    // to at most one instead, so that no part overflows.
-    const float boost = kBf16 ? 0.0f : 10.0f;
+    // FP16: probabilities carry a factor of 2^15, which keeps the parts of small ones out of the subnormals
+    // and cancels in O / l.  It is multiplied on, exactly: added to the exponent it costs the argument
+    // of a probability near one its last three bits.
+    constexpr float kBoost = kBf16 ? 1.0f : 32768.0f;
+    // (With value scales above one they also carry the power of two that brings the largest to at most one.)
     float v_mul = 1.0f, v_undo = 1.0f;
     if (!kBf16 && a.val_scale != nullptr) {
         float mx = 0.0f;
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
                 float p[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    p[i] = fast_exp2(x[i] - m_use + boost);
+                    p[i] = fast_exp2(x[i] - m_use) * kBoost;
                     l_run[t][hf] += p[i];
                     p[i] *= vs[i];
                 }

@@ -47,6 +47,25 @@ def test_head_dims_above_128(bd, oracle, storage, hd, nh, Lq, Lk, opt):
     assert np.abs(got - ref).max() <= half_ulp + 1e-4 * np.abs(ref).max()
 
 
+def test_head_dims_above_128_probabilities_near_one(bd):
+    """Two keys of almost the same score and opposite values: the output is V * tanh(d / 2), all of it what
+    the second probability 1 - d lacks to one.  Root mean square error of that probability over 256 rows:
+    2^-23 / sqrt(12) from its two parts, as much from the exponential and less from the output's
+    rounding, 0.6e-7 in all; an exponent rounded at 2^-20 makes 1.9e-7."""
+    hd, rows, big = 160, 256, 32768.0
+    d = np.exp2(-14.0 + 2.0 * np.arange(rows) / rows)
+    c = synth.round_fp16((d * np.sqrt(hd)).astype(np.float32))
+    q = np.zeros((rows, hd), np.float32)
+    q[:, 0] = c
+    k = np.zeros((2, hd), np.float32)
+    k[1, 0] = -1.0
+    v = np.full((2, hd), big, np.float32)
+    v[1] = -big
+    got = G.sdpa(bd, q, k, v, 1, dtype=torch.float16)
+    err = (got[:, 0].astype(np.float64) / big - np.tanh(c.astype(np.float64) / np.sqrt(hd) / 2.0)) * 2.0
+    assert np.sqrt(np.mean(err ** 2)) < 1e-7
+
+
 def test_head_dims_above_128_segments_and_groups(bd, oracle):
     """Two segments on both sides whose border is inside a tile, two query heads per K/V head."""
     hd, nh, nkv = 160, 4, 2
