@@ -81,10 +81,14 @@ __device__ __forceinline__ uint32_t gen_part(float& x, float& y) {
     return w;
 }
 
-template <int HD, int MT, bool kBf16>
+// kWide (FP16 with value scales): a weight, the probability times its scale, has the range of FP32, which
+// FP16 parts do not.  Weights are split into BF16 parts as with BF16 values, and a value of FP16 into
+// two BF16 parts that add up to it.
+template <int HD, int MT, bool kBf16, bool kWide>
 __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGeneralArgs a, int q_ctas0) {
     using C = GenCfg<HD>;
-    constexpr int kParts = kBf16 ? 3 : 2;
+    constexpr bool kBf16Parts = kBf16 || kWide;
+    constexpr int kParts = kBf16Parts ? 3 : 2;
     extern __shared__ __align__(16) uint8_t gsm[];
     uint16_t* Qs = reinterpret_cast<uint16_t*>(gsm);                                    // [16 * MT][kLd]
     uint8_t* ring = gsm + 16 * MT * C::kLd * 2;
@@ -148,21 +152,7 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
     // FP16: probabilities carry a factor of 2^15, which keeps the parts of small ones out of the subnormals
     // and cancels in O / l.  It is multiplied on, exactly: added to the exponent it costs the argument
     // of a probability near one its last three bits.
-    constexpr float kBoost = kBf16 ? 1.0f : 32768.0f;
-    // (With value scales above one they also carry the power of two that brings the largest to at most one.)
-    float v_mul = 1.0f, v_undo = 1.0f;
-    if (!kBf16 && a.val_scale != nullptr) {
-        float mx = 0.0f;
-        for (int i = lane; i < Lk; i += 32) mx = fmaxf(mx, fabsf(__ldg(a.val_scale + i)));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (mx > 1.0f && mx < INFINITY) {
-            int e;
-            frexpf(mx, &e);                       // mx <= 2^e
-            v_mul = ldexpf(1.0f, -e / 2) * ldexpf(1.0f, -(e - e / 2));
-            v_undo = 1.0f / v_mul;
-        }
-    }
+    constexpr float kBoost = kBf16Parts ? 1.0f : 32768.0f;
 
     float o[MT][HD / 8][4];
     float m_run[MT][2], l_run[MT][2];
@@ -216,7 +206,7 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
             const bool in = kg < Lk;
             seen[i] = in && (a.key_mask == nullptr || __ldg(a.key_mask + kg) != 0.0f);
             ks[i] = sl2 * (in && a.key_scale != nullptr ? __ldg(a.key_scale + kg) : 1.0f);
-            vs[i] = in && a.val_scale != nullptr ? __ldg(a.val_scale + kg) * v_mul : 1.0f;
+            vs[i] = kBf16Parts && in && a.val_scale != nullptr ? __ldg(a.val_scale + kg) : 1.0f;
         }
         uint32_t pa[MT][kParts][4];
 #pragma unroll
@@ -252,12 +242,12 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
                 for (int i = 0; i < 4; ++i) {
                     p[i] = fast_exp2(x[i] - m_use) * kBoost;
                     l_run[t][hf] += p[i];
-                    p[i] *= vs[i];
+                    if constexpr (kBf16Parts) p[i] *= vs[i];
                 }
 #pragma unroll
                 for (int k = 0; k < kParts; ++k) {
-                    pa[t][k][hf] = gen_part<kBf16>(p[0], p[1]);          // keys 2 q4, 2 q4 + 1
-                    pa[t][k][2 + hf] = gen_part<kBf16>(p[2], p[3]);      // the same + 8
+                    pa[t][k][hf] = gen_part<kBf16Parts>(p[0], p[1]);          // keys 2 q4, 2 q4 + 1
+                    pa[t][k][2 + hf] = gen_part<kBf16Parts>(p[2], p[3]);      // the same + 8
                 }
             }
         }
@@ -265,12 +255,30 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
         for (int n = 0; n < HD / 16; ++n) {
             uint32_t b[4];
             gen_ldsm4_t(b, v_addr + n * 32);
+            if constexpr (kWide) {
+                uint32_t rest[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const __half2 h = *reinterpret_cast<const __half2*>(&b[i]);
+                    float lo = __low2float(h), hi = __high2float(h);
+                    b[i] = gen_part<true>(lo, hi);
+                    rest[i] = pack2<true>(lo, hi);
+                }
+#pragma unroll
+                for (int t = 0; t < MT; ++t) {
+#pragma unroll
+                    for (int k = kParts - 1; k >= 0; --k) {
+                        gen_mma<true>(o[t][2 * n], pa[t][k], rest[0], rest[1]);
+                        gen_mma<true>(o[t][2 * n + 1], pa[t][k], rest[2], rest[3]);
+                    }
+                }
+            }
 #pragma unroll
             for (int t = 0; t < MT; ++t) {
 #pragma unroll
                 for (int k = kParts - 1; k >= 0; --k) {                  // smallest part first
-                    gen_mma<kBf16>(o[t][2 * n], pa[t][k], b[0], b[1]);
-                    gen_mma<kBf16>(o[t][2 * n + 1], pa[t][k], b[2], b[3]);
+                    gen_mma<kBf16Parts>(o[t][2 * n], pa[t][k], b[0], b[1]);
+                    gen_mma<kBf16Parts>(o[t][2 * n + 1], pa[t][k], b[2], b[3]);
                 }
             }
         }
@@ -324,7 +332,7 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
             f[0] = fmaf(c, u0.x, f[0]); f[1] = fmaf(c, u0.y, f[1]); f[2] = fmaf(c, u0.z, f[2]); f[3] = fmaf(c, u0.w, f[3]);
             f[4] = fmaf(c, u1.x, f[4]); f[5] = fmaf(c, u1.y, f[5]); f[6] = fmaf(c, u1.z, f[6]); f[7] = fmaf(c, u1.w, f[7]);
         }
-        const float inv = l > 0.0f ? v_undo / l : 0.0f;
+        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
         uint4 w4;
         w4.x = pack2<kBf16>(f[0] * inv, f[1] * inv); w4.y = pack2<kBf16>(f[2] * inv, f[3] * inv);
         w4.z = pack2<kBf16>(f[4] * inv, f[5] * inv); w4.w = pack2<kBf16>(f[6] * inv, f[7] * inv);
@@ -332,9 +340,9 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
     }
 }
 
-template <int HD, int MT, bool kBf16>
+template <int HD, int MT, bool kBf16, bool kWide>
 cudaError_t launch_general_t(const SdpaGeneralArgs& a, int num_heads, int batch, cudaStream_t stream) {
-    auto kern = sdpa_general_kernel<HD, MT, kBf16>;
+    auto kern = sdpa_general_kernel<HD, MT, kBf16, kWide>;
     constexpr int smem = GenCfg<HD>::smem(MT);
     cudaError_t e = set_max_smem_once(kern, smem);
     if (e != cudaSuccess) return e;
@@ -345,20 +353,23 @@ cudaError_t launch_general_t(const SdpaGeneralArgs& a, int num_heads, int batch,
     return launch_dependent(kern, grid, dim3(kGThreads), smem, stream, a, q_ctas0);
 }
 
+template <int HD, int MT>
+cudaError_t launch_general_hd(const SdpaGeneralArgs& a, int num_heads, int batch, bool bf16, cudaStream_t stream) {
+    if (bf16) return launch_general_t<HD, MT, true, false>(a, num_heads, batch, stream);
+    return a.val_scale != nullptr ? launch_general_t<HD, MT, false, true>(a, num_heads, batch, stream)
+                                  : launch_general_t<HD, MT, false, false>(a, num_heads, batch, stream);
+}
+
 }  // namespace
 
 cudaError_t launch_sdpa_general(const SdpaGeneralArgs& a, int num_heads, int batch, bool bf16,
                                 cudaStream_t stream) {
-    if (a.head_dim > 160)
-        return bf16 ? launch_general_t<256, 1, true>(a, num_heads, batch, stream)
-                    : launch_general_t<256, 1, false>(a, num_heads, batch, stream);
+    if (a.head_dim > 160) return launch_general_hd<256, 1>(a, num_heads, batch, bf16, stream);
     // two row tiles per CTA once that still leaves one CTA per SM
     const long long rows = static_cast<long long>(a.q_rows[0]) + a.q_rows[1];
     if ((rows + 31) / 32 * num_heads * batch >= sm_count())
-        return bf16 ? launch_general_t<160, 2, true>(a, num_heads, batch, stream)
-                    : launch_general_t<160, 2, false>(a, num_heads, batch, stream);
-    return bf16 ? launch_general_t<160, 1, true>(a, num_heads, batch, stream)
-                : launch_general_t<160, 1, false>(a, num_heads, batch, stream);
+        return launch_general_hd<160, 2>(a, num_heads, batch, bf16, stream);
+    return launch_general_hd<160, 1>(a, num_heads, batch, bf16, stream);
 }
 
 }  // namespace bdattn

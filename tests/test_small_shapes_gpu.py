@@ -66,6 +66,31 @@ def test_head_dims_above_128_probabilities_near_one(bd):
     assert np.sqrt(np.mean(err ** 2)) < 1e-7
 
 
+# Value scales far from one with FP16 values: a scale of 1e8 on a key nobody sees, scales of 1e-8 on values
+# near 5e4, scales that span twelve decades.  Only the output is rounded (bound as above, for the largest
+# value of a row's 160 columns: what cancels there leaves FP32 errors of that size).
+@pytest.mark.parametrize("hd,nh,Lq,Lk", [(160, 2, 40, 50), (160, 8, 600, 36), (256, 2, 20, 4)])
+@pytest.mark.parametrize("kind", ["masked", "small", "wide"])
+def test_head_dims_above_128_value_scales_far_from_one(bd, oracle, hd, nh, Lq, Lk, kind):
+    q, k, v = _acts([(Lq, nh * hd), (Lk, nh * hd), (Lk, nh * hd)], 9540 + hd, "fp16")
+    scale = 0.5 + 0.5 * synth.uniform01(Lk, 9541).astype(np.float32)
+    mask = np.ones(Lk, np.float32)
+    if kind == "masked":
+        scale[1], mask[1] = 1e8, 0.0
+    elif kind == "small":
+        v = synth.round_fp16((5e4 * (0.5 + 0.5 * synth.uniform01(v.size, 9542))).astype(np.float32).reshape(v.shape))
+        scale *= 1e-8
+    else:
+        scale *= np.power(10.0, np.linspace(-10, 2, Lk)).astype(np.float32)
+        v = synth.round_fp16(v * 16.0)
+    got = G.sdpa(bd, q, k, v, nh, dtype=torch.float16, key_mask=mask, val_scale=scale)
+    ref = oracle.sdpa(q, k, v * scale[:, None], nh, key_mask=mask)
+    half_ulp = np.exp2(np.maximum(np.floor(np.log2(np.abs(ref) + 1e-30)), -14.0) - 11.0)
+    top = np.abs(ref.reshape(Lq, nh, hd)).max(axis=2, keepdims=True)
+    slack = np.broadcast_to(1e-4 * top, (Lq, nh, hd)).reshape(Lq, nh * hd)
+    assert (np.abs(got - ref) <= half_ulp + slack).all()
+
+
 def test_head_dims_above_128_segments_and_groups(bd, oracle):
     """Two segments on both sides whose border is inside a tile, two query heads per K/V head."""
     hd, nh, nkv = 160, 4, 2
