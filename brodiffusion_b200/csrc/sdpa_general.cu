@@ -81,11 +81,134 @@ __device__ __forceinline__ uint32_t gen_part(float& x, float& y) {
     return w;
 }
 
+// Eight 16-bit values as floats.
+template <bool kBf16>
+__device__ __forceinline__ void gen_wide8(const uint16_t* src, float (&out)[8]) {
+    const uint4 w = *reinterpret_cast<const uint4*>(src);
+    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if constexpr (kBf16) {
+            out[2 * e] = __uint_as_float(ws[e] << 16);
+            out[2 * e + 1] = __uint_as_float(ws[e] & 0xffff0000u);
+        } else {
+            const __half2 h = *reinterpret_cast<const __half2*>(&ws[e]);
+            out[2 * e] = __low2float(h);
+            out[2 * e + 1] = __high2float(h);
+        }
+    }
+}
+
+// The output of a CTA again, with plain FP32 products, when some value of it was not finite (an infinity
+// or NaN among the inputs): a weight split into parts has parts that are zero or negative, whose
+// product with an infinite value is NaN.  Q rows in Qs; the four warps' row maxima and sums of the first
+// pass in the merge area.  `boost`: the factor those sums carry.
+// A function of its own that is not inlined: in line it changed how the loop of the first pass
+// was compiled (576 x 576, 24 heads of 160: 53.9 -> 65.6 us); called, it costs that pass nothing.
+template <int HD, int MT, bool kBf16>
+__device__ __noinline__ void gen_plain(const SdpaGeneralArgs& a, int q_ctas0, float boost, const uint16_t* Qs, uint8_t* ring) {
+    using C = GenCfg<HD>;
+    constexpr int kRows = 16 * MT;
+    const int hd = a.head_dim, vecs = hd >> 3;
+    const int head = blockIdx.y, batch = blockIdx.z;
+    const int qseg = static_cast<int>(blockIdx.x) >= q_ctas0 ? 1 : 0;
+    const int qrow0 = (qseg ? static_cast<int>(blockIdx.x) - q_ctas0 : static_cast<int>(blockIdx.x)) * kRows;
+    const int seg_rows = qseg ? a.q_rows[1] : a.q_rows[0];
+    const int q_glob0 = (qseg ? a.q_rows[0] : 0) + qrow0;
+    const int Lk = a.kv_rows[0] + a.kv_rows[1];
+    int k_end = Lk;
+    if (a.mask_mode == 1) k_end = max(0, min(Lk, q_glob0 + min(kRows, seg_rows - qrow0) + a.q_offset));
+    const long long kv_col = static_cast<long long>(head / a.kv_group) * hd;
+    const float sl2 = a.scale * 1.4426950408889634f;
+
+    float* Om = reinterpret_cast<float*>(ring);
+    const float* Sm = Om + kGWarps * kRows * C::kMergeLd;
+    float* const Ms = Om;                        // [kRows] maximum, [kRows] 1 / sum
+    float* const Ps = Om + 2 * kRows;            // [kRows][33]
+    if (threadIdx.x < kRows) {
+        float m = -INFINITY, l = 0.0f;
+        for (int w = 0; w < kGWarps; ++w) m = fmaxf(m, Sm[(w * kRows + threadIdx.x) * 2]);
+        for (int w = 0; w < kGWarps; ++w) {
+            const float mw = Sm[(w * kRows + threadIdx.x) * 2];
+            l += mw == -INFINITY ? 0.0f : fast_exp2(mw - m) * Sm[(w * kRows + threadIdx.x) * 2 + 1];
+        }
+        Ms[threadIdx.x] = m == -INFINITY ? 0.0f : m;
+        Ms[kRows + threadIdx.x] = l > 0.0f ? boost / l : 0.0f;
+    }
+    auto row_of = [&](const void* const (&p)[2], const long long (&ld)[2], const long long (&bs)[2], int kg) {
+        const int seg = kg >= a.kv_rows[0] ? 1 : 0;
+        const long long rr = seg ? kg - a.kv_rows[0] : kg;
+        return static_cast<const uint16_t*>(seg ? p[1] : p[0]) + (batch * (seg ? bs[1] : bs[0]) + rr * (seg ? ld[1] : ld[0]) + kv_col);
+    };
+    constexpr int kItems = (kRows * (HD / 8) + kGThreads - 1) / kGThreads;    // output vectors of a thread
+    float acc[kItems][8];
+#pragma unroll
+    for (int j = 0; j < kItems; ++j)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[j][e] = 0.0f;
+#pragma unroll 1
+    for (int k0 = 0; k0 < k_end; k0 += 32) {
+        __syncthreads();
+#pragma unroll 1
+        for (int i = threadIdx.x; i < kRows * 32; i += kGThreads) {
+            const int r = i >> 5, kg = k0 + (i & 31);
+            const bool vis = kg < Lk && (a.mask_mode != 1 || kg <= q_glob0 + r + a.q_offset) &&
+                             (a.key_mask == nullptr || __ldg(a.key_mask + kg) != 0.0f);
+            float p = 0.0f;
+            if (vis) {
+                const uint16_t* kr = row_of(a.k, a.k_ld, a.k_bs, kg);
+                float dot = 0.0f;
+#pragma unroll 1
+                for (int d = 0; d < hd; d += 8) {
+                    float qv[8], kv[8];
+                    gen_wide8<kBf16>(Qs + r * C::kLd + d, qv);
+                    gen_wide8<kBf16>(kr + d, kv);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) dot = fmaf(qv[e], kv[e], dot);
+                }
+                p = fast_exp2(dot * (sl2 * (a.key_scale != nullptr ? __ldg(a.key_scale + kg) : 1.0f)) - Ms[r]) * Ms[kRows + r];
+            }
+            Ps[r * 33 + (i & 31)] = p;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int kk = 0; kk < min(32, Lk - k0); ++kk) {
+            const uint16_t* vr = row_of(a.v, a.v_ld, a.v_bs, k0 + kk);
+            const float sc = a.val_scale != nullptr ? __ldg(a.val_scale + k0 + kk) : 1.0f;
+#pragma unroll
+            for (int j = 0; j < kItems; ++j) {
+                const int i = threadIdx.x + j * kGThreads, r = i / vecs;
+                if (r < kRows) {
+                    const float p = Ps[r * 33 + kk];
+                    float vv[8];
+                    gen_wide8<kBf16>(vr + (i - r * vecs) * 8, vv);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[j][e] = fmaf(p, vv[e] * sc, acc[j][e]);
+                }
+            }
+        }
+    }
+    uint16_t* op = static_cast<uint16_t*>(qseg ? a.o[1] : a.o[0]) + batch * (qseg ? a.o_bs[1] : a.o_bs[0]) +
+                   static_cast<long long>(head) * hd;
+    const long long o_ld = qseg ? a.o_ld[1] : a.o_ld[0];
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+        const int i = threadIdx.x + j * kGThreads, r = i / vecs;
+        if (r < kRows && qrow0 + r < seg_rows) {
+            uint4 w4;
+            w4.x = pack2<kBf16>(acc[j][0], acc[j][1]); w4.y = pack2<kBf16>(acc[j][2], acc[j][3]);
+            w4.z = pack2<kBf16>(acc[j][4], acc[j][5]); w4.w = pack2<kBf16>(acc[j][6], acc[j][7]);
+            *reinterpret_cast<uint4*>(op + static_cast<long long>(qrow0 + r) * o_ld + (i - r * vecs) * 8) = w4;
+        }
+    }
+}
+
 // kWide (FP16 with value scales): a weight, the probability times its scale, has the range of FP32, which
 // FP16 parts do not.  Weights are split into BF16 parts as with BF16 values, and a value of FP16 into
 // two BF16 parts that add up to it.
 template <int HD, int MT, bool kBf16, bool kWide>
-__global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGeneralArgs a, int q_ctas0) {
+__global__ void __launch_bounds__(kGThreads)
+sdpa_general_kernel(const __grid_constant__ SdpaGeneralArgs a, int q_ctas0) {
     using C = GenCfg<HD>;
     constexpr bool kBf16Parts = kBf16 || kWide;
     constexpr int kParts = kBf16Parts ? 3 : 2;
@@ -313,6 +436,7 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
     uint16_t* op = static_cast<uint16_t*>(qseg ? a.o[1] : a.o[0]) + batch * (qseg ? a.o_bs[1] : a.o_bs[0]) +
                    static_cast<long long>(head) * hd;
     const long long o_ld = qseg ? a.o_ld[1] : a.o_ld[0];
+    bool finite = true;
     for (int i = threadIdx.x; i < kRows * vecs; i += kGThreads) {
         const int r = i / vecs, v = i - r * vecs;
         if (qrow0 + r >= seg_rows) break;        // rows only grow from here on
@@ -333,11 +457,19 @@ __global__ void __launch_bounds__(kGThreads) sdpa_general_kernel(const SdpaGener
             f[4] = fmaf(c, u1.x, f[4]); f[5] = fmaf(c, u1.y, f[5]); f[6] = fmaf(c, u1.z, f[6]); f[7] = fmaf(c, u1.w, f[7]);
         }
         const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        float t = 0.0f;                          // NaN once a value is not finite
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            f[e] *= inv;
+            t = fmaf(f[e], 0.0f, t);
+        }
+        finite = finite && t == 0.0f;
         uint4 w4;
-        w4.x = pack2<kBf16>(f[0] * inv, f[1] * inv); w4.y = pack2<kBf16>(f[2] * inv, f[3] * inv);
-        w4.z = pack2<kBf16>(f[4] * inv, f[5] * inv); w4.w = pack2<kBf16>(f[6] * inv, f[7] * inv);
+        w4.x = pack2<kBf16>(f[0], f[1]); w4.y = pack2<kBf16>(f[2], f[3]);
+        w4.z = pack2<kBf16>(f[4], f[5]); w4.w = pack2<kBf16>(f[6], f[7]);
         *reinterpret_cast<uint4*>(op + static_cast<long long>(qrow0 + r) * o_ld + v * 8) = w4;
     }
+    if (__syncthreads_or(!finite)) gen_plain<HD, MT, kBf16>(a, q_ctas0, kBoost, Qs, ring);
 }
 
 template <int HD, int MT, bool kBf16, bool kWide>

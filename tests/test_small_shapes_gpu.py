@@ -104,6 +104,28 @@ def test_head_dims_above_128_segments_and_groups(bd, oracle):
     G.check(G.host(out), oracle.sdpa(q, rep(k), rep(v), nh), what="segments and groups, head_dim 160")
 
 
+# Infinite and NaN values stay what a sum of products makes of them, in their own columns only; the
+# key that carries them is in the first, a middle or the last (ragged) chunk of sixteen.
+@pytest.mark.parametrize("storage", ["bf16", "fp16"])
+@pytest.mark.parametrize("hd,Lq,Lk,key", [(160, 40, 70, 3), (160, 600, 70, 37), (136, 17, 70, 69), (256, 20, 33, 32)])
+def test_head_dims_above_128_values_that_are_not_finite(bd, oracle, storage, hd, Lq, Lk, key):
+    nh = 8 if Lq > 100 else 2
+    q, k, v = _acts([(Lq, nh * hd), (Lk, nh * hd), (Lk, nh * hd)], 9530 + hd, storage)
+    ref = oracle.sdpa(q, k, v, nh)
+    other = (key + 29) % Lk
+    for col, vals in ((1, (np.inf,)), (7, (-np.inf,)), (hd - 1, (np.inf, -np.inf)), (64, (np.nan,)), (hd + 5, (np.inf, np.inf))):
+        for row, val in zip((key, other), vals):
+            v[row, col] = val
+        ref[:, col] = sum(vals) if len(set(vals)) == 1 else np.nan
+    got = G.sdpa(bd, q, k, v, nh, dtype=torch.bfloat16 if storage == "bf16" else torch.float16)
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    inf = np.isinf(ref)
+    assert np.array_equal(got[inf], ref[inf])
+    fin = np.isfinite(ref)
+    half_ulp = np.exp2(np.ceil(np.log2(np.abs(ref[fin]).max()))) * (2.0 ** -9 if storage == "bf16" else 2.0 ** -12)
+    assert np.abs(got[fin] - ref[fin]).max() <= half_ulp + 1e-4 * np.abs(ref[fin]).max()
+
+
 # Few output tiles, so that 2, 4 or 8 CTAs share a tile: ragged rows and columns, K not a
 # multiple of a K block, the smallest K that is split and one just below it.
 @pytest.mark.parametrize("M,N,K", [(64, 1280, 1280), (64, 1280, 5120), (1, 72, 2048), (77, 1280, 768), (130, 200, 1000),
