@@ -7,10 +7,11 @@
 //   warp  8    : issues the Q.K^T MMAs (one lane), owns the TMEM allocation
 //   warp  9    : TMA producer for Q, K and V tiles (one lane)
 //   warp  10   : issues the P.V MMAs (one lane)
-//   warp  11   : with per-key scale vectors (kScale): multiplies the rows of a K or
-//                V tile in shared memory by their factors before the MMAs read it;
-//                otherwise idle (it completes the third warpgroup, so that registers
-//                can be moved to the softmax warpgroups with setmaxnreg)
+//   warp  11   : idle (it completes the third warpgroup, so that registers can be moved
+//                to the softmax warpgroups with setmaxnreg)
+//   warps 12-15: only with per-key scale vectors (kScale): multiply the rows of a K or V
+//                tile in shared memory by their factors before the MMAs read it, 32
+//                rows each
 // Tensor memory (512 columns) at head_dim 128:
 //   P0 [0,64)  S [64,192)  P1 [192,256)  O0 [256,384)  O1 [384,512)
 // and at 64: S0 [0,128) S1 [128,256) P0 [256,320) P1 [320,384) O0 [384,448)
@@ -79,11 +80,17 @@ struct Cfg {
     static constexpr uint32_t kColO1 = kColO0 + HD;
 };
 
-constexpr int kThreads = 384;
-// Registers per thread after the hand-over (setmaxnreg): 8 x 216 + 4 x 64 stays within
-// the 12 x 168 the CTA is launched with.
-constexpr int kRegsSoftmax = 216;
-constexpr int kRegsOther = 64;
+// Threads of a CTA, and registers per thread after the hand-over (setmaxnreg), which stay within what the
+// CTA is launched with: 8 x 216 + 4 x 64 within 12 x 168; with scaling warps 8 x 208 + 8 x 48 = 16 x 128.
+// Scaling a tile costs one warp 5000 cycles beside the softmax warps, a key step has two tiles and
+// 2790 cycles: four warps (256 + 1024 keys of which 256 are scaled, 24 heads of 128: 24.6 us; 31.5 with
+// one warp, 21.9 without scales; all of 2048 + 512 keys 53.6, 106 and 35.2).
+template <bool kScale>
+struct Roles {
+    static constexpr int kThreads = kScale ? 512 : 384;
+    static constexpr int kRegsSoftmax = kScale ? 208 : 216;
+    static constexpr int kRegsOther = kScale ? 48 : 64;
+};
 
 struct TileInfo {
     int seg;
@@ -151,11 +158,11 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 // HOOKS: 0 = none; 1 = key_mask only; 2 = key_mask, bias and the per-row softmax
 // statistics (slower softmax path).
 // SCALE: key_scale / val_scale are applied to the K / V tiles in shared memory by
-// warp 10 (rounded to the storage type, as the reference's scale_inplace on its
+// warps 12-15 (rounded to the storage type, as the reference's scale_inplace on its
 // k_full_ / v_full_ copies does, src/dit/qwenimage21_forward.cpp:606-645); the
 // softmax code does not change.
 template <int HD, bool kBf16, int kHooks, bool kScale>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Roles<kScale>::kThreads, 1)
 sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant__ CUtensorMap tmQ1,
                  const __grid_constant__ CUtensorMap tmK0, const __grid_constant__ CUtensorMap tmK1,
                  const __grid_constant__ CUtensorMap tmV0, const __grid_constant__ CUtensorMap tmV1,
@@ -210,12 +217,12 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
         for (int i = 0; i < KS; ++i) {
             mbar_init(&k_full[i], 1);
             mbar_init(&k_empty[i], 1);
-            mbar_init(&k_ready[i], 1);
+            mbar_init(&k_ready[i], 4);
         }
         for (int i = 0; i < VS; ++i) {
             mbar_init(&v_full[i], 1);
             mbar_init(&v_empty[i], 1);
-            mbar_init(&v_ready[i], 1);
+            mbar_init(&v_ready[i], 4);
         }
         for (int t = 0; t < 2; ++t) {
             mbar_init(&q_full[t], 1);
@@ -268,7 +275,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             }
             __syncwarp();
 #pragma unroll 2
-            for (int t = warp; t < n_kv; t += kThreads / 32) {
+            for (int t = warp; t < n_kv; t += Roles<kScale>::kThreads / 32) {
                 const TileInfo ti = kv_tile(a, t);
                 float mv[4];
 #pragma unroll
@@ -299,7 +306,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
 
     if (warp < 8) {
         // ------------------------------------------------ softmax + epilogue
-        setmaxnreg_inc<kRegsSoftmax>();
+        setmaxnreg_inc<Roles<kScale>::kRegsSoftmax>();
         const int t = warp >> 2;
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t tS = tmem_base + lane_base + (t ? C::kColS1 : C::kColS0);
@@ -695,7 +702,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             }
         }
     } else {
-        setmaxnreg_dec<kRegsOther>();
+        setmaxnreg_dec<Roles<kScale>::kRegsOther>();
         if (warp == 8) {
             // -------------------------------------------------- Q.K^T issuer
             // One tcgen05.mma costs its issuing thread 46-59 cycles and the pipe 64, the
@@ -810,90 +817,71 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                 }
             }
             __syncwarp();
-        } else {
+        } else if (kScale && warp >= 12) {
             // ------------------------------------------- K / V row scaling
-            // Warp 11 walks the K and V tiles in order (it sees every phase of the
-            // barriers it waits on).  The row
-            // factors of an item are fetched before the wait for its tile.  A tile
-            // none of whose factors differs from one is passed on as it is; otherwise
-            // every row is multiplied by its factor (FP32 product rounded to the
-            // storage type).
+            // The four warps walk the K and V tiles in order (they see every phase of the barriers they
+            // wait on); a lane has one row of a tile and its factor, fetched one tile ahead.  Rows none of
+            // whose factors differs from one are passed on as they are, the others multiplied by
+            // theirs (FP32 product rounded to the storage type).
             if constexpr (kScale) {
                 bool ok = true;
-                // row factors of item i (rows lane, lane + 32, ...), fetched one item ahead
-                auto fetch = [&](int i, float (&f)[4]) {
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) f[w] = 1.0f;
+                const int row = (warp - 12) * 32 + lane;
+                auto fetch = [&](int i) {
                     const float* sc = (i & 1) ? a.val_scale : a.key_scale;
-                    if (sc != nullptr && i < 2 * n_kv) {
-                        const TileInfo ti = kv_tile(a, i >> 1);
-#pragma unroll
-                        for (int w = 0; w < 4; ++w) {
-                            const int r = lane + 32 * w;
-                            if (r < ti.valid) f[w] = __ldg(sc + ti.kbase + r);
-                        }
-                    }
+                    if (sc == nullptr || i >= 2 * n_kv) return 1.0f;
+                    const TileInfo ti = kv_tile(a, i >> 1);
+                    return row < ti.valid ? __ldg(sc + ti.kbase + row) : 1.0f;
                 };
-                float f[4], fn[4];
-                fetch(0, fn);
-                for (int i = 0; ok && i < 2 * n_kv; ++i) {
-                    const int n = i >> 1;
-                    const int slot = (i & 1) ? n % VS : n % KS;
-                    const uint32_t phase = static_cast<uint32_t>(((i & 1) ? n / VS : n / KS) & 1);
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) f[w] = fn[w];
-                    fetch(i + 1, fn);
-                    const bool ne = f[0] != 1.0f || f[1] != 1.0f || f[2] != 1.0f || f[3] != 1.0f;
-                    const bool scale_tile = __any_sync(0xffffffffu, ne);
-                    ok = mbar_wait((i & 1) ? &v_full[slot] : &k_full[slot], phase);
+                float next = fetch(0);
+                int kslot = 0, vslot = 0;
+                uint32_t kphase = 0, vphase = 0;
+                for (int i = 0; i < 2 * n_kv; ++i) {
+                    const float f = next;
+                    next = fetch(i + 1);
+                    const bool is_v = (i & 1) != 0;
+                    ok = is_v ? mbar_wait(&v_full[vslot], vphase) : mbar_wait(&k_full[kslot], kphase);
                     if (!ok) break;
-                    if (scale_tile) {
-                        uint8_t* tile = ((i & 1) ? smem_v : smem_k) + slot * C::kTileBytes;
-                        // A lane owns whole rows (lane, lane + 32, ...: the rows whose factors it
-                        // holds).  Within a 64-column chunk a row is one 128-byte line whose 16-byte
-                        // pieces the swizzle permutes; the factor is the same for all of them, so
-                        // the pieces are walked in physical order, rotated by the lane's row so that
-                        // the 32 rows of one access fall into different banks.
+                    if (__any_sync(0xffffffffu, f != 1.0f)) {
+                        // Within a 64-column chunk a row is one 128-byte line whose 16-byte pieces the
+                        // swizzle permutes; the factor is the same for all of them, so the pieces are
+                        // walked in physical order, rotated by the lane's row so that the 32 rows of
+                        // one access fall into different banks.
+                        uint8_t* line = (is_v ? smem_v + vslot * C::kTileBytes : smem_k + kslot * C::kTileBytes) + row * 128;
+#pragma unroll 1
+                        for (int h = 0; h < 2 * C::kChunks; ++h) {
+                            uint8_t* const half = line + (h >> 1) * kChunkBytes;
+                            const int rot = (lane & 7) ^ ((h & 1) * 4);
+                            uint4 v[4];
 #pragma unroll
-                        for (int pi = 0; pi < 4 * C::kChunks; ++pi) {
-                            const int w = pi / C::kChunks, ch = pi % C::kChunks;
-                            if (!__any_sync(0xffffffffu, f[w] != 1.0f)) continue;
-                            uint8_t* line = tile + ch * kChunkBytes + (lane + 32 * w) * 128;
-                            const float fw = f[w];
+                            for (int b = 0; b < 4; ++b) v[b] = *reinterpret_cast<const uint4*>(half + ((b ^ rot) << 4));
 #pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                uint4 v[4];
+                            for (int b = 0; b < 4; ++b) {
+                                uint32_t* w32 = reinterpret_cast<uint32_t*>(&v[b]);
 #pragma unroll
-                                for (int b = 0; b < 4; ++b)
-                                    v[b] = *reinterpret_cast<const uint4*>(line + (((h * 4 + b) ^ (lane & 7)) << 4));
-#pragma unroll
-                                for (int b = 0; b < 4; ++b) {
-                                    uint32_t* w32 = reinterpret_cast<uint32_t*>(&v[b]);
-#pragma unroll
-                                    for (int e = 0; e < 4; ++e) {
-                                        float lo, hi;
-                                        if constexpr (kBf16) {
-                                            lo = __uint_as_float(w32[e] << 16);
-                                            hi = __uint_as_float(w32[e] & 0xffff0000u);
-                                        } else {
-                                            const __half2 hh = *reinterpret_cast<const __half2*>(&w32[e]);
-                                            lo = __low2float(hh);
-                                            hi = __high2float(hh);
-                                        }
-                                        // x * f + (-0) = x * f with the sign of a zero product kept
-                                        ffma2(lo, hi, lo, hi, fw, fw, -0.0f, -0.0f);
-                                        w32[e] = pack2<kBf16>(lo, hi);
+                                for (int e = 0; e < 4; ++e) {
+                                    float lo, hi;
+                                    if constexpr (kBf16) {
+                                        lo = __uint_as_float(w32[e] << 16);
+                                        hi = __uint_as_float(w32[e] & 0xffff0000u);
+                                    } else {
+                                        const __half2 hh = *reinterpret_cast<const __half2*>(&w32[e]);
+                                        lo = __low2float(hh);
+                                        hi = __high2float(hh);
                                     }
+                                    // x * f + (-0) = x * f with the sign of a zero product kept
+                                    ffma2(lo, hi, lo, hi, f, f, -0.0f, -0.0f);
+                                    w32[e] = pack2<kBf16>(lo, hi);
                                 }
-#pragma unroll
-                                for (int b = 0; b < 4; ++b)
-                                    *reinterpret_cast<uint4*>(line + (((h * 4 + b) ^ (lane & 7)) << 4)) = v[b];
                             }
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) *reinterpret_cast<uint4*>(half + ((b ^ rot) << 4)) = v[b];
                         }
                         fence_proxy_async_smem();      // the MMA reads the tile through the async proxy
                     }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive((i & 1) ? &v_ready[slot] : &k_ready[slot]);
+                    if (lane == 0) mbar_arrive(is_v ? &v_ready[vslot] : &k_ready[kslot]);
+                    if (is_v) { if (++vslot == VS) { vslot = 0; vphase ^= 1; } }
+                    else { if (++kslot == KS) { kslot = 0; kphase ^= 1; } }
                 }
             }
         }
@@ -915,7 +903,7 @@ cudaError_t launch_t(const SdpaLaunch& L, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     dim3 grid(static_cast<unsigned>(L.q_ctas), static_cast<unsigned>(L.num_heads),
               static_cast<unsigned>(L.batch));
-    return launch_dependent(kern, grid, dim3(kThreads), C::kSmemBytes, stream, L.tmQ[0], L.tmQ[1], L.tmK[0],
+    return launch_dependent(kern, grid, dim3(Roles<kScale>::kThreads), C::kSmemBytes, stream, L.tmQ[0], L.tmQ[1], L.tmK[0],
                             L.tmK[1], L.tmV[0], L.tmV[1], L.args);
 }
 

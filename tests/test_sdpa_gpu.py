@@ -505,3 +505,25 @@ def test_argument_errors_carry_the_operator_prefix(bd):
     q192 = torch.zeros(16, 192, device="cuda", dtype=torch.bfloat16)
     with pytest.raises(bd.BdattnError, match=r"^bdattn_sdpa_fwd_allgather_multicast: .*head_dim <= 128"):
         bd.sdpa_fwd(q192, q192, q192, q192.clone(), 1, multicast_out_ptrs=[q192.data_ptr()])
+
+
+# Every row of a K or V tile has a factor of its own, the last tile is ragged, more tiles than the rings
+# hold; one vector or both.  The rows are scaled in FP32 and rounded to the storage type: the same bits as
+# K and V scaled beforehand.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hd,Lk", [(128, 1100), (64, 1100), (40, 333), (128, 1)])
+@pytest.mark.parametrize("which", ["k", "v", "kv"])
+def test_row_scales_have_the_bits_of_scaled_rows(bd, dtype, hd, Lk, which):
+    nh, Lq = 3, 300
+    gen = torch.Generator(device="cuda").manual_seed(8700 + hd)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    q, k, v = rnd(Lq, nh * hd).to(dtype), rnd(Lk, nh * hd).to(dtype), rnd(Lk, nh * hd).to(dtype)
+    factor = 0.25 + torch.rand(Lk, device="cuda", generator=gen)
+    factor[Lk // 3:Lk // 2] = 1.0
+    scaled = lambda t: (t.float() * factor[:, None]).to(dtype)
+    got, ref = torch.empty_like(q), torch.empty_like(q)
+    bd.sdpa_fwd(q, k, v, got, nh, key_scale=factor if "k" in which else None,
+                val_scale=factor if "v" in which else None)
+    bd.sdpa_fwd(q, scaled(k) if "k" in which else k, scaled(v) if "v" in which else v, ref, nh)
+    assert bd.device_status() == 0
+    assert torch.equal(got, ref)
