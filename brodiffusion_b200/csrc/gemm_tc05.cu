@@ -160,7 +160,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // only now: a dependent CTA that took tensor memory first could keep this one from getting its own
-    dependents_may_launch();
+    if (!kNormRope || g.one_wave) dependents_may_launch();
     wait_for_prior_grid();
 
     if (warp == 0) {
@@ -404,6 +404,10 @@ cudaError_t launch_gemm_tc05(const GemmLaunch& L, cudaStream_t stream) {
     args.n_tile_max = nt_max;
     args.any_geglu = any_geglu;
     const long long ctas = static_cast<long long>(tn) * tm * L.n_problems * args.split;
+    // With norm + RoPE the CTAs of Q and K are the slow ones and come first, those of V fill up; the next
+    // kernel's CTAs in the slots of the first finishers would undo that order for a kernel of this
+    // kind (4096 rows, 2 heads of 64, K = 1024: 28.8 us a launch, 20.7 kept back).
+    args.one_wave = ctas <= sm_count();
     const int stage = gemm_stage_bytes(nt_max, any_geglu != 0);
     // three stages with the gate tile: the stage ring stays below 114 KB and two CTAs fit per SM
     args.stages = any_geglu ? 3 : 4;

@@ -183,6 +183,7 @@ struct GemmArgs {
     int any_geglu;
     int stages;
     int split;        // CTAs (a cluster) that share the K blocks of a tile
+    bool one_wave;    // no more CTAs than SMs
 };
 struct GemmLaunch {
     CUtensorMap tmA[3], tmB[3];
