@@ -146,8 +146,6 @@ int make_map_2d(const char* op, CUtensorMap* m, const void* base, bool bf16, lon
     return 0;
 }
 
-int round_up(int x, int m) { return (x + m - 1) / m * m; }
-
 // One GEMM problem  C[M, N] = A[M, K] . W[N, K]^T (+ bias).  head_dim > 0 asks for
 // tiles of whole heads (norm + RoPE epilogue).
 int add_gemm_problem(const char* op, bdattn::GemmLaunch& L, int idx, const void* A, long long lda,
@@ -163,7 +161,7 @@ int add_gemm_problem(const char* op, bdattn::GemmLaunch& L, int idx, const void*
     if (N % 8 != 0) return fail("%s: output width must be a multiple of 8 (got %d)", op, N);
     bdattn::GemmProblem& p = L.args.p[idx];
     p.M = M; p.N = N; p.K = K; p.C = Cout; p.ldc = ldc; p.bias = bias;
-    p.tiles_m = (M + 127) / 128;
+    p.tiles_m = bdattn::gemm_row_tiles(M);
     p.geglu_offset = geglu_offset;
     p.n_tile = head_dim;       // 0: chosen at the launch
     if (make_map_2d(op, &L.tmA[idx], A, L.bf16, K, M, lda, 128)) return -1;
@@ -171,8 +169,7 @@ int add_gemm_problem(const char* op, bdattn::GemmLaunch& L, int idx, const void*
     L.W[idx] = W;
     L.ldw[idx] = ldw;
     L.w_rows[idx] = geglu_offset > 0 ? static_cast<long long>(N) + geglu_offset : N;
-    // the pair kernel's tiles are 256 columns (GEGLU: 128 value columns + their gate columns)
-    L.whole[idx] = N % (geglu_offset > 0 ? 128 : 256) == 0;
+    L.whole[idx] = N % bdattn::gemm_pair_cols(geglu_offset > 0) == 0;
     return 0;
 }
 
@@ -772,7 +769,9 @@ int bdattn_add_row_bias(void* y, const void* bias, int rows, int cols, long long
 
 size_t bdattn_qkvo_workspace_bytes(int q_rows, int kv_rows, int num_heads, int head_dim) {
     if (q_rows < 0 || kv_rows < 0 || num_heads < 1 || head_dim < 1) return 0;
-    // room for heads padded to 64 or 128 columns, which the projections once wrote
+    // Heads take no padding in the workspace; the size asked for is that of heads padded to 64 or 128 columns
+    // all the same, so that the sizes callers keep, and which calls the fixed scratch array of
+    // bdattn_qkvo_fwd_static takes, stay what they were.
     const int pad = head_dim % 8 != 0 || head_dim > 128 ? head_dim : (head_dim <= 64 ? 64 : 128);
     const size_t wq = static_cast<size_t>(q_rows) * num_heads * pad * 2;
     const size_t wkv = static_cast<size_t>(kv_rows) * num_heads * pad * 2;

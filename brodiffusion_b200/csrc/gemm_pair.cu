@@ -2,7 +2,8 @@
 // src/dit/flux.cpp:471-484; out-projection: src/dit/flux.cpp:519-525):
 //   C[M,N] = A[M,K] . W[N,K]^T (+ bias) [-> per-head RMSNorm -> RoPE]
 // Same operand layout and epilogue arithmetic as gemm_tc05_kernel; what differs is the
-// schedule, for problems that fill the SMs with 256 x 256 tiles:
+// schedule, for problems that fill SMs with 256 x 256 tiles and, whatever their size, for whole heads
+// with norm + RoPE:
 //   * a cluster of two CTAs owns a 256-row x 256-column tile and computes it with
 //     tcgen05.mma.cta_group::2: every CTA stages its 128 rows of A and 128 of the tile's 256
 //     weight rows, so a K block costs an SM 32 KB of L2 reads and 8 KB of operand reads per
@@ -50,10 +51,8 @@ struct PairTile {
 
 // Output columns of one tile: 256, or 128 for GEGLU (the other 128 accumulator
 // columns hold the gate).
-__host__ __device__ __forceinline__ int pair_out_cols(const GemmProblem& p) {
-    return p.geglu_offset > 0 ? kPTile / 2 : kPTile;
-}
-__host__ __device__ __forceinline__ int pair_tiles_m(const GemmProblem& p) { return (p.tiles_m + 1) / 2; }
+__host__ __device__ __forceinline__ int pair_out_cols(const GemmProblem& p) { return gemm_pair_cols(p.geglu_offset > 0); }
+__host__ __device__ __forceinline__ int pair_tiles_m(const GemmProblem& p) { return gemm_pair_row_tiles(p.tiles_m); }
 
 __device__ __forceinline__ PairTile pair_tile(const GemmArgs& g, int tile) {
     int z = 0;
@@ -416,15 +415,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
 
 }  // namespace
 
-int gemm_pair_tiles(const GemmLaunch& L) {
+cudaError_t launch_gemm_pair(const GemmLaunch& L, cudaStream_t stream) {
     int total = 0;
     for (int i = 0; i < L.n_problems; ++i)
         total += pair_tiles_m(L.args.p[i]) * (L.args.p[i].N / pair_out_cols(L.args.p[i]));
-    return total;
-}
-
-cudaError_t launch_gemm_pair(const GemmLaunch& L, cudaStream_t stream) {
-    const int total = gemm_pair_tiles(L);
     const int pairs = sm_count() / 2;
     const dim3 grid(static_cast<unsigned>(2 * (total < pairs ? total : pairs)));
     auto go = [&](auto kern) {

@@ -42,7 +42,7 @@ __host__ __device__ inline int gemm_stage_bytes(int n_tile, bool geglu) {
 // Partial sums of a split tile in shared memory: row-major, four floats of padding per
 // row so that both a thread per row and several threads per row read and write
 // float4 without bank conflicts.
-__host__ __device__ inline int gemm_red_ld(int n_tile, bool geglu) { return (geglu ? 2 : 1) * n_tile + 4; }
+__host__ __device__ inline int gemm_red_ld(int n_tile) { return n_tile + 4; }
 
 template <bool kBf16>
 __device__ __forceinline__ float gemm_ld16(const void* base, long long i) {
@@ -54,10 +54,10 @@ __device__ __forceinline__ float gemm_ld16(const void* base, long long i) {
 // Epilogue of a split tile.  Every CTA of the cluster holds a partial 128 x n_tile sum
 // at the same shared-memory address; this one finishes 128 / split rows, `split`
 // threads to a row with n_tile / split columns (a multiple of eight) each.
-template <bool kBf16, bool kGeglu>
+template <bool kBf16>
 __device__ __forceinline__ void epilogue_split(const GemmProblem& p, cooperative_groups::cluster_group& cluster,
                                                float* red, int split, int part, int tid, int m0, int n0) {
-    const int ld = gemm_red_ld(p.n_tile, kGeglu);
+    const int ld = gemm_red_ld(p.n_tile);
     const int r = part * (128 / split) + tid / split;
     const int per = p.n_tile / split;
     const int row = m0 + r;
@@ -83,17 +83,6 @@ __device__ __forceinline__ void epilogue_split(const GemmProblem& p, cooperative
 #pragma unroll
             for (int i = 0; i < 8; ++i) f[i] += gemm_ld16<kBf16>(p.bias, n0 + c + i);
         }
-        if constexpr (kGeglu) {
-            if (p.geglu_offset > 0) {
-                float gt[8];
-                sum8(p.n_tile + c, gt);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if (p.bias != nullptr) gt[i] += gemm_ld16<kBf16>(p.bias, n0 + p.geglu_offset + c + i);
-                    f[i] *= gelu_exact(gt[i]);
-                }
-            }
-        }
         uint4 w;
         w.x = pack2<kBf16>(f[0], f[1]); w.y = pack2<kBf16>(f[2], f[3]);
         w.z = pack2<kBf16>(f[4], f[5]); w.w = pack2<kBf16>(f[6], f[7]);
@@ -101,7 +90,7 @@ __device__ __forceinline__ void epilogue_split(const GemmProblem& p, cooperative
     }
 }
 
-// One instantiation per epilogue (plain, GEGLU, norm + RoPE; whole or split tiles): the
+// One instantiation per epilogue (plain, GEGLU, norm + RoPE, plain split tiles): the
 // GEGLU and the norm + RoPE code are long, and an epilogue that only branches around them
 // spent more time fetching instructions than storing (5.6 us for one 128 x 128 tile
 // against 2.3 us).
@@ -228,13 +217,11 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         const int n_valid = min(p.n_tile, p.N - n0);      // a ragged last tile stops at the matrix edge
         if constexpr (kSplit) {
             // partial sums to shared memory: the ring is at rest, its last MMA has completed
-            float* rrow = reinterpret_cast<float*>(smem) + (q * 32 + lane) * gemm_red_ld(p.n_tile, kGeglu);
+            float* rrow = reinterpret_cast<float*>(smem) + (q * 32 + lane) * gemm_red_ld(p.n_tile);
 #pragma unroll 1
-            for (int c = 0; ok && c < (kGeglu ? 2 : 1) * p.n_tile; c += 32) {
-                const bool gate = kGeglu && c >= p.n_tile;
-                if (gate && !geglu) break;
+            for (int c = 0; ok && c < p.n_tile; c += 32) {
                 uint32_t v[32];
-                tmem_ld32(tacc + (gate ? 128 + c - p.n_tile : c), v);
+                tmem_ld32(tacc + c, v);
                 tmem_wait_ld();
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
@@ -371,7 +358,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         cg::cluster_group cluster = cg::this_cluster();
         cluster_sync();
         if (warp >= 2)
-            epilogue_split<kBf16, kGeglu>(p, cluster, reinterpret_cast<float*>(smem), split, part,
+            epilogue_split<kBf16>(p, cluster, reinterpret_cast<float*>(smem), split, part,
                                           static_cast<int>(threadIdx.x) - 64, m0, n0);
         cluster_sync_relaxed();      // the peers' shared memory stays until everyone has read it
     }
@@ -388,9 +375,13 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
 
 cudaError_t launch_gemm_tc05(const GemmLaunch& L, cudaStream_t stream) {
     int tn = 0, tm = 0, nt_max = 16, any_geglu = 0, any_norm_rope = 0, k_max = 0;
-    // a CTA without a K block would wait for an accumulator that nobody computes
-    for (int i = 0; i < L.n_problems; ++i)
-        if (L.args.split > gemm_k_blocks(L.args.p[i].K)) return cudaErrorInvalidValue;
+    // a CTA without a K block would wait for an accumulator that nobody computes; the epilogues of GEGLU and
+    // norm + RoPE take whole tiles
+    for (int i = 0; i < L.n_problems; ++i) {
+        const GemmProblem& p = L.args.p[i];
+        if (L.args.split > gemm_k_blocks(p.K) || (L.args.split > 1 && (p.geglu_offset > 0 || p.norm_rope != 0)))
+            return cudaErrorInvalidValue;
+    }
     for (int i = 0; i < L.n_problems; ++i) {
         const GemmProblem& p = L.args.p[i];
         tn = p.tiles_n > tn ? p.tiles_n : tn;
@@ -432,7 +423,6 @@ cudaError_t launch_gemm_tc05(const GemmLaunch& L, cudaStream_t stream) {
     auto pick = [&](auto bf16) {
         constexpr bool kB = decltype(bf16)::value;
         if (any_norm_rope) go(gemm_tc05_kernel<kB, false, true, false>);        // never split
-        else if (any_geglu && args.split > 1) go(gemm_tc05_kernel<kB, true, false, true>);
         else if (any_geglu) go(gemm_tc05_kernel<kB, true, false, false>);
         else if (args.split > 1) go(gemm_tc05_kernel<kB, false, false, true>);
         else go(gemm_tc05_kernel<kB, false, false, false>);

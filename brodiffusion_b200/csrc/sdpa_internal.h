@@ -198,7 +198,6 @@ cudaError_t launch_gemm_tc05(const GemmLaunch& L, cudaStream_t stream);
 // Persistent kernel of CTA pairs and 256 x 256 tiles; every problem of the launch must
 // have whole[i] set.
 cudaError_t launch_gemm_pair(const GemmLaunch& L, cudaStream_t stream);
-int gemm_pair_tiles(const GemmLaunch& L);
 
 // Elementwise helpers.
 cudaError_t launch_add_inplace(void* y, const void* x, long long n, bool bf16, cudaStream_t stream);
@@ -206,7 +205,6 @@ cudaError_t launch_axpby_inplace(void* y, const void* x, long long n, float a, f
                                  cudaStream_t stream);
 cudaError_t launch_add_row_bias(void* y, const void* bias, long long rows, long long cols, long long ld,
                                 bool bf16, cudaStream_t stream);
-
 
 // Device-side RoPE table build.
 constexpr int kMaxRopeSegments = 64;

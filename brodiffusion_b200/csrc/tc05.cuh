@@ -315,8 +315,9 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // The same without ordering memory: for the start (behind fence_mbar_init) and for the end of a
-// kernel, where a CTA only has to outlive its peers' accesses.  The release of the other
-// form waits for the global stores in flight.
+// kernel whose CTAs have waited for every arrival and read every value that comes from a peer, and only
+// have to outlive the peers' accesses to them.  The release of the other form waits for the global
+// stores in flight.
 __device__ __forceinline__ void cluster_sync_relaxed() {
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

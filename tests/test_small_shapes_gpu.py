@@ -127,9 +127,11 @@ def test_head_dims_above_128_values_that_are_not_finite(bd, oracle, storage, hd,
 
 
 # Few output tiles, so that 2, 4 or 8 CTAs share a tile: ragged rows and columns, K not a
-# multiple of a K block, the smallest K that is split and one just below it.
+# multiple of a K block, the smallest K that is split (eleven blocks) and shorter ones that are not
+# (tests/test_gemm_plan.py has the rule).
 @pytest.mark.parametrize("M,N,K", [(64, 1280, 1280), (64, 1280, 5120), (1, 72, 2048), (77, 1280, 768), (130, 200, 1000),
-                                   (256, 3072, 3072), (128, 64, 384), (128, 64, 320), (300, 640, 2560)])
+                                   (256, 3072, 3072), (128, 64, 384), (128, 64, 320), (300, 640, 2560),
+                                   (128, 64, 648), (128, 64, 640)])
 def test_linear_split_over_a_cluster(bd, oracle, M, N, K):
     x, w, b = synth.activations((M, K), 9600 + M), synth.weights((N, K), 9601 + N), synth.weights((N,), 9602)
     for bias in (b, None):
@@ -141,15 +143,16 @@ def test_linear_split_over_a_cluster(bd, oracle, M, N, K):
         assert np.abs(G.host(y) - ref).max() <= np.abs(ref).max() * (2.0 ** -8 + 1e-5)
 
 
+# Few rows: GEGLU is never split, these take 64 columns (the ragged ones) or pairs.
 @pytest.mark.parametrize("B,Din,Dout", [(64, 1280, 5120), (33, 1280, 264), (130, 520, 72)])
-def test_geglu_split_over_a_cluster(bd, oracle, B, Din, Dout):
+def test_geglu_few_rows(bd, oracle, B, Din, Dout):
     x, w = synth.activations((B, Din), 9700, "fp16"), synth.weights((2 * Dout, Din), 9701, "fp16")
     b = synth.weights((2 * Dout,), 9702, "fp16")
     y = torch.full((B, Dout), float("nan"), device="cuda", dtype=torch.float16)
     bd.linear_geglu_fwd(G.dev(x, torch.float16), G.dev(w, torch.float16), G.dev(b, torch.float16), y)
     assert bd.device_status() == 0
     ref = oracle.linear_geglu(x, w, b)
-    assert np.abs(G.host(y) - ref).max() <= 0.01 * np.abs(ref).max() + 0.008   # as for the unsplit kernel
+    assert np.abs(G.host(y) - ref).max() <= 0.01 * np.abs(ref).max() + 0.008   # the reference's own bound
 
 
 # Tiles of 256 x 256 shared by two CTAs: row counts that leave the second CTA empty or
