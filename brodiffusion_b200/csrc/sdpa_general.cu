@@ -13,7 +13,7 @@
 // exponential itself is good to 2^-22.5).
 // Two row tiles per CTA (MT = 2) halve the reads of K and V where there are still
 // enough CTAs for that.
-// 64 x 64 with 8 heads of 160: 4.2 us, 576 x 576: 22.8 us (97 and 840 on the CUDA-core kernel
+// 64 x 64 with 8 heads of 160: 4.2 us, 576 x 576: 22.3 us (97 and 840 on the CUDA-core kernel
 // that stood here before).
 // Same arithmetic as src/dit/common.cpp:246-305 with FP32 scores.
 #include "sdpa_internal.h"

@@ -83,7 +83,7 @@ def test_wide_tile_projection_matches_oracle(bd, oracle):
     rv = oracle.linear(x, wv)
     assert np.abs(G.host(q) - rq).max() < 2.5e-2
     assert np.abs(G.host(k) - rk).max() < 2.5e-2
-    G.check(G.host(v), rv, max_abs=2.5e-2, what="V projection (wide tiles)")
+    G.check(G.host(v), rv, max_abs=2.5e-2, what="V projection (pairs)")
 
 
 @pytest.mark.parametrize("dtype", ["bf16", "f16"])
@@ -101,7 +101,7 @@ def test_wide_tile_linear_matches_oracle(bd, oracle, dtype, hd):
         y = torch.full((rows, N), float("nan"), device="cuda", dtype=tdt)
         bd.linear_fwd(G.dev(x, tdt), G.dev(w, tdt), G.dev(b, tdt), y)
         assert bd.device_status() == 0
-        G.check(G.host(y), oracle.linear(x, w, b), max_abs=2.5e-2, what="linear (wide tiles)")
+        G.check(G.host(y), oracle.linear(x, w, b), max_abs=2.5e-2, what="linear (pairs)")
     else:
         rows, din, nh = 2304, 136, 16
         D = nh * hd

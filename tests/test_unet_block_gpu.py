@@ -116,7 +116,7 @@ def test_linear(bd, oracle):
 def test_fused_linear_geglu(bd, oracle, golden, B, Din, Dout):
     """Reference shapes (tests/test_fused_parity.cpp:268-269) plus the SD1.5
     top-level FF1 (4096, 320) -> 1280 and a ragged case; the last two are large
-    enough for the persistent wide-tile kernel (value + gate tile per MMA)."""
+    enough for the persistent pair kernel (value + gate tile per MMA)."""
     if (B, Din, Dout) == (40, 64, 48):
         x, w, b = golden["geglu_x"], golden["geglu_w"], golden["geglu_b"]
         ref = golden["geglu_y"]
