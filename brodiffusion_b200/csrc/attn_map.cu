@@ -66,7 +66,7 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_free + 2);
     float* ks_s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 128);   // [kMapKeys]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
     const int kt = blockIdx.x, rt = blockIdx.y;
     const int kseg = kt >= a.key_tiles0 ? 1 : 0;
@@ -116,7 +116,7 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
     const int qi = row_base + row;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             const CUtensorMap* tmQ = rseg ? &tmQ1 : &tmQ0;
             const CUtensorMap* tmK = kseg ? &tmK1 : &tmK0;
             bool ok = true;
@@ -143,14 +143,14 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
         __syncwarp();
     } else if (warp == 1) {
         constexpr uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, kMapRows, kMapKeys, 0, 0);
-        bool ok = true;
-        for (int i = 0; ok && i < n_heads; ++i) {
-            const int s = i % kMapStages, b = i & 1;
-            if (i >= 2) ok = mbar_wait(&s_free[b], static_cast<uint32_t>((i / 2 - 1) & 1));
-            if (ok) ok = mbar_wait(&full[s], static_cast<uint32_t>((i / kMapStages) & 1));
-            if (!ok) break;
-            tc_fence_after();
-            if (lane == 0) {
+        if (elect_one()) {
+            bool ok = true;
+            for (int i = 0; ok && i < n_heads; ++i) {
+                const int s = i % kMapStages, b = i & 1;
+                if (i >= 2) ok = mbar_wait(&s_free[b], static_cast<uint32_t>((i / 2 - 1) & 1));
+                if (ok) ok = mbar_wait(&full[s], static_cast<uint32_t>((i / kMapStages) & 1));
+                if (!ok) break;
+                tc_fence_after();
                 const uint32_t qa = smem_u32(smem + s * C::kStageBytes);
                 const uint32_t kb = qa + C::kChunks * kMapQChunk;
 #pragma unroll
@@ -163,8 +163,8 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
                 umma_commit(&empty[s]);
                 umma_commit(&s_full[b]);
             }
-            __syncwarp();
         }
+        __syncwarp();
     } else {
         const uint32_t tS = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
         const bool row_ok = row < rows;

@@ -196,7 +196,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     float* gain_s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);   // [3][128]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -289,16 +289,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             const int chunks = (K + 63) / 64;
             const int as = ti & 1;
             if (ti >= 2) {       // both epilogues must have drained this accumulator (tile ti - 2)
-                ok = mbar_wait(&acc_empty[as], static_cast<uint32_t>(((ti >> 1) - 1) & 1));
+                ok = mbar_wait_warp(&acc_empty[as], static_cast<uint32_t>(((ti >> 1) - 1) & 1));
                 if (!ok) break;
                 tc_fence_after();
             }
             const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(as * kPTile);
             for (int c = 0; c < chunks; c += 2) {
-                ok = mbar_wait(&full[slot], phase);
+                ok = mbar_wait_warp(&full[slot], phase);
                 if (!ok) break;
                 tc_fence_after();
-                if (lane == 0) {
+                // (the lane is elected for each stage: with one thread running the loop GEGLU over
+                // 9216 x 320 -> 1280 takes 28.4 us, this way 26.2)
+                if (elect_one()) {
                     const uint64_t ad = a0 + slot * (kPStageBytes >> 4), bd = b0 + slot * (kPStageBytes >> 4);
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)

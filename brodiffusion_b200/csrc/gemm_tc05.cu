@@ -122,7 +122,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     uint64_t* acc_done = empty + kGemmMaxStages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
     const int k_all = gemm_k_blocks(p.K);
     const int k_begin = kSplit ? gemm_part_begin(k_all, split, part) : 0;
@@ -153,7 +153,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     wait_for_prior_grid();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t bytes = kGemmABytes + (geglu ? 2u : 1u) * static_cast<uint32_t>(p.n_tile) * 128u;
             bool ok = true;
             int issued = 0;
@@ -178,20 +178,20 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         }
         __syncwarp();
     } else if (warp == 1) {
-        // The issuing thread is what a long K loop waits for (with the loads left out it ran no
-        // faster): the slot and its parity are counted on, a division by the runtime ring size
-        // cost more than the four MMAs.
+        // One elected thread runs the whole loop (with the warp in step and the lane elected for each
+        // block 576 x 1280 x 1280 takes 7.3 us, this way 6.5).  The slot and its parity are counted on, a
+        // division by the runtime ring size cost more than the four MMAs.
         const uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, 128, p.n_tile, 0, 0);
         const uint64_t a0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
         const uint64_t b0 = make_smem_desc_sw128(smem_u32(smem) + kGemmABytes, 16, 1024);
         const uint32_t stage_units = static_cast<uint32_t>(kGemmStageBytes) >> 4;   // descriptors count 16 bytes
         const uint32_t gate_units = static_cast<uint32_t>(kGemmBBytes) >> 4;
-        int slot = 0;
-        uint32_t phase = 0;
-        for (int kb = 0; kb < k_blocks; ++kb) {
-            if (!mbar_wait(&full[slot], phase)) break;
-            tc_fence_after();
-            if (lane == 0) {
+        if (elect_one()) {
+            int slot = 0;
+            uint32_t phase = 0;
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!mbar_wait(&full[slot], phase)) break;
+                tc_fence_after();
                 const uint64_t ad = a0 + slot * stage_units, bd = b0 + slot * stage_units;
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) {
@@ -200,10 +200,10 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 }
                 umma_commit(&empty[slot]);
                 if (kb == k_blocks - 1) umma_commit(acc_done);
+                if (++slot == kGemmStages) { slot = 0; phase ^= 1; }
             }
-            __syncwarp();
-            if (++slot == kGemmStages) { slot = 0; phase ^= 1; }
         }
+        __syncwarp();
     } else {
         // epilogue: warp w reads TMEM lanes 32 * (w % 4) ..
         const int q = warp & 3;

@@ -192,7 +192,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_ready + VS);
     uint16_t* tile_list = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(bars) + C::kBarBytes);   // [kMaxListed]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
     const int head = blockIdx.y;
     const int batch = blockIdx.z;
@@ -705,11 +705,11 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
         setmaxnreg_dec<Roles<kScale>::kRegsOther>();
         if (warp == 8) {
             // -------------------------------------------------- Q.K^T issuer
-            // One tcgen05.mma costs its issuing thread 46-59 cycles and the pipe 64, the
-            // queue between them holds about sixteen, and every commit and completed wait
-            // costs another 46-50 cycles of the thread: a single warp issuing both products
-            // of both tiles could not keep the pipe fed, two warps can (65.5 cycles per MMA
-            // measured with a wait and a commit after every eight).
+            // The queue between the issuing thread and the tensor pipe holds about sixteen MMAs, and
+            // every commit and completed wait costs the thread 46-50 cycles: a single warp issuing both
+            // products of both tiles could not keep the pipe fed, two warps can.  All lanes wait (a
+            // wait that runs out is voted on behind the MMAs, where nothing waits for the vote) and one
+            // elected lane of the converged warp issues: see elect_one.
             constexpr uint32_t idesc_qk = make_idesc_f16(kBf16 ? 1 : 0, kBM, kBN, 0, 0);
             const uint32_t q_base = smem_u32(smem_q);
             const uint32_t k_base = smem_u32(smem_k);
@@ -727,9 +727,8 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                     // was that buffer's last user, with two this keeps the tiles in turns
                     if (ok && (j > 0 || t > 0)) ok = mbar_wait(&s_free[t ^ 1], static_cast<uint32_t>((t ? j : j - 1) & 1));
                     if (ok && t == 0) ok = mbar_wait(&k_rdy[slot], phase);
-                    if (!ok) break;
                     tc_fence_after();
-                    if (lane == 0) {
+                    if (elect_one() && ok) {
                         const uint32_t qa = q_base + t * C::kQBytes;
                         const uint32_t kb = k_base + slot * C::kTileBytes;
                         const uint32_t d = tmem_base + (t ? C::kColS1 : C::kColS0);
@@ -742,7 +741,8 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                         umma_commit(&s_full[t]);
                         if (t == 1) umma_commit(&k_empty[slot]);
                     }
-                    __syncwarp();
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
                 }
                 if (++slot == KS) { slot = 0; phase ^= 1; }
             }
@@ -758,9 +758,8 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                 ok = mbar_wait(&v_rdy[slot], phase);
                 for (int t = 0; t < 2; ++t) {
                     if (ok) ok = mbar_wait(&p_full[t], static_cast<uint32_t>(j & 1));
-                    if (!ok) break;
                     tc_fence_after();
-                    if (lane == 0) {
+                    if (elect_one() && ok) {
                         const uint32_t vb = v_base + slot * C::kTileBytes;
                         const uint32_t d = tmem_base + (t ? C::kColO1 : C::kColO0);
                         const uint32_t p = tmem_base + (t ? C::kColP1 : C::kColP0);
@@ -772,7 +771,8 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                         umma_commit(&pv_done[t]);
                         if (t == 1) umma_commit(&v_empty[slot]);
                     }
-                    __syncwarp();
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
                 }
                 if (++slot == VS) { slot = 0; phase ^= 1; }
             }
