@@ -16,9 +16,13 @@
 //     reads few weight and few activation tiles);
 //   * the accumulator is double-buffered in tensor memory (2 x 256 columns), so the epilogue
 //     of tile i (bias, RMSNorm, RoPE, stores) runs while the MMAs of tile i+1 are issued;
-//   * the cos / sin rows and the outputs go through 4 KB of shared memory per epilogue warp, so
+//   * the cos / sin rows and the outputs go through 2 KB of shared memory per epilogue warp, so
 //     that global accesses are whole row pieces (a load or store with a row per lane touches 32
-//     cache lines; the exposed last epilogue of a short prompt's projections took ten of 30 us).
+//     cache lines), and everything the epilogue reads from global memory is on its way before it is
+//     needed: the bias in shared memory and the first table rows in registers before the
+//     accumulator is ready, the next rows while a piece is worked on.  With bias values and table rows
+//     loaded where they are used the epilogue of norm + RoPE took 19300 cycles a tile, 10 of the 31 us of
+//     a 256-row prompt's projections, where the last one has nothing to hide behind.
 // GEGLU (src/fused_transformer.cu:89-92,275-282) runs here too: a tile is then 128 value
 // columns + their 128 gate columns (the first CTA stages the value rows of the weight, the
 // second the gate rows), one MMA computes both and the epilogue stores
@@ -40,7 +44,7 @@ constexpr int kPTile = 256;                   // rows and accumulator columns of
 constexpr int kPChunk = 128 * 64 * 2;         // 128 rows x 64 columns: one TMA box of A or B
 // A stage of a CTA: two chunks (128 columns of K) of its 128 rows of A, two of its 128 weight rows
 constexpr int kPStageBytes = 4 * kPChunk;
-constexpr int kPStgBytes = 4096;              // staging of one epilogue warp
+constexpr int kPStgBytes = 2048 + 512;        // one epilogue warp: staging, and 128 bias values as FP32
 constexpr int kPSmemBytes = kPStages * kPStageBytes + 8 * kPStgBytes + 256 + 3 * 128 * 4 + 1024;
 static_assert(kPSmemBytes <= 227 * 1024, "shared memory of one CTA");
 constexpr int kPGroup = 16;                   // row blocks of a group
@@ -84,97 +88,139 @@ __device__ __forceinline__ float load16(const void* base, long long i) {
                  : __half2float(*reinterpret_cast<const __half*>(&b));
 }
 
-// Epilogue of a tile that holds 256 / HD whole heads; this thread owns one
-// token's row of each: RMSNorm over the head and the rotary embedding are
-// thread-local (src/dit/flux.cpp:462-469, src/dit/common.cpp:192-193).  Two
-// passes over the accumulator (tensor memory reads are cheap): sum of squares
-// per head first, then 32 columns at a time so that one load of the token's
-// cos / sin serves every head of the tile.  gain_s: the HD gains in shared
-// memory as FP32, or null for no RMSNorm.  row0: the warp's first row; c0: the
-// first of the 128 output columns it takes.
-template <int HD, bool kBf16>
-__device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t tacc, int row0, int c0,
-                                               const float* gain_s, uint8_t* stg, int lane) {
-    constexpr int kHeads = kPTile / HD / 2;
-    const int rows = min(32, p.M - row0);
-    uint16_t* cbase = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row0) * p.ldc + c0;
-    float inv[kHeads];
+// The cos / sin values of 32 rows and 16 pairs, spread over a warp: lane -> (row lane / 4 of a group of eight,
+// 16-byte piece lane % 4).
+struct TablePiece {
+    float4 c[4], s[4];
+    __device__ __forceinline__ void load(const GemmProblem& p, int half_hd, int row0, int rows, int first_pair, int lane) {
+        const long long at = static_cast<long long>(p.rope_row0 + row0 + (lane >> 2)) * half_hd + first_pair + (lane & 3) * 4;
 #pragma unroll
-    for (int h = 0; h < kHeads; ++h) inv[h] = 1.0f;
-    if (gain_s != nullptr) {
+        for (int i = 0; i < 4; ++i) {
+            if (i * 8 + (lane >> 2) < rows) {
+                c[i] = __ldg(reinterpret_cast<const float4*>(p.cos + at + static_cast<long long>(i * 8) * half_hd));
+                s[i] = __ldg(reinterpret_cast<const float4*>(p.sin + at + static_cast<long long>(i * 8) * half_hd));
+            } else {
+                c[i] = s[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        }
+    }
+    // This lane's own row, through 2 KB of shared memory: sixteen rows at a time.
+    __device__ __forceinline__ void rows_of_lanes(uint8_t* stg, int lane, float (&cs)[16], float (&sn)[16]) const {
+        const int tr = lane >> 2, tq = lane & 3;
 #pragma unroll
-        for (int h = 0; h < kHeads; ++h) {
-            float ss0 = 0.0f, ss1 = 0.0f;
-#pragma unroll 1
-            for (int c = 0; c < HD / 32; ++c) {
-                uint32_t v[32];
-                tmem_ld32(tacc + h * HD + c * 32, v);
-                tmem_wait_ld();
+        for (int h = 0; h < 2; ++h) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float x0 = __uint_as_float(v[i]), x1 = __uint_as_float(v[i + 1]);
-                    if (p.bias != nullptr) {
-                        x0 += load16<kBf16>(p.bias, c0 + h * HD + c * 32 + i);
-                        x1 += load16<kBf16>(p.bias, c0 + h * HD + c * 32 + i + 1);
-                    }
-                    ss0 = fmaf(x0, x0, ss0);
-                    ss1 = fmaf(x1, x1, ss1);
+            for (int i = 0; i < 2; ++i) {
+                uint8_t* const row = stg + (i * 8 + tr) * 128;
+                *reinterpret_cast<float4*>(row + ((tq ^ tr) << 4)) = c[2 * h + i];
+                *reinterpret_cast<float4*>(row + (((tq + 4) ^ tr) << 4)) = s[2 * h + i];
+            }
+            __syncwarp();
+            if ((lane >> 4) == h) {
+                const uint8_t* const row = stg + (lane & 15) * 128;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float4 a = *reinterpret_cast<const float4*>(row + ((i ^ (lane & 7)) << 4));
+                    const float4 b = *reinterpret_cast<const float4*>(row + (((i + 4) ^ (lane & 7)) << 4));
+                    cs[4 * i] = a.x; cs[4 * i + 1] = a.y; cs[4 * i + 2] = a.z; cs[4 * i + 3] = a.w;
+                    sn[4 * i] = b.x; sn[4 * i + 1] = b.y; sn[4 * i + 2] = b.z; sn[4 * i + 3] = b.w;
                 }
             }
-            inv[h] = rsqrtf((ss0 + ss1) / static_cast<float>(HD) + p.eps);
+            __syncwarp();
+        }
+    }
+};
+
+// v + bias of N columns (bias in shared memory, read by all lanes alike).
+template <int N>
+__device__ __forceinline__ void add_bias(const uint32_t (&v)[N], const float* bias_w, float (&f)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+        const float4 b = *reinterpret_cast<const float4*>(bias_w + i);
+        f[i] = __uint_as_float(v[i]) + b.x;
+        f[i + 1] = __uint_as_float(v[i + 1]) + b.y;
+        f[i + 2] = __uint_as_float(v[i + 2]) + b.z;
+        f[i + 3] = __uint_as_float(v[i + 3]) + b.w;
+    }
+}
+
+// Epilogue of 128 columns of a tile of whole heads, one of 128 columns or two of 64; this thread owns one
+// token's row of them: RMSNorm over the head and the rotary embedding are
+// thread-local (src/dit/flux.cpp:462-469, src/dit/common.cpp:192-193).  Two
+// passes over the accumulator (tensor memory reads are cheap): sum of squares
+// per head first, then 32 columns at a time.  One loop for both head dims: two instantiations do not
+// fit the registers.  gain_s: the gains of a head in shared
+// memory as FP32, or null for no RMSNorm.  row0: the warp's first row; cbase: its first
+// output element; bias_w: the bias of its columns; tab: the table values of the first 32
+// columns of a head, where there is RoPE.
+template <bool kBf16>
+__device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t tacc, int row0, uint16_t* cbase,
+                                               const float* gain_s, const float* bias_w, uint8_t* stg, TablePiece& tab,
+                                               int lane) {
+    const int rows = min(32, p.M - row0);
+    const int hd = p.n_tile;
+    float inv0 = 1.0f, inv1 = 1.0f;
+    if (gain_s != nullptr) {
+        float ss0 = 0.0f, ss1 = 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < 128; c += 32) {
+            uint32_t v[32];
+            tmem_ld32(tacc + c, v);
+            tmem_wait_ld();
+            float f[32];
+            add_bias(v, bias_w + c, f);
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+                ss0 = fmaf(f[i], f[i], ss0);
+                ss1 = fmaf(f[i + 1], f[i + 1], ss1);
+            }
+            if (((c + 32) & (hd - 1)) == 0) {          // the head's last columns
+                const float inv = rsqrtf((ss0 + ss1) / static_cast<float>(hd) + p.eps);
+                if (c < hd) inv0 = inv;
+                else inv1 = inv;
+                ss0 = ss1 = 0.0f;
+            }
         }
     }
     const bool rope = p.cos != nullptr;
-    // lane -> (row lane / 4 of a group of eight, 16-byte piece lane % 4) for the table rows
-    const int tr = lane >> 2, tq = lane & 3;
-    const long long tb = static_cast<long long>(p.rope_row0 + row0) * (HD / 2) + tq * 4;
 #pragma unroll 1
-    for (int c = 0; c < HD / 32; ++c) {
+    for (int c = 0; c < 128; c += 32) {
+        const float inv = c < hd ? inv0 : inv1;
+        const float* const gain_c = gain_s + (c & (hd - 1));
         float cs[16], sn[16];
-        if (rope) {
+        if (rope) tab.rows_of_lanes(stg, lane, cs, sn);
+        // sixteen columns at a time: with 32 the registers do not suffice
+        uint32_t packed[16];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = i * 8 + tr;
-                if (r < rows) {
-                    const float4 a = __ldg(reinterpret_cast<const float4*>(p.cos + tb + static_cast<long long>(r) * (HD / 2) + c * 16));
-                    const float4 b = __ldg(reinterpret_cast<const float4*>(p.sin + tb + static_cast<long long>(r) * (HD / 2) + c * 16));
-                    *reinterpret_cast<float4*>(stg + r * 128 + ((tq ^ (r & 7)) << 4)) = a;
-                    *reinterpret_cast<float4*>(stg + r * 128 + (((tq + 4) ^ (r & 7)) << 4)) = b;
-                }
-            }
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 a = *reinterpret_cast<const float4*>(stg + lane * 128 + ((i ^ (lane & 7)) << 4));
-                const float4 b = *reinterpret_cast<const float4*>(stg + lane * 128 + (((i + 4) ^ (lane & 7)) << 4));
-                cs[4 * i] = a.x; cs[4 * i + 1] = a.y; cs[4 * i + 2] = a.z; cs[4 * i + 3] = a.w;
-                sn[4 * i] = b.x; sn[4 * i + 1] = b.y; sn[4 * i + 2] = b.z; sn[4 * i + 3] = b.w;
-            }
-            __syncwarp();
-        }
-#pragma unroll
-        for (int h = 0; h < kHeads; ++h) {
-            uint32_t v[32];
-            tmem_ld32(tacc + h * HD + c * 32, v);
+        for (int hf = 0; hf < 2; ++hf) {
+            uint32_t v[16];
+            tmem_ld16(tacc + c + hf * 16, v);
             tmem_wait_ld();
-            float f[32];
+            float f[16];
+            add_bias(v, bias_w + c + hf * 16, f);
+            if (gain_s != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                float x = __uint_as_float(v[i]);
-                if (p.bias != nullptr) x += load16<kBf16>(p.bias, c0 + h * HD + c * 32 + i);
-                if (gain_s != nullptr) x *= inv[h] * gain_s[c * 32 + i];
-                f[i] = x;
+                for (int i = 0; i < 16; i += 4) {
+                    const float4 g = *reinterpret_cast<const float4*>(gain_c + hf * 16 + i);
+                    f[i] *= inv * g.x;
+                    f[i + 1] *= inv * g.y;
+                    f[i + 2] *= inv * g.z;
+                    f[i + 3] *= inv * g.w;
+                }
             }
             if (rope) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
+                for (int i = 0; i < 8; ++i) {
                     const float a0 = f[2 * i], b0 = f[2 * i + 1];
-                    f[2 * i] = a0 * cs[i] - b0 * sn[i];
-                    f[2 * i + 1] = a0 * sn[i] + b0 * cs[i];
+                    f[2 * i] = a0 * cs[hf * 8 + i] - b0 * sn[hf * 8 + i];
+                    f[2 * i + 1] = a0 * sn[hf * 8 + i] + b0 * cs[hf * 8 + i];
                 }
             }
-            store_tile32<kBf16>(f, stg, lane, cbase + h * HD + c * 32, p.ldc, rows, 32);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) packed[hf * 8 + i] = pack2<kBf16>(f[2 * i], f[2 * i + 1]);
         }
+        if (rope && c < 96) tab.load(p, hd >> 1, row0, rows, ((c + 32) & (hd - 1)) >> 1, lane);
+        store_words32(packed, stg, lane, cbase + c, p.ldc, rows, 32);
     }
 }
 
@@ -214,9 +260,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         tmem_alloc_pair(tmem_slot, 512);
         tmem_relinquish_pair();
     }
+    // The first tile of this pair: found before the wait for the kernel before this one, so that the first
+    // look at the problems in the parameters is behind it too.
+    const int rank = static_cast<int>(cluster_ctarank());
+    const int pairs = static_cast<int>(gridDim.x) >> 1;
+    const int first_tile = static_cast<int>(blockIdx.x) >> 1;
+    const PairTile first = pair_tile(g, first_tile);
     if (warp == 0 && lane == 0) {
-        tma_prefetch_desc(&tmA0);
-        tma_prefetch_desc(&tmB0);
+        tma_prefetch_desc(first.z == 0 ? &tmA0 : (first.z == 1 ? &tmA1 : &tmA2));
+        tma_prefetch_desc(first.z == 0 ? &tmB0 : (first.z == 1 ? &tmB1 : &tmB2));
     }
     tc_fence_before();
     __syncthreads();
@@ -227,9 +279,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     dependents_may_launch();
     // barriers, tensor memory and descriptors are set up; from here on global memory is touched
     wait_for_prior_grid();
-    const int rank = static_cast<int>(cluster_ctarank());
-    const int pairs = static_cast<int>(gridDim.x) >> 1;
-    const int first_tile = static_cast<int>(blockIdx.x) >> 1;
 
     if (warp == 0) {
         // ---------------------------------------------------- TMA producer
@@ -241,7 +290,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             uint32_t phase = 1;  // parity that a fresh barrier passes
             bool ok = true;
             for (int tile = first_tile; ok && tile < total_tiles; tile += pairs) {
-                const PairTile t = pair_tile(g, tile);
+                const PairTile t = tile == first_tile ? first : pair_tile(g, tile);
                 const CUtensorMap* tmA = t.z == 0 ? &tmA0 : (t.z == 1 ? &tmA1 : &tmA2);
                 const CUtensorMap* tmB = t.z == 0 ? &tmB0 : (t.z == 1 ? &tmB1 : &tmB2);
                 const int K = t.z == 0 ? g.p[0].K : (t.z == 1 ? g.p[1].K : g.p[2].K);
@@ -284,7 +333,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         int ti = 0;              // tiles done by this pair
         bool ok = rank == 0;
         for (int tile = first_tile; ok && tile < total_tiles; tile += pairs, ++ti) {
-            const PairTile t = pair_tile(g, tile);
+            const PairTile t = tile == first_tile ? first : pair_tile(g, tile);
             const int K = t.z == 0 ? g.p[0].K : (t.z == 1 ? g.p[1].K : g.p[2].K);
             const int chunks = (K + 63) / 64;
             const int as = ti & 1;
@@ -336,10 +385,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         int ti = 0;
         bool ok = true;
         for (int tile = first_tile; tile < total_tiles; tile += pairs, ++ti) {
-            const PairTile t = pair_tile(g, tile);
+            const PairTile t = tile == first_tile ? first : pair_tile(g, tile);
             const GemmProblem& p = t.z == 0 ? g.p[0] : (t.z == 1 ? g.p[1] : g.p[2]);
             const int as = ti & 1;
-            if (!p.norm_rope) {
+            const int row0 = t.m0 + rank * 128 + q * 32;
+            const int rows = min(32, p.M - row0);
+            // a projection without norm and RoPE (V) has nothing but its bias to add
+            const bool heads = p.norm_rope && (p.gain != nullptr || p.cos != nullptr);
+            {
                 // the 128 bias values this warp needs (GEGLU: 64 and those of their gates), fetched
                 // while the tile is computed
                 const int lc = lane * 4;
@@ -353,35 +406,41 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 *reinterpret_cast<float4*>(bias_w + lc) = b;
                 __syncwarp();
             }
+            TablePiece tab;
+            if (heads && p.cos != nullptr && rows > 0) tab.load(p, p.n_tile >> 1, row0, rows, 0, lane);
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[as], static_cast<uint32_t>((ti >> 1) & 1)));
             if (!ok) break;
             tc_fence_after();
-            const int row0 = t.m0 + rank * 128 + q * 32;
-            const int rows = min(32, p.M - row0);
             const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(as * kPTile);
             uint16_t* cbase = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row0) * p.ldc + t.n0;
             if (rows <= 0) {
                 // rows past the matrix: nothing to store
-            } else if (p.norm_rope) {
+            } else if (heads) {
                 const float* gs = p.gain != nullptr ? gain_s + t.z * 128 : nullptr;
                 const int c0 = half * (kPTile / 2);
-                if (p.n_tile == 128) epilogue_heads<128, kBf16>(p, tacc + c0, row0, t.n0 + c0, gs, stg, lane);
-                else epilogue_heads<64, kBf16>(p, tacc + c0, row0, t.n0 + c0, gs, stg, lane);
+                epilogue_heads<kBf16>(p, tacc + c0, row0, cbase + c0, gs, bias_w, stg, tab, lane);
             } else if (p.geglu_offset > 0) {
                 // value in accumulator columns [0, 128), gate in [128, 256); this group
                 // stores 64 of the tile's 128 output columns
 #pragma unroll 1
                 for (int c = half * 64; c < half * 64 + 64; c += 32) {
-                    uint32_t v[32], gt[32];
-                    tmem_ld32(tacc + c, v);
-                    tmem_ld32(tacc + 128 + c, gt);
-                    tmem_wait_ld();
                     const float* bv = bias_w + (c - half * 64);
-                    float f[32];
+                    uint32_t packed[16];
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        f[i] = (__uint_as_float(v[i]) + bv[i]) * gelu_exact(__uint_as_float(gt[i]) + bv[64 + i]);
-                    store_tile32<kBf16>(f, stg, lane, cbase + c, p.ldc, rows, 32);
+                    for (int hf = 0; hf < 2; ++hf) {
+                        uint32_t v[16], gt[16];
+                        tmem_ld16(tacc + c + hf * 16, v);
+                        tmem_ld16(tacc + 128 + c + hf * 16, gt);
+                        tmem_wait_ld();
+                        float f[16], gate[16];
+                        add_bias(v, bv + hf * 16, f);
+                        add_bias(gt, bv + 64 + hf * 16, gate);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            packed[hf * 8 + i] = pack2<kBf16>(f[2 * i] * gelu_exact(gate[2 * i]),
+                                                              f[2 * i + 1] * gelu_exact(gate[2 * i + 1]));
+                    }
+                    store_words32(packed, stg, lane, cbase + c, p.ldc, rows, 32);
                 }
             } else {
 #pragma unroll 1
@@ -389,10 +448,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                     uint32_t v[32];
                     tmem_ld32(tacc + c, v);
                     tmem_wait_ld();
-                    const float* bv = bias_w + (c - half * (kPTile / 2));
                     float f[32];
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]) + bv[i];
+                    add_bias(v, bias_w + (c - half * (kPTile / 2)), f);
                     store_tile32<kBf16>(f, stg, lane, cbase + c, p.ldc, rows, 32);
                 }
             }

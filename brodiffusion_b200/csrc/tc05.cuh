@@ -310,7 +310,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
           "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -533,22 +533,16 @@ __device__ __forceinline__ void load32_as_float(const void* base, long long i, f
     }
 }
 
-// Stores a warp's 32 x 32 tile (thread = row) as 16-bit values: through `stg` (2 KB of this
+// Stores a warp's 32 x 32 tile (thread = row) of 16-bit values, two to a word: through `stg` (2 KB of this
 // warp's shared memory), so that four lanes write 64 consecutive bytes of a row.  Straight
 // from the registers a store instruction touches 32 rows, 32 cache lines.
 // base: element (first row, first column); rows / cols: how many of each exist.
-template <bool kBf16>
-__device__ __forceinline__ void store_tile32(const float (&f)[32], uint8_t* stg, int lane, uint16_t* base,
-                                             long long ld, int rows, int cols) {
+__device__ __forceinline__ void store_words32(const uint32_t (&w)[16], uint8_t* stg, int lane, uint16_t* base,
+                                              long long ld, int rows, int cols) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        uint4 w;
-        w.x = pack2<kBf16>(f[c * 8 + 0], f[c * 8 + 1]);
-        w.y = pack2<kBf16>(f[c * 8 + 2], f[c * 8 + 3]);
-        w.z = pack2<kBf16>(f[c * 8 + 4], f[c * 8 + 5]);
-        w.w = pack2<kBf16>(f[c * 8 + 6], f[c * 8 + 7]);
-        *reinterpret_cast<uint4*>(stg + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = w;
-    }
+    for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<uint4*>(stg + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
+            make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
     __syncwarp();
     const int c = lane & 3;
 #pragma unroll
@@ -559,6 +553,14 @@ __device__ __forceinline__ void store_tile32(const float (&f)[32], uint8_t* stg,
                 *reinterpret_cast<const uint4*>(stg + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
     }
     __syncwarp();
+}
+template <bool kBf16>
+__device__ __forceinline__ void store_tile32(const float (&f)[32], uint8_t* stg, int lane, uint16_t* base,
+                                             long long ld, int rows, int cols) {
+    uint32_t w[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) w[i] = pack2<kBf16>(f[2 * i], f[2 * i + 1]);
+    store_words32(w, stg, lane, base, ld, rows, cols);
 }
 
 }  // namespace bdattn
