@@ -131,19 +131,6 @@ struct TablePiece {
     }
 };
 
-// v + bias of N columns (bias in shared memory, read by all lanes alike).
-template <int N>
-__device__ __forceinline__ void add_bias(const uint32_t (&v)[N], const float* bias_w, float (&f)[N]) {
-#pragma unroll
-    for (int i = 0; i < N; i += 4) {
-        const float4 b = *reinterpret_cast<const float4*>(bias_w + i);
-        f[i] = __uint_as_float(v[i]) + b.x;
-        f[i + 1] = __uint_as_float(v[i + 1]) + b.y;
-        f[i + 2] = __uint_as_float(v[i + 2]) + b.z;
-        f[i + 3] = __uint_as_float(v[i + 3]) + b.w;
-    }
-}
-
 // Epilogue of 128 columns of a tile of whole heads, one of 128 columns or two of 64; this thread owns one
 // token's row of them: RMSNorm over the head and the rotary embedding are
 // thread-local (src/dit/flux.cpp:462-469, src/dit/common.cpp:192-193).  Two

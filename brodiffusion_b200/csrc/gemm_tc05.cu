@@ -29,6 +29,7 @@ namespace bdattn {
 namespace {
 
 constexpr int kGemmThreads = 192;
+constexpr int kGemmPrefetch = 20;            // K blocks whose weights are asked for ahead
 constexpr int kGemmMaxStages = 8;
 constexpr int kGemmABytes = 128 * 64 * 2;   // A stage
 // A B (or gate) tile is n_tile rows x 128 B; a stage holds A, B and, for GEGLU,
@@ -52,41 +53,48 @@ __device__ __forceinline__ float gemm_ld16(const void* base, long long i) {
 }
 
 // Epilogue of a split tile.  Every CTA of the cluster holds a partial 128 x n_tile sum
-// at the same shared-memory address; this one finishes 128 / split rows, `split`
-// threads to a row with n_tile / split columns (a multiple of eight) each.
+// at the same shared-memory address; this one finishes every split-th row, eight columns to a thread, so that the
+// rows that exist are spread over the cluster and eight threads read and write a whole row piece, and asks for
+// all partial sums of a piece before it adds the first (a thread walking the columns of a row, one remote read
+// behind the other, took 2 to 4 us; with the bias ahead 64 x 1280 x 1280 over four 5.3 -> 4.7 us, 1024 x 640 x 2560
+// over two 13.4 -> 11.5).
 template <bool kBf16>
 __device__ __forceinline__ void epilogue_split(const GemmProblem& p, cooperative_groups::cluster_group& cluster,
-                                               float* red, int split, int part, int tid, int m0, int n0) {
+                                               float* red, const float* bias_s, int split, int part, int tid, int m0, int n0) {
     const int ld = gemm_red_ld(p.n_tile);
-    const int r = part * (128 / split) + tid / split;
-    const int per = p.n_tile / split;
-    const int row = m0 + r;
-    const int c_first = (tid % split) * per;
-    if (row >= p.M) return;
-    auto sum8 = [&](int c, float (&f)[8]) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = 0.0f;
-        for (int k = 0; k < split; ++k) {
-            const float4* src = reinterpret_cast<const float4*>(cluster.map_shared_rank(red, k) + r * ld + c);
-            const float4 u = src[0], v = src[1];
-            f[0] += u.x; f[1] += u.y; f[2] += u.z; f[3] += u.w;
-            f[4] += v.x; f[5] += v.y; f[6] += v.z; f[7] += v.w;
-        }
-    };
-    uint16_t* crow = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row) * p.ldc + n0;
+    const int units = p.n_tile / 8;
     const int n_valid = min(p.n_tile, p.N - n0);           // a multiple of eight
-    for (int c = c_first; c < c_first + per; c += 8) {
-        if (c >= n_valid) break;
-        float f[8];
-        sum8(c, f);
-        if (p.bias != nullptr) {
+    const int rows = min(128, p.M - m0);
+    const float* src[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] += gemm_ld16<kBf16>(p.bias, n0 + c + i);
+    for (int k = 0; k < 8; ++k) src[k] = cluster.map_shared_rank(red, min(k, split - 1));
+#pragma unroll 2
+    for (int i = tid; i < 128 / split * units; i += 128) {
+        const int r = part + split * (i / units), c = i % units * 8;
+        if (r >= rows || c >= n_valid) continue;
+        float4 u[8], v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k < split) {
+                const float4* at = reinterpret_cast<const float4*>(src[k] + r * ld + c);
+                u[k] = at[0];
+                v[k] = at[1];
+            }
         }
+        float f[8] = {};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k < split) {
+                f[0] += u[k].x; f[1] += u[k].y; f[2] += u[k].z; f[3] += u[k].w;
+                f[4] += v[k].x; f[5] += v[k].y; f[6] += v[k].z; f[7] += v[k].w;
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] += bias_s[c + e];
         uint4 w;
         w.x = pack2<kBf16>(f[0], f[1]); w.y = pack2<kBf16>(f[2], f[3]);
         w.z = pack2<kBf16>(f[4], f[5]); w.w = pack2<kBf16>(f[6], f[7]);
-        *reinterpret_cast<uint4*>(crow + c) = w;
+        *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(m0 + r) * p.ldc + n0 + c) = w;
     }
 }
 
@@ -121,6 +129,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     uint64_t* empty = bars + kGemmMaxStages;
     uint64_t* acc_done = empty + kGemmMaxStages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+    float* bias_s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);    // [128] and [128] of the gate
 
     const int warp = warp_index();
     const int lane = threadIdx.x & 31;
@@ -150,6 +159,15 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     const uint32_t tmem_base = *tmem_slot;
     // only now: a dependent CTA that took tensor memory first could keep this one from getting its own
     if (!kNormRope || g.one_wave) dependents_may_launch();
+    // While the kernel before this one ends, this tile's weights come into the L2 (its activations may still
+    // be being written): once for the row tiles that share them (the eleven calls of a 64-token block of 1280
+    // channels, weights cold, 62.2 -> 59.4 us).
+    if (warp == 0 && tile_m == 0 && elect_one()) {
+        for (int kb = 0; kb < k_blocks && kb < kGemmPrefetch; ++kb) {
+            tma_prefetch_l2_2d(tmB, (k_begin + kb) * 64, n0);
+            if (geglu) tma_prefetch_l2_2d(tmB, (k_begin + kb) * 64, n0 + p.geglu_offset);
+        }
+    }
     wait_for_prior_grid();
 
     if (warp == 0) {
@@ -208,6 +226,15 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         // epilogue: warp w reads TMEM lanes 32 * (w % 4) ..
         const int q = warp & 3;
         const int row = m0 + q * 32 + lane;
+        if constexpr (!kNormRope) {
+            // the tile's bias, zero where there is none, while the tile is computed
+            const int t = static_cast<int>(threadIdx.x) - 64;
+            const bool on = p.bias != nullptr && t < p.n_tile && n0 + t < p.N;
+            bias_s[t] = on ? gemm_ld16<kBf16>(p.bias, n0 + t) : 0.0f;
+            if constexpr (kGeglu)
+                bias_s[128 + t] = on && geglu ? gemm_ld16<kBf16>(p.bias, static_cast<long long>(n0) + p.geglu_offset + t) : 0.0f;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
         bool ok = mbar_wait(acc_done, 0);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
@@ -304,48 +331,15 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 tmem_ld32(tacc + c, v);
                 if (geglu) tmem_ld32(tacc + 128 + c, gt);
                 tmem_wait_ld();
-                // the 32 bias values of this piece (and of its gate), zero where there is none
-                float bx[32], bg[kGeglu ? 32 : 1];
-                const bool whole = c + 32 <= n_valid;
-                if (p.bias != nullptr && whole) {
-                    load32_as_float<kBf16>(p.bias, n0 + c, bx);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        bx[i] = 0.0f;
-                        if (p.bias != nullptr && c + i < n_valid) {
-                            const uint16_t b = reinterpret_cast<const uint16_t*>(p.bias)[n0 + c + i];
-                            bx[i] = kBf16 ? __uint_as_float(static_cast<uint32_t>(b) << 16)
-                                          : __half2float(*reinterpret_cast<const __half*>(&b));
-                        }
-                    }
-                }
-                if constexpr (kGeglu) {
-                    if (p.bias != nullptr && geglu && whole) {
-                        load32_as_float<kBf16>(p.bias, n0 + p.geglu_offset + c, bg);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            bg[i] = 0.0f;
-                            if (p.bias != nullptr && geglu && c + i < n_valid) {
-                                const uint16_t b = reinterpret_cast<const uint16_t*>(p.bias)[n0 + p.geglu_offset + c + i];
-                                bg[i] = kBf16 ? __uint_as_float(static_cast<uint32_t>(b) << 16)
-                                              : __half2float(*reinterpret_cast<const __half*>(&b));
-                            }
-                        }
-                    }
-                }
                 float f[32];
+                add_bias(v, bias_s + c, f);
+                if constexpr (kGeglu) {
+                    if (geglu) {
+                        float gate[32];
+                        add_bias(gt, bias_s + 128 + c, gate);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    float x = __uint_as_float(v[i]) + bx[i];
-                    if constexpr (kGeglu) {
-                        if (geglu) {
-                            const float gate = __uint_as_float(gt[i]) + bg[i];
-                            x *= gelu_exact(gate);
-                        }
+                        for (int i = 0; i < 32; ++i) f[i] *= gelu_exact(gate[i]);
                     }
-                    f[i] = x;
                 }
                 // (the ring is at rest, its last MMA has completed: it holds the staging)
                 store_tile32<kBf16>(f, smem + q * 2048, lane, crow0 + c, p.ldc, p.M - m0 - q * 32, n_valid - c);
@@ -358,8 +352,8 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         cg::cluster_group cluster = cg::this_cluster();
         cluster_sync();
         if (warp >= 2)
-            epilogue_split<kBf16>(p, cluster, reinterpret_cast<float*>(smem), split, part,
-                                          static_cast<int>(threadIdx.x) - 64, m0, n0);
+            epilogue_split<kBf16>(p, cluster, reinterpret_cast<float*>(smem), bias_s, split, part,
+                                  static_cast<int>(threadIdx.x) - 64, m0, n0);
         cluster_sync_relaxed();      // the peers' shared memory stays until everyone has read it
     }
 
@@ -410,7 +404,7 @@ cudaError_t launch_gemm_tc05(const GemmLaunch& L, cudaStream_t stream) {
         // so that one CTA's epilogue runs under the others' loads (4096 x 320 -> 960: 18.1 -> 12.2 us).
         args.stages = 2;
     }
-    const int smem = args.stages * stage + 256 + 1024;
+    const int smem = args.stages * stage + 256 + 1024 + 1024;    // barriers, bias, alignment
     const dim3 grid(static_cast<unsigned>(tn), static_cast<unsigned>(tm),
                     static_cast<unsigned>(L.n_problems * args.split));
     cudaError_t e = cudaSuccess;

@@ -254,6 +254,14 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
         : "memory");
 }
 
+// Asks for a box to be brought into the L2, where every later access sees it, whoever wrote it last: so this may
+// run ahead of wait_for_prior_grid().
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
+                 ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y)
+                 : "memory");
+}
+
 // ---------------------------------------------------------- tensor memory
 // Allocate ncols (power of two, 32..512) TMEM columns; the base address is
 // written to *smem_slot.  Executed by one full warp.
@@ -503,33 +511,16 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     return r;
 }
 
-// 32 consecutive 16-bit values from element i of `base` as floats: four 16-byte loads
-// when the address allows (every lane of a warp reads the same words: a broadcast), else
-// one load per value.
-template <bool kBf16>
-__device__ __forceinline__ void load32_as_float(const void* base, long long i, float (&out)[32]) {
-    const uint16_t* p = reinterpret_cast<const uint16_t*>(base) + i;
-    auto widen = [](uint32_t h) {
-        if constexpr (kBf16) return __uint_as_float(h << 16);
-        else {
-            const uint16_t b = static_cast<uint16_t>(h);
-            return __half2float(*reinterpret_cast<const __half*>(&b));
-        }
-    };
-    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+// v + bias of N columns (bias in shared memory, read by all lanes alike).
+template <int N>
+__device__ __forceinline__ void add_bias(const uint32_t (&v)[N], const float* bias_w, float (&f)[N]) {
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const uint4 w = __ldg(reinterpret_cast<const uint4*>(p) + v);
-            const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                out[v * 8 + 2 * e] = widen(ws[e] & 0xffffu);
-                out[v * 8 + 2 * e + 1] = widen(ws[e] >> 16);
-            }
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) out[e] = widen(__ldg(p + e));
+    for (int i = 0; i < N; i += 4) {
+        const float4 b = *reinterpret_cast<const float4*>(bias_w + i);
+        f[i] = __uint_as_float(v[i]) + b.x;
+        f[i + 1] = __uint_as_float(v[i + 1]) + b.y;
+        f[i + 2] = __uint_as_float(v[i + 2]) + b.z;
+        f[i + 3] = __uint_as_float(v[i + 3]) + b.w;
     }
 }
 

@@ -1,0 +1,20 @@
+"""Linear layers whose tiles are split over a cluster."""
+import pytest
+import torch
+
+import gpu_util as G
+import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 72, 768), (127, 200, 1536), (200, 1280, 1288), (64, 136, 5120)])
+def test_linear_split_rows_over_the_cluster(bd, oracle, M, N, K):
+    """The rows of a split tile are dealt out to the CTAs of its cluster: ragged rows and columns, two to eight CTAs."""
+    x, w = synth.activations((M, K), 9950), synth.round_bf16(synth.normal((N, K), 9951, 0, 1.0 / K ** 0.5))
+    b = synth.weights((N,), 9952)
+    y = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    bd.linear_fwd(G.dev(x), G.dev(w), G.dev(b), y[:M, :N])
+    assert bd.device_status() == 0
+    G.check(G.host(y[:M, :N]), oracle.linear(x, w, b), max_abs=2.5e-2, what=f"linear {M}x{N}x{K}")
+    assert bool((y[M] == 7.0).all()) and bool((y[:, N:] == 7.0).all())
