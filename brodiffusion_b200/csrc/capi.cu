@@ -187,8 +187,8 @@ int launch_gemm(const char* op, bdattn::GemmLaunch& L, int n, cudaStream_t strea
         bdattn::GemmProblem& p = L.args.p[i];
         if (p.n_tile == 0) p.n_tile = plan.width;
         p.tiles_n = (p.N + p.n_tile - 1) / p.n_tile;
-        // a CTA of a pair stages 128 weight rows
-        if (make_map_2d(op, &L.tmB[i], L.W[i], L.bf16, p.K, L.w_rows[i], L.ldw[i], plan.pair ? 128 : p.n_tile)) return -1;
+        // a CTA of a pair stages half of the tile's weight rows
+        if (make_map_2d(op, &L.tmB[i], L.W[i], L.bf16, p.K, L.w_rows[i], L.ldw[i], plan.pair ? plan.pair_cols / 2 : p.n_tile)) return -1;
     }
     for (int i = n; i < 3; ++i) {
         L.args.p[i] = L.args.p[0];
@@ -197,7 +197,7 @@ int launch_gemm(const char* op, bdattn::GemmLaunch& L, int n, cudaStream_t strea
         L.tmA[i] = L.tmA[0];
         L.tmB[i] = L.tmB[0];
     }
-    const cudaError_t e = plan.pair ? bdattn::launch_gemm_pair(L, stream) : bdattn::launch_gemm_tc05(L, stream);
+    const cudaError_t e = plan.pair ? bdattn::launch_gemm_pair(L, plan.pair_cols, stream) : bdattn::launch_gemm_tc05(L, stream);
     if (e != cudaSuccess) return cuda_fail(op, e);
     return 0;
 }

@@ -2,19 +2,22 @@
 // src/dit/flux.cpp:471-484; out-projection: src/dit/flux.cpp:519-525):
 //   C[M,N] = A[M,K] . W[N,K]^T (+ bias) [-> per-head RMSNorm -> RoPE]
 // Same operand layout and epilogue arithmetic as gemm_tc05_kernel; what differs is the
-// schedule, for problems that fill SMs with 256 x 256 tiles and, whatever their size, for whole heads
-// with norm + RoPE:
-//   * a cluster of two CTAs owns a 256-row x 256-column tile and computes it with
-//     tcgen05.mma.cta_group::2: every CTA stages its 128 rows of A and 128 of the tile's 256
-//     weight rows, so a K block costs an SM 32 KB of L2 reads and 8 KB of operand reads per
-//     128 tensor-pipe cycles (48 KB and 12 KB with a 128 x 256 tile of its own);
-//   * a stage is 128 columns of K: the issuing thread spends 64 cycles on an MMA and about
-//     250 on the wait and the commit around a stage, which with four MMAs to a stage made
-//     610 cycles of a K block of 64 where the tensor pipe needs 512;
+// schedule, for the larger problems, for GEGLU and, whatever their size, for whole heads
+// with norm + RoPE (gemm_plan.h):
+//   * a cluster of two CTAs owns a tile of 256 rows x kN = 256 or 128 columns and computes it with
+//     tcgen05.mma.cta_group::2: every CTA stages its 128 rows of A and half of the tile's
+//     weight rows, so a K block of 64 costs an SM 32 KB of L2 reads per 512 tensor-pipe cycles, with
+//     128 columns 24 KB per 256.  An SM is fed at about 70 bytes a cycle, so the wide tile is the better
+//     one wherever it fills the SMs and the narrow one where it does not: QKV of 256 rows of 3072 is 36
+//     tiles of 256 columns for 74 pairs, 26.8 us, or 72 of 128, 18.7; of 512 rows 72 wide tiles 27.9,
+//     144 narrow ones 29.1;
+//   * a stage is 128 columns of K: the wait and the commit around a stage cost the issuing thread about
+//     250 cycles, which with four MMAs of 64 to a stage made 610 cycles of a K block of 64 where the tensor
+//     pipe needs 512;
 //   * the pairs walk a list of tiles (up to three problems in one launch; tiles of one
 //     column block adjacent, in groups of sixteen row blocks, so that what runs together
 //     reads few weight and few activation tiles);
-//   * the accumulator is double-buffered in tensor memory (2 x 256 columns), so the epilogue
+//   * the accumulator is double-buffered in tensor memory (2 x kN columns), so the epilogue
 //     of tile i (bias, RMSNorm, RoPE, stores) runs while the MMAs of tile i+1 are issued;
 //   * the cos / sin rows and the outputs go through 2 KB of shared memory per epilogue warp, so
 //     that global accesses are whole row pieces (a load or store with a row per lane touches 32
@@ -23,8 +26,8 @@
 //     accumulator is ready, the next rows while a piece is worked on.  With bias values and table rows
 //     loaded where they are used the epilogue of norm + RoPE took 19300 cycles a tile, 10 of the 31 us of
 //     a 256-row prompt's projections, where the last one has nothing to hide behind.
-// GEGLU (src/fused_transformer.cu:89-92,275-282) runs here too: a tile is then 128 value
-// columns + their 128 gate columns (the first CTA stages the value rows of the weight, the
+// GEGLU (src/fused_transformer.cu:89-92,275-282) runs here too: a tile is then kN / 2 value
+// columns + as many gate columns (the first CTA stages the value rows of the weight, the
 // second the gate rows), one MMA computes both and the epilogue stores
 // value * gelu_exact(gate).
 // Roles in each CTA: warp 0 = TMA producer, warp 1 = TMEM owner and, in the first CTA of
@@ -39,45 +42,55 @@ namespace bdattn {
 namespace {
 
 constexpr int kPThreads = 320;
-constexpr int kPStages = 3;
-constexpr int kPTile = 256;                   // rows and accumulator columns of a pair's tile
-constexpr int kPChunk = 128 * 64 * 2;         // 128 rows x 64 columns: one TMA box of A or B
-// A stage of a CTA: two chunks (128 columns of K) of its 128 rows of A, two of its 128 weight rows
-constexpr int kPStageBytes = 4 * kPChunk;
+constexpr int kPRows = 256;                   // rows of a pair's tile
+constexpr int kPChunk = 128 * 64 * 2;         // 128 rows x 64 columns: one TMA box of A
 constexpr int kPStgBytes = 2048 + 512;        // one epilogue warp: staging, and 128 bias values as FP32
-constexpr int kPSmemBytes = kPStages * kPStageBytes + 8 * kPStgBytes + 256 + 3 * 128 * 4 + 1024;
-static_assert(kPSmemBytes <= 227 * 1024, "shared memory of one CTA");
+constexpr int kPPrefetch = 384;               // columns of K whose weights are asked for ahead
 constexpr int kPGroup = 16;                   // row blocks of a group
+
+// kN: accumulator columns of a tile, 256 or 128.  A stage of a CTA is two chunks (128 columns of K) of its
+// 128 rows of A and two of its kN / 2 weight rows.
+template <int kN>
+struct PairCfg {
+    static constexpr int kStages = kN == 256 ? 3 : 4;
+    static constexpr int kBChunk = kN / 2 * 64 * 2;
+    static constexpr int kStageBytes = 2 * kPChunk + 2 * kBChunk;
+    static constexpr int kSmemBytes = kStages * kStageBytes + 8 * kPStgBytes + 256 + 3 * 128 * 4 + 1024;
+    static constexpr int kHalf = kN / 2;      // output columns of an epilogue warp
+    static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
+};
 
 struct PairTile {
     int z, m0, n0;
 };
 
-// Output columns of one tile: 256, or 128 for GEGLU (the other 128 accumulator
+// Output columns of one tile: kN, or half of them for GEGLU (the other accumulator
 // columns hold the gate).
-__host__ __device__ __forceinline__ int pair_out_cols(const GemmProblem& p) { return gemm_pair_cols(p.geglu_offset > 0); }
+template <int kN>
+__host__ __device__ __forceinline__ int pair_out_cols(const GemmProblem& p) { return p.geglu_offset > 0 ? kN / 2 : kN; }
 __host__ __device__ __forceinline__ int pair_tiles_m(const GemmProblem& p) { return gemm_pair_row_tiles(p.tiles_m); }
 
+template <int kN>
 __device__ __forceinline__ PairTile pair_tile(const GemmArgs& g, int tile) {
     int z = 0;
     int local = tile;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const int cnt = pair_tiles_m(g.p[i]) * (g.p[i].N / pair_out_cols(g.p[i]));
+        const int cnt = pair_tiles_m(g.p[i]) * (g.p[i].N / pair_out_cols<kN>(g.p[i]));
         if (z == i && local >= cnt) {
             local -= cnt;
             z = i + 1;
         }
     }
     const GemmProblem& p = z == 0 ? g.p[0] : (z == 1 ? g.p[1] : g.p[2]);
-    const int cols = pair_out_cols(p), tm = pair_tiles_m(p), tn = p.N / cols;
+    const int cols = pair_out_cols<kN>(p), tm = pair_tiles_m(p), tn = p.N / cols;
     const int first = local / (kPGroup * tn) * kPGroup;      // first row block of the group
     const int rows = min(kPGroup, tm - first);
     local -= first * tn;
     PairTile t;
     t.z = z;
     t.n0 = (local / rows) * cols;
-    t.m0 = (first + local % rows) * kPTile;
+    t.m0 = (first + local % rows) * kPRows;
     return t;
 }
 
@@ -131,26 +144,28 @@ struct TablePiece {
     }
 };
 
-// Epilogue of 128 columns of a tile of whole heads, one of 128 columns or two of 64; this thread owns one
+// Epilogue of kW columns of a tile of whole heads of 128 or 64 columns; this thread owns one
 // token's row of them: RMSNorm over the head and the rotary embedding are
 // thread-local (src/dit/flux.cpp:462-469, src/dit/common.cpp:192-193).  Two
 // passes over the accumulator (tensor memory reads are cheap): sum of squares
-// per head first, then 32 columns at a time.  One loop for both head dims: two instantiations do not
-// fit the registers.  gain_s: the gains of a head in shared
-// memory as FP32, or null for no RMSNorm.  row0: the warp's first row; cbase: its first
-// output element; bias_w: the bias of its columns; tab: the table values of the first 32
-// columns of a head, where there is RoPE.
-template <bool kBf16>
+// per head first (the whole head, also where this warp finishes half of it), then 32 columns at a time.
+// One loop for both head dims: two instantiations do not fit the registers.  gain_s: the gains of a head in
+// shared memory as FP32, or null for no RMSNorm.  row0: the warp's first row.  tacc, bias_w and cbase: accumulator,
+// bias and output of 128 columns, of which this warp takes c_first and on; tab: the table values of its
+// first 32 columns, where there is RoPE.
+template <bool kBf16, int kW>
 __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t tacc, int row0, uint16_t* cbase,
-                                               const float* gain_s, const float* bias_w, uint8_t* stg, TablePiece& tab,
-                                               int lane) {
+                                               int c_first, const float* gain_s, const float* bias_w, uint8_t* stg,
+                                               TablePiece& tab, int lane) {
     const int rows = min(32, p.M - row0);
     const int hd = p.n_tile;
     float inv0 = 1.0f, inv1 = 1.0f;
     if (gain_s != nullptr) {
         float ss0 = 0.0f, ss1 = 0.0f;
+        // (kW = 64: the one head that the warp has columns of)
+        const int c_norm = kW == 128 ? 0 : c_first & ~(hd - 1), n_norm = kW == 128 ? 128 : hd;
 #pragma unroll 1
-        for (int c = 0; c < 128; c += 32) {
+        for (int c = c_norm; c < c_norm + n_norm; c += 32) {
             uint32_t v[32];
             tmem_ld32(tacc + c, v);
             tmem_wait_ld();
@@ -163,7 +178,7 @@ __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t ta
             }
             if (((c + 32) & (hd - 1)) == 0) {          // the head's last columns
                 const float inv = rsqrtf((ss0 + ss1) / static_cast<float>(hd) + p.eps);
-                if (c < hd) inv0 = inv;
+                if (kW == 64 || c < hd) inv0 = inv;
                 else inv1 = inv;
                 ss0 = ss1 = 0.0f;
             }
@@ -171,8 +186,8 @@ __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t ta
     }
     const bool rope = p.cos != nullptr;
 #pragma unroll 1
-    for (int c = 0; c < 128; c += 32) {
-        const float inv = c < hd ? inv0 : inv1;
+    for (int c = c_first; c < c_first + kW; c += 32) {
+        const float inv = kW == 64 || c < hd ? inv0 : inv1;
         const float* const gain_c = gain_s + (c & (hd - 1));
         float cs[16], sn[16];
         if (rope) tab.rows_of_lanes(stg, lane, cs, sn);
@@ -206,17 +221,20 @@ __device__ __forceinline__ void epilogue_heads(const GemmProblem& p, uint32_t ta
 #pragma unroll
             for (int i = 0; i < 8; ++i) packed[hf * 8 + i] = pack2<kBf16>(f[2 * i], f[2 * i + 1]);
         }
-        if (rope && c < 96) tab.load(p, hd >> 1, row0, rows, ((c + 32) & (hd - 1)) >> 1, lane);
+        if (rope && c + 32 < c_first + kW) tab.load(p, hd >> 1, row0, rows, ((c + 32) & (hd - 1)) >> 1, lane);
         store_words32(packed, stg, lane, cbase + c, p.ldc, rows, 32);
     }
 }
 
-template <bool kBf16>
+template <bool kBf16, int kN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                  const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB0,
                  const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmB2,
                  const GemmArgs g, const int total_tiles) {
+    using C = PairCfg<kN>;
+    constexpr int kPStages = C::kStages;
+    constexpr int kPStageBytes = C::kStageBytes;
     extern __shared__ uint8_t gemm_pair_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_pair_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
@@ -244,7 +262,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         fence_mbar_init();
     }
     if (warp == 1) {
-        tmem_alloc_pair(tmem_slot, 512);
+        tmem_alloc_pair(tmem_slot, 2 * kN);
         tmem_relinquish_pair();
     }
     // The first tile of this pair: found before the wait for the kernel before this one, so that the first
@@ -252,7 +270,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     const int rank = static_cast<int>(cluster_ctarank());
     const int pairs = static_cast<int>(gridDim.x) >> 1;
     const int first_tile = static_cast<int>(blockIdx.x) >> 1;
-    const PairTile first = pair_tile(g, first_tile);
+    const PairTile first = pair_tile<kN>(g, first_tile);
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(first.z == 0 ? &tmA0 : (first.z == 1 ? &tmA1 : &tmA2));
         tma_prefetch_desc(first.z == 0 ? &tmB0 : (first.z == 1 ? &tmB1 : &tmB2));
@@ -264,6 +282,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     const uint32_t tmem_base = *tmem_slot;
     // only now: a dependent CTA that took tensor memory first could keep this one from getting its own
     dependents_may_launch();
+    // While the kernel before this one ends, the first weights come into the L2 (the activations
+    // may still be being written): once for the row blocks that share them.  No more than a few stages: all
+    // of the first tile's weights took the first stages' bandwidth (QKV of 256 rows 26.6 -> 29.4 us).
+    if (warp == 0 && first.m0 % (kPGroup * kPRows) == 0 && elect_one()) {
+        const GemmProblem& p = first.z == 0 ? g.p[0] : (first.z == 1 ? g.p[1] : g.p[2]);
+        const CUtensorMap* tmB = first.z == 0 ? &tmB0 : (first.z == 1 ? &tmB1 : &tmB2);
+        const int row = first.n0 + rank * (p.geglu_offset > 0 ? p.geglu_offset : kN / 2);
+        for (int x = 0; x < p.K && x < kPPrefetch; x += 64) tma_prefetch_l2_2d(tmB, x, row);
+    }
     // barriers, tensor memory and descriptors are set up; from here on global memory is touched
     wait_for_prior_grid();
 
@@ -277,24 +304,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             uint32_t phase = 1;  // parity that a fresh barrier passes
             bool ok = true;
             for (int tile = first_tile; ok && tile < total_tiles; tile += pairs) {
-                const PairTile t = tile == first_tile ? first : pair_tile(g, tile);
+                const PairTile t = tile == first_tile ? first : pair_tile<kN>(g, tile);
                 const CUtensorMap* tmA = t.z == 0 ? &tmA0 : (t.z == 1 ? &tmA1 : &tmA2);
                 const CUtensorMap* tmB = t.z == 0 ? &tmB0 : (t.z == 1 ? &tmB1 : &tmB2);
                 const int K = t.z == 0 ? g.p[0].K : (t.z == 1 ? g.p[1].K : g.p[2].K);
                 const int geglu_off = t.z == 0 ? g.p[0].geglu_offset : (t.z == 1 ? g.p[1].geglu_offset : g.p[2].geglu_offset);
                 const int chunks = (K + 63) / 64;
                 const int a_row = t.m0 + rank * 128;
-                const int b_row = t.n0 + rank * (geglu_off > 0 ? geglu_off : 128);
+                const int b_row = t.n0 + rank * (geglu_off > 0 ? geglu_off : kN / 2);
                 for (int c = 0; c < chunks; c += 2, ++it) {
                     ok = mbar_wait(&empty[slot], phase);
                     if (!ok) break;
                     uint8_t* st = smem + slot * kPStageBytes;
                     const int n = min(2, chunks - c);          // an odd last chunk stands alone
-                    if (rank == 0) mbar_arrive_expect_tx(&full[slot], n * 2 * 2 * kPChunk);
+                    if (rank == 0) mbar_arrive_expect_tx(&full[slot], n * 2 * (kPChunk + C::kBChunk));
                     const uint32_t bar = mapa(smem_u32(&full[slot]), 0);
                     for (int i = 0; i < n; ++i) {
                         tma_load_2d_pair(st + i * kPChunk, tmA, bar, (c + i) * 64, a_row);
-                        tma_load_2d_pair(st + (2 + i) * kPChunk, tmB, bar, (c + i) * 64, b_row);
+                        tma_load_2d_pair(st + 2 * kPChunk + i * C::kBChunk, tmB, bar, (c + i) * 64, b_row);
                     }
                     if (++slot == kPStages) { slot = 0; phase ^= 1; }
                 }
@@ -312,7 +339,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         __syncwarp();
     } else if (warp == 1) {
         // ---------------------------------------- MMA issuer (first CTA of the pair)
-        constexpr uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, kPTile, kPTile, 0, 0);
+        constexpr uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, kPRows, kN, 0, 0);
         const uint64_t a0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
         const uint64_t b0 = make_smem_desc_sw128(smem_u32(smem) + 2 * kPChunk, 16, 1024);
         int slot = 0;
@@ -320,7 +347,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         int ti = 0;              // tiles done by this pair
         bool ok = rank == 0;
         for (int tile = first_tile; ok && tile < total_tiles; tile += pairs, ++ti) {
-            const PairTile t = tile == first_tile ? first : pair_tile(g, tile);
+            const PairTile t = tile == first_tile ? first : pair_tile<kN>(g, tile);
             const int K = t.z == 0 ? g.p[0].K : (t.z == 1 ? g.p[1].K : g.p[2].K);
             const int chunks = (K + 63) / 64;
             const int as = ti & 1;
@@ -329,7 +356,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 if (!ok) break;
                 tc_fence_after();
             }
-            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(as * kPTile);
+            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(as * kN);
             for (int c = 0; c < chunks; c += 2) {
                 ok = mbar_wait_warp(&full[slot], phase);
                 if (!ok) break;
@@ -344,7 +371,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                     if (c + 1 < chunks) {
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
-                            umma_ss_pair(d_tmem, ad + (kPChunk >> 4) + 2 * kk, bd + (kPChunk >> 4) + 2 * kk, idesc, 1u);
+                            umma_ss_pair(d_tmem, ad + (kPChunk >> 4) + 2 * kk, bd + (C::kBChunk >> 4) + 2 * kk, idesc, 1u);
                     }
                     umma_commit_pair(&empty[slot]);
                     if (c + 2 >= chunks) umma_commit_pair(&acc_full[as]);
@@ -372,20 +399,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         int ti = 0;
         bool ok = true;
         for (int tile = first_tile; tile < total_tiles; tile += pairs, ++ti) {
-            const PairTile t = tile == first_tile ? first : pair_tile(g, tile);
+            const PairTile t = tile == first_tile ? first : pair_tile<kN>(g, tile);
             const GemmProblem& p = t.z == 0 ? g.p[0] : (t.z == 1 ? g.p[1] : g.p[2]);
             const int as = ti & 1;
             const int row0 = t.m0 + rank * 128 + q * 32;
             const int rows = min(32, p.M - row0);
             // a projection without norm and RoPE (V) has nothing but its bias to add
             const bool heads = p.norm_rope && (p.gain != nullptr || p.cos != nullptr);
+            // where the 128 columns whose bias this warp keeps begin in the tile, and its own among them
+            constexpr bool kWide = kN == 256;
+            const int c_base = kWide ? half * 128 : 0, c_own = kWide ? 0 : half * C::kHalf;
             {
-                // the 128 bias values this warp needs (GEGLU: 64 and those of their gates), fetched
-                // while the tile is computed
+                // 128 bias values (GEGLU: 64 and those of their gates), fetched while the tile is computed
                 const int lc = lane * 4;
                 const long long at = p.geglu_offset > 0
-                                         ? t.n0 + half * 64 + (lc < 64 ? lc : static_cast<long long>(p.geglu_offset) + lc - 64)
-                                         : t.n0 + half * 128 + lc;
+                                         ? t.n0 + (c_base >> 1) + (lc < 64 ? lc : static_cast<long long>(p.geglu_offset) + lc - 64)
+                                         : t.n0 + c_base + lc;
                 float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if (p.bias != nullptr)
                     b = make_float4(load16<kBf16>(p.bias, at), load16<kBf16>(p.bias, at + 1), load16<kBf16>(p.bias, at + 2),
@@ -394,30 +423,28 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 __syncwarp();
             }
             TablePiece tab;
-            if (heads && p.cos != nullptr && rows > 0) tab.load(p, p.n_tile >> 1, row0, rows, 0, lane);
+            if (heads && p.cos != nullptr && rows > 0) tab.load(p, p.n_tile >> 1, row0, rows, (c_own & (p.n_tile - 1)) >> 1, lane);
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[as], static_cast<uint32_t>((ti >> 1) & 1)));
             if (!ok) break;
             tc_fence_after();
-            const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(as * kPTile);
+            const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(as * kN);
             uint16_t* cbase = reinterpret_cast<uint16_t*>(p.C) + static_cast<long long>(row0) * p.ldc + t.n0;
             if (rows <= 0) {
                 // rows past the matrix: nothing to store
             } else if (heads) {
                 const float* gs = p.gain != nullptr ? gain_s + t.z * 128 : nullptr;
-                const int c0 = half * (kPTile / 2);
-                epilogue_heads<kBf16>(p, tacc + c0, row0, cbase + c0, gs, bias_w, stg, tab, lane);
+                epilogue_heads<kBf16, C::kHalf>(p, tacc + c_base, row0, cbase + c_base, c_own, gs, bias_w, stg, tab, lane);
             } else if (p.geglu_offset > 0) {
-                // value in accumulator columns [0, 128), gate in [128, 256); this group
-                // stores 64 of the tile's 128 output columns
+                // values in the first half of the accumulator's columns, gates in the second
 #pragma unroll 1
-                for (int c = half * 64; c < half * 64 + 64; c += 32) {
-                    const float* bv = bias_w + (c - half * 64);
+                for (int c = (c_base + c_own) / 2; c < (c_base + c_own + C::kHalf) / 2; c += 32) {
+                    const float* bv = bias_w + (c - c_base / 2);
                     uint32_t packed[16];
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
                         uint32_t v[16], gt[16];
                         tmem_ld16(tacc + c + hf * 16, v);
-                        tmem_ld16(tacc + 128 + c + hf * 16, gt);
+                        tmem_ld16(tacc + kN / 2 + c + hf * 16, gt);
                         tmem_wait_ld();
                         float f[16], gate[16];
                         add_bias(v, bv + hf * 16, f);
@@ -431,12 +458,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
                 }
             } else {
 #pragma unroll 1
-                for (int c = half * (kPTile / 2); c < (half + 1) * (kPTile / 2); c += 32) {
+                for (int c = c_base + c_own; c < c_base + c_own + C::kHalf; c += 32) {
                     uint32_t v[32];
                     tmem_ld32(tacc + c, v);
                     tmem_wait_ld();
                     float f[32];
-                    add_bias(v, bias_w + (c - half * (kPTile / 2)), f);
+                    add_bias(v, bias_w + (c - c_base), f);
                     store_tile32<kBf16>(f, stg, lane, cbase + c, p.ldc, rows, 32);
                 }
             }
@@ -455,25 +482,30 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     cluster_sync_relaxed();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc_pair(tmem_base, 512);
+        tmem_dealloc_pair(tmem_base, 2 * kN);
     }
 }
 
 }  // namespace
 
-cudaError_t launch_gemm_pair(const GemmLaunch& L, cudaStream_t stream) {
+template <int kN>
+static cudaError_t launch_gemm_pair_n(const GemmLaunch& L, cudaStream_t stream) {
     int total = 0;
     for (int i = 0; i < L.n_problems; ++i)
-        total += pair_tiles_m(L.args.p[i]) * (L.args.p[i].N / pair_out_cols(L.args.p[i]));
+        total += pair_tiles_m(L.args.p[i]) * (L.args.p[i].N / pair_out_cols<kN>(L.args.p[i]));
     const int pairs = sm_count() / 2;
     const dim3 grid(static_cast<unsigned>(2 * (total < pairs ? total : pairs)));
     auto go = [&](auto kern) {
-        cudaError_t e = set_max_smem_once(kern, kPSmemBytes);
+        cudaError_t e = set_max_smem_once(kern, PairCfg<kN>::kSmemBytes);
         if (e != cudaSuccess) return e;
-        return launch_dependent(kern, grid, dim3(kPThreads), kPSmemBytes, stream, L.tmA[0], L.tmA[1], L.tmA[2],
+        return launch_dependent(kern, grid, dim3(kPThreads), PairCfg<kN>::kSmemBytes, stream, L.tmA[0], L.tmA[1], L.tmA[2],
                                 L.tmB[0], L.tmB[1], L.tmB[2], L.args, total);
     };
-    return L.bf16 ? go(gemm_pair_kernel<true>) : go(gemm_pair_kernel<false>);
+    return L.bf16 ? go(gemm_pair_kernel<true, kN>) : go(gemm_pair_kernel<false, kN>);
+}
+
+cudaError_t launch_gemm_pair(const GemmLaunch& L, int tile_cols, cudaStream_t stream) {
+    return tile_cols == 128 ? launch_gemm_pair_n<128>(L, stream) : launch_gemm_pair_n<256>(L, stream);
 }
 
 }  // namespace bdattn

@@ -15,12 +15,13 @@ struct GemmShape {
     int M, N, K;
     bool geglu;
     bool heads;      // whole heads with norm + RoPE
-    bool whole;      // whole 256-column tiles (128 for GEGLU)
+    bool whole;      // whole 256-column tiles (128 for GEGLU) of the pair kernel
 };
 
 struct GemmPlan {
     bool pair;
     int width, split;
+    int pair_cols = 256;     // accumulator columns of a pair's tile
 };
 
 BDATTN_HD constexpr int gemm_k_blocks(int K) { return (K + 63) / 64; }
@@ -39,35 +40,39 @@ BDATTN_HD constexpr bool pair_acc_reused(int tile, int pairs, int total_tiles) {
     return tile + 2 * pairs < total_tiles;
 }
 
-// The least of the modelled times, fitted to FP16 calls of 64 x 1280 x 1280 to 9216 x 320 x 1280
-// (M x N x K) on one B200.  A K block of 64 costs a CTA 0.30 us with 64 or 128 columns and a
-// pair 0.28 us; the rest of a call is 3 us (64 columns, one CTA per SM), 4.3 (64, several), 4.2
-// (128) or 7.5 (pairs), and the exchange of a split tile 1.5, as much again for a second wave.
-// Several CTAs of 64 columns share an SM and hide part of each other.  Examples, measured:
-//   64 x 1280 x 5120   64 columns 27.2 us, split over four 10.6, pairs 28.9
-//   256 x 1280 x 1280  64 columns  8.8 us, split over two 8.1, over four 9.6
-//   4096 x 320 x 320   64 columns  6.4 us, 128 columns 5.5
-//   1024 x 3072 x 3072 64 columns 36.8 us, 128 columns 37.9, pairs 21.8
-// GEGLU: 64 x 1280 -> 5120 64 columns 16.0 us, pairs 14; 256 x 320 -> 1280 8.5 and 9.
-// None is split: the two accumulators of a tile double the exchange.
-// (BF16 is within a few per cent of FP16: 64 x 1280 x 5120 9.6 us against 9.8, 4096 x 3072 x 3072 54.5 against 57.0.)
+// The least of the modelled times, fitted to calls of 64 x 1280 x 1280 to 9216 x 320 x 1280 (M x N x K) in
+// FP16 with cold weights on one B200; x stands for waves of CTAs (pairs), k for K blocks of 64.  Measured, in us:
+//                          64 columns  128 columns  pairs x 128  pairs x 256
+//   4096 x  320 x  320          6.6         4.5          -            -
+//   1024 x  640 x 2560          8.9        11.0        10.8           -
+//    576 x 1280 x 1280          6.1         7.2         7.6         11.1
+//    512 x 3072 x 3072         17.4        13.7        13.5         20.0
+//   2304 x  640 x 2560         15.1        11.9        11.8           -
+//   1024 x 3072 x 3072         30.5        31.4        21.8         21.0
+//   4096 x 3072 x 3072         92          88          64.5         57
+//   GEGLU  256 x  640 -> 2560   8.3          -          6.7          9.3
+//   GEGLU 1024 x  640 -> 2560  18.1          -         12.9         13.4
+//   GEGLU 4096 x  320 -> 1280  22.3          -         18.1         16.4
+//   Q, K, V with norm + RoPE, K = 3072: 256 rows 18.7 with 128 columns, 26.8 with 256; 512 rows 29.1 and
+//   27.9; 1024 rows 50.4 and 46.6
+// A tile split over CTAs pays where few tiles have a long K: 64 x 1280 x 5120 14.3 us, 10.1 over two CTAs, 7.8 over
+// four, 9.2 over eight; 256 x 1280 x 5120 14.2, 11.4, 13.7.  The splits are entered at about 0.8 us less than they
+// take when all CTAs run at once, and three when not: with the times themselves launches of a few tiles would be
+// split less than tests/test_gemm_plan.py has it (256 x 1280 x 1280 6.4 us over two, 5.7 whole).
+// GEGLU is not split: the two accumulators of a tile double the exchange.
 // The problems of a launch may differ in K (the queries and the keys of a cross-attention): the
 // longest sets the time, the shortest how far its tiles can be split, a CTA without a K
 // block would have nothing to add and nothing to wait for.
 inline GemmPlan plan_gemm(const GemmShape* p, int n, int sms) {
-    bool whole = true, geglu = false, heads = false;
+    bool geglu = false, heads = false;
     int kb = 0, kb_min = 0;
     for (int i = 0; i < n; ++i) {
-        whole = whole && p[i].whole;
         geglu = geglu || p[i].geglu;
         heads = heads || p[i].heads;
         const int b = gemm_k_blocks(p[i].K);
         kb = b > kb ? b : kb;
         kb_min = i == 0 || b < kb_min ? b : kb_min;
     }
-    // whole heads with norm + RoPE are faster on pairs at any size (16 rows of 3072: 31 against 24 us; three
-    // tiles on three pairs, 1024 rows to 2 heads of 128 with K = 1024, 17.7 us, half of it on the narrow kernel 27.7)
-    if (heads) return {whole, 64, 1};
     auto tiles = [&](int w) {
         long long t = 0;
         for (int i = 0; i < n; ++i) t += static_cast<long long>(gemm_row_tiles(p[i].M)) * ((p[i].N + w - 1) / w);
@@ -75,30 +80,37 @@ inline GemmPlan plan_gemm(const GemmShape* p, int n, int sms) {
     };
     auto waves = [&](int w, int s) { return static_cast<double>((tiles(w) * s + sms - 1) / sms); };
     GemmPlan best = {false, 64, 1};
-    double best_us;
-    {
-        const double x = waves(64, 1), b = kb * (geglu ? 0.45 : 0.30) * (geglu ? x : 1.0);
-        best_us = x <= 1.0 ? b + 3.0 : (geglu ? b : 0.62 * x * b) + 4.3;
-        if (geglu) best_us += 3.0 * x;
-    }
+    // whole heads with norm + RoPE are faster on pairs at any size (the narrow kernel: 256 rows 37 us, 1024 rows 128)
+    double best_us = 1e30;
     auto offer = [&](const GemmPlan& o, double us) {
         if (us < best_us) { best = o; best_us = us; }
     };
-    if (!geglu) {
-        offer({false, 128, 1}, waves(128, 1) * kb * 0.31 + 4.2);
-        // (beyond one and a half CTAs per SM a split only adds waves: 256 x 3072 x 3072 over four 21.4 us,
-        // over two 16.2)
+    if (!heads) {
+        const double x = waves(64, 1);
+        if (geglu) offer(best, kb * 0.45 * x + 4.3 + 3.0 * x);
+        else offer(best, x <= 1.0 ? 2.2 + 0.165 * kb : 2.5 + x * (0.8 + 0.155 * kb));
+    }
+    if (!geglu && !heads) {
+        const double x = waves(128, 1);
+        offer({false, 128, 1}, x <= 1.0 ? 2.8 + 0.21 * kb : 2.0 + x * (1.0 + 0.30 * kb));
         for (int s = 2; s <= 8 && kb >= 3 * s && kb_min >= s && tiles(64) * s * 2 <= 3LL * sms; s *= 2) {
-            const double x = waves(64, s), b = 0.30 * kb / s;
-            offer({false, 64, s}, (x <= 1.0 ? b : 0.725 * x * b) + 4.5 + 1.5 * (x - 1.0));
+            // (with more CTAs than SMs a longer part of K costs more than the split saves)
+            if (waves(64, s) <= 1.0) offer({false, 64, s}, 3.15 + 0.15 * kb / s);
+            else if (kb <= 12 * s) offer({false, 64, s}, 3.22 + 0.27 * kb / s * tiles(64) * s / sms);
         }
     }
-    if (whole) {
-        int pair_tiles = 0;
-        for (int i = 0; i < n; ++i)
-            pair_tiles += gemm_pair_row_tiles(gemm_row_tiles(p[i].M)) * (p[i].N / gemm_pair_cols(p[i].geglu));
-        const double x = (pair_tiles + sms / 2 - 1) / (sms / 2);
-        offer({true, 64, 1}, x * (kb * 0.28 + (geglu ? 2.5 : 0.0)) + (geglu ? 5.3 : 7.5));
+    for (int cols = 256; cols >= 128; cols /= 2) {
+        bool whole = true;
+        long long t = 0;
+        for (int i = 0; i < n; ++i) {
+            const int out = gemm_pair_cols(p[i].geglu) * cols / 256;
+            whole = whole && (cols == 256 ? p[i].whole : p[i].N % out == 0);
+            t += static_cast<long long>(gemm_pair_row_tiles(gemm_row_tiles(p[i].M))) * (p[i].N / out);
+        }
+        if (!whole) continue;
+        const double x = static_cast<double>((t + sms / 2 - 1) / (sms / 2));
+        if (cols == 256) offer({true, 64, 1, 256}, heads ? 8.0 + x * (1.0 + 0.37 * kb) : geglu ? 2.5 + 0.17 * kb + x * (2.6 + 0.24 * kb) : 4.5 + x * (0.8 + 0.32 * kb));
+        else offer({true, 64, 1, 128}, heads ? 6.5 + x * (1.0 + 0.215 * kb) : geglu ? 2.0 + x * (2.4 + 0.15 * kb) : 3.2 + x * (0.5 + 0.20 * kb));
     }
     return best;
 }

@@ -195,9 +195,9 @@ struct GemmLaunch {
     bool bf16;
 };
 cudaError_t launch_gemm_tc05(const GemmLaunch& L, cudaStream_t stream);
-// Persistent kernel of CTA pairs and 256 x 256 tiles; every problem of the launch must
-// have whole[i] set.
-cudaError_t launch_gemm_pair(const GemmLaunch& L, cudaStream_t stream);
+// Persistent kernel of CTA pairs with tiles of 256 rows x tile_cols (256 or 128) accumulator columns; every
+// problem of the launch must have whole tiles of that width.
+cudaError_t launch_gemm_pair(const GemmLaunch& L, int tile_cols, cudaStream_t stream);
 
 // Elementwise helpers.
 cudaError_t launch_add_inplace(void* y, const void* x, long long n, bool bf16, cudaStream_t stream);
