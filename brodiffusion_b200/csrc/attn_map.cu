@@ -12,12 +12,12 @@
 // heads in turn, so that a small block (32 such tiles at 1024 rows x 256 keys) still
 // fills the SMs, and add up their sums through distributed shared memory.  Per head:
 // TMA brings the Q and K tile of the head (zero-filled past head_dim), one lane issues
-// S = Q.K^T into one of two tensor-memory buffers, and four warps (one thread per query
-// row) turn the scores into weights and add them to 64 registers; the bias of the tile
+// S = Q.K^T into one of two tensor-memory buffers, and eight warps (two threads per query
+// row) turn the scores into weights and add them to 32 registers each; the bias of the tile
 // and its visibility bits are fetched once, not per head.
-// Bound by the L2 reads of Q and K (48 KB per head and tile; 37 MB in all at 1024 x 256,
-// 24 heads of 128).  With dot products on the CUDA cores out of shared memory that block
-// took nine tenths of a traced call of 770 us (1280 x 1280); the call now takes 54 us.
+// A tile is a chain of latencies: with four warps, bias rows fetched in eight batches, a test per key for its
+// visibility and remote sums read by four bytes it took 35000 cycles at 1024 x 256, 24 heads of 128 (bias 9000, bits
+// 4000, six heads 11000, sums and stores 10000), 21 of the 54 us of a traced call; now 10 of 40.
 #include <cooperative_groups.h>
 
 #include "sdpa_internal.h"
@@ -29,7 +29,7 @@ namespace {
 constexpr int kMapRows = 128;
 constexpr int kMapKeys = 64;
 constexpr int kMapStages = 3;
-constexpr int kMapThreads = 192;          // TMA warp, MMA warp, four warps for the rows
+constexpr int kMapThreads = 320;          // TMA warp, MMA warp, eight warps for the rows: 32 rows x 32 keys each
 constexpr uint32_t kMapTmemCols = 128;    // two score buffers of 64 columns
 constexpr int kMapQChunk = kMapRows * 128;   // 64 head columns of the Q tile
 constexpr int kMapKChunk = kMapKeys * 128;
@@ -38,11 +38,16 @@ template <int HD>
 struct MapCfg {
     static constexpr int kChunks = HD / 64;
     static constexpr int kStageBytes = kChunks * (kMapQChunk + kMapKChunk);
-    // the ring also holds the CTA's 128 x 64 sums on their way to the cluster (32 KB)
+    // the ring also holds the CTA's 128 x 64 sums on their way out
     static constexpr int kSmemBytes = kMapStages * kStageBytes + 128 + kMapKeys * 4 + 1024;
-    // with a bias: 32 x 32 values of it for each of the four row warps, one float of padding per row
-    static constexpr int kBiasBytes = 4 * 32 * 33 * 4;
+    // with a bias: 32 x 32 values of it for each of the row warps
+    static constexpr int kBiasBytes = 8 * 4096;
 };
+
+constexpr int kMapSumLd = kMapKeys + 4;       // floats of a row of sums: no bank conflicts, a thread per row or per 16 bytes
+
+// The first n of 32 bits.
+__device__ __forceinline__ uint32_t first_bits(int n) { return n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u); }
 
 template <int HD, bool kBf16>
 __global__ void __launch_bounds__(kMapThreads, 1)
@@ -87,7 +92,7 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&s_full[b], 1);
-            mbar_init(&s_free[b], 4);
+            mbar_init(&s_free[b], 8);
         }
         fence_mbar_init();
     }
@@ -109,10 +114,11 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
         __syncthreads();
     }
 
-    float acc[kMapKeys];
+    float acc[32];
 #pragma unroll
-    for (int c = 0; c < kMapKeys; ++c) acc[c] = 0.0f;
+    for (int c = 0; c < 32; ++c) acc[c] = 0.0f;
     const int row = (warp & 3) * 32 + lane;
+    const int col0 = ((warp - 2) >> 2) * 32;       // the keys of this warp (warps 2-9)
     const int qi = row_base + row;
 
     if (warp == 0) {
@@ -166,48 +172,38 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
         }
         __syncwarp();
     } else {
-        const uint32_t tS = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        const uint32_t tS = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(col0);
         const bool row_ok = row < rows;
-        // the row's bias in log2 units, and which of its 64 keys it sees (the attention kernel's
+        // the row's bias in log2 units, and which of its 32 keys it sees (the attention kernel's
         // rules: a masked key has weight 0)
         const float log2e = 1.4426950408889634f;
-        float bias[kMapKeys];
-        uint32_t vis[2] = {0u, 0u};
+        float bias[32];
+        uint8_t* const bs = reinterpret_cast<uint8_t*>(ks_s + kMapKeys) + (warp - 2) * 4096;
         if (a.bias != nullptr) {
-            // rows of the bias through shared memory, so that a load takes 32 columns of one row (a row per
-            // lane touches 32 cache lines: 64 rows x 77 keys, one head of 40: a traced call 27.3 -> 21.2 us)
-            float* const bs = ks_s + kMapKeys + (warp & 3) * 32 * 33;
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                const int col = hf * 32 + lane, kg = key_base + col;
-                const bool col_ok = col < keys && kg < a.bias_cols;
-#pragma unroll 8
-                for (int r = 0; r < 32; ++r) {
-                    const int tr = (warp & 3) * 32 + r, br = row_base + tr - a.bias_row0;
-                    const bool on = col_ok && tr < rows && br >= 0 && br < a.bias_rows;
-                    bs[r * 33 + lane] = on ? __ldg(a.bias + static_cast<long long>(br) * a.bias_ld + kg) * log2e : 0.0f;
-                }
-                __syncwarp();
-#pragma unroll
-                for (int c = 0; c < 32; ++c) bias[hf * 32 + c] = bs[lane * 33 + c];
-                __syncwarp();
-            }
-        } else {
-#pragma unroll
-            for (int c = 0; c < kMapKeys; ++c) bias[c] = 0.0f;
+            const int kg = key_base + col0;
+            copy_rows32(bs, a.bias + kg, a.bias_ld, row_base + (warp & 3) * 32 - a.bias_row0, a.bias_rows,
+                        min(keys - col0, a.bias_cols - kg), lane);
         }
-#pragma unroll
-        for (int c = 0; c < kMapKeys; ++c) {
-            const int kg = key_base + c;
-            bool v = row_ok && c < keys;
-            if (a.mask_mode == 1) v = v && kg <= qi + a.q_offset;
-            if (a.key_mask != nullptr) v = v && __ldg(a.key_mask + kg) != 0.0f;
-            vis[c >> 5] |= (v ? 1u : 0u) << (c & 31);
+        uint32_t vis = first_bits(keys - col0);
+        if (a.mask_mode == 1) vis &= first_bits(qi + a.q_offset - key_base - col0 + 1);
+        if (a.key_mask != nullptr) {
+            const float seen = col0 + lane < keys ? __ldg(a.key_mask + key_base + col0 + lane) : 0.0f;
+            vis &= __ballot_sync(0xffffffffu, seen != 0.0f);
         }
+        if (!row_ok) vis = 0u;
         const float* st = a.lse + (static_cast<long long>(rank) * a.lq_total + qi) * 2;
         const long long st_step = static_cast<long long>(cs) * a.lq_total * 2;
         float2 stat = make_float2(0.0f, 0.0f);
         if (row_ok && n_heads > 0) stat = make_float2(st[0], st[1]);
+        if (a.bias != nullptr) {
+            cp_async_wait_all();
+            __syncwarp();
+        }
+#pragma unroll
+        for (int c = 0; c < 32; c += 4) {
+            const float4 b = a.bias != nullptr ? row_piece32(bs, lane, c >> 2) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            bias[c] = b.x * log2e; bias[c + 1] = b.y * log2e; bias[c + 2] = b.z * log2e; bias[c + 3] = b.w * log2e;
+        }
         bool ok = true;
         for (int i = 0; i < n_heads; ++i) {
             const int b = i & 1;
@@ -216,60 +212,69 @@ attn_map_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant_
             st += st_step;
             if (row_ok && i + 1 < n_heads) stat = make_float2(st[0], st[1]);
             // a row whose reference maximum is -inf saw no key: its map row is zero
-            const bool seen = m2 != -INFINITY;
+            const uint32_t bits = m2 != -INFINITY ? vis : 0u;
             ok = __all_sync(0xffffffffu, mbar_wait(&s_full[b], static_cast<uint32_t>((i >> 1) & 1)));
             if (!ok) break;
             tc_fence_after();
+            uint32_t v[32];
+            tmem_ld32(tS + b * kMapKeys, v);
+            tmem_wait_ld();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[b]);
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                uint32_t v[32];
-                tmem_ld32(tS + b * kMapKeys + hf * 32, v);
-                tmem_wait_ld();
-                if (hf == 1) {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&s_free[b]);
-                }
-                const uint32_t bits = seen ? vis[hf] : 0u;
-#pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    float x = __uint_as_float(v[c]);
-                    if (a.key_scale != nullptr) x *= ks_s[hf * 32 + c];
-                    const float p = fast_exp2(fmaf(x, a.scale_log2, bias[hf * 32 + c]) - m2) * inv_l;
-                    acc[hf * 32 + c] += ((bits >> c) & 1u) != 0u ? p : 0.0f;
-                }
+            for (int c = 0; c < 32; ++c) {
+                float x = __uint_as_float(v[c]);
+                if (a.key_scale != nullptr) x *= ks_s[col0 + c];
+                const float p = fast_exp2(fmaf(x, a.scale_log2, bias[c]) - m2) * inv_l;
+                acc[c] += ((bits >> c) & 1u) != 0u ? p : 0.0f;
             }
         }
     }
 
+    // Sums to shared memory (the ring is at rest: every MMA that read it has completed); then every CTA of the
+    // cluster adds up and stores its share of the columns, four to a thread.
     const float inv_h = 1.0f / static_cast<float>(a.num_heads);
-    float* out = a.map + static_cast<long long>(qi - a.map_row0) * a.map_ld + key_base;
-    if (cs == 1) {
-        if (warp >= 2 && row < rows) {
+    float* const out = a.map + static_cast<long long>(row_base - a.map_row0) * a.map_ld + key_base;
+    float* const red = reinterpret_cast<float*>(smem);
+    if (warp >= 2) {
 #pragma unroll
-            for (int c = 0; c < kMapKeys; ++c)
-                if (c < keys) out[c] = acc[c] * inv_h;
-        }
-    } else {
-        // sums to shared memory (the ring is at rest: every MMA that read it has completed), column
-        // by column so that a warp's accesses are consecutive; then every CTA of the cluster adds
-        // up and stores its share of the columns
-        float* red = reinterpret_cast<float*>(smem);
-        if (warp >= 2) {
+        for (int c = 0; c < 32; c += 4)
+            *reinterpret_cast<float4*>(red + row * kMapSumLd + col0 + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
+    }
+    if (cs > 1) cluster_sync();
+    else __syncthreads();
+    if (warp >= 2) {
+        const float* src[8];
 #pragma unroll
-            for (int c = 0; c < kMapKeys; ++c) red[c * kMapRows + row] = acc[c];
-        }
-        cluster_sync();
-        if (warp >= 2 && row < rows) {
-            const int per = kMapKeys / cs;
-            for (int c = rank * per; c < (rank + 1) * per; ++c) {
-                float sum = 0.0f;
-                for (int r = 0; r < cs; ++r) sum += cluster.map_shared_rank(red, r)[c * kMapRows + row];
-                if (c < keys) out[c] = sum * inv_h;
+        for (int k = 0; k < 8; ++k) src[k] = cs > 1 ? cluster.map_shared_rank(red, min(k, cs - 1)) : red;
+        const int units = kMapKeys / 4 / cs;                                   // a power of two, as cs is
+        const bool vec = (a.map_ld & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+#pragma unroll 2
+        for (int i = static_cast<int>(threadIdx.x) - 64; i < kMapRows * units; i += 256) {
+            const int r = i / units, c = (rank * units + (i & (units - 1))) * 4;
+            if (r >= rows || c >= keys) continue;
+            float4 u[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (k < cs) u[k] = *reinterpret_cast<const float4*>(src[k] + r * kMapSumLd + c);
+            float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (k < cs) { sum.x += u[k].x; sum.y += u[k].y; sum.z += u[k].z; sum.w += u[k].w; }
+            sum.x *= inv_h; sum.y *= inv_h; sum.z *= inv_h; sum.w *= inv_h;
+            float* const at = out + r * a.map_ld + c;
+            if (vec && c + 4 <= keys) {
+                *reinterpret_cast<float4*>(at) = sum;
+            } else {
+                at[0] = sum.x;
+                if (c + 1 < keys) at[1] = sum.y;
+                if (c + 2 < keys) at[2] = sum.z;
+                if (c + 3 < keys) at[3] = sum.w;
             }
         }
-        cluster_sync_relaxed();      // the peers' shared memory stays until everyone has read it
     }
+    if (cs > 1) cluster_sync_relaxed();      // the peers' shared memory stays until everyone has read it
 
     tc_fence_before();
     __syncthreads();

@@ -262,6 +262,43 @@ __device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, 
                  : "memory");
 }
 
+// Asynchronous copy of kBytes (4 or 16) to shared memory, zeros where `on` is false (src is then not read).
+template <int kBytes>
+__device__ __forceinline__ void cp_async_zfill(void* dst, const void* src, bool on) {
+    const int n = on ? kBytes : 0;
+    if constexpr (kBytes == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// 32 x 32 values of an FP32 matrix to 4 KB of a warp's shared memory (cp.async), rows [row, row + 32) from column 0
+// of `src`, zeros outside rows [0, n_rows) and columns [0, n_cols).  The 16-byte pieces of a row are permuted by
+// the row, so that a copy takes whole rows and a lane reads its own without bank conflicts (row_piece32): a
+// load with a row per lane touches 32 cache lines.
+__device__ __forceinline__ void copy_rows32(uint8_t* dst, const float* src, long long ld, int row, int n_rows, int n_cols,
+                                            int lane) {
+    if ((n_cols >= 32 || (n_cols & 3) == 0) && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = i * 4 + (lane >> 3), p = lane & 7;
+            const bool on = row + r >= 0 && row + r < n_rows && p * 4 < n_cols;
+            cp_async_zfill<16>(dst + r * 128 + ((p ^ (r & 7)) << 4), on ? src + (row + r) * ld + p * 4 : src, on);
+        }
+    } else {
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) {
+            const bool on = row + r >= 0 && row + r < n_rows && lane < n_cols;
+            cp_async_zfill<4>(dst + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4,
+                              on ? src + (row + r) * ld + lane : src, on);
+        }
+    }
+}
+// Values 4 i .. 4 i + 3 of the lane's row.
+__device__ __forceinline__ float4 row_piece32(const uint8_t* rows, int lane, int i) {
+    return *reinterpret_cast<const float4*>(rows + lane * 128 + ((i ^ (lane & 7)) << 4));
+}
+
 // ---------------------------------------------------------- tensor memory
 // Allocate ncols (power of two, 32..512) TMEM columns; the base address is
 // written to *smem_slot.  Executed by one full warp.
