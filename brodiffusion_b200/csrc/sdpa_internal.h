@@ -13,7 +13,9 @@ struct SdpaDevArgs {
     void* o[2];
     long long o_ld[2];
     long long o_bs[2];
-    int q_ctas0;    // CTAs covering query segment 0
+    int q_ctas0;    // pairs of query tiles covering query segment 0
+    int q_ctas, num_heads;
+    int whole_items;   // items (pair of tiles, head, batch) that a CTA does as a whole; the others are two CTAs
     int kv_tiles0;  // 128-key tiles covering key segment 0
     int kv_tiles;   // key tiles in total
     int mask_mode;

@@ -1,6 +1,7 @@
 // Softmax attention forward for head_dim 64 / 128 on the sm_100a tensor cores.
 //
-// One CTA owns two 128-row query tiles of one (batch, head) and walks the key
+// One CTA owns two 128-row query tiles of one (batch, head), or in the last wave of a launch
+// a single one (launch_t), and walks the key
 // tiles (128 keys each).  Roles (12 warps, three warpgroups):
 //   warps 0-3  : softmax of query tile 0   (one thread per query row)
 //   warps 4-7  : softmax of query tile 1
@@ -27,7 +28,7 @@
 // a step apart, take turns in it (it is occupied from the first MMA until the fetch
 // is over, about 1100 cycles of a step per tile).  At 64 each tile has its own, and the
 // scores are issued in turns all the same: two tiles in step want the exponential unit at
-// the same time (4096 x 4096, 8 heads of 40, FP16: 57.9 us in step, 53.9 in turns).  A key step takes 2790 cycles (3550
+// the same time (4096 x 4096, 8 heads of 40, FP16: 57.9 us in step, 53.9 in turns).  A key step takes 2720 cycles (3550
 // when P overwrote S and Q.K^T of step j+1 had to wait for P.V of step j): 4608 x 4608,
 // 24 heads of 128, 224 -> 199 us before the power cap sets in; 16896 x 16896, two batch
 // items, under the cap (SM clock 1.48 GHz instead of 1.85) 6.34 -> 5.77 ms.
@@ -164,7 +165,8 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 // warps 12-15 (rounded to the storage type, as the reference's scale_inplace on its
 // k_full_ / v_full_ copies does, src/dit/qwenimage21_forward.cpp:606-645); the
 // softmax code does not change.
-template <int HD, bool kBf16, int kHooks, bool kScale>
+// kMixed: some CTAs of the launch have one query tile (launch_t); without it every CTA has two.
+template <int HD, bool kBf16, int kHooks, bool kScale, bool kMixed>
 __global__ void __launch_bounds__(Roles<kScale>::kThreads, 1)
 sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant__ CUtensorMap tmQ1,
                  const __grid_constant__ CUtensorMap tmK0, const __grid_constant__ CUtensorMap tmK1,
@@ -197,17 +199,34 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
 
     const int warp = warp_index();
     const int lane = threadIdx.x & 31;
-    const int head = blockIdx.y;
-    const int batch = blockIdx.z;
-    const int qseg = (static_cast<int>(blockIdx.x) >= a.q_ctas0) ? 1 : 0;
-    const int qrow0 = (qseg ? static_cast<int>(blockIdx.x) - a.q_ctas0 : static_cast<int>(blockIdx.x)) * 2 * kBM;
+    // Work item of this CTA: two query tiles of one (batch, head), or one of them.
+    int q_cta = static_cast<int>(blockIdx.x), head = static_cast<int>(blockIdx.y), batch = static_cast<int>(blockIdx.z);
+    int tile0 = 0, n_tiles = 2;
+    if constexpr (kMixed) {
+        int item = static_cast<int>(blockIdx.x);
+        if (item >= a.whole_items) {
+            n_tiles = 1;
+            tile0 = (item - a.whole_items) & 1;
+            item = a.whole_items + ((item - a.whole_items) >> 1);
+        }
+        q_cta = item % a.q_ctas;
+        head = item / a.q_ctas % a.num_heads;
+        batch = item / a.q_ctas / a.num_heads;
+    }
+    const int qseg = q_cta >= a.q_ctas0 ? 1 : 0;
+    const int qrow0 = ((qseg ? q_cta - a.q_ctas0 : q_cta) * 2 + tile0) * kBM;
     const int seg_rows = qseg ? a.q_rows[1] : a.q_rows[0];
     const int q_global0 = (qseg ? a.q_rows[0] : 0) + qrow0;
+    if constexpr (kMixed) {
+        if (qrow0 >= seg_rows) return;               // the second tile of a segment's last rows
+        if (seg_rows - qrow0 <= kBM) n_tiles = 1;
+    }
+    const int n_t = kMixed ? n_tiles : 2;
 
     // Key tiles this CTA has to visit.
     int n_kv = a.kv_tiles;
     if (a.mask_mode == 1) {
-        const int last = q_global0 + min(2 * kBM, seg_rows - qrow0) - 1;
+        const int last = q_global0 + min(n_t * kBM, seg_rows - qrow0) - 1;
         const int max_key = last + a.q_offset;
         int n = 0;
         for (int t = 0; t < a.kv_tiles; ++t) {
@@ -274,7 +293,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             listed = true;
             if (warp == 9 && lane == 0) {      // the query tiles travel meanwhile
                 load_q(0);
-                load_q(1);
+                if (n_t == 2) load_q(1);
             }
             __syncwarp();
 #pragma unroll 2
@@ -307,7 +326,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
     // the j-th key tile of this CTA
     auto tile_at = [&](int j) { return kv_tile(a, listed ? tile_list[j] : j); };
 
-    if (warp < 8) {
+    if (warp < 4 * n_t) {
         // ------------------------------------------------ softmax + epilogue
         setmaxnreg_inc<Roles<kScale>::kRegsSoftmax>();
         const int t = warp >> 2;
@@ -623,7 +642,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
         const float inv = (l_sum > 0.0f) ? 1.0f / l_sum : 0.0f;
         if constexpr (kHooks == 2) {
             if (a.lse != nullptr && ok && row_in_seg < seg_rows) {
-                float* st = a.lse + ((static_cast<long long>(batch) * gridDim.y + head) * a.lq_total + q_glob) * 2;
+                float* st = a.lse + ((static_cast<long long>(batch) * a.num_heads + head) * a.lq_total + q_glob) * 2;
                 st[0] = m_ref * sl2;
                 st[1] = l_sum;
             }
@@ -705,7 +724,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                 }
             }
         }
-    } else {
+    } else if (warp >= 8) {
         setmaxnreg_dec<Roles<kScale>::kRegsOther>();
         if (warp == 8) {
             // -------------------------------------------------- Q.K^T issuer
@@ -722,14 +741,16 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             uint32_t phase = 0;
             bool ok = true;
             for (int j = 0; ok && j < n_kv; ++j) {
+#pragma unroll
                 for (int t = 0; t < 2; ++t) {
+                    if (t == 1 && n_t == 1) continue;
                     if (j == 0) {
                         ok = mbar_wait(&q_full[t], 0);
                         if (ok && a.q_fused) ok = mbar_wait(&q_ready[t], 0);
                     }
                     // the other tile holds the scores before these in registers: with one buffer it
                     // was that buffer's last user, with two this keeps the tiles in turns
-                    if (ok && (j > 0 || t > 0)) ok = mbar_wait(&s_free[t ^ 1], static_cast<uint32_t>((t ? j : j - 1) & 1));
+                    if (ok && (j > 0 || t > 0)) ok = mbar_wait(&s_free[n_t == 2 ? t ^ 1 : 0], static_cast<uint32_t>((t ? j : j - 1) & 1));
                     if (ok && t == 0) ok = mbar_wait(&k_rdy[slot], phase);
                     tc_fence_after();
                     if (elect_one() && ok) {
@@ -743,7 +764,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                                     make_smem_desc_sw128(kb + off, 16, 1024), idesc_qk, kk > 0 ? 1u : 0u);
                         }
                         umma_commit(&s_full[t]);
-                        if (t == 1) umma_commit(&k_empty[slot]);
+                        if (t == 1 || n_t == 1) umma_commit(&k_empty[slot]);
                     }
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
@@ -760,7 +781,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             bool ok = true;
             for (int j = 0; ok && j < n_kv; ++j) {
                 ok = mbar_wait(&v_rdy[slot], phase);
-                for (int t = 0; t < 2; ++t) {
+                for (int t = 0; t < n_t; ++t) {
                     if (ok) ok = mbar_wait(&p_full[t], static_cast<uint32_t>(j & 1));
                     tc_fence_after();
                     if (elect_one() && ok) {
@@ -773,7 +794,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                                     (j > 0 || kk > 0) ? 1u : 0u);
                         }
                         umma_commit(&pv_done[t]);
-                        if (t == 1) umma_commit(&v_empty[slot]);
+                        if (t == 1 || n_t == 1) umma_commit(&v_empty[slot]);
                     }
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
@@ -797,7 +818,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                         tma_load_4d(smem_k + ks * C::kTileBytes + c * kChunkBytes, ti.seg ? &tmK1 : &tmK0, &k_full[ks],
                                     c * 64, kv_head, ti.row0, batch);
                     }
-                    if (j == 0 && !listed) load_q(1);         // after what the first scores need
+                    if (j == 0 && !listed && n_t == 2) load_q(1);         // after what the first scores need
                     issued = 2 * j + 1;
                     if (++ks == KS) { ks = 0; kph ^= 1; }
                     if (j >= VS) ok = mbar_wait(&v_empty[vs], vph);
@@ -814,7 +835,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                     // Unwinding after a wait ran out: let the copies already in
                     // flight land before the CTA gives its shared memory back.
                     mbar_wait(&q_full[0], 0);
-                    mbar_wait(&q_full[1], 0);
+                    if (n_t == 2) mbar_wait(&q_full[1], 0);
                     const int nk = (issued + 1) / 2, nv = issued / 2;
                     for (int i = max(0, nk - KS); i < nk; ++i) mbar_wait(&k_full[i % KS], static_cast<uint32_t>((i / KS) & 1));
                     for (int i = max(0, nv - VS); i < nv; ++i) mbar_wait(&v_full[i % VS], static_cast<uint32_t>((i / VS) & 1));
@@ -902,13 +923,28 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
 template <int HD, bool kBf16, int kHooks, bool kScale>
 cudaError_t launch_t(const SdpaLaunch& L, cudaStream_t stream) {
     using C = Cfg<HD, kHooks == 2>;
-    auto kern = sdpa_tc05_kernel<HD, kBf16, kHooks, kScale>;
-    cudaError_t e = set_max_smem_once(kern, C::kSmemBytes);
-    if (e != cudaSuccess) return e;
-    dim3 grid(static_cast<unsigned>(L.q_ctas), static_cast<unsigned>(L.num_heads),
-              static_cast<unsigned>(L.batch));
-    return launch_dependent(kern, grid, dim3(Roles<kScale>::kThreads), C::kSmemBytes, stream, L.tmQ[0], L.tmQ[1], L.tmK[0],
-                            L.tmK[1], L.tmV[0], L.tmV[1], L.args);
+    // The CTAs of a last wave that fills no more than half of the SMs have one query tile each: a key step of
+    // one tile takes about 1900 cycles, of two 2720, so that the wave ends after two thirds of the time.  A
+    // row's arithmetic is the same in both.  1024 x 1024, 8 heads of 80 (32 items) 16.4 -> 13.7 us, 2042 x 2042,
+    // 24 heads of 128 (192 items) 58.2 -> 53.6; a wave of 92 (2499 x 2499) would be two.  Calls without such a
+    // wave keep the kernel whose CTAs all have two tiles: it issues its MMAs a little faster (4096 x 4096, 8 heads of
+    // 40, 50.1 us against 53.1).
+    const int sms = sm_count();
+    const long long items = static_cast<long long>(L.q_ctas) * L.num_heads * L.batch, rest = items % sms;
+    SdpaDevArgs args = L.args;
+    args.q_ctas = L.q_ctas;
+    args.num_heads = L.num_heads;
+    args.whole_items = static_cast<int>(items - rest);
+    const bool mixed = rest > 0 && 2 * rest <= sms && items < (1LL << 30);
+    const dim3 grid = mixed ? dim3(static_cast<unsigned>(items + rest))
+                            : dim3(static_cast<unsigned>(L.q_ctas), static_cast<unsigned>(L.num_heads), static_cast<unsigned>(L.batch));
+    auto go = [&](auto kern) {
+        cudaError_t e = set_max_smem_once(kern, C::kSmemBytes);
+        if (e != cudaSuccess) return e;
+        return launch_dependent(kern, grid, dim3(Roles<kScale>::kThreads), C::kSmemBytes, stream, L.tmQ[0], L.tmQ[1], L.tmK[0],
+                                L.tmK[1], L.tmV[0], L.tmV[1], args);
+    };
+    return mixed ? go(sdpa_tc05_kernel<HD, kBf16, kHooks, kScale, true>) : go(sdpa_tc05_kernel<HD, kBf16, kHooks, kScale, false>);
 }
 
 template <int HD, bool kBf16>

@@ -527,3 +527,37 @@ def test_row_scales_have_the_bits_of_scaled_rows(bd, dtype, hd, Lk, which):
     bd.sdpa_fwd(q, scaled(k) if "k" in which else k, scaled(v) if "v" in which else v, ref, nh)
     assert bd.device_status() == 0
     assert torch.equal(got, ref)
+
+
+# One hundred and ninety-two pairs of query tiles: the last forty-four run as single tiles.  Ninety-six (half the
+# heads) all run as pairs, and the rows' arithmetic is the same: the bits have to be.  Segments end in one
+# tile, in two, and in part of the second.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hd", [128, 40])
+@pytest.mark.parametrize("kind", ["plain", "causal", "masked", "scaled"])
+def test_single_query_tiles_have_the_bits_of_pairs(bd, dtype, hd, kind):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms != 148:
+        pytest.skip("the wave sizes below are those of 148 SMs")
+    nh, rows, Lk = 24, [300, 1400], 700                      # 2 + 6 pairs of tiles a head
+    gen = torch.Generator(device="cuda").manual_seed(8900 + hd)
+    rnd = lambda n: torch.randn(n, nh * hd, device="cuda", generator=gen).to(dtype)
+    q, k, v = [rnd(n) for n in rows], rnd(Lk), rnd(Lk)
+    kw = {}
+    if kind == "causal":
+        kw["mask_mode"] = bd.MASK_CAUSAL
+    if kind == "masked":
+        kw["key_mask"] = (torch.rand(Lk, device="cuda", generator=gen) > 0.4).float()
+        kw["key_mask"][128:384] = 0.0
+    if kind == "scaled":
+        kw["key_scale"] = 0.5 + torch.rand(Lk, device="cuda", generator=gen)
+        kw["val_scale"] = 0.5 + torch.rand(Lk, device="cuda", generator=gen)
+    out = [torch.full_like(x, float("nan")) for x in q]
+    bd.sdpa_fwd(q, k, v, out, nh, **kw)
+    ref = [torch.full_like(x, float("nan")) for x in q]
+    for h in (0, nh // 2):
+        cols = slice(h * hd, (h + nh // 2) * hd)
+        bd.sdpa_fwd([x[:, cols] for x in q], k[:, cols], v[:, cols], [x[:, cols] for x in ref], nh // 2, **kw)
+    assert bd.device_status() == 0
+    for a, b in zip(out, ref):
+        assert torch.equal(a, b)
