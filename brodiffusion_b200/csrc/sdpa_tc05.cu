@@ -58,6 +58,7 @@ constexpr int kBN = 128;           // keys per tile
 constexpr int kChunkBytes = 128 * 128;  // one 64-column (128 B) x 128-row TMA box
 
 constexpr int kMaxListed = 512;    // key tiles a list of the tiles with a visible key has room for
+constexpr int kPartTile = 0x8000;  // set in its entries for tiles that have a masked key too
 
 // kBias: the softmax warps have 4 KB of shared memory each for rows of a logit bias, in the place of the third K tile.
 template <int HD, bool kBias>
@@ -306,17 +307,22 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                     mv[w] = c < ti.valid ? __ldg(a.key_mask + ti.kbase + c) : 0.0f;
                 }
                 const bool seen = __any_sync(0xffffffffu, mv[0] != 0.0f || mv[1] != 0.0f || mv[2] != 0.0f || mv[3] != 0.0f);
-                if (lane == 0) tile_list[t] = seen ? 1 : 0;
+                bool hidden = false;
+#pragma unroll
+                for (int w = 0; w < 4; ++w) hidden = hidden || (mv[w] == 0.0f && lane + 32 * w < ti.valid);
+                const bool part = __any_sync(0xffffffffu, hidden);
+                if (lane == 0) tile_list[t] = seen ? (part ? kPartTile | 1 : 1) : 0;
             }
             __syncthreads();
             // every warp counts and one writes (in place: an entry is read before it is overwritten)
             int n = 0;
             for (int t0 = 0; t0 < n_kv; t0 += 32) {
                 const int t = t0 + lane;
-                const bool on = t < n_kv && tile_list[t] != 0;
+                const int f = t < n_kv ? tile_list[t] : 0;
+                const bool on = f != 0;
                 const uint32_t m = __ballot_sync(0xffffffffu, on);
                 __syncthreads();
-                if (warp == 0 && on) tile_list[n + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(t);
+                if (warp == 0 && on) tile_list[n + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(t | (f & kPartTile));
                 n += __popc(m);
             }
             __syncthreads();
@@ -324,7 +330,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
         }
     }
     // the j-th key tile of this CTA
-    auto tile_at = [&](int j) { return kv_tile(a, listed ? tile_list[j] : j); };
+    auto tile_at = [&](int j) { return kv_tile(a, listed ? tile_list[j] & (kPartTile - 1) : j); };
 
     if (warp < 4 * n_t) {
         // ------------------------------------------------ softmax + epilogue
@@ -477,7 +483,8 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             // per lane), fetched before the wait for S so that its latency is hidden.
             uint32_t mbits[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
             if constexpr (kHooks >= 1) {
-                if (a.key_mask != nullptr) {
+                // (a list says which tiles have none, and they are passed over: 2042 keys of which 1717 are visible, 24 heads, 56.7 -> 54.2 us)
+                if (a.key_mask != nullptr && (!listed || (tile_list[j] & kPartTile) != 0)) {
                     const TileInfo tm = tile_at(j);
                     float mv[4];
 #pragma unroll
