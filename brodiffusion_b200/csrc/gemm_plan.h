@@ -42,17 +42,19 @@ BDATTN_HD constexpr bool pair_acc_reused(int tile, int pairs, int total_tiles) {
 
 // The least of the modelled times, fitted to calls of 64 x 1280 x 1280 to 9216 x 320 x 1280 (M x N x K) in
 // FP16 with cold weights on one B200; x stands for waves of CTAs (pairs), k for K blocks of 64.  Measured, in us:
-//                          64 columns  128 columns  pairs x 128  pairs x 256
-//   4096 x  320 x  320          6.6         4.5          -            -
-//   1024 x  640 x 2560          8.9        11.0        10.8           -
-//    576 x 1280 x 1280          6.1         7.2         7.6         11.1
-//    512 x 3072 x 3072         17.4        13.7        13.5         20.0
-//   2304 x  640 x 2560         15.1        11.9        11.8           -
-//   1024 x 3072 x 3072         30.5        31.4        21.8         21.0
-//   4096 x 3072 x 3072         92          88          64.5         57
-//   GEGLU  256 x  640 -> 2560   8.3          -          6.7          9.3
-//   GEGLU 1024 x  640 -> 2560  18.1          -         12.9         13.4
-//   GEGLU 4096 x  320 -> 1280  22.3          -         18.1         16.4
+//                          64 columns  80     96     128 columns  pairs x 128  pairs x 256
+//   4096 x  320 x  320          6.6      4.2    4.2       4.5          -            -
+//   4096 x  320 x 1280          9.3      6.9    7.4       7.9          -            -
+//   9216 x  320 x 1280         16.8     10.9   16.8      17.4          -            -
+//   1024 x  640 x 2560          8.9      9.4   10.5      11.0        10.7           -
+//    576 x 1280 x 1280          6.1      6.5    6.7       7.2         7.4         11.1
+//    512 x 3072 x 3072         17.5     17.4   12.6      13.7        13.2         20.0
+//   2304 x  640 x 2560         15.3     10.0   11.1      11.9        11.5           -
+//   1024 x 3072 x 3072         30.5       -      -       31.4        21.8         21.0
+//   4096 x 3072 x 3072         92         -      -       88          64.5         57
+//   GEGLU  256 x  640 -> 2560   8.3       -      -         -          6.4          8.8
+//   GEGLU 1024 x  640 -> 2560  18.1       -      -         -         12.0         12.6
+//   GEGLU 4096 x  320 -> 1280  22.3       -      -         -         16.5         14.9
 //   Q, K, V with norm + RoPE, K = 3072: 256 rows 18.7 with 128 columns, 26.8 with 256; 512 rows 29.1 and
 //   27.9; 1024 rows 50.4 and 46.6
 // A tile split over CTAs pays where few tiles have a long K: 64 x 1280 x 5120 14.3 us, 10.1 over two CTAs, 7.8 over
@@ -91,6 +93,13 @@ inline GemmPlan plan_gemm(const GemmShape* p, int n, int sms) {
         else offer(best, x <= 1.0 ? 2.2 + 0.165 * kb : 2.5 + x * (0.8 + 0.155 * kb));
     }
     if (!geglu && !heads) {
+        // Between 64 and 128 columns for widths that these divide badly (320, 640) and for what 64 columns make two
+        // waves of; with several CTAs to an SM only 80 columns, whose rings still fit twice (a short K has
+        // rings of two stages there and gains nothing: 9216 x 320 x 320 8.0 us, 7.7 with 64 or 128).
+        for (int w = 80; w < 128; w += 16) {
+            if (waves(w, 1) <= 1.0) offer({false, w, 1}, 1.6 + 0.6 * w / 64 + (0.12 + 0.045 * w / 64) * kb);
+            else if (w == 80 && kb > 8) offer({false, w, 1}, 2.5 + waves(w, 1) * (1.15 + 0.14 * kb));
+        }
         const double x = waves(128, 1);
         offer({false, 128, 1}, x <= 1.0 ? 2.8 + 0.21 * kb : 2.0 + x * (1.0 + 0.30 * kb));
         for (int s = 2; s <= 8 && kb >= 3 * s && kb_min >= s && tiles(64) * s * 2 <= 3LL * sms; s *= 2) {

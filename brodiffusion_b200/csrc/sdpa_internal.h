@@ -168,7 +168,7 @@ struct GemmProblem {
     long long ldc;
     const void* bias;   // N values of the output dtype, or null
     int tiles_m, tiles_n;
-    int n_tile;         // MMA N of a tile, 64 or 128 = rows of the B box; the head_dim with norm_rope
+    int n_tile;         // MMA N of a tile, 64 to 128 = rows of the B box; the head_dim with norm_rope
     int geglu_offset;   // 0, or D_out
     // Per-head RMSNorm + RoPE epilogue (head tiles with n_tile == head_dim only):
     const void* gain;   // head_dim values, or null

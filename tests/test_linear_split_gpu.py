@@ -1,4 +1,4 @@
-"""Linear layers whose tiles are split over a cluster."""
+"""Linear layers on the one-tile kernel: tiles split over a cluster, and tiles of widths between 64 and 128."""
 import pytest
 import torch
 
@@ -13,6 +13,19 @@ def test_linear_split_rows_over_the_cluster(bd, oracle, M, N, K):
     """The rows of a split tile are dealt out to the CTAs of its cluster: ragged rows and columns, two to eight CTAs."""
     x, w = synth.activations((M, K), 9950), synth.round_bf16(synth.normal((N, K), 9951, 0, 1.0 / K ** 0.5))
     b = synth.weights((N,), 9952)
+    y = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    bd.linear_fwd(G.dev(x), G.dev(w), G.dev(b), y[:M, :N])
+    assert bd.device_status() == 0
+    G.check(G.host(y[:M, :N]), oracle.linear(x, w, b), max_abs=2.5e-2, what=f"linear {M}x{N}x{K}")
+    assert bool((y[M] == 7.0).all()) and bool((y[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(2300, 640, 640), (4000, 320, 72), (500, 3072, 200), (5000, 328, 600), (1024, 648, 1288)])
+def test_linear_tile_widths_between_64_and_128(bd, oracle, M, N, K):
+    """Widths of 80, 96 and 112 columns (csrc/gemm_plan.h): no multiple of the epilogue's 32, ragged rows, columns and
+    K, one CTA to an SM and two.  Bound as in test_qkv_proj_gpu.py: one rounding of values of up to five."""
+    x, w = synth.activations((M, K), 9960), synth.round_bf16(synth.normal((N, K), 9961, 0, 1.0 / K ** 0.5))
+    b = synth.weights((N,), 9962)
     y = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
     bd.linear_fwd(G.dev(x), G.dev(w), G.dev(b), y[:M, :N])
     assert bd.device_status() == 0
