@@ -5,6 +5,9 @@
 // src/dit/qwenimage21_forward.cpp:301-302 -> 124-200).  Here one thread
 // computes one (token, pair) cell with the same double-precision formula, so
 // the tables never cross PCIe.  Tables are FP32 (rows, head_dim / 2).
+// The kernel reads nothing but its arguments: it waits for the kernel before it only when it stores, so that the
+// power and the sine and cosine, a chain of double-precision latencies, run while that one ends (320 rows behind
+// another kernel 2.6 -> 2.3 us, a 256-token extract step 44.8 -> 43.7).
 #include "sdpa_internal.h"
 #include "tc05.cuh"
 
@@ -13,7 +16,6 @@ namespace {
 
 __global__ void rope_tables_kernel(const RopeTableArgs a) {
     dependents_may_launch();
-    wait_for_prior_grid();
     const int half = a.half;
     const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= static_cast<long long>(a.rows) * half) return;
@@ -48,16 +50,15 @@ __global__ void rope_tables_kernel(const RopeTableArgs a) {
             const double omega = 1.0 / pow(static_cast<double>(a.theta),
                                            (2.0 * pl) / static_cast<double>(a.axes[axis]));
             const double ang = static_cast<double>(pos) * omega;
-            c = cos(ang);
-            sn = sin(ang);
+            sincos(ang, &sn, &c);
         }
     } else {
         const double freq = pow(static_cast<double>(a.theta),
                                 -2.0 * static_cast<double>(pl) / static_cast<double>(a.axes[axis]));
         const double ang = static_cast<double>(pos) * freq;
-        c = cos(ang);
-        sn = sin(ang);
+        sincos(ang, &sn, &c);
     }
+    wait_for_prior_grid();
     a.cos_out[idx] = static_cast<float>(c);
     a.sin_out[idx] = static_cast<float>(sn);
 }
