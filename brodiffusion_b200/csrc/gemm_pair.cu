@@ -9,11 +9,10 @@
 //     weight rows, so a K block of 64 costs an SM 32 KB of L2 reads per 512 tensor-pipe cycles, with
 //     128 columns 24 KB per 256.  An SM is fed at about 70 bytes a cycle, so the wide tile is the better
 //     one wherever it fills the SMs and the narrow one where it does not: QKV of 256 rows of 3072 is 36
-//     tiles of 256 columns for 74 pairs, 26.8 us, or 72 of 128, 18.7; of 512 rows 72 wide tiles 27.9,
-//     144 narrow ones 29.1;
-//   * a stage is 128 columns of K: the wait and the commit around a stage cost the issuing thread about
-//     250 cycles, which with four MMAs of 64 to a stage made 610 cycles of a K block of 64 where the tensor
-//     pipe needs 512;
+//     tiles of 256 columns for 74 pairs, 26.5 us, or 72 of 128, 18.2; of 512 rows 72 wide tiles 27.7,
+//     144 narrow ones 29.2;
+//   * a stage is 128 columns of K: the wait and the commit around a stage stand against sixteen MMAs' worth of the
+//     tensor pipe and not eight (with stages of 64 a K block took 610 cycles where the pipe needs 512);
 //   * the pairs walk a list of tiles (up to three problems in one launch; tiles of one
 //     column block adjacent, in groups of sixteen row blocks, so that what runs together
 //     reads few weight and few activation tiles);

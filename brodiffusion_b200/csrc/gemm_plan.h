@@ -52,11 +52,11 @@ BDATTN_HD constexpr bool pair_acc_reused(int tile, int pairs, int total_tiles) {
 //   2304 x  640 x 2560         15.3     10.0   11.1      11.9        11.5           -
 //   1024 x 3072 x 3072         30.5       -      -       31.4        21.8         21.0
 //   4096 x 3072 x 3072         92         -      -       88          64.5         57
-//   GEGLU  256 x  640 -> 2560   8.3       -      -         -          6.4          8.8
-//   GEGLU 1024 x  640 -> 2560  18.1       -      -         -         12.0         12.6
-//   GEGLU 4096 x  320 -> 1280  22.3       -      -         -         16.5         14.9
-//   Q, K, V with norm + RoPE, K = 3072: 256 rows 18.7 with 128 columns, 26.8 with 256; 512 rows 29.1 and
-//   27.9; 1024 rows 50.4 and 46.6
+//   GEGLU  256 x  640 -> 2560   8.3       -      -         -          6.3          8.8
+//   GEGLU 1024 x  640 -> 2560  18.1       -      -         -         12.0         12.5
+//   GEGLU 4096 x  320 -> 1280  22.2       -      -         -         17.0         14.9
+//   Q, K, V with norm + RoPE, K = 3072: 256 rows 18.2 with 128 columns, 26.5 with 256; 512 rows 29.2 and
+//   27.7; 1024 rows 50.3 and 46.7
 // A tile split over CTAs pays where few tiles have a long K: 64 x 1280 x 5120 14.3 us, 10.1 over two CTAs, 7.8 over
 // four, 9.2 over eight; 256 x 1280 x 5120 14.2, 11.4, 13.7.  The splits are entered at about 0.8 us less than they
 // take when all CTAs run at once, and three when not: with the times themselves launches of a few tiles would be

@@ -112,3 +112,30 @@ def test_errors(bd):
     b = torch.zeros(100, 10, device="cuda")
     with pytest.raises(bd.BdattnError, match=r"^joint_attention_traced: bias block"):
         bd.sdpa_traced_fwd(q, q, q, q.clone(), 2, bias=b)
+
+
+@pytest.mark.parametrize("hd,split,row0,rows,cols,offset,ld", [
+    (128, 70, 75, 300, 200, 0, 200), (128, 256, 256, 250, 256, 4, 264),      # rows of 16-byte pieces
+    (128, 70, 40, 170, 131, 0, 131), (64, 129, 1, 377, 130, 1, 200),         # rows and bases that are no multiple of them
+    (40, 128, 128, 1, 1, 3, 8), (64, 300, 0, 506, 506, 2, 510)])
+def test_bias_rows_of_any_alignment(bd, oracle, hd, split, row0, rows, cols, offset, ld):
+    """The bias is copied in pieces of 32 rows x 32 columns: blocks that begin and end inside a piece, a tile and a
+    segment, strides above the width, bases off a 16-byte boundary."""
+    nh, L = 3, 506
+    q, k, v = (synth.activations((L, nh * hd), 9950 + i) for i in range(3))
+    wide = torch.full((rows, ld + offset), 1e30, device="cuda")              # what lies around it must not be read as bias
+    bias = wide[:, offset:offset + cols]
+    ref_bias = synth.normal((rows, cols), 9953, 0, 1.0)
+    bias.copy_(G.dev(ref_bias, torch.float32))
+    tq, tk, tv = G.dev(q), G.dev(k), G.dev(v)
+    out = torch.full_like(tq, float("nan"))
+    seg = lambda t: [t[:split], t[split:]]
+    amap = bd.sdpa_traced_fwd(seg(tq), seg(tk), seg(tv), seg(out), nh, bias=bias, bias_row0=row0, map_row0=row0,
+                              map_rows=rows, map_cols=cols)
+    assert bd.device_status() == 0
+    # (the oracle's bias reaches to the last query: rows without one are zero there)
+    to_the_end = np.concatenate([ref_bias, np.zeros((L - row0 - rows, cols), np.float32)])
+    ref, avg = oracle.sdpa(q, k, v, nh, bias=to_the_end, bias_row0=row0, want_avg=True)
+    G.check(G.host(out), ref, what="biased output")
+    # FP32 scores on both sides; 2^-22 from each exponential and 1e-5 from the sums
+    assert np.abs(G.host(amap) - avg[row0:row0 + rows, :cols]).max() <= 1e-4 * avg.max()
