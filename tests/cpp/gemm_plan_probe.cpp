@@ -5,7 +5,7 @@ using namespace bdattn;
 
 extern "C" {
 
-// shapes: n rows of M, N, K; out: pair, width, split
+// shapes: n rows of M, N, K; out: pair, width, split, pair_cols
 void probe_plan(const int* shapes, int n, int geglu, int heads, int sms, int* out) {
     GemmShape s[3];
     for (int i = 0; i < n; ++i)
@@ -15,6 +15,7 @@ void probe_plan(const int* shapes, int n, int geglu, int heads, int sms, int* ou
     out[0] = p.pair;
     out[1] = p.width;
     out[2] = p.split;
+    out[3] = p.pair_cols;
 }
 
 // the fewest K blocks that any CTA of a tile has

@@ -19,10 +19,17 @@ def plan(tmp_path_factory):
 
     def run(shapes, geglu=False, heads=False, sms=148):
         flat = (C.c_int * (3 * len(shapes)))(*itertools.chain(*shapes))
-        out = (C.c_int * 3)()
+        out = (C.c_int * 4)()
         lib.probe_plan(flat, len(shapes), int(geglu), int(heads), sms, out)
+        run.pair_cols = out[3]
         return bool(out[0]), out[1], out[2]
 
+    def kernel(shapes, **kw):
+        """Name of the kernel and tile width, and over how many CTAs a tile is split."""
+        pair, width, split = run(shapes, **kw)
+        return f"p{run.pair_cols}" if pair else str(width), split
+
+    run.kernel = kernel
     run.fewest_blocks = lib.probe_fewest_blocks
     run.acc_reused = lib.probe_acc_reused
     return run
@@ -52,6 +59,20 @@ def test_every_cta_of_a_split_tile_has_a_k_block(plan):
     ([(128, 64, 640)], 1)])
 def test_split_is_bounded_by_the_shortest_k(plan, shapes, split):
     assert plan(shapes)[2] == split
+
+
+# kernel (64 to 128: columns of the one-tile kernel; p128, p256: pairs) that the measurements beside the rule have as
+# the fastest or within 3 % of it: short K, where a pair waits for its epilogues; long K; rows off 32 bytes
+@pytest.mark.parametrize("kind,shape,kernels", [
+    ("plain", (2304, 2560, 320), ("80", "112", "128")), ("plain", (4096, 1280, 320), ("80", "112", "128")),
+    ("plain", (9216, 640, 320), ("80", "112", "128")), ("plain", (4096, 2560, 112), ("96", "128")),
+    ("plain", (9216, 1280, 640), ("p256",)), ("plain", (2240, 2304, 2240), ("p128",)),
+    ("plain", (576, 5120, 448), ("p128",)), ("plain", (576, 4096, 936), ("p256",)), ("plain", (2240, 1024, 2240), ("128",)),
+    ("geglu", (4096, 1280, 2808), ("p256",)), ("geglu", (64, 5120, 1280), ("p128",)), ("geglu", (4096, 1280, 320), ("p256",)),
+    ("heads", (3580, 1024, 1288), ("p256",)), ("heads", (256, 3072, 3072), ("p128",)), ("heads", (1024, 3072, 3072), ("p256",))])
+def test_plan_is_the_measured_best(plan, kind, shape, kernels):
+    n = 3 if kind == "heads" else 1
+    assert plan.kernel([shape] * n, geglu=kind == "geglu", heads=kind == "heads")[0] in kernels
 
 
 def test_geglu_is_never_split(plan):
