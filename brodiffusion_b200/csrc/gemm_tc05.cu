@@ -226,7 +226,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
         // epilogue: warp w reads TMEM lanes 32 * (w % 4) ..
         const int q = warp & 3;
         const int row = m0 + q * 32 + lane;
-        if constexpr (!kNormRope) {
+        if (!kNormRope || !p.norm_rope) {
             // the tile's bias, zero where there is none, while the tile is computed
             const int t = static_cast<int>(threadIdx.x) - 64;
             const bool on = p.bias != nullptr && t < p.n_tile && n0 + t < p.N;
