@@ -129,6 +129,8 @@ def _packer(cls):
 _pack_sdpa, _pack_qkv, _pack_qkvo = _packer(SdpaParams), _packer(QkvProjParams), _packer(QkvoParams)
 _pack_job = _packer(NormRopeJob)
 
+_STRUCTURES = [C.POINTER(t) for t in (SdpaParams, QkvProjParams, QkvoParams, NormRopeJob)]
+
 _lib = None
 
 
@@ -146,26 +148,25 @@ def lib():
                 f"{path} is missing: build it with `python -m brodiffusion_b200._build` "
                 "(there is no fallback implementation)")
         L = C.CDLL(path)
-        # (parameter structures are passed as void pointers: a structure by reference or its packed bytes)
         L.bdattn_version.restype = C.c_int
         L.bdattn_last_error.restype = C.c_char_p
         L.bdattn_device_status.argtypes = [C.POINTER(C.c_int), C.c_int]
-        L.bdattn_sdpa_fwd.argtypes = [C.c_void_p, C.c_void_p]
-        L.bdattn_sdpa_fwd_allgather.argtypes = [C.c_void_p, C.POINTER(C.c_void_p),
+        L.bdattn_sdpa_fwd.argtypes = [C.POINTER(SdpaParams), C.c_void_p]
+        L.bdattn_sdpa_fwd_allgather.argtypes = [C.POINTER(SdpaParams), C.POINTER(C.c_void_p),
                                                 C.POINTER(C.c_void_p), C.c_int, C.c_void_p]
-        L.bdattn_sdpa_fwd_allgather_multicast.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p,
+        L.bdattn_sdpa_fwd_allgather_multicast.argtypes = [C.POINTER(SdpaParams), C.c_void_p, C.c_void_p,
                                                           C.c_void_p]
         L.bdattn_mgpu_init.argtypes = [C.POINTER(C.c_void_p), C.POINTER(C.c_int), C.c_int]
         L.bdattn_mgpu_destroy.argtypes = [C.c_void_p]
         L.bdattn_mgpu_size.argtypes = [C.c_void_p]
         L.bdattn_mgpu_barrier.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_void_p]
-        L.bdattn_mgpu_sdpa_fwd_headsharded.argtypes = [C.c_void_p, C.c_int, C.c_void_p,
+        L.bdattn_mgpu_sdpa_fwd_headsharded.argtypes = [C.c_void_p, C.c_int, C.POINTER(SdpaParams),
                                                        C.POINTER(C.c_void_p), C.c_longlong, C.c_longlong,
                                                        C.c_int, C.c_void_p]
         L.bdattn_sdpa_traced_workspace_bytes.restype = C.c_size_t
         L.bdattn_sdpa_traced_workspace_bytes.argtypes = [C.c_int, C.c_int]
-        L.bdattn_sdpa_traced_fwd.argtypes = [C.c_void_p, C.POINTER(TraceParams), C.c_void_p]
-        L.bdattn_rmsnorm_rope.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int,
+        L.bdattn_sdpa_traced_fwd.argtypes = [C.POINTER(SdpaParams), C.POINTER(TraceParams), C.c_void_p]
+        L.bdattn_rmsnorm_rope.argtypes = [C.POINTER(NormRopeJob), C.c_int, C.c_int, C.c_int,
                                           C.c_int, C.c_float, C.c_int, C.c_void_p]
         L.bdattn_linear_attn_relu_fwd.argtypes = [
             C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,
@@ -180,10 +181,10 @@ def lib():
                                               C.c_void_p, C.c_void_p, C.c_void_p]
         L.bdattn_qkvo_workspace_bytes.restype = C.c_size_t
         L.bdattn_qkvo_workspace_bytes.argtypes = [C.c_int] * 4
-        L.bdattn_qkvo_fwd.argtypes = [C.c_void_p, C.c_void_p]
+        L.bdattn_qkvo_fwd.argtypes = [C.POINTER(QkvoParams), C.c_void_p]
         L.bdattn_qkvo_static_capacity.restype = C.c_size_t
-        L.bdattn_qkvo_fwd_static.argtypes = [C.c_void_p, C.c_void_p]
-        L.bdattn_qkv_norm_rope_fwd.argtypes = [C.c_void_p, C.c_void_p]
+        L.bdattn_qkvo_fwd_static.argtypes = [C.POINTER(QkvoParams), C.c_void_p]
+        L.bdattn_qkv_norm_rope_fwd.argtypes = [C.POINTER(QkvProjParams), C.c_void_p]
         L.bdattn_project_kv.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_longlong, C.c_void_p,
                                         C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                         C.c_longlong, C.c_int, C.c_int, C.c_void_p]
@@ -197,6 +198,13 @@ def lib():
                                            C.c_int, C.c_void_p]
         L.bdattn_add_row_bias.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_longlong,
                                           C.c_int, C.c_void_p]
+        # The same entry points for this module's own calls, which pass packed structures (bytes) as pointers
+        L.packed = {}
+        for name in ("sdpa_fwd", "sdpa_fwd_allgather", "sdpa_fwd_allgather_multicast", "mgpu_sdpa_fwd_headsharded",
+                     "sdpa_traced_fwd", "rmsnorm_rope", "qkvo_fwd", "qkvo_fwd_static", "qkv_norm_rope_fwd"):
+            fn = L["bdattn_" + name]             # a function object of its own
+            fn.argtypes = [C.c_void_p if t in _STRUCTURES else t for t in getattr(L, "bdattn_" + name).argtypes]
+            L.packed[name] = fn
         _lib = L
     return _lib
 
@@ -341,25 +349,25 @@ def sdpa_fwd(q, k, v, out, num_heads, *, mask_mode=MASK_NONE, key_mask=None, key
                    mask_mode, _addr(key_mask), _addr(key_scale), _addr(val_scale), softmax_scale, num_kv_heads,
                    gain[0], gain[1], gain_dtype, eps, cos, sin, rope_row0)
     if _trace is not None:
-        _check(lib().bdattn_sdpa_traced_fwd(p, C.byref(_trace), _stream(stream)))
+        _check(lib().packed["sdpa_traced_fwd"](p, C.byref(_trace), _stream(stream)))
         return
     if _mgpu is not None:
         ctx, rank, replica_ptrs, replica_ld, replica_bs, total_heads = _mgpu
         arr = (C.c_void_p * len(replica_ptrs))(*replica_ptrs)
-        _check(lib().bdattn_mgpu_sdpa_fwd_headsharded(ctx, rank, p, arr, replica_ld, replica_bs,
+        _check(lib().packed["mgpu_sdpa_fwd_headsharded"](ctx, rank, p, arr, replica_ld, replica_bs,
                                                       total_heads, _stream(stream)))
         return
     if multicast_out_ptrs:
         m1 = multicast_out_ptrs[1] if len(multicast_out_ptrs) > 1 else None
-        _check(lib().bdattn_sdpa_fwd_allgather_multicast(p, multicast_out_ptrs[0], m1, _stream(stream)))
+        _check(lib().packed["sdpa_fwd_allgather_multicast"](p, multicast_out_ptrs[0], m1, _stream(stream)))
         return
     if peer_out_ptrs:
         n = len(peer_out_ptrs[0])
         a0 = (C.c_void_p * max(n, 1))(*peer_out_ptrs[0])
         a1 = (C.c_void_p * max(n, 1))(*(peer_out_ptrs[1] if len(peer_out_ptrs) > 1 else [None] * n))
-        _check(lib().bdattn_sdpa_fwd_allgather(p, a0, a1, n, _stream(stream)))
+        _check(lib().packed["sdpa_fwd_allgather"](p, a0, a1, n, _stream(stream)))
         return
-    _check(lib().bdattn_sdpa_fwd(p, _stream(stream)))
+    _check(lib().packed["sdpa_fwd"](p, _stream(stream)))
 
 
 class MultiGpu:
@@ -406,7 +414,7 @@ def rmsnorm_rope(jobs, num_heads, head_dim, *, eps=1e-6, pair_mode=ROPE_INTERLEA
         packed.append(_pack_job(x.data_ptr(), out.data_ptr(), x.shape[0], x.stride(0), out.stride(0),
                                 _addr(g), _dtype_code(g) if g is not None else F32,
                                 _addr(j.get("cos")), _addr(j.get("sin")), j.get("rope_row0", 0)))
-    _check(lib().bdattn_rmsnorm_rope(b"".join(packed), len(jobs), dtype, num_heads, head_dim, eps, pair_mode,
+    _check(lib().packed["rmsnorm_rope"](b"".join(packed), len(jobs), dtype, num_heads, head_dim, eps, pair_mode,
                                      _stream(stream)))
 
 
@@ -487,9 +495,9 @@ def qkvo_fwd(x, ctx, wq, wk, wv, wo, bo, num_heads, out, workspace, *, bq=None, 
                    *cached, _addr(key_mask), out.data_ptr(), out.shape[1], out.stride(0),
                    _addr(workspace), workspace.numel() * workspace.element_size() if workspace is not None else 0)
     if workspace is None:
-        _check(lib().bdattn_qkvo_fwd_static(p, _stream(stream)))
+        _check(lib().packed["qkvo_fwd_static"](p, _stream(stream)))
         return
-    _check(lib().bdattn_qkvo_fwd(p, _stream(stream)))
+    _check(lib().packed["qkvo_fwd"](p, _stream(stream)))
 
 
 def qkvo_static_capacity() -> int:
@@ -578,4 +586,4 @@ def qkv_norm_rope_fwd(x, wq, wk, wv, q_out, k_out, v_out, num_heads, head_dim, *
                   _addr(q_out), _addr(k_out), _addr(v_out),
                   q_out.stride(0) if q_out is not None else 0, k_out.stride(0) if k_out is not None else 0,
                   v_out.stride(0) if v_out is not None else 0)
-    _check(lib().bdattn_qkv_norm_rope_fwd(p, _stream(stream)))
+    _check(lib().packed["qkv_norm_rope_fwd"](p, _stream(stream)))
