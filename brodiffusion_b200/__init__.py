@@ -128,6 +128,13 @@ def _packer(cls):
 
 _pack_sdpa, _pack_qkv, _pack_qkvo = _packer(SdpaParams), _packer(QkvProjParams), _packer(QkvoParams)
 _pack_job = _packer(NormRopeJob)
+_FLT_MAX = struct.unpack("f", b"\xff\xff\x7f\x7f")[0]
+
+
+def _f32(x):
+    """A float that ``struct`` packs: beyond FP32 it is infinite, as in a ctypes field."""
+    return x if -_FLT_MAX <= x <= _FLT_MAX else C.c_float(x).value
+
 
 _STRUCTURES = [C.POINTER(t) for t in (SdpaParams, QkvProjParams, QkvoParams, NormRopeJob)]
 
@@ -341,13 +348,16 @@ def sdpa_fwd(q, k, v, out, num_heads, *, mask_mode=MASK_NONE, key_mask=None, key
         cos, sin = _addr(q_norm.get("cos")), _addr(q_norm.get("sin"))
         rope_row0 = q_norm.get("rope_row0", 0)
     (q0, q1), (o0, o1), (k0, k1), (v0, v1) = qd, od, kd, vd
-    p = _pack_sdpa(dtype, batch, num_heads, head_dim,
-                   len(qs), q0[0], q1[0], o0[0], o1[0], q0[1], q1[1], q0[2], q1[2], o0[2], o1[2],
-                   q0[3], q1[3], o0[3], o1[3],
-                   len(ks), k0[0], k1[0], v0[0], v1[0], k0[1], k1[1], k0[2], k1[2], v0[2], v1[2],
-                   k0[3], k1[3], v0[3], v1[3],
-                   mask_mode, _addr(key_mask), _addr(key_scale), _addr(val_scale), softmax_scale, num_kv_heads,
-                   gain[0], gain[1], gain_dtype, eps, cos, sin, rope_row0)
+    try:
+        p = _pack_sdpa(dtype, batch, num_heads, head_dim,
+                       len(qs), q0[0], q1[0], o0[0], o1[0], q0[1], q1[1], q0[2], q1[2], o0[2], o1[2],
+                       q0[3], q1[3], o0[3], o1[3],
+                       len(ks), k0[0], k1[0], v0[0], v1[0], k0[1], k1[1], k0[2], k1[2], v0[2], v1[2],
+                       k0[3], k1[3], v0[3], v1[3],
+                       mask_mode, _addr(key_mask), _addr(key_scale), _addr(val_scale), _f32(softmax_scale), num_kv_heads,
+                       gain[0], gain[1], gain_dtype, _f32(eps), cos, sin, rope_row0)
+    except struct.error as e:
+        raise TypeError(str(e)) from None
     if _trace is not None:
         _check(lib().packed["sdpa_traced_fwd"](p, C.byref(_trace), _stream(stream)))
         return
@@ -411,9 +421,12 @@ def rmsnorm_rope(jobs, num_heads, head_dim, *, eps=1e-6, pair_mode=ROPE_INTERLEA
     packed = []
     for j in jobs:
         x, out, g = j["x"], j["out"], j.get("gain")
-        packed.append(_pack_job(x.data_ptr(), out.data_ptr(), x.shape[0], x.stride(0), out.stride(0),
-                                _addr(g), _dtype_code(g) if g is not None else F32,
-                                _addr(j.get("cos")), _addr(j.get("sin")), j.get("rope_row0", 0)))
+        try:
+            packed.append(_pack_job(x.data_ptr(), out.data_ptr(), x.shape[0], x.stride(0), out.stride(0),
+                                    _addr(g), _dtype_code(g) if g is not None else F32,
+                                    _addr(j.get("cos")), _addr(j.get("sin")), j.get("rope_row0", 0)))
+        except struct.error as e:
+            raise TypeError(str(e)) from None
     _check(lib().packed["rmsnorm_rope"](b"".join(packed), len(jobs), dtype, num_heads, head_dim, eps, pair_mode,
                                      _stream(stream)))
 
@@ -489,11 +502,14 @@ def qkvo_fwd(x, ctx, wq, wk, wv, wo, bo, num_heads, out, workspace, *, bq=None, 
     cached = (0, 0, 0, 0, 0)
     if k_cached is not None:
         cached = (k_cached.data_ptr(), v_cached.data_ptr(), k_cached.shape[0], k_cached.stride(0), v_cached.stride(0))
-    p = _pack_qkvo(_dtype_code(x), num_heads, wq.shape[0], 1 if causal else 0,
-                   x.data_ptr(), x.shape[0], x.shape[1], x.stride(0), *context,
-                   _addr(wq), _addr(bq), _addr(wk), _addr(bk), _addr(wv), _addr(bv), _addr(wo), _addr(bo),
-                   *cached, _addr(key_mask), out.data_ptr(), out.shape[1], out.stride(0),
-                   _addr(workspace), workspace.numel() * workspace.element_size() if workspace is not None else 0)
+    try:
+        p = _pack_qkvo(_dtype_code(x), num_heads, wq.shape[0], 1 if causal else 0,
+                       x.data_ptr(), x.shape[0], x.shape[1], x.stride(0), *context,
+                       _addr(wq), _addr(bq), _addr(wk), _addr(bk), _addr(wv), _addr(bv), _addr(wo), _addr(bo),
+                       *cached, _addr(key_mask), out.data_ptr(), out.shape[1], out.stride(0),
+                       _addr(workspace), workspace.numel() * workspace.element_size() if workspace is not None else 0)
+    except struct.error as e:
+        raise TypeError(str(e)) from None
     if workspace is None:
         _check(lib().packed["qkvo_fwd_static"](p, _stream(stream)))
         return
@@ -580,10 +596,13 @@ def qkv_norm_rope_fwd(x, wq, wk, wv, q_out, k_out, v_out, num_heads, head_dim, *
     """``bdattn_qkv_norm_rope_fwd``: Q/K/V projections with per-head RMSNorm and
     RoPE in the GEMM epilogue."""
     g = gain_q if gain_q is not None else gain_k
-    p = _pack_qkv(_dtype_code(x), num_heads, head_dim, x.data_ptr(), x.shape[0], x.shape[1], x.stride(0),
-                  _addr(wq), _addr(wk), _addr(wv), _addr(bq), _addr(bk), _addr(bv), _addr(gain_q), _addr(gain_k),
-                  _dtype_code(g) if g is not None else F32, eps, _addr(cos), _addr(sin), rope_row0,
-                  _addr(q_out), _addr(k_out), _addr(v_out),
-                  q_out.stride(0) if q_out is not None else 0, k_out.stride(0) if k_out is not None else 0,
-                  v_out.stride(0) if v_out is not None else 0)
+    try:
+        p = _pack_qkv(_dtype_code(x), num_heads, head_dim, x.data_ptr(), x.shape[0], x.shape[1], x.stride(0),
+                      _addr(wq), _addr(wk), _addr(wv), _addr(bq), _addr(bk), _addr(bv), _addr(gain_q), _addr(gain_k),
+                      _dtype_code(g) if g is not None else F32, _f32(eps), _addr(cos), _addr(sin), rope_row0,
+                      _addr(q_out), _addr(k_out), _addr(v_out),
+                      q_out.stride(0) if q_out is not None else 0, k_out.stride(0) if k_out is not None else 0,
+                      v_out.stride(0) if v_out is not None else 0)
+    except struct.error as e:
+        raise TypeError(str(e)) from None
     _check(lib().packed["qkv_norm_rope_fwd"](p, _stream(stream)))
