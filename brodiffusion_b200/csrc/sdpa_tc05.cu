@@ -160,8 +160,8 @@ __device__ __forceinline__ void setmaxnreg_dec() {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// HOOKS: 0 = none; 1 = key_mask only; 2 = key_mask, bias and the per-row softmax
-// statistics (slower softmax path).
+// HOOKS: 0 = none; 1 = key_mask only; 2 = key_mask and the per-row softmax statistics; 3 = a logit
+// bias besides (slower softmax path).
 // SCALE: key_scale / val_scale are applied to the K / V tiles in shared memory by
 // warps 12-15 (rounded to the storage type, as the reference's scale_inplace on its
 // k_full_ / v_full_ copies does, src/dit/qwenimage21_forward.cpp:606-645); the
@@ -173,7 +173,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                  const __grid_constant__ CUtensorMap tmK0, const __grid_constant__ CUtensorMap tmK1,
                  const __grid_constant__ CUtensorMap tmV0, const __grid_constant__ CUtensorMap tmV1,
                  const SdpaDevArgs a) {
-    using C = Cfg<HD, kHooks == 2>;
+    using C = Cfg<HD, kHooks == 3>;
     constexpr int KS = C::kKStages;
     constexpr int VS = C::kVStages;
     extern __shared__ uint8_t smem_raw[];
@@ -498,7 +498,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             }
             const TileInfo ti = tile_at(j);
             int bias_lim = 0;              // columns of this tile that have a bias, none where the warp's rows have none
-            if constexpr (kHooks == 2) {
+            if constexpr (kHooks == 3) {
                 if (a.bias != nullptr && w_row + 32 > 0 && w_row < a.bias_rows) bias_lim = min(ti.valid, a.bias_cols - ti.kbase);
                 if (bias_lim > 0) load_bias(ti.kbase, bias_lim, 0);
             }
@@ -520,7 +520,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             __syncwarp();
             if (lane == 0) mbar_arrive(&s_free[t]);
 
-            if constexpr (kHooks == 2) {
+            if constexpr (kHooks == 3) {
                 if (bias_lim > 0) {
 #pragma unroll
                     for (int c = 0; c < kBN; c += 32) {
@@ -647,7 +647,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             ok = __all_sync(0xffffffffu, mbar_wait(&q_full[t], 0));
         }
         const float inv = (l_sum > 0.0f) ? 1.0f / l_sum : 0.0f;
-        if constexpr (kHooks == 2) {
+        if constexpr (kHooks >= 2) {
             if (a.lse != nullptr && ok && row_in_seg < seg_rows) {
                 float* st = a.lse + ((static_cast<long long>(batch) * a.num_heads + head) * a.lq_total + q_glob) * 2;
                 st[0] = m_ref * sl2;
@@ -929,7 +929,7 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
 
 template <int HD, bool kBf16, int kHooks, bool kScale>
 cudaError_t launch_t(const SdpaLaunch& L, cudaStream_t stream) {
-    using C = Cfg<HD, kHooks == 2>;
+    using C = Cfg<HD, kHooks == 3>;
     // The CTAs of a last wave that fills no more than half of the SMs have one query tile each: a key step of
     // one tile takes about 1900 cycles, of two 2720, so that the wave ends after two thirds of the time.  A
     // row's arithmetic is the same in both.  1024 x 1024, 8 heads of 80 (32 items) 16.4 -> 13.7 us, 2042 x 2042,
@@ -956,16 +956,17 @@ cudaError_t launch_t(const SdpaLaunch& L, cudaStream_t stream) {
 
 template <int HD, bool kBf16>
 cudaError_t launch_hd(const SdpaLaunch& L, cudaStream_t stream) {
-    // 2: every softmax hook; 1: key mask only (the common case: padded captions), kept
-    // free of the other hooks' code; 0: none.  The per-key scale vectors are handled
-    // outside the softmax (kScale) and combine with 0 or 2.
-    const bool all_hooks = L.args.bias != nullptr || L.args.lse != nullptr;
+    // 3: a logit bias and every other softmax hook; 2: key mask and statistics (a map), free of the bias's code
+    // and with the third K tile that its rows take (mask and scales, 1033 x 1137, 24 heads of 128, 28.6 -> 27.1 us;
+    // statistics 8.8 -> 8.1 at 344 tokens); 1: key mask only (the common case: padded captions; with the statistics'
+    // store at its end 441 x 2365, 3 heads, takes 35.1 us instead of 32.9); 0: none.  The per-key scale vectors are
+    // handled outside the softmax (kScale) and combine with 0, 2 and 3.
     const bool scale = L.args.key_scale != nullptr || L.args.val_scale != nullptr;
-    if (scale) {
-        if (all_hooks || L.args.key_mask != nullptr) return launch_t<HD, kBf16, 2, true>(L, stream);
-        return launch_t<HD, kBf16, 0, true>(L, stream);
-    }
-    if (all_hooks) return launch_t<HD, kBf16, 2, false>(L, stream);
+    if (L.args.bias != nullptr) return scale ? launch_t<HD, kBf16, 3, true>(L, stream) : launch_t<HD, kBf16, 3, false>(L, stream);
+    if (scale)
+        return L.args.lse != nullptr || L.args.key_mask != nullptr ? launch_t<HD, kBf16, 2, true>(L, stream)
+                                                                   : launch_t<HD, kBf16, 0, true>(L, stream);
+    if (L.args.lse != nullptr) return launch_t<HD, kBf16, 2, false>(L, stream);
     if (L.args.key_mask != nullptr) return launch_t<HD, kBf16, 1, false>(L, stream);
     return launch_t<HD, kBf16, 0, false>(L, stream);
 }

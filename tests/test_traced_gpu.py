@@ -139,3 +139,39 @@ def test_bias_rows_of_any_alignment(bd, oracle, hd, split, row0, rows, cols, off
     G.check(G.host(out), ref, what="biased output")
     # FP32 scores on both sides; 2^-22 from each exponential and 1e-5 from the sums
     assert np.abs(G.host(amap) - avg[row0:row0 + rows, :cols]).max() <= 1e-4 * avg.max()
+
+
+# Two segments of query rows, 24 heads: 48 pairs of query tiles, all run as single tiles; 120, all pairs; 192, pairs and
+# single tiles (148 SMs)
+ROWS = {"single": [200, 100], "pairs": [600, 400], "both": [300, 1400]}
+
+
+@pytest.mark.parametrize("hd", [128, 40])
+@pytest.mark.parametrize("tiles", list(ROWS))
+def test_hooks_without_an_effect_keep_the_bits(bd, tiles, hd):
+    """Statistics, a mask of ones, scale vectors of ones and a bias of zeros, each alone and together: every combination
+    has a kernel of its own, and all have the bits of the call without hooks."""
+    nh, Lk = 24, 700
+    gen = torch.Generator(device="cuda").manual_seed(9800 + hd)
+    rnd = lambda n: torch.randn(n, nh * hd, device="cuda", generator=gen).to(torch.bfloat16)
+    q, k, v = [rnd(n) for n in ROWS[tiles]], rnd(Lk), rnd(Lk)
+    ref = [torch.full_like(x, float("nan")) for x in q]
+    bd.sdpa_fwd(q, k, v, ref, nh)
+    ones, Lq = torch.ones(Lk, device="cuda"), sum(ROWS[tiles])
+    ws = torch.empty(8 * nh * Lq, device="cuda", dtype=torch.uint8)
+    bias = torch.zeros(Lq, Lk, device="cuda")
+    for hooks in range(1, 16):
+        t = None
+        if hooks & 3:                                        # statistics (a traced call), with a bias or without
+            t = bd.TraceParams()
+            t.workspace, t.workspace_bytes = ws.data_ptr(), ws.numel()
+            if hooks & 2:
+                t.bias, t.bias_rows, t.bias_cols, t.bias_ld = bias.data_ptr(), Lq, Lk, Lk
+        kw = dict(key_mask=ones) if hooks & 4 else {}
+        if hooks & 8:
+            kw.update(key_scale=ones, val_scale=ones)
+        out = [torch.full_like(x, float("nan")) for x in q]
+        bd.sdpa_fwd(q, k, v, out, nh, _trace=t, **kw)
+        assert bd.device_status() == 0
+        for a, b in zip(out, ref):
+            assert torch.equal(a, b), hooks
