@@ -60,7 +60,8 @@ constexpr int kChunkBytes = 128 * 128;  // one 64-column (128 B) x 128-row TMA b
 constexpr int kMaxListed = 512;    // key tiles a list of the tiles with a visible key has room for
 constexpr int kPartTile = 0x8000;  // set in its entries for tiles that have a masked key too
 
-// kBias: the softmax warps have 4 KB of shared memory each for rows of a logit bias, in the place of the third K tile.
+// kBias: the softmax warps have 4 KB of shared memory each for rows of a logit bias, at 128 columns in the place of the
+// third K tile; at 64 columns 16 KB more for the CTAs with a single query tile.
 template <int HD, bool kBias>
 struct Cfg {
     static constexpr int kChunks = HD / 64;
@@ -72,7 +73,7 @@ struct Cfg {
     static constexpr int kVStages = HD == 128 ? 2 : 4;
     static constexpr int kBarBytes = 512;
     static constexpr int kListBytes = 2 * kMaxListed;      // key tiles to visit (calls with a key mask)
-    static constexpr int kBiasBytes = kBias ? 8 * 4096 : 0;
+    static constexpr int kBiasBytes = kBias ? (HD == 128 ? 8 : 12) * 4096 : 0;
     static constexpr int kSmemBytes =
         2 * kQBytes + (kKStages + kVStages) * kTileBytes + kBarBytes + kListBytes + kBiasBytes + 1024;
     // Tensor memory columns (512 in all).  At 64 columns per head every tile has its
@@ -471,11 +472,20 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
 
         // Logit bias: the warp's 32 rows, 32 columns at a time through shared memory; the first piece travels while
         // the scores are computed (a load with a row per lane: 256 + 1024 tokens, 24 heads, bias on two of ten tiles,
-        // 33.1 us, now 29.4, 21.1 without a bias).
+        // 33.1 us, now 29.4, 21.1 without a bias).  The others follow one by one, a latency each, as far as there are
+        // columns.  A CTA with a single query tile has nothing to hide that behind, but the room of the other tile: there
+        // all four pieces travel ahead of the scores (23 + 512 tokens, 24 heads of 40, bias on the 23: 22.3 us one by one, 16.3).
+        constexpr int kOwn = C::kBiasBytes / (4 * 4096);             // pieces of a lone tile that the bias area holds
+        const int lone = n_t == 1 ? 1 : 0;
         uint8_t* const bias_s = reinterpret_cast<uint8_t*>(tile_list + kMaxListed) + warp * 4096;
         const int w_row = q_global0 + t * kBM + (warp & 3) * 32 - a.bias_row0;      // the warp's first bias row
-        auto load_bias = [&](int kbase, int lim, int c) {
-            copy_rows32(bias_s, a.bias + kbase + c, a.bias_ld, w_row, a.bias_rows, lim - c, lane);
+        auto bias_piece = [&](int i) {
+            // (from the end of the bias area back to the second tile's Q buffer)
+            constexpr int kBack = kOwn * 4 * 4096 + C::kListBytes + C::kBarBytes + (KS + VS) * C::kTileBytes + C::kQBytes;
+            return bias_s + lone * (i * 4 * 4096 - (i < kOwn ? 0 : kBack));
+        };
+        auto load_bias = [&](int kbase, int lim, int i) {
+            copy_rows32(bias_piece(i), a.bias + kbase + i * 32, a.bias_ld, w_row, a.bias_rows, lim - i * 32, lane);
         };
 
         for (int j = 0; j < n_kv; ++j) {
@@ -499,8 +509,12 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             const TileInfo ti = tile_at(j);
             int bias_lim = 0;              // columns of this tile that have a bias, none where the warp's rows have none
             if constexpr (kHooks == 3) {
-                if (a.bias != nullptr && w_row + 32 > 0 && w_row < a.bias_rows) bias_lim = min(ti.valid, a.bias_cols - ti.kbase);
-                if (bias_lim > 0) load_bias(ti.kbase, bias_lim, 0);
+                if (w_row + 32 > 0 && w_row < a.bias_rows) bias_lim = min(ti.valid, a.bias_cols - ti.kbase);
+                if (bias_lim > 0) {
+                    const int ahead = lone ? (bias_lim + 31) >> 5 : 1;
+#pragma unroll 1
+                    for (int i = 0; i < ahead; ++i) load_bias(ti.kbase, bias_lim, i);
+                }
             }
             int lim = ti.valid - 1;
             if (a.mask_mode == 1) lim = min(lim, q_glob + a.q_offset - ti.kbase);
@@ -528,14 +542,15 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                         __syncwarp();
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            const float4 b = row_piece32(bias_s, lane, i);
+                            const float4 b = row_piece32(bias_piece(c >> 5), lane, i);
                             s[c + 4 * i] += b.x * a.bias_mul;
                             s[c + 4 * i + 1] += b.y * a.bias_mul;
                             s[c + 4 * i + 2] += b.z * a.bias_mul;
                             s[c + 4 * i + 3] += b.w * a.bias_mul;
                         }
                         __syncwarp();
-                        if (c + 32 < kBN) load_bias(ti.kbase, bias_lim, c + 32);
+                        if (c + 32 >= bias_lim) break;
+                        if (!lone) load_bias(ti.kbase, bias_lim, (c >> 5) + 1);
                     }
                 }
             }

@@ -175,3 +175,31 @@ def test_hooks_without_an_effect_keep_the_bits(bd, tiles, hd):
         assert bd.device_status() == 0
         for a, b in zip(out, ref):
             assert torch.equal(a, b), hooks
+
+
+@pytest.mark.parametrize("hd", [128, 40])
+@pytest.mark.parametrize("tiles", ["pairs", "both"])
+@pytest.mark.parametrize("cols,row0,rows", [(1, 0, 5), (31, 3, 40), (33, 130, 200), (64, 255, 2), (97, 500, 400), (128, 290, 333),
+                                            (131, 590, 60), (500, 700, 300)])
+def test_biased_pairs_have_the_bits_of_single_tiles(bd, tiles, hd, cols, row0, rows):
+    """A single query tile has all pieces of a key tile's bias in flight at once, a tile of a pair one after the other: a
+    head's bits are the same, and the map is the mean of the maps of its parts."""
+    nh, part, Lk = 24, 3, 600
+    n_rows = ROWS[tiles]
+    Lq = sum(n_rows)
+    rows = min(rows, Lq - row0)
+    gen = torch.Generator(device="cuda").manual_seed(9900 + cols)
+    rnd = lambda n: torch.randn(n, nh * hd, device="cuda", generator=gen).to(torch.bfloat16)
+    q, k, v = [rnd(n) for n in n_rows], rnd(Lk), rnd(Lk)
+    kw = dict(bias=torch.randn(rows, cols, device="cuda", generator=gen), bias_row0=row0, map_row0=row0, map_rows=rows, map_cols=cols)
+    out, ref = [torch.full_like(x, float("nan")) for x in q], [torch.full_like(x, float("nan")) for x in q]
+    amap = bd.sdpa_traced_fwd(q, k, v, out, nh, **kw)
+    mean = torch.zeros_like(amap)
+    for h in range(0, nh, part):
+        c = slice(h * hd, (h + part) * hd)
+        mean += bd.sdpa_traced_fwd([x[:, c] for x in q], k[:, c], v[:, c], [x[:, c] for x in ref], part, **kw) * (part / nh)
+    assert bd.device_status() == 0
+    for a, b in zip(out, ref):
+        assert torch.equal(a, b)
+    # FP32 sums of the same terms in another order
+    assert (amap - mean).abs().max() <= 1e-5 * mean.max()
