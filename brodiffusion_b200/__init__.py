@@ -206,12 +206,11 @@ def lib():
         L.bdattn_add_row_bias.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_longlong,
                                           C.c_int, C.c_void_p]
         # The same entry points for this module's own calls, which pass packed structures (bytes) as pointers
-        L.packed = {}
         for name in ("sdpa_fwd", "sdpa_fwd_allgather", "sdpa_fwd_allgather_multicast", "mgpu_sdpa_fwd_headsharded",
                      "sdpa_traced_fwd", "rmsnorm_rope", "qkvo_fwd", "qkvo_fwd_static", "qkv_norm_rope_fwd"):
             fn = L["bdattn_" + name]             # a function object of its own
             fn.argtypes = [C.c_void_p if t in _STRUCTURES else t for t in getattr(L, "bdattn_" + name).argtypes]
-            L.packed[name] = fn
+            setattr(L, "packed_" + name, fn)
         _lib = L
     return _lib
 
@@ -344,7 +343,7 @@ def sdpa_fwd(q, k, v, out, num_heads, *, mask_mode=MASK_NONE, key_mask=None, key
         gain = tuple(_addr(gt) for gt in (gains[:2] + [None, None])[:2])
         g0 = next((gt for gt in gains if gt is not None), None)
         gain_dtype = _dtype_code(g0) if g0 is not None else F32
-        eps = q_norm.get("eps", 1e-6)
+        eps = _f32(q_norm.get("eps", 1e-6))
         cos, sin = _addr(q_norm.get("cos")), _addr(q_norm.get("sin"))
         rope_row0 = q_norm.get("rope_row0", 0)
     (q0, q1), (o0, o1), (k0, k1), (v0, v1) = qd, od, kd, vd
@@ -354,30 +353,31 @@ def sdpa_fwd(q, k, v, out, num_heads, *, mask_mode=MASK_NONE, key_mask=None, key
                        q0[3], q1[3], o0[3], o1[3],
                        len(ks), k0[0], k1[0], v0[0], v1[0], k0[1], k1[1], k0[2], k1[2], v0[2], v1[2],
                        k0[3], k1[3], v0[3], v1[3],
-                       mask_mode, _addr(key_mask), _addr(key_scale), _addr(val_scale), _f32(softmax_scale), num_kv_heads,
-                       gain[0], gain[1], gain_dtype, _f32(eps), cos, sin, rope_row0)
+                       mask_mode, _addr(key_mask), _addr(key_scale), _addr(val_scale),
+                       softmax_scale and _f32(softmax_scale), num_kv_heads,
+                       gain[0], gain[1], gain_dtype, eps, cos, sin, rope_row0)
     except struct.error as e:
         raise TypeError(str(e)) from None
     if _trace is not None:
-        _check(lib().packed["sdpa_traced_fwd"](p, C.byref(_trace), _stream(stream)))
+        _check(lib().packed_sdpa_traced_fwd(p, C.byref(_trace), _stream(stream)))
         return
     if _mgpu is not None:
         ctx, rank, replica_ptrs, replica_ld, replica_bs, total_heads = _mgpu
         arr = (C.c_void_p * len(replica_ptrs))(*replica_ptrs)
-        _check(lib().packed["mgpu_sdpa_fwd_headsharded"](ctx, rank, p, arr, replica_ld, replica_bs,
+        _check(lib().packed_mgpu_sdpa_fwd_headsharded(ctx, rank, p, arr, replica_ld, replica_bs,
                                                       total_heads, _stream(stream)))
         return
     if multicast_out_ptrs:
         m1 = multicast_out_ptrs[1] if len(multicast_out_ptrs) > 1 else None
-        _check(lib().packed["sdpa_fwd_allgather_multicast"](p, multicast_out_ptrs[0], m1, _stream(stream)))
+        _check(lib().packed_sdpa_fwd_allgather_multicast(p, multicast_out_ptrs[0], m1, _stream(stream)))
         return
     if peer_out_ptrs:
         n = len(peer_out_ptrs[0])
         a0 = (C.c_void_p * max(n, 1))(*peer_out_ptrs[0])
         a1 = (C.c_void_p * max(n, 1))(*(peer_out_ptrs[1] if len(peer_out_ptrs) > 1 else [None] * n))
-        _check(lib().packed["sdpa_fwd_allgather"](p, a0, a1, n, _stream(stream)))
+        _check(lib().packed_sdpa_fwd_allgather(p, a0, a1, n, _stream(stream)))
         return
-    _check(lib().packed["sdpa_fwd"](p, _stream(stream)))
+    _check(lib().packed_sdpa_fwd(p, _stream(stream)))
 
 
 class MultiGpu:
@@ -427,7 +427,7 @@ def rmsnorm_rope(jobs, num_heads, head_dim, *, eps=1e-6, pair_mode=ROPE_INTERLEA
                                     _addr(j.get("cos")), _addr(j.get("sin")), j.get("rope_row0", 0)))
         except struct.error as e:
             raise TypeError(str(e)) from None
-    _check(lib().packed["rmsnorm_rope"](b"".join(packed), len(jobs), dtype, num_heads, head_dim, eps, pair_mode,
+    _check(lib().packed_rmsnorm_rope(b"".join(packed), len(jobs), dtype, num_heads, head_dim, eps, pair_mode,
                                      _stream(stream)))
 
 
@@ -511,9 +511,9 @@ def qkvo_fwd(x, ctx, wq, wk, wv, wo, bo, num_heads, out, workspace, *, bq=None, 
     except struct.error as e:
         raise TypeError(str(e)) from None
     if workspace is None:
-        _check(lib().packed["qkvo_fwd_static"](p, _stream(stream)))
+        _check(lib().packed_qkvo_fwd_static(p, _stream(stream)))
         return
-    _check(lib().packed["qkvo_fwd"](p, _stream(stream)))
+    _check(lib().packed_qkvo_fwd(p, _stream(stream)))
 
 
 def qkvo_static_capacity() -> int:
@@ -605,4 +605,4 @@ def qkv_norm_rope_fwd(x, wq, wk, wv, q_out, k_out, v_out, num_heads, head_dim, *
                       v_out.stride(0) if v_out is not None else 0)
     except struct.error as e:
         raise TypeError(str(e)) from None
-    _check(lib().packed["qkv_norm_rope_fwd"](p, _stream(stream)))
+    _check(lib().packed_qkv_norm_rope_fwd(p, _stream(stream)))
