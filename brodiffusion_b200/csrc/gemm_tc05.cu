@@ -53,24 +53,28 @@ __device__ __forceinline__ float gemm_ld16(const void* base, long long i) {
 }
 
 // Epilogue of a split tile.  Every CTA of the cluster holds a partial 128 x n_tile sum
-// at the same shared-memory address; this one finishes every split-th row, eight columns to a thread, so that the
-// rows that exist are spread over the cluster and eight threads read and write a whole row piece, and asks for
+// at the same shared-memory address; this one finishes its share of the rows, eight columns to a thread, so that
+// eight threads read and write a whole row piece, and asks for
 // all partial sums of a piece before it adds the first (a thread walking the columns of a row, one remote read
 // behind the other, took 2 to 4 us; with the bias ahead 64 x 1280 x 1280 over four 5.3 -> 4.7 us, 1024 x 640 x 2560
-// over two 13.4 -> 11.5).
+// over two 13.4 -> 11.5).  Up to 64 rows are dealt out one by one, so that every CTA has some; more are
+// taken as blocks (128 x 640 x 5120 over eight 7.8 us dealt out, 7.4; 64 x 1280 x 1280 4.7, 5.2 in blocks).  Of a narrow
+// tile no thread gets columns that do not exist: 5251 x 8 x 1064 8.0 -> 6.9 us, 113 x 8 x 680 5.4 -> 4.2.
 template <bool kBf16>
 __device__ __forceinline__ void epilogue_split(const GemmProblem& p, cooperative_groups::cluster_group& cluster,
                                                float* red, const float* bias_s, int split, int part, int tid, int m0, int n0) {
     const int ld = gemm_red_ld(p.n_tile);
-    const int units = p.n_tile / 8;
     const int n_valid = min(p.n_tile, p.N - n0);           // a multiple of eight
+    const int sh = n_valid > 64 ? 4 : n_valid > 32 ? 3 : n_valid > 16 ? 2 : n_valid > 8 ? 1 : 0;
     const int rows = min(128, p.M - m0);
+    const bool dealt = rows <= 64;
     const float* src[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) src[k] = cluster.map_shared_rank(red, min(k, split - 1));
 #pragma unroll 2
-    for (int i = tid; i < 128 / split * units; i += 128) {
-        const int r = part + split * (i / units), c = i % units * 8;
+    for (int i = tid; i < (128 / split) << sh; i += 128) {
+        const int j = i >> sh, c = (i & ((1 << sh) - 1)) * 8;
+        const int r = dealt ? part + split * j : part * (128 / split) + j;
         if (r >= rows || c >= n_valid) continue;
         float4 u[8], v[8];
 #pragma unroll

@@ -31,3 +31,18 @@ def test_linear_tile_widths_between_64_and_128(bd, oracle, M, N, K):
     assert bd.device_status() == 0
     G.check(G.host(y[:M, :N]), oracle.linear(x, w, b), max_abs=2.5e-2, what=f"linear {M}x{N}x{K}")
     assert bool((y[M] == 7.0).all()) and bool((y[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("N", [8, 16, 24, 40, 64, 72, 104])
+@pytest.mark.parametrize("M", [1, 64, 65, 128, 190])
+def test_linear_split_shares_of_narrow_and_ragged_tiles(bd, oracle, M, N):
+    """Tiles of one to eight pieces of eight columns; up to 64 rows, more, all: how a cluster shares the rows and a
+    warp the pieces depends on both. The K give two, four and eight CTAs to a tile.  Bound as above."""
+    for K in (696, 776, 1544):
+        x, w = synth.activations((M, K), 9980), synth.round_bf16(synth.normal((N, K), 9981, 0, 1.0 / K ** 0.5))
+        b = synth.weights((N,), 9982)
+        y = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+        bd.linear_fwd(G.dev(x), G.dev(w), G.dev(b), y[:M, :N])
+        assert bd.device_status() == 0
+        G.check(G.host(y[:M, :N]), oracle.linear(x, w, b), max_abs=2.5e-2, what=f"linear {M}x{N}x{K}")
+        assert bool((y[M] == 7.0).all()) and bool((y[:, N:] == 7.0).all())
