@@ -80,11 +80,12 @@ BDATTN_HD constexpr bool pair_acc_reused(int tile, int pairs, int total_tiles) {
 // block would have nothing to add and nothing to wait for.
 inline GemmPlan plan_gemm(const GemmShape* p, int n, int sms) {
     bool geglu = false, heads = false, odd = false;
-    int kb = 0, kb_min = 0;
+    int kb = 0, kb_min = 0, m_max = 0;
     for (int i = 0; i < n; ++i) {
         geglu = geglu || p[i].geglu;
         heads = heads || p[i].heads;
         odd = odd || p[i].K % 16 != 0;
+        m_max = p[i].M > m_max ? p[i].M : m_max;
         const int b = gemm_k_blocks(p[i].K);
         kb = b > kb ? b : kb;
         kb_min = i == 0 || b < kb_min ? b : kb_min;
@@ -132,9 +133,10 @@ inline GemmPlan plan_gemm(const GemmShape* p, int n, int sms) {
                                                (rounds(tiles(128), 3LL * sms) - 1.0) * (2.5 + 0.45 * k128)
                                          : y * (3.0 + (odd ? 0.41 : 0.265) * kb));
         for (int s = 2; s <= 8 && kb >= 3 * s && kb_min >= s && tiles(64) * s * 2 <= 3LL * sms; s *= 2) {
-            // (with more CTAs than SMs a longer part of K costs more than the split saves)
+            // (with more CTAs than SMs a longer part of K costs more than the split saves, and of tiles with more than 64 rows
+            // any: 135 x 640 x 5120 over eight 11.5 us, over four 8.0, and the same for 100 shapes drawn at random)
             if (waves(64, s) <= 1.0) offer({false, 64, s}, 3.15 + 0.15 * kb / s);
-            else if (kb <= 12 * s) offer({false, 64, s}, 3.22 + 0.27 * kb / s * tiles(64) * s / sms);
+            else if (kb <= 12 * s && m_max <= 64) offer({false, 64, s}, 3.22 + 0.27 * kb / s * tiles(64) * s / sms);
         }
     }
     for (int cols = 256; cols >= 128; cols /= 2) {

@@ -89,3 +89,10 @@ def test_every_release_of_an_accumulator_is_waited_for(plan, pairs, total):
         tiles = list(range(first, total, pairs))
         released = [ti for ti, tile in enumerate(tiles) if plan.acc_reused(tile, pairs, total)]
         assert released == [ti - 2 for ti in range(2, len(tiles))]
+
+
+@pytest.mark.parametrize("shape", [(65, 1280, 5120), (100, 1280, 5120), (135, 640, 5120), (131, 608, 4736), (223, 1264, 2640)])
+def test_no_split_beyond_the_sms_above_64_rows(plan, shape):
+    """Where the parts do not all run at once the exchange of full tiles costs more than the shorter K saves."""
+    m, n, _ = shape
+    assert -(-m // 128) * -(-n // 64) * plan([shape])[2] <= 148
