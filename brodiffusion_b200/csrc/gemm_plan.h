@@ -112,14 +112,24 @@ inline GemmPlan plan_gemm(const GemmShape* p, int n, int sms) {
         // 11.5; 10.1 on pairs).  With a longer K an SM has two CTAs of 64 or 80 columns (1024 x 2560 x 1280, 256 tiles
         // of 80, 10.1, 1024 x 3072 x 1280, 312, 16.5) and one of 128.
         const bool short_k = kb <= 8;
-        const double k64 = odd ? 1.7 * kb : kb, k80 = odd ? 2.4 * kb : kb, k128 = odd ? 1.3 * kb : kb;
+        const double k64 = odd ? (short_k ? 1.7 : 1.85) * kb : kb, k80 = odd ? 2.4 * kb : kb;
         auto per_sm = [&](int w) { return static_cast<double>(tiles(w)) / sms; };
         auto late = [](double a) { return a > 0.0 ? a : 0.0; };
         const double x = waves(64, 1), t64 = per_sm(64), y = waves(128, 1), t128 = per_sm(128);
-        offer(best, x <= 1.0  ? 2.2 + 0.165 * kb
-                    : short_k ? 4.4 + 0.61 * k64 - late(2.0 - t64) * (1.7 + 0.1 * k64) + late(t64 - 4.0) * 0.9 +
-                                    (rounds(tiles(64), 4LL * sms) - 1.0) * (1.0 + 0.48 * k64)
-                              : 1.15 + x * (0.6 + 0.05 * k64) + rounds(tiles(64), 2LL * sms) * (1.45 + 0.176 * k64));
+        // Short K off 32 bytes and more tiles than SMs: the L2 sets the pace, in proportion to the tiles, so that wide ones
+        // are better but for the CTAs that they leave over: two CTAs of 64 columns to an SM, or four, that run at once
+        // instead of 128 columns in a second round (64, 96 and 128 columns: 3573 x 704 x 152 7.2, 7.3, 8.1 us,
+        // 7290 x 392 x 216 8.4, 8.0, 10.3, 1911 x 2112 x 200 9.1, 8.0, 9.4, 3829 x 5016 x 392 44.7, 39.7, 35.1; with the terms
+        // for even rows up to 30 % longer than the best of 64 and 128, over 183 shapes now 3 % on average).
+        const bool odd_short = odd && short_k && y > 1.0;
+        if (odd_short) {
+            offer({false, t64 <= 2.0 ? 64 : t64 <= 4.0 ? 96 : 128, 1}, 3.0 + 0.11 * kb + t128 * (1.46 + 0.37 * kb));
+        } else {
+            offer(best, x <= 1.0  ? 2.2 + 0.165 * kb
+                        : short_k ? 4.4 + 0.61 * k64 - late(2.0 - t64) * (1.7 + 0.1 * k64) + late(t64 - 4.0) * 0.9 +
+                                        (rounds(tiles(64), 4LL * sms) - 1.0) * (1.0 + 0.48 * k64)
+                                  : 1.15 + x * (0.6 + 0.05 * k64) + rounds(tiles(64), 2LL * sms) * (1.45 + 0.176 * k64));
+        }
         // Between 64 and 128 columns for widths that these divide badly (320, 640) and for what 64 columns make two
         // waves of; with several CTAs to an SM only 80 columns, whose rings still fit twice (a short K has
         // rings of two stages there and gains nothing: 9216 x 320 x 320 8.0 us, 7.7 with 64 or 128).
@@ -127,11 +137,11 @@ inline GemmPlan plan_gemm(const GemmShape* p, int n, int sms) {
             if (waves(w, 1) <= 1.0) offer({false, w, 1}, 1.6 + 0.6 * w / 64 + (0.12 + 0.045 * w / 64) * kb);
             else if (w == 80 && !short_k) offer({false, w, 1}, 1.0 + waves(w, 1) * (1.4 + 0.065 * k80) + rounds(tiles(w), 2LL * sms) * (0.5 + 0.166 * k80));
         }
-        offer({false, 128, 1}, y <= 1.0  ? 2.8 + 0.21 * kb
-                               : short_k ? 5.6 + 0.68 * k128 - late(3.0 - t128) * (0.4 + 0.05 * k128) + late(t128 - 3.0) * 0.9 +
-                                               (odd ? 0.06 * kb * kb * (t128 - 1.0) : 0.0) +
-                                               (rounds(tiles(128), 3LL * sms) - 1.0) * (2.5 + 0.45 * k128)
-                                         : y * (3.0 + (odd ? 0.41 : 0.265) * kb));
+        if (!odd_short)
+            offer({false, 128, 1}, y <= 1.0  ? 2.8 + 0.21 * kb
+                                   : short_k ? 5.6 + 0.68 * kb - late(3.0 - t128) * (0.4 + 0.05 * kb) + late(t128 - 3.0) * 0.9 +
+                                                   (rounds(tiles(128), 3LL * sms) - 1.0) * (2.5 + 0.45 * kb)
+                                             : odd ? y * (2.9 + 0.38 * kb) : y * (3.0 + 0.265 * kb));
         for (int s = 2; s <= 8 && kb >= 3 * s && kb_min >= s && tiles(64) * s * 2 <= 3LL * sms; s *= 2) {
             // (with more CTAs than SMs a longer part of K costs more than the split saves, and of tiles with more than 64 rows
             // any: 135 x 640 x 5120 over eight 11.5 us, over four 8.0, and the same for 100 shapes drawn at random)

@@ -96,3 +96,12 @@ def test_no_split_beyond_the_sms_above_64_rows(plan, shape):
     """Where the parts do not all run at once the exchange of full tiles costs more than the shorter K saves."""
     m, n, _ = shape
     assert -(-m // 128) * -(-n // 64) * plan([shape])[2] <= 148
+
+
+@pytest.mark.parametrize("shape,kernels", [
+    ((3829, 5016, 392), ("128",)), ((8128, 1696, 504), ("128",)), ((2341, 3320, 280), ("128",)), ((2079, 4608, 392), ("p256",)),
+    ((1895, 1184, 136), ("64",)), ((7290, 392, 216), ("64", "96")), ((2569, 1288, 248), ("64", "96")), ((1911, 2112, 200), ("64", "96")),
+    ((8256, 2848, 1208), ("80", "128")), ((4399, 3768, 1032), ("80", "128")), ((8218, 1728, 1032), ("80", "128"))])
+def test_k_off_32_bytes(plan, shape, kernels):
+    """More tiles than SMs: a width that was measured to be no slower than 128 columns were before the pair kernel's narrow tiles."""
+    assert plan.kernel([shape])[0] in kernels
