@@ -162,7 +162,7 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 }
 
 // HOOKS: 0 = none; 1 = key_mask only; 2 = key_mask and the per-row softmax statistics; 3 = a logit
-// bias besides (slower softmax path).
+// bias besides (slower softmax path); 4 = a bias of a few rows, read without shared memory (launch_hd).
 // SCALE: key_scale / val_scale are applied to the K / V tiles in shared memory by
 // warps 12-15 (rounded to the storage type, as the reference's scale_inplace on its
 // k_full_ / v_full_ copies does, src/dit/qwenimage21_forward.cpp:606-645); the
@@ -508,8 +508,9 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
             }
             const TileInfo ti = tile_at(j);
             int bias_lim = 0;              // columns of this tile that have a bias, none where the warp's rows have none
-            if constexpr (kHooks == 3) {
+            if constexpr (kHooks >= 3)
                 if (w_row + 32 > 0 && w_row < a.bias_rows) bias_lim = min(ti.valid, a.bias_cols - ti.kbase);
+            if constexpr (kHooks == 3) {
                 if (bias_lim > 0) {
                     const int ahead = lone ? (bias_lim + 31) >> 5 : 1;
 #pragma unroll 1
@@ -551,6 +552,29 @@ sdpa_tc05_kernel(const __grid_constant__ CUtensorMap tmQ0, const __grid_constant
                         __syncwarp();
                         if (c + 32 >= bias_lim) break;
                         if (!lone) load_bias(ti.kbase, bias_lim, (c >> 5) + 1);
+                    }
+                }
+            }
+            if constexpr (kHooks == 4) {
+                // a thread reads its own row, all loads in flight at once
+                const int br = q_glob - a.bias_row0;
+                if (bias_lim > 0 && br >= 0 && br < a.bias_rows) {
+                    const float* const brow = a.bias + static_cast<long long>(br) * a.bias_ld + ti.kbase;
+                    if ((bias_lim & 3) == 0 && (a.bias_ld & 3) == 0 && (reinterpret_cast<uintptr_t>(a.bias + ti.kbase) & 15u) == 0) {
+#pragma unroll
+                        for (int c = 0; c < kBN; c += 4) {
+                            if (c < bias_lim) {
+                                const float4 b = __ldg(reinterpret_cast<const float4*>(brow + c));
+                                s[c] += b.x * a.bias_mul;
+                                s[c + 1] += b.y * a.bias_mul;
+                                s[c + 2] += b.z * a.bias_mul;
+                                s[c + 3] += b.w * a.bias_mul;
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < kBN; ++c)
+                            if (c < bias_lim) s[c] += __ldg(brow + c) * a.bias_mul;
                     }
                 }
             }
@@ -977,7 +1001,17 @@ cudaError_t launch_hd(const SdpaLaunch& L, cudaStream_t stream) {
     // store at its end 441 x 2365, 3 heads, takes 35.1 us instead of 32.9); 0: none.  The per-key scale vectors are
     // handled outside the softmax (kScale) and combine with 0, 2 and 3.
     const bool scale = L.args.key_scale != nullptr || L.args.val_scale != nullptr;
-    if (L.args.bias != nullptr) return scale ? launch_t<HD, kBf16, 3, true>(L, stream) : launch_t<HD, kBf16, 3, false>(L, stream);
+    if (L.args.bias != nullptr) {
+        // A bias of few rows concerns a warp or two, and a piece of it behind the other through shared memory held up
+        // the whole call: 32 rows x 1280 columns, 24 heads of 128, 49.2 us, a row per thread 37.4; 26 x 1096, 24 heads of 64, 31.7
+        // and 27.4 (1024 rows x 256, 29.2 and 32.4).  Where every CTA has a single tile the pieces are all in flight
+        // and the better choice (23 x 512, 24 heads of 40, 16.4 and 19.0) unless the rows are off 16 bytes (one row of 537, 25.7 and 22.1).
+        const bool lone = 2LL * L.q_ctas * L.num_heads * L.batch <= sm_count();
+        const bool rows16 = (L.args.bias_ld & 3) == 0 && (reinterpret_cast<uintptr_t>(L.args.bias) & 15u) == 0;
+        if (L.args.bias_rows <= 32 && !(lone && rows16))
+            return scale ? launch_t<HD, kBf16, 4, true>(L, stream) : launch_t<HD, kBf16, 4, false>(L, stream);
+        return scale ? launch_t<HD, kBf16, 3, true>(L, stream) : launch_t<HD, kBf16, 3, false>(L, stream);
+    }
     if (scale)
         return L.args.lse != nullptr || L.args.key_mask != nullptr ? launch_t<HD, kBf16, 2, true>(L, stream)
                                                                    : launch_t<HD, kBf16, 0, true>(L, stream);
