@@ -5,6 +5,7 @@
 
 #include <cmath>
 #include <cstdarg>
+#include <cfloat>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -340,7 +341,8 @@ static int sdpa_fwd_impl(const char* op, const bdattn_sdpa_params* p, void* cons
             a.bias = tr->bias;
             a.bias_row0 = tr->bias_row0; a.bias_rows = tr->bias_rows; a.bias_cols = tr->bias_cols;
             a.bias_ld = tr->bias_ld > 0 ? tr->bias_ld : tr->bias_cols;
-            a.bias_mul = 1.0f / scale;
+            // (finite: a row without a bias adds zeros)
+            a.bias_mul = fminf(1.0f / scale, FLT_MAX);
             a.lse = static_cast<float*>(tr->workspace);
             a.lq_total = static_cast<int>(Lq);
         }

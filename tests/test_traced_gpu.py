@@ -203,3 +203,21 @@ def test_biased_pairs_have_the_bits_of_single_tiles(bd, tiles, hd, cols, row0, r
         assert torch.equal(a, b)
     # FP32 sums of the same terms in another order
     assert (amap - mean).abs().max() <= 1e-5 * mean.max()
+
+
+def test_rows_without_a_bias_at_the_smallest_scale(bd):
+    """The reciprocal of the softmax scale is beyond FP32; rows that have no bias must not notice."""
+    nh, hd, L, rows, scale = 2, 64, 200, 40, 1e-39
+    gen = torch.Generator(device="cuda").manual_seed(9950)
+    q, k, v = (torch.randn(L, nh * hd, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(3))
+    out, ref = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    bd.sdpa_fwd(q, k, v, ref, nh, softmax_scale=scale)
+    bias = torch.randn(rows, 100, device="cuda", generator=gen)
+    ws = torch.empty(8 * nh * L, device="cuda", dtype=torch.uint8)
+    t = bd.TraceParams()
+    t.workspace, t.workspace_bytes = ws.data_ptr(), ws.numel()
+    t.bias, t.bias_row0, t.bias_rows, t.bias_cols, t.bias_ld = bias.data_ptr(), 10, rows, 100, 100
+    bd.sdpa_fwd(q, k, v, out, nh, softmax_scale=scale, _trace=t)
+    assert bd.device_status() == 0
+    assert bool(torch.isfinite(ref).all())
+    assert torch.equal(out[:10], ref[:10]) and torch.equal(out[10 + rows:], ref[10 + rows:])
