@@ -105,3 +105,25 @@ def test_no_split_beyond_the_sms_above_64_rows(plan, shape):
 def test_k_off_32_bytes(plan, shape, kernels):
     """More tiles than SMs: a width that was measured to be no slower than 128 columns were before the pair kernel's narrow tiles."""
     assert plan.kernel([shape])[0] in kernels
+
+
+# What the GPU tests of single kernels say that they run (148 SMs): a change of the modelled times must not empty them
+@pytest.mark.parametrize("kind,shapes,kernel", [
+    ("heads", [(509, 3072, 1000), (1000, 3072, 1000)], "p256"), ("heads", [(129, 384, 200), (77, 384, 72), (1500, 1024, 72)], "p128"),
+    ("geglu", [(130, 192, 520), (1, 64, 64), (1000, 2560, 616), (2300, 1152, 200)], "p128"), ("geglu", [(4096, 1280, 320)], "p256"),
+    ("plain", [(1100, 2176, 712), (577, 4992, 456)], "p128"), ("plain", [(1000, 3072, 616), (999, 3072, 1000)], "p256"),
+    ("plain", [(2300, 640, 640), (4000, 320, 72)], "80"), ("plain", [(500, 3072, 200)], "96"), ("plain", [(5000, 328, 600)], "112"),
+    ("several", [(9200, 320, 648), (7000, 328, 648), (4800, 480, 1280), (7000, 328, 1288)], "80")])
+def test_kernels_of_the_gpu_tests(plan, kind, shapes, kernel):
+    for m, n, k in shapes:
+        got = plan.kernel([(m, n, k)] * (3 if kind == "heads" else 1), geglu=kind == "geglu", heads=kind == "heads")
+        assert got == (kernel, 1), (m, n, k)
+        if kernel.isdigit():
+            assert (-(-m // 128) * -(-n // int(kernel)) > 148) == (kind == "several")
+
+
+@pytest.mark.parametrize("rows", [1, 64, 65, 128, 190])
+@pytest.mark.parametrize("k,split", [(696, 2), (776, 4), (1544, 8)])
+def test_splits_of_the_gpu_tests(plan, rows, k, split):
+    for n in (8, 16, 24, 40, 64, 72, 104):
+        assert plan([(rows, n, k)])[2] == split

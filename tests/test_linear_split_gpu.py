@@ -46,3 +46,16 @@ def test_linear_split_shares_of_narrow_and_ragged_tiles(bd, oracle, M, N):
         assert bd.device_status() == 0
         G.check(G.host(y[:M, :N]), oracle.linear(x, w, b), max_abs=2.5e-2, what=f"linear {M}x{N}x{K}")
         assert bool((y[M] == 7.0).all()) and bool((y[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(9200, 320, 648), (7000, 328, 648), (4800, 480, 1280), (7000, 328, 1288)])
+def test_linear_80_columns_several_ctas_to_an_sm(bd, oracle, M, N, K):
+    """80 columns with more tiles than SMs, where a ring of four stages lets two CTAs share one (tests/test_gemm_plan.py
+    has the width of each).  Bound as above."""
+    x, w = synth.activations((M, K), 9990), synth.round_bf16(synth.normal((N, K), 9991, 0, 1.0 / K ** 0.5))
+    b = synth.weights((N,), 9992)
+    y = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    bd.linear_fwd(G.dev(x), G.dev(w), G.dev(b), y[:M, :N])
+    assert bd.device_status() == 0
+    G.check(G.host(y[:M, :N]), oracle.linear(x, w, b), max_abs=2.5e-2, what=f"linear {M}x{N}x{K}")
+    assert bool((y[M] == 7.0).all()) and bool((y[:, N:] == 7.0).all())

@@ -63,3 +63,16 @@ def test_geglu_64_columns(bd, oracle, B, Din, Dout):
     got = G.host(y)
     assert np.isfinite(got).all()
     assert np.abs(got - ref).max() <= 0.01 * np.abs(ref).max() + 0.008
+
+
+@pytest.mark.parametrize("M,N,K", [(1100, 2176, 712), (577, 4992, 456),           # 128 columns
+                                   (1000, 3072, 616), (999, 3072, 1000)])         # 256 columns
+def test_linear_both_widths(bd, oracle, M, N, K):
+    """Plain layers on pairs (tests/test_gemm_plan.py has the width of each), ragged rows and K."""
+    x, w = synth.activations((M, K), 9740), synth.round_bf16(synth.normal((N, K), 9741, 0, 1.0 / K ** 0.5))
+    b = synth.weights((N,), 9742)
+    y = torch.full((M + 1, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    bd.linear_fwd(G.dev(x), G.dev(w), G.dev(b), y[:M, :N])
+    assert bd.device_status() == 0
+    G.check(G.host(y[:M, :N]), oracle.linear(x, w, b), max_abs=2.5e-2, what=f"linear {M}x{N}x{K}")
+    assert bool((y[M] == 7.0).all()) and bool((y[:, N:] == 7.0).all())
