@@ -75,8 +75,10 @@ inline int sm_count() {
 // become resident while the kernel before it in the stream is still running (as that
 // one's CTAs retire, once all of them have passed dependents_may_launch()); it does
 // its set-up and then holds at wait_for_prior_grid() until the earlier grid has
-// completed and its writes are visible.  Every kernel launched this way calls
-// wait_for_prior_grid() before its first access to global memory.
+// completed and its writes are visible.  A kernel launched this way reads and writes no global memory ahead of
+// wait_for_prior_grid(); what may come before it are requests that bring data into the L2
+// (tma_prefetch_l2_2d).  CTAs and threads that have nothing to do may end without the wait: the grid is complete
+// only when those that have have waited, so that a grid behind it still finds all earlier ones complete.
 // With a cluster of more than one CTA, `cluster` gives its size.
 template <class... KArgs, class... Args>
 inline cudaError_t launch_dependent_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
@@ -363,15 +365,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
           "=r"(r[15])
         : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-          "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
-          "r"(r[14]), "r"(r[15])
         : "memory");
 }
 
