@@ -124,6 +124,19 @@ inline GemmPlan plan_gemm(const GemmShape* p, int n, int sms) {
         const bool odd_short = odd && short_k && y > 1.0;
         if (odd_short) {
             offer({false, t64 <= 2.0 ? 64 : t64 <= 4.0 ? 96 : 128, 1}, 3.0 + 0.11 * kb + t128 * (1.46 + 0.37 * kb));
+        } else if (short_k && y > 1.0 && t128 <= 3.0) {
+            // All of these CTAs run at once, three to an SM with 96 columns and more: the width that leaves no SM with one more
+            // than the others.  Measured behind another kernel, where nothing of the launch before is left to run
+            // beside (64, 96, 112, 128 columns and pairs with 128): 4096 x 960 x 320 7.8, 7.0, 6.8, 7.2 us, 1564 x 2752 x 256 7.8,
+            // 7.1, 7.6, 6.4, 4096 x 1280 x 320 10.6, 9.9, 8.2, 8.7, 10.9, 3628 x 896 x 320 7.2, 6.3, 6.7, 6.8, 8.4, 1672 x 1792 x 512
+            // 8.6, 7.5, 8.0, 8.1, 9.3.  (Behind itself a launch starts in the SMs that its predecessor leaves, and
+            // pairs look up to 1 us better than they are.)
+            const double t96 = per_sm(96), t112 = per_sm(112);
+            if (t64 <= 2.0) offer({false, 64, 1}, 3.5 + 0.25 * kb + t64 * (0.3 + 0.07 * kb));
+            else if (t128 > 1.78 && t128 <= 2.0) offer({false, 128, 1}, 3.5 + 0.25 * kb + t128 * (0.5 + 0.09 * kb));
+            else if (t96 <= 3.0) offer({false, 96, 1}, 3.5 + 0.25 * kb + t96 * (0.5 + 0.08 * kb));
+            else if (t112 <= 3.0) offer({false, 112, 1}, 3.9 + 0.25 * kb + t112 * (0.6 + 0.1 * kb));
+            else offer({false, 128, 1}, 3.9 + 0.25 * kb + t128 * (0.7 + 0.11 * kb));
         } else {
             offer(best, x <= 1.0  ? 2.2 + 0.165 * kb
                         : short_k ? 4.4 + 0.61 * k64 - late(2.0 - t64) * (1.7 + 0.1 * k64) + late(t64 - 4.0) * 0.9 +
@@ -137,7 +150,7 @@ inline GemmPlan plan_gemm(const GemmShape* p, int n, int sms) {
             if (waves(w, 1) <= 1.0) offer({false, w, 1}, 1.6 + 0.6 * w / 64 + (0.12 + 0.045 * w / 64) * kb);
             else if (w == 80 && !short_k) offer({false, w, 1}, 1.0 + waves(w, 1) * (1.4 + 0.065 * k80) + rounds(tiles(w), 2LL * sms) * (0.5 + 0.166 * k80));
         }
-        if (!odd_short)
+        if (!odd_short && !(short_k && y > 1.0 && t128 <= 3.0))
             offer({false, 128, 1}, y <= 1.0  ? 2.8 + 0.21 * kb
                                    : short_k ? 5.6 + 0.68 * kb - late(3.0 - t128) * (0.4 + 0.05 * kb) + late(t128 - 3.0) * 0.9 +
                                                    (rounds(tiles(128), 3LL * sms) - 1.0) * (2.5 + 0.45 * kb)

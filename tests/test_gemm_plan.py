@@ -67,7 +67,7 @@ def test_split_is_bounded_by_the_shortest_k(plan, shapes, split):
     ("plain", (2304, 2560, 320), ("80", "112", "128")), ("plain", (4096, 1280, 320), ("80", "112", "128")),
     ("plain", (9216, 640, 320), ("80", "112", "128")), ("plain", (4096, 2560, 112), ("96", "128")),
     ("plain", (9216, 1280, 640), ("p256",)), ("plain", (2240, 2304, 2240), ("p128",)),
-    ("plain", (576, 5120, 448), ("p128",)), ("plain", (576, 4096, 936), ("p256",)), ("plain", (2240, 1024, 2240), ("128",)),
+    ("plain", (576, 5120, 448), ("96", "p128")), ("plain", (576, 4096, 936), ("p256",)), ("plain", (2240, 1024, 2240), ("128",)),
     ("geglu", (4096, 1280, 2808), ("p256",)), ("geglu", (64, 5120, 1280), ("p128",)), ("geglu", (4096, 1280, 320), ("p256",)),
     ("heads", (3580, 1024, 1288), ("p256",)), ("heads", (256, 3072, 3072), ("p128",)), ("heads", (1024, 3072, 3072), ("p256",))])
 def test_plan_is_the_measured_best(plan, kind, shape, kernels):
