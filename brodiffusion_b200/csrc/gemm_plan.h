@@ -71,9 +71,9 @@ BDATTN_HD constexpr bool pair_acc_reused(int tile, int pairs, int total_tiles) {
 // 2808) a box row touches five sectors instead of four, and a K block takes 1.6 times as long with a CTA for every tile and
 // several rounds of them (2.4 with 80 columns), 1.35 on pairs with 128 columns, 1.15 with 256.
 // A tile split over CTAs pays where few tiles have a long K: 64 x 1280 x 5120 14.3 us, 10.1 over two CTAs, 7.8 over
-// four, 9.2 over eight; 256 x 1280 x 5120 14.2, 11.4, 13.7.  The splits are entered at about 0.8 us less than they
+// four, 8.8 over eight; 256 x 1280 x 5120 14.2, 11.4, 13.7.  The splits are entered at about 0.8 us less than they
 // take when all CTAs run at once, and three when not: with the times themselves launches of a few tiles would be
-// split less than tests/test_gemm_plan.py has it (256 x 1280 x 1280 6.4 us over two, 5.7 whole).
+// split less than tests/test_gemm_plan.py has it (256 x 1280 x 1280 6.1 us over two, 5.7 whole).
 // GEGLU is not split: the two accumulators of a tile double the exchange.
 // The problems of a launch may differ in K (the queries and the keys of a cross-attention): the
 // longest sets the time, the shortest how far its tiles can be split, a CTA without a K
