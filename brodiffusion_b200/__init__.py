@@ -599,7 +599,7 @@ def qkv_norm_rope_fwd(x, wq, wk, wv, q_out, k_out, v_out, num_heads, head_dim, *
     try:
         p = _pack_qkv(_dtype_code(x), num_heads, head_dim, x.data_ptr(), x.shape[0], x.shape[1], x.stride(0),
                       _addr(wq), _addr(wk), _addr(wv), _addr(bq), _addr(bk), _addr(bv), _addr(gain_q), _addr(gain_k),
-                      _dtype_code(g) if g is not None else F32, _f32(eps), _addr(cos), _addr(sin), rope_row0,
+                      _dtype_code(g) if g is not None else F32, eps if eps == 1e-6 else _f32(eps), _addr(cos), _addr(sin), rope_row0,
                       _addr(q_out), _addr(k_out), _addr(v_out),
                       q_out.stride(0) if q_out is not None else 0, k_out.stride(0) if k_out is not None else 0,
                       v_out.stride(0) if v_out is not None else 0)
